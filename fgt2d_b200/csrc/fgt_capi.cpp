@@ -998,7 +998,17 @@ int fgt_plan_expansion(fgt_plan* p, int which, int box, double* out) {
   const HostPlan& H = p->H;
   if (box < 0 || box >= H.tree.nboxes) return FGT_ERR_BADARG;
   const std::vector<int>& slots = which == 0 ? H.mp_slot : H.loc_slot;
-  if ((int)slots.size() <= box || slots[box] < 0) return FGT_ERR_BADARG;
+  if ((int)slots.size() <= box) return FGT_ERR_BADARG;
+  const int lcut = std::max(H.P.npwlevel, 0);
+  if (which == 0 && slots[box] < 0 && H.P.dim == 3 && H.P.scheme == 0 && H.tree.level[box] > lcut &&
+      H.tree.ns(box) > 0) {
+    // below the cut level the transform forms none: formed here on request
+    CKS(cudaSetDevice(p->ctx->device));
+    if (p->done) CKS(cudaEventSynchronize(p->done));
+    CKS(device_plan_box_expansion(H, p->D, box, out, p->ctx->stream));
+    return FGT_OK;
+  }
+  if (slots[box] < 0) return FGT_ERR_BADARG;
   const double2* pool = which == 0 ? p->D.mp : p->D.loc;
   const size_t per = (size_t)H.P.nd * H.P.nexp;
   CKS(cudaSetDevice(p->ctx->device));

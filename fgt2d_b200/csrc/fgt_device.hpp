@@ -66,6 +66,53 @@ struct HornerTask {
   long long off;
 };
 
+// A leaf below (or at) a root box, with its place in the root's grid of boxes
+// of its level: the root holds 2^d boxes per dimension at depth d.
+struct SepItem {
+  int box = 0, root = 0;  // boxes; root by its position in the list of roots
+  int p = 0, d = 0;       // order of the block, depth below the root
+  int x[3] = {0, 0, 0};   // place in the root's grid
+  long long off = 0;      // the leaf's block (doubles)
+  int n = 1;              // partial blocks at off, off + P^3, ... (Hermite blocks)
+  int index = 0;          // the caller's number of the leaf
+};
+// A leaf's plane-wave expansion added to a cut-level one: its slot and its
+// phase rows in x, y and z.
+struct SepShift {
+  int src, row[3];
+};
+// Separable 3D transforms (fgt_sep3d.hpp).  A leaf's block with its z phase
+// row; a node of the levels above: a column (x, y) of leaves, a slab (x) of
+// columns, a cut-level box of slabs.
+struct SepLeaf {
+  long long off;  // block, doubles per density
+  int row, n;     // phase row; partial blocks
+};
+struct SepNode {
+  long long off;       // columns, slabs: intermediate, doubles per density; boxes: expansion slot
+  int beg, cnt, row, p;  // children [beg, beg + cnt), own phase row, order + 1
+};
+struct SepGroup {  // columns and slabs of one order
+  int p, cbeg, cend, sbeg, send;
+};
+struct SepLists {
+  std::vector<SepLeaf> leaves;
+  std::vector<SepNode> cols, slabs, boxes;
+  std::vector<int> box_slabs;  // the boxes' slabs (a box has slabs of several orders)
+  std::vector<SepGroup> groups;
+  size_t t1 = 0, t2 = 0;  // doubles per density of all columns and all slabs
+};
+struct SepDev {
+  SepLeaf* leaves = nullptr;
+  SepNode *cols = nullptr, *slabs = nullptr, *boxes = nullptr;
+  int* box_slabs = nullptr;
+  int nboxes = 0;
+  std::vector<SepGroup> groups;
+  double2* ph = nullptr;
+  double *t1 = nullptr, *t2 = nullptr;
+  int sms = 148;
+};
+
 struct StageTimes {
   float ms[8];  // gather, form, merge, m2l, split, eval, direct, scatter
   // the dominant tensor-core launch: the Hermite-block MMA kernel of the
@@ -131,11 +178,17 @@ struct DevicePlan {
   int nfchunks = 0;
   int* fcbeg = nullptr;      // per Hermite form task, first chunk (size n+1)
   double* hbuf = nullptr;    // partial Hermite blocks
-  bool form3_smem = false, eval3_smem = false;
+  // 3D plane-wave scheme: the leaves' Hermite blocks to the cut level's
+  // expansions; the leaves' own expansions (plane-wave route) added to them
+  SepDev up;
+  MergeGroup* upw_groups = nullptr;
+  SepShift* upw = nullptr;
+  int nupw_groups = 0;
+  std::vector<SepItem> up_items;  // the Hermite leaves (host copy)
+  bool eval3_smem = false;
   bool eval3_split = false;  // 3D Taylor eval in two kernels (conversion, Horner)
   int eval3_nsplit = 0;      // 3D Taylor tasks [0, eval3_nsplit) take the two kernels
-  int form3_nsplit = 0;      // 3D Hermite form tasks [0, form3_nsplit) take the shared-memory kernels
-  size_t form3_shB = 0, eval3_sh = 0;
+  size_t eval3_sh = 0;
   std::vector<OrderGroup> fchunk_groups;  // chunk ranges of equal order
   // per-CTA scratch of the 3D separable transforms (fallback path)
   double2* scratch = nullptr;
@@ -234,6 +287,12 @@ cudaError_t device_plan_set_points(DevicePlan& D, const double* src, const doubl
 // the cut level between the two).
 cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& out,
                                 int precision, cudaStream_t stream, StageTimes* times, int phase = 0);
+
+// The multipole expansion of a box below the cut level after the last
+// execute (3D plane-wave scheme, which forms none there): its leaves' blocks
+// and expansions taken to the box instead of the cut level, nd * nexp complex
+// in out (host); synchronous on st.
+cudaError_t device_plan_box_expansion(const HostPlan& H, DevicePlan& D, int box, double* out, cudaStream_t st);
 
 // Sets *d_flag (device int, not cleared here) when any of x[0, n) is not
 // finite; asynchronous on st.

@@ -88,6 +88,12 @@ __device__ __forceinline__ double2 cexpi(double th) {
   sincos(th, &s, &c);
   return make_double2(c, s);
 }
+// One FP64 tensor-core step, mma.m8n8k4 (fragment layout: PTX ISA).
+__device__ __forceinline__ void dmma_884(double& d0, double& d1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(d0), "+d"(d1)
+               : "d"(a), "d"(b));
+}
 // Packed FP32 pairs on the sm_100 f32x2 pipe: one instruction computes both
 // lanes of a float2 (d.x = a.x b.x + c.x, d.y = a.y b.y + c.y), each rounded
 // as the scalar FP32 operation.

@@ -29,6 +29,7 @@
 
 #include "fgt_device.hpp"
 #include "fgt_kcommon.cuh"
+#include "fgt_sep3d.hpp"
 
 namespace fgtb {
 
@@ -265,118 +266,6 @@ __global__ void __launch_bounds__(256) k_form2d(KP k, const FormTask* __restrict
   }
 }
 
-// ------------------------------------------------------------ (a) form, 3D Hermite
-// Persistent CTAs; H (P^3) in shared memory, accumulated by (j,k) pairs with
-// the P values of l in registers; the three 1D passes go through this CTA's
-// scratch slab in global memory (z pass, y pass, x pass into the slot).
-template <int MAXP>
-__global__ void __launch_bounds__(256) k_form3d_hermite(KP k, const FormTask* __restrict__ tasks,
-                                                        int ntasks, double2* __restrict__ scratch,
-                                                        size_t slab, const double* __restrict__ isq) {
-  extern __shared__ double sm[];
-  const int npw = k.npw, n2 = k.n2;
-  double2* T1 = scratch + slab * blockIdx.x;
-  for (int w = blockIdx.x; w < ntasks * k.nd; w += gridDim.x) {
-    const FormTask T = tasks[w / k.nd];
-    const int ind = w % k.nd;
-    const int Pn = T.p + 1, P2 = Pn * Pn, P3 = P2 * Pn;
-    double* H = sm;
-    double* X = H + P3;
-    double* Y = X + FORM_CH * Pn;
-    double* Z = Y + FORM_CH * Pn;
-    const double cx = k.centers[3 * T.box], cy = k.centers[3 * T.box + 1],
-                 cz = k.centers[3 * T.box + 2];
-    for (int e = threadIdx.x; e < P3; e += blockDim.x) H[e] = 0.0;
-    __syncthreads();
-    // dipoles: three columns per source (dip3_coef), 10 sources per chunk
-    const int vc = k.ifdipole ? 3 : 1, chs = FORM_CH / vc;
-    for (int c0 = 0; c0 < T.n; c0 += chs) {
-      const int m = vc * min(chs, T.n - c0);
-      if (threadIdx.x < m) {
-        const int i = T.s0 + c0 + threadIdx.x / vc;
-        const double x = (k.src[3 * i] - cx) * k.dsq, y = (k.src[3 * i + 1] - cy) * k.dsq,
-                     z = (k.src[3 * i + 2] - cz) * k.dsq;
-        double* xr = X + threadIdx.x * Pn;
-        double* yr = Y + threadIdx.x * Pn;
-        double* zr = Z + threadIdx.x * Pn;
-        if (!k.ifdipole) {
-          double xv = 1.0, yv = 1.0, zv = k.chg[(size_t)i * k.nd + ind];
-          xr[0] = xv; yr[0] = yv; zr[0] = zv;
-          for (int j = 1; j < Pn; j++) {
-            double sj = sqrt((double)j);
-            xv = xv * x / sj; yv = yv * y / sj; zv = zv * z / sj;
-            xr[j] = xv; yr[j] = yv; zr[j] = zv;
-          }
-        } else {
-          double dv[3], a, b;
-          src_dipole<3>(k, i, ind, dv);
-          const double q = src_charge(k, i, ind), cv[3] = {x, y, z};
-          double* rows[3] = {xr, yr, zr};
-          for (int d = 0; d < 3; d++) {
-            dip3_coef(threadIdx.x % vc, d, q, dv, a, b);
-            dip_row(rows[d], 1, Pn, cv[d], a, b, k.dsq, isq);
-          }
-        }
-      }
-      __syncthreads();
-      for (int pr = threadIdx.x; pr < P2; pr += blockDim.x) {
-        const int j = pr % Pn, kk = pr / Pn;
-        double acc[MAXP];
-#pragma unroll
-        for (int l = 0; l < MAXP; l++) acc[l] = l < Pn ? H[j + Pn * (kk + Pn * l)] : 0.0;
-        for (int t = 0; t < m; t++) {
-          const double a = X[t * Pn + j] * Y[t * Pn + kk];
-          const double* zr = Z + t * Pn;
-#pragma unroll
-          for (int l = 0; l < MAXP; l++)
-            if (l < Pn) acc[l] = fma(a, zr[l], acc[l]);
-        }
-#pragma unroll
-        for (int l = 0; l < MAXP; l++)
-          if (l < Pn) H[j + Pn * (kk + Pn * l)] = acc[l];
-      }
-      __syncthreads();
-    }
-    // z pass: T1[(j3 + P j2) n2 + k1] = sum_j1 A(j1,k1) i^j1 H[j3 + P(j2 + P j1)]
-    // (k1 over the first half of the ascending 3D nodes, as pwexp(:,:,npw/2))
-    double2* T2 = T1 + (size_t)P2 * n2;
-    for (int idx = threadIdx.x; idx < P2 * n2; idx += blockDim.x) {
-      const int k1 = idx % n2, jj = idx / n2;
-      double2 a = make_double2(0.0, 0.0);
-      for (int j1 = 0; j1 < Pn; j1++) addrot(a, k.h2x[j1 * npw + k1] * H[jj + P2 * j1], j1);
-      T1[idx] = a;
-    }
-    __syncthreads();
-    // y pass: T2[(j3 npw + k2) n2 + k1] = sum_j2 A(j2,k2) i^j2 T1[(j3 + P j2) n2 + k1]
-    for (int idx = threadIdx.x; idx < Pn * npw * n2; idx += blockDim.x) {
-      const int k1 = idx % n2, r = idx / n2, k2 = r % npw, j3 = r / npw;
-      double2 a = make_double2(0.0, 0.0);
-      for (int j2 = 0; j2 < Pn; j2++) {
-        const double h = k.h2x[j2 * npw + k2];
-        const double2 z = rot(T1[(j3 + Pn * j2) * n2 + k1], j2);
-        a.x = fma(h, z.x, a.x);
-        a.y = fma(h, z.y, a.y);
-      }
-      T2[idx] = a;
-    }
-    __syncthreads();
-    // x pass into the slot: pw[k3 + npw (k2 + npw k1)]
-    double2* out = k.mp + ((size_t)T.slot * k.nd + ind) * k.nexp;
-    for (int e = threadIdx.x; e < k.nexp; e += blockDim.x) {
-      const int k3 = e % npw, r = e / npw, k2 = r % npw, k1 = r / npw;
-      double2 a = make_double2(0.0, 0.0);
-      for (int j3 = 0; j3 < Pn; j3++) {
-        const double h = k.h2x[j3 * npw + k3];
-        const double2 z = rot(T2[(j3 * npw + k2) * n2 + k1], j3);
-        a.x = fma(h, z.x, a.x);
-        a.y = fma(h, z.y, a.y);
-      }
-      out[e] = a;
-    }
-    __syncthreads();
-  }
-}
-
 // ------------------------------------------------------------ (a) form, 2D on FP64 MMA
 // Hermite block of a leaf, H[j][k] = sum_t q_t x_t^j y_t^k (g2dformhc_vec,
 // g2drouts.f:100-168, without the 1/sqrt(j! k!) factors, which k_h2pw2d
@@ -390,12 +279,6 @@ __global__ void __launch_bounds__(256) k_form3d_hermite(KP k, const FormTask* __
 // each fragment load is two conflict-free wavefronts.  Four warps split the
 // leaf's sources; their tiles are summed in shared memory and the P x P block
 // goes to the leaf's slot of the Hermite buffer.
-__device__ __forceinline__ void dmma_884(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
-}
-
 // Leading dimensions (in doubles) of zero-padded shared-memory operands of
 // the m8n8k4 FP64 MMA: an A operand with K columns is stored with a stride of
 // 4 (mod 16) and a B operand with N columns with a stride of 8 (mod 16), so
@@ -674,16 +557,11 @@ __global__ void __launch_bounds__(128) k_h2pw2d(KP k, const FormTask* __restrict
   }
 }
 
-// ------------------------------------------------------------ (a) form, 3D, two kernels
-// Kernel A: one CTA per chunk of <= FORM3_CHK sources of a leaf; the chunk's
-// Hermite block H[j + P (k + P l)] (g3dformhc_vec, g3drouts.f:109-192) is
-// accumulated in shared memory -- each thread owns (j,k) pairs and keeps the
-// P values of l in registers -- and written to its slot of the partial buffer.
-// Kernel B: one CTA per leaf sums the leaf's partial blocks in chunk order
-// (deterministic) and runs the separable Hermite -> plane-wave transform
-// (g3dh2pw_real_vec, g3drouts.f:1565-1685) in shared memory: z pass over the
-// stored half, then y and x passes over the positive half using the mirror
-// symmetry A(j, mirror k) = (-1)^j A(j, k) of the ascending node set.
+// ------------------------------------------------------------ (a) form, 3D
+// One CTA per chunk of <= 4096 sources of a leaf accumulates the chunk's
+// Hermite block H[j + P (k + P l)] (g3dformhc_vec, g3drouts.f:109-192) and
+// writes it to its slot of the partial buffer; fgt_sep3d.cu sums a leaf's
+// blocks in chunk order and takes them to the cut level's expansions.
 
 // The chunk's Hermite block on the FP64 tensor cores: H[j][(k, l)] =
 // sum_t x_t^j (q_t y_t^k z_t^l) (with the 1/sqrt(j!) factors, g3dformhc_vec,
@@ -694,7 +572,7 @@ __global__ void __launch_bounds__(128) k_h2pw2d(KP k, const FormTask* __restrict
 // two staged powers, with (k, l) of the lane's column fixed per tile.  The
 // eight warps split the N tiles (up to four each per pass over the sources).
 // The partial block goes to the chunk's slot of the Hermite buffer, laid out
-// H[j + P (k + P l)] as k_form3d_h2pw reads it.
+// H[j + P (k + P l)] as k_up_z reads it.
 // With dipoles (DIP) every source stages three columns (dip3_coef), 21
 // sources (63 columns) per batch.
 template <int MT, bool DIP>
@@ -790,343 +668,8 @@ __global__ void __launch_bounds__(256) k_form3d_mma(KP k, const FormTask* __rest
   }
 }
 
-__global__ void __launch_bounds__(512) k_form3d_h2pw(KP k, const FormTask* __restrict__ tasks,
-                                                     const int* __restrict__ cbeg,
-                                                     const FormChunk* __restrict__ chunks,
-                                                     const double* __restrict__ hbuf) {
-  const int tk = blockIdx.x, ind = blockIdx.y;
-  const FormTask T = tasks[tk];
-  const int npw = k.npw, n2 = k.n2;
-  const int Pn = T.p + 1, P2 = Pn * Pn, P3 = P2 * Pn;
-  extern __shared__ double sm[];
-  // region A: H, later T2 [(j3 npw + k2) n2 + k1]; region B: T1 [(j3 + P j2) n2 + k1];
-  // then the signed table hs[j][k] = h2x[j][k] (j mod 4 < 2 ? 1 : -1).  The
-  // factor i^j of each pass is then a sign (in hs) times 1 (even j) or i
-  // (odd j): even and odd j are summed apart, E + i O, and the mirror node
-  // of k (A(j, mirror k) = (-1)^j A(j, k)) gets E - i O.
-  const size_t szA = max((size_t)P3, (size_t)2 * Pn * npw * n2);
-  double* H = sm;
-  double2* T2 = reinterpret_cast<double2*>(sm);
-  double2* T1 = reinterpret_cast<double2*>(sm + ((szA + 1) & ~size_t(1)));
-  double* hs = reinterpret_cast<double*>(T1 + (size_t)P2 * n2);
-  for (int e = threadIdx.x; e < Pn * npw; e += blockDim.x) {
-    const int j = e / npw;
-    hs[e] = (j & 2) ? -k.h2x[e] : k.h2x[e];
-  }
-  for (int e = threadIdx.x; e < P3; e += blockDim.x) {
-    double v = 0.0;
-    for (int c = cbeg[tk]; c < cbeg[tk + 1]; c++) v += hbuf[(size_t)chunks[c].hoff * k.nd + (size_t)ind * P3 + e];
-    H[e] = v;
-  }
-  __syncthreads();
-  // z pass over the stored half (the first n2 ascending nodes)
-  for (int idx = threadIdx.x; idx < P2 * n2; idx += blockDim.x) {
-    const int k1 = idx % n2, jj = idx / n2;
-    double ev = 0.0, od = 0.0;
-    int j1 = 0;
-    for (; j1 + 1 < Pn; j1 += 2) {
-      ev = fma(hs[j1 * npw + k1], H[jj + P2 * j1], ev);
-      od = fma(hs[(j1 + 1) * npw + k1], H[jj + P2 * (j1 + 1)], od);
-    }
-    if (j1 < Pn) ev = fma(hs[j1 * npw + k1], H[jj + P2 * j1], ev);
-    T1[idx] = make_double2(ev, od);
-  }
-  __syncthreads();
-  // y pass over the positive half k2 = n2 + m and its mirror n2 - 1 - m
-  for (int idx = threadIdx.x; idx < Pn * n2 * n2; idx += blockDim.x) {
-    const int k1 = idx % n2, r = idx / n2, m = r % n2, j3 = r / n2;
-    const int kp = n2 + m, km = n2 - 1 - m;
-    double2 E = make_double2(0.0, 0.0), O = make_double2(0.0, 0.0);
-    const double2* zc = T1 + (size_t)j3 * n2 + k1;
-    int j2 = 0;
-    for (; j2 + 1 < Pn; j2 += 2) {
-      const double he = hs[j2 * npw + kp], ho = hs[(j2 + 1) * npw + kp];
-      const double2 ze = zc[(size_t)Pn * j2 * n2], zo = zc[(size_t)Pn * (j2 + 1) * n2];
-      E.x = fma(he, ze.x, E.x);
-      E.y = fma(he, ze.y, E.y);
-      O.x = fma(ho, zo.x, O.x);
-      O.y = fma(ho, zo.y, O.y);
-    }
-    if (j2 < Pn) {
-      const double he = hs[j2 * npw + kp];
-      const double2 ze = zc[(size_t)Pn * j2 * n2];
-      E.x = fma(he, ze.x, E.x);
-      E.y = fma(he, ze.y, E.y);
-    }
-    T2[((size_t)j3 * npw + kp) * n2 + k1] = make_double2(E.x - O.y, E.y + O.x);
-    T2[((size_t)j3 * npw + km) * n2 + k1] = make_double2(E.x + O.y, E.y - O.x);
-  }
-  __syncthreads();
-  double2* out = k.mp + ((size_t)T.slot * k.nd + ind) * k.nexp;
-  // x pass into the slot, positive half k3 = n2 + m and mirror
-  for (int idx = threadIdx.x; idx < n2 * npw * n2; idx += blockDim.x) {
-    const int m = idx % n2, r = idx / n2, k2 = r % npw, k1 = r / npw;
-    const int kp = n2 + m, km = n2 - 1 - m;
-    double2 E = make_double2(0.0, 0.0), O = make_double2(0.0, 0.0);
-    const double2* zc = T2 + (size_t)k2 * n2 + k1;
-    const size_t zs = (size_t)npw * n2;
-    int j3 = 0;
-    for (; j3 + 1 < Pn; j3 += 2) {
-      const double he = hs[j3 * npw + kp], ho = hs[(j3 + 1) * npw + kp];
-      const double2 ze = zc[zs * j3], zo = zc[zs * (j3 + 1)];
-      E.x = fma(he, ze.x, E.x);
-      E.y = fma(he, ze.y, E.y);
-      O.x = fma(ho, zo.x, O.x);
-      O.y = fma(ho, zo.y, O.y);
-    }
-    if (j3 < Pn) {
-      const double he = hs[j3 * npw + kp];
-      const double2 ze = zc[zs * j3];
-      E.x = fma(he, ze.x, E.x);
-      E.y = fma(he, ze.y, E.y);
-    }
-    const size_t base = (size_t)npw * (k2 + (size_t)npw * k1);
-    out[base + kp] = make_double2(E.x - O.y, E.y + O.x);
-    out[base + km] = make_double2(E.x + O.y, E.y - O.x);
-  }
-}
-
-// k_form3d_h2pw_mma: the transform of k_form3d_h2pw with its three passes on
-// the FP64 tensor cores.  Each pass is a real product against the signed node
-// table hs, the even and odd j in separate k-steps so that i^j becomes E + i O
-// and the mirror node gets E - i O from the same accumulators (K = j, KS
-// k-steps of 4 per parity):
-//   z pass  E/O[m][kz]   = sum_l  H[m][l] hs[l][kz],        m = jx + P jy, kz < n2
-//           -> T1[jy][(jx, kz)] = E + i O                    (M = P^2, N = n2)
-//   y pass  E/O[m][col]  = sum_jy hs[jy][n2 + m] T1[jy][col], col = (jx, kz, re/im)
-//           -> T2[jx][(ky, kz)], ky = n2 + m and n2 - 1 - m  (M = n2, N = 2 P n2)
-//   x pass  E/O[m][col]  = sum_jx hs[jx][n2 + m] T2[jx][col], col = (ky, kz, re/im)
-//           -> the slot, kx = n2 + m and n2 - 1 - m          (M = n2, N = 2 npw n2)
-// The y and x passes run per 8-row tile t of the node half: the y pass of tile
-// t fills T2 with its 16 ky and the x pass of tile t drains it, so T2 holds 16
-// ky instead of npw.  The node tables are register fragments, loaded once per
-// CTA (a launch covers one order); rows j >= P are zero fragments, not loads.
-// Row strides are 4 (mod 8) doubles, so the rows two apart that one fragment
-// reads fall in opposite halves of the banks.  Persistent CTAs of 8 warps, two
-// per SM at the orders of eps >= 1e-6, stride over the leaves of the order
-// group; where shared memory allows, the next leaf's Hermite block is copied
-// into its own buffer with cp.async while the y and x passes of the current
-// leaf run (else it is staged over T2 at the leaf's start).  Each warp takes
-// two N tiles per step (independent accumulator chains in flight).
-struct H3Dims {
-  int ldh, ld1, ld2;
-  size_t total_pf, total_ov;  // doubles: H in its own buffer (prefetched) / H over T2
-  __host__ __device__ H3Dims(int Pn, int n2) {
-    ldh = ((Pn * Pn + 3) & ~7) + 4;
-    ld1 = 8 * ((2 * Pn * n2 + 7) / 8) + 4;
-    ld2 = 32 * n2 + 4;
-    total_pf = (size_t)Pn * (ld1 + ld2 + ldh) + 8;
-    const size_t t2 = (size_t)Pn * ld2, hb = (size_t)Pn * ldh + 8;
-    total_ov = (size_t)Pn * ld1 + (t2 > hb ? t2 : hb);
-  }
-};
-
-// Stage the Hermite block of task tk (the sum of its chunk partials) into H
-// with row stride ldh, row l of P^2 doubles per warp: a single partial block
-// by asynchronous copies (16 bytes where the rows allow; waited for by the
-// caller), several by plain loads in chunk order.
-// The task's chunk range [cb0, cb1) and its first chunk's offset hoff0 are
-// loaded by the caller ahead of time.
-__device__ __forceinline__ void h2pw_stage(const KP& k, int ind, int Pn, int ldh, int cb0, int cb1, long long hoff0,
-                                           const FormChunk* __restrict__ chunks, const double* __restrict__ hbuf,
-                                           double* H) {
-  const int P2 = Pn * Pn, P3 = P2 * Pn, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  if (cb1 - cb0 == 1) {
-    const double* src = hbuf + (size_t)hoff0 * k.nd + (size_t)ind * P3;
-    const unsigned dst = (unsigned)__cvta_generic_to_shared(H);
-    if (((P2 | (int)(reinterpret_cast<size_t>(src) >> 3)) & 1) == 0) {
-      for (int l = threadIdx.x >> 5; l < Pn; l += nw)
-        for (int m = 2 * lane; m < P2; m += 64)
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 8u * (unsigned)(l * ldh + m)),
-                       "l"(src + l * P2 + m) : "memory");
-    } else {
-      for (int l = threadIdx.x >> 5; l < Pn; l += nw)
-        for (int m = lane; m < P2; m += 32)
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 8u * (unsigned)(l * ldh + m)),
-                       "l"(src + l * P2 + m) : "memory");
-    }
-  } else {
-    for (int l = threadIdx.x >> 5; l < Pn; l += nw)
-      for (int m = lane; m < P2; m += 32) {
-        double v = 0.0;
-        for (int ch = cb0; ch < cb1; ch++) v += hbuf[(size_t)chunks[ch].hoff * k.nd + (size_t)ind * P3 + l * P2 + m];
-        H[l * ldh + m] = v;
-      }
-  }
-}
-
 // q / d for 0 <= q < 1115 and 1 <= d <= 64, with mg = ceil(2^16 / d)
 __device__ __forceinline__ int div16(int q, int mg) { return (q * mg) >> 16; }
-
-template <int KS, int MT>
-__global__ void __launch_bounds__(256, (KS * MT <= 4) ? 2 : 1)
-    k_form3d_h2pw_mma(KP k, const FormTask* __restrict__ tasks, int ntask, const int* __restrict__ cbeg,
-                      const FormChunk* __restrict__ chunks, const double* __restrict__ hbuf, bool pf) {
-  const int ind = blockIdx.y;
-  const int npw = k.npw, n2 = k.n2;
-  const int Pn = tasks[0].p + 1, P2 = Pn * Pn;
-  const int mgP = (65536 + Pn - 1) / Pn, mgN = (65536 + n2 - 1) / n2;  // div16 factors
-  const H3Dims Z(Pn, n2);
-  extern __shared__ double sm[];
-  double* T1 = sm;                       // [Pn][ld1]: (jx, kz, re/im)
-  double* T2 = T1 + (size_t)Pn * Z.ld1;  // [Pn][ld2]: (kyl, kz, re/im)
-  // H [Pn][ldh] (+ 8: the last M tile's rows past P^2): its own buffer when
-  // pf (the next leaf's block is prefetched), else over T2 (staged per leaf)
-  double* H = pf ? T2 + (size_t)Pn * Z.ld2 : T2;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = lane >> 2, c = lane & 3;
-  int tk = blockIdx.x;
-  if (tk >= ntask) return;
-  // chunk range and first partial block of the current task
-  int cb0 = cbeg[tk], cb1 = cbeg[tk + 1];
-  long long hoff0 = chunks[cb0].hoff;
-  if (pf) h2pw_stage(k, ind, Pn, Z.ldh, cb0, cb1, hoff0, chunks, hbuf, H);
-  // B fragments of the stored-half table for the z pass (B[k = j][n = kz]) and
-  // A fragments of the positive-half table for the y and x passes (A[m][k = j])
-  double hz[MT][2][KS], hn[MT][2][KS];
-#pragma unroll
-  for (int t = 0; t < MT; t++)
-#pragma unroll
-    for (int par = 0; par < 2; par++)
-#pragma unroll
-      for (int s = 0; s < KS; s++) {
-        const int j = 8 * s + 2 * c + par, m = 8 * t + r;
-        const bool ok = j < Pn && m < n2;
-        const double sg = (j & 2) ? -1.0 : 1.0;
-        hz[t][par][s] = ok ? sg * k.h2x[j * npw + m] : 0.0;
-        hn[t][par][s] = ok ? sg * k.h2x[j * npw + n2 + m] : 0.0;
-      }
-  const int mtiles = (P2 + 7) / 8, nt1 = (2 * Pn * n2 + 7) / 8;
-  for (; tk < ntask; tk += gridDim.x) {
-    if (!pf) h2pw_stage(k, ind, Pn, Z.ldh, cb0, cb1, hoff0, chunks, hbuf, H);  // T2 is free: the last pass ended in a barrier
-    // the next task's chunk range and first block offset, loaded while this one runs
-    const int tn = tk + gridDim.x;
-    if (tn < ntask) {
-      cb0 = cbeg[tn];
-      cb1 = cbeg[tn + 1];
-      hoff0 = chunks[cb0].hoff;
-    }
-    const int slot = tasks[tk].slot;
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
-    // z pass: H -> T1
-    for (int mt = warp; mt < mtiles; mt += 8) {
-      const int m = 8 * mt + r;
-      double a[2][KS];
-#pragma unroll
-      for (int par = 0; par < 2; par++)
-#pragma unroll
-        for (int s = 0; s < KS; s++) {
-          const int j = 8 * s + 2 * c + par;
-          a[par][s] = j < Pn ? H[m + j * Z.ldh] : 0.0;
-        }
-      const int jy = div16(m, mgP), jx = m - jy * Pn;
-#pragma unroll
-      for (int t = 0; t < MT; t++) {
-        double e0 = 0.0, e1 = 0.0, o0 = 0.0, o1 = 0.0;
-#pragma unroll
-        for (int s = 0; s < KS; s++) {
-          dmma_884(e0, e1, a[0][s], hz[t][0][s]);
-          dmma_884(o0, o1, a[1][s], hz[t][1][s]);
-        }
-        const int kz = 8 * t + 2 * c;  // the lane's accumulator columns kz, kz + 1
-        if (m < P2) {
-          double* row = T1 + jy * Z.ld1 + 2 * (jx * n2 + kz);
-          if (kz < n2) *reinterpret_cast<double2*>(row) = make_double2(e0, o0);
-          if (kz + 1 < n2) *reinterpret_cast<double2*>(row + 2) = make_double2(e1, o1);
-        }
-      }
-    }
-    __syncthreads();
-    // the next leaf's Hermite block lands while this leaf's y and x passes run
-    if (pf && tn < ntask) h2pw_stage(k, ind, Pn, Z.ldh, cb0, cb1, hoff0, chunks, hbuf, H);
-    double2* out = k.mp + ((size_t)slot * k.nd + ind) * k.nexp;
-#pragma unroll
-    for (int t = 0; t < MT; t++) {
-      const int nv = min(8, n2 - 8 * t);  // node rows of tile t
-      // y pass of tile t into T2[jx][(kyl n2 + kz)], kyl = 2 i (ky = n2 + 8t + i) or 2 i + 1 (ky = n2 - 1 - 8t - i)
-      for (int nt0 = warp; nt0 < nt1; nt0 += 16) {
-        double b[2][2][KS], acc[2][4];
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const int col = 8 * (nt0 + 8 * h) + r;
-          const bool ok = nt0 + 8 * h < nt1;
-#pragma unroll
-          for (int par = 0; par < 2; par++)
-#pragma unroll
-            for (int s = 0; s < KS; s++) {
-              const int j = 8 * s + 2 * c + par;
-              b[h][par][s] = (ok && j < Pn) ? T1[j * Z.ld1 + col] : 0.0;
-            }
-          acc[h][0] = acc[h][1] = acc[h][2] = acc[h][3] = 0.0;
-        }
-#pragma unroll
-        for (int s = 0; s < KS; s++)
-#pragma unroll
-          for (int h = 0; h < 2; h++) {
-            dmma_884(acc[h][0], acc[h][1], hn[t][0][s], b[h][0][s]);
-            dmma_884(acc[h][2], acc[h][3], hn[t][1][s], b[h][1][s]);
-          }
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const int q = 4 * (nt0 + 8 * h) + c;  // the lane's complex column (jx, kz)
-          if (r < nv && q < Pn * n2) {
-            const int jx = div16(q, mgN), kz = q - jx * n2;
-            double* row = T2 + jx * Z.ld2 + 2 * kz + 4 * n2 * r;
-            *reinterpret_cast<double2*>(row) = make_double2(acc[h][0] - acc[h][3], acc[h][1] + acc[h][2]);
-            *reinterpret_cast<double2*>(row + 2 * n2) = make_double2(acc[h][0] + acc[h][3], acc[h][1] - acc[h][2]);
-          }
-        }
-      }
-      __syncthreads();
-      // x pass of tile t: all node rows of kx against T2's columns (kyl, kz)
-      const int nq = 2 * nv * n2, nt2 = (2 * nq + 7) / 8;
-      for (int nt0 = warp; nt0 < nt2; nt0 += 16) {
-        double b[2][2][KS], acc[2][MT][4];
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const int col = 8 * (nt0 + 8 * h) + r;
-          const bool ok = nt0 + 8 * h < nt2;
-#pragma unroll
-          for (int par = 0; par < 2; par++)
-#pragma unroll
-            for (int s = 0; s < KS; s++) {
-              const int j = 8 * s + 2 * c + par;
-              b[h][par][s] = (ok && j < Pn) ? T2[j * Z.ld2 + col] : 0.0;
-            }
-#pragma unroll
-          for (int u = 0; u < MT; u++) acc[h][u][0] = acc[h][u][1] = acc[h][u][2] = acc[h][u][3] = 0.0;
-        }
-#pragma unroll
-        for (int s = 0; s < KS; s++)
-#pragma unroll
-          for (int h = 0; h < 2; h++)
-#pragma unroll
-            for (int u = 0; u < MT; u++) {
-              dmma_884(acc[h][u][0], acc[h][u][1], hn[u][0][s], b[h][0][s]);
-              dmma_884(acc[h][u][2], acc[h][u][3], hn[u][1][s], b[h][1][s]);
-            }
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const int q = 4 * (nt0 + 8 * h) + c;  // the lane's complex column (kyl, kz)
-          if (q < nq) {
-            const int kyl = div16(q, mgN), kz = q - kyl * n2, i = kyl >> 1;
-            const int ky = (kyl & 1) ? n2 - 1 - 8 * t - i : n2 + 8 * t + i;
-            double2* o = out + npw * (ky + npw * kz);
-#pragma unroll
-            for (int u = 0; u < MT; u++) {
-              const int mx = 8 * u + r;
-              if (mx < n2) {
-                o[n2 + mx] = make_double2(acc[h][u][0] - acc[h][u][3], acc[h][u][1] + acc[h][u][2]);
-                o[n2 - 1 - mx] = make_double2(acc[h][u][0] + acc[h][u][3], acc[h][u][1] - acc[h][u][2]);
-              }
-            }
-          }
-        }
-      }
-      __syncthreads();
-    }
-  }
-}
 
 // ------------------------------------------------------------ (c) eval, 2D Taylor in two kernels
 // k_pw2taylor2d: one warp per evaluation leaf converts the leaf's plane-wave
@@ -3382,12 +2925,6 @@ struct Staged {
     if (e_ != cudaSuccess) return e_;       \
   } while (0)
 
-// Shared memory of k_form3d_h2pw (the SIMT passes) at order Pn.
-size_t form3_simt_smem(int Pn_, int npw) {
-  const size_t Pn = Pn_, n2 = npw / 2, P3 = Pn * Pn * Pn;
-  const size_t szA = std::max(P3, 2 * Pn * npw * n2);
-  return (((szA + 1) & ~size_t(1)) + 2 * Pn * Pn * n2 + Pn * npw) * 8;
-}
 // Stable sort of tasks by (route, order): a counting sort (the keys are few
 // small integers), linear in the number of tasks.
 template <typename Task>
@@ -3417,18 +2954,6 @@ std::vector<Task> route_order_sort(const std::vector<Task>& in) {
   }
   return out;
 }
-// Whether the 3D Hermite form of order Pn runs on the shared-memory kernels:
-// k_form3d_mma's staging ((8 ceil(P/8) + 2 P) power rows of 68 doubles) and
-// one of the Hermite -> PW kernels (tensor-core or SIMT passes).
-bool form3_fits(int Pn, int npw) {
-  const size_t lim = 227 * 1024;
-  const size_t shA = ((size_t)8 * ((Pn + 7) / 8) + 2 * Pn) * 68 * 8;
-  if (Pn > 32 || shA > lim) return false;
-  const H3Dims Z(Pn, npw / 2);
-  const bool mma = (Pn + 7) / 8 <= 4 && (npw / 2 + 7) / 8 <= 4 && std::min(Z.total_pf, Z.total_ov) * 8 <= lim;
-  return mma || form3_simt_smem(Pn, npw) <= lim;
-}
-
 cudaError_t device_pool_setup() {
   // keep freed stream-ordered allocations in the device's default pool
   // instead of returning them at every synchronisation (process-local
@@ -3469,7 +2994,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   tq[nq++] = tnow();
   // order form and eval tasks by route so each kernel gets a contiguous range
   // (then by order; stable)
-  const std::vector<FormTask> form = route_order_sort(H.form);
+  std::vector<FormTask> form = route_order_sort(H.form);
   D.nform = (int)form.size();
   for (auto& f : form) {
     (f.route == ROUTE_PW ? D.form_pw_n : D.form_hermite_n)++;
@@ -3480,6 +3005,74 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   for (auto& e : ev) {
     (e.route == ROUTE_PW ? D.eval_pw_n : D.eval_taylor_n)++;
     if (e.route == ROUTE_TAYLOR) D.eval_pmax = std::max(D.eval_pmax, e.p);
+  }
+  // 3D plane-wave scheme: the Hermite leaves in the order of the columns and
+  // slabs of their cut-level boxes, and the leaves with their own expansions
+  const int lcut = std::max(P.npwlevel, 0);
+  const bool sep = P.dim == 3 && P.scheme == 0 && !P.all_direct;
+  SepLists up;
+  std::vector<MergeGroup> upw_groups;
+  std::vector<SepShift> upw;
+  std::vector<double> sep_ph;
+  if (sep) {
+    const Tree& tr = H.tree;
+    auto cut_box = [&](int b) {
+      while (tr.level[b] > lcut) b = tr.parent[b];
+      return b;
+    };
+    std::vector<int> roots, root_slot, rank(tr.llast[lcut] + 1, -1);
+    auto root_of = [&](int b) {
+      const int a = cut_box(b);
+      if (rank[a] < 0) {
+        rank[a] = (int)roots.size();
+        roots.push_back(a);
+        root_slot.push_back(H.mp_slot[a]);
+      }
+      return rank[a];
+    };
+    std::vector<SepItem> items(D.form_hermite_n), pw;
+    for (int i = 0; i < D.nform; i++) {
+      const FormTask& f = form[i];
+      if (i >= D.form_hermite_n && tr.level[f.box] == lcut) continue;  // forms the cut level's expansion itself
+      SepItem s;
+      s.box = f.box;
+      s.root = root_of(f.box);
+      s.p = f.p;
+      s.index = i;
+      if (i < D.form_hermite_n) items[i] = s;
+      else pw.push_back(s);
+    }
+    sep_sort(tr, roots, items);
+    {
+      const std::vector<FormTask> in(form.begin(), form.begin() + D.form_hermite_n);
+      long long hoff = 0;
+      for (int i = 0; i < D.form_hermite_n; i++) {
+        SepItem& s = items[i];
+        form[i] = in[s.index];
+        s.index = i;
+        s.off = hoff;
+        s.n = (form[i].n + 4095) / 4096;
+        hoff += (long long)s.n * (s.p + 1) * (s.p + 1) * (s.p + 1);
+      }
+    }
+    sep_lists(items, root_slot, P.npw, up);
+    sep_sort(tr, roots, pw);
+    std::stable_sort(pw.begin(), pw.end(), [](const SepItem& a, const SepItem& b) { return a.root < b.root; });
+    int dmax = 0;
+    for (const SepItem& s : items) dmax = std::max(dmax, s.d);
+    for (size_t i = 0; i < pw.size(); i++) {
+      const SepItem& s = pw[i];
+      dmax = std::max(dmax, s.d);
+      if (i == 0 || pw[i - 1].root != s.root) upw_groups.push_back({root_slot[s.root], (int)i, 0});
+      upw_groups.back().cnt++;
+      const int r0 = (1 << s.d) - 1;
+      upw.push_back({form[s.index].slot, {r0 + s.x[0], r0 + s.x[1], r0 + s.x[2]}});
+    }
+    sep_phases(H, dmax, H.tree.boxsize[lcut], sep_ph);
+    D.up_items = items;
+    for (SepItem& s : D.up_items) s.root = 0;
+    D.up_items.insert(D.up_items.end(), pw.begin(), pw.end());  // (their index: the form task)
+    for (size_t i = items.size(); i < D.up_items.size(); i++) D.up_items[i].index = form[D.up_items[i].index].slot;
   }
   tq[nq++] = tnow();
   // launch groups of equal order among the Hermite form / Taylor eval tasks
@@ -3537,7 +3130,6 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     while (gs2 > 1 && C3Dims2(Pn, P.npw, gs2).total * 8 > 227 * 1024) gs2 >>= 1;
     return C3Dims2(Pn, P.npw, gs2).total * 8 <= 227 * 1024;
   };
-  const int lcut = std::max(P.npwlevel, 0);
   std::vector<uint8_t> fused_leaf(H.tree.nboxes, 0);
   tq[nq++] = tnow();
   if ((P.dim == 2 || D.eval3_split) && !P.all_direct) {
@@ -3708,7 +3300,6 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   tp[np_++] = tnow();
   // 3D: shared-memory paths when the largest order fits, else the scratch path
   std::vector<FormChunk> fchunks;
-  std::vector<int> fcbeg;
   size_t hbuf_doubles = 0;
   // 2D: Hermite blocks of the MMA form (orders <= 31), nd P^2 doubles per leaf
   std::vector<long long> form_hoff;
@@ -3725,41 +3316,30 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     const size_t lim = 227 * 1024;
     const int n2 = P.npw / 2;
     if (D.form_hermite_n > 0) {
-      // the Hermite block kernel and one of the two Hermite -> PW kernels
-      // take the tasks whose order fits their shared memory (a prefix: the
-      // tasks are sorted by order); the rest take the scratch fallback
-      int t = 0;
-      while (t < D.form_hermite_n && form3_fits(form[t].p + 1, P.npw)) t++;
-      D.form3_nsplit = t;
-      D.form3_smem = t > 0;
-      if (D.form3_smem) {
-        long long hoff = 0;
-        for (int t = 0; t < D.form3_nsplit; t++) {
-          fcbeg.push_back((int)fchunks.size());
-          const FormTask& f = form[t];
-          long long p3 = (long long)(f.p + 1) * (f.p + 1) * (f.p + 1);
-          for (int c = 0; c < f.n; c += 4096) {
-            fchunks.push_back({t, f.s0 + c, std::min(4096, f.n - c), hoff});
-            hoff += p3;
-          }
+      long long hoff = 0;
+      for (int t = 0; t < D.form_hermite_n; t++) {
+        const FormTask& f = form[t];
+        long long p3 = (long long)(f.p + 1) * (f.p + 1) * (f.p + 1);
+        for (int c = 0; c < f.n; c += 4096) {
+          fchunks.push_back({t, f.s0 + c, std::min(4096, f.n - c), hoff});
+          hoff += p3;
         }
-        fcbeg.push_back((int)fchunks.size());
-        hbuf_doubles = (size_t)hoff * P.nd;
-        D.nfchunks = (int)fchunks.size();
-        // chunk ranges of equal order (the tasks are sorted by order)
-        long long best = -1;
-        for (size_t t = 0; t < fchunks.size();) {
-          size_t u = t;
-          const int pt = form[fchunks[t].task].p;
-          long long n = 0;
-          while (u < fchunks.size() && form[fchunks[u].task].p == pt) n += fchunks[u++].n;
-          const double Pn = pt + 1;
-          D.group_flops.push_back(2.0 * (double)n * Pn * Pn * Pn * P.nd);
-          D.group_alg_flops.push_back(4.0 * (double)n * P.npw * P.npw * P.npw * P.nd);
-          if (n > best) { best = n; D.dom_fchunk_group = (int)D.fchunk_groups.size(); }
-          D.fchunk_groups.push_back({pt, (int)t, (int)u});
-          t = u;
-        }
+      }
+      hbuf_doubles = (size_t)hoff * P.nd;
+      D.nfchunks = (int)fchunks.size();
+      // chunk ranges of equal order (the tasks are sorted by order)
+      long long best = -1;
+      for (size_t t = 0; t < fchunks.size();) {
+        size_t u = t;
+        const int pt = form[fchunks[t].task].p;
+        long long n = 0;
+        while (u < fchunks.size() && form[fchunks[u].task].p == pt) n += fchunks[u++].n;
+        const double Pn = pt + 1;
+        D.group_flops.push_back(2.0 * (double)n * Pn * Pn * Pn * P.nd);
+        D.group_alg_flops.push_back(4.0 * (double)n * P.npw * P.npw * P.npw * P.nd);
+        if (n > best) { best = n; D.dom_fchunk_group = (int)D.fchunk_groups.size(); }
+        D.fchunk_groups.push_back({pt, (int)t, (int)u});
+        t = u;
       }
     }
     if (D.eval_taylor_n > 0) {
@@ -3773,15 +3353,10 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     }
   }
   // scratch for the 3D separable transforms (fallback path)
-  const bool form3_fallback = P.dim == 3 && D.form3_nsplit < D.form_hermite_n;
-  if (P.dim == 3 && !P.all_direct && (form3_fallback || !D.eval3_smem)) {
+  if (P.dim == 3 && !P.all_direct && !D.eval3_smem) {
     size_t slab = 0;
     int n2 = P.npw / 2;
-    if (form3_fallback)
-      for (auto& f : form)
-        if (f.route == ROUTE_HERMITE) slab = std::max(slab, (size_t)(f.p + 1) * (f.p + 1) * n2 + (size_t)(f.p + 1) * P.npw * n2);
-    if (!D.eval3_smem)
-      for (auto& e : ev)
+    for (auto& e : ev)
         if (e.route == ROUTE_TAYLOR) {
         size_t Pn = e.p + 1;
         slab = std::max(slab, Pn * P.npw * n2 + Pn * Pn * n2 + (Pn * Pn * Pn + 1) / 2);
@@ -3811,8 +3386,11 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
                  al(P.ifdipole ? ns * dim * 8 : 0) + al(P.ifdipole ? ns * nd * 8 : 0) +
                  al(nt * nd * out_comps(dim, P.ifpghtarg) * 8) +
                  al((size_t)D.scratch_ctas * D.scratch_per_cta * 16) + bytes_of(fchunks) +
+                 bytes_of(up.leaves) + bytes_of(up.cols) + bytes_of(up.slabs) + bytes_of(up.boxes) +
+                 bytes_of(up.box_slabs) + bytes_of(upw_groups) + bytes_of(upw) + bytes_of(sep_ph) +
+                 al(up.t1 * nd * 8) + al(up.t2 * nd * 8) +
                  al((size_t)D.conv3_ctas * nd * D.uscr_per_cta * 8) +
-                 bytes_of(fcbeg) + al(hbuf_doubles * 8) + bytes_of(form_hoff) + bytes_of(tables) + bytes_of(conv) + bytes_of(horner) +
+                 al(hbuf_doubles * 8) + bytes_of(form_hoff) + bytes_of(tables) + bytes_of(conv) + bytes_of(horner) +
                  al(lo_doubles * 8) + 4096;
   D.bytes = total;
   if (size_only) {
@@ -3861,7 +3439,20 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
       st.add(cur, D.dir_src, H.dir_src);
     }
     st.add(cur, D.fchunks, fchunks);
-    st.add(cur, D.fcbeg, fcbeg);
+    st.add(cur, D.up.leaves, up.leaves);
+    st.add(cur, D.up.cols, up.cols);
+    st.add(cur, D.up.slabs, up.slabs);
+    st.add(cur, D.up.boxes, up.boxes);
+    st.add(cur, D.up.box_slabs, up.box_slabs);
+    st.add(cur, D.upw_groups, upw_groups);
+    st.add(cur, D.upw, upw);
+    double* ph = nullptr;
+    st.add(cur, ph, sep_ph);
+    D.up.ph = reinterpret_cast<double2*>(ph);
+    D.up.nboxes = (int)up.boxes.size();
+    D.up.groups = up.groups;
+    D.up.sms = D.psm();
+    D.nupw_groups = (int)upw_groups.size();
     st.add(cur, D.form_hoff, form_hoff);
     st.add(cur, D.tables, tables);
     st.add(cur, D.conv, conv);
@@ -3927,6 +3518,8 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   }
   D.lo = reinterpret_cast<double*>(cur); cur += al(lo_doubles * 8);
   D.hbuf = reinterpret_cast<double*>(cur); cur += al(hbuf_doubles * 8);
+  D.up.t1 = reinterpret_cast<double*>(cur); cur += al(up.t1 * nd * 8);
+  D.up.t2 = reinterpret_cast<double*>(cur); cur += al(up.t2 * nd * 8);
   D.mp = reinterpret_cast<double2*>(cur); cur += al((size_t)H.nmp * nd * P.nexp * 16);
   D.loc = reinterpret_cast<double2*>(cur); cur += al((size_t)H.nloc * nd * P.nexp * 16);
   D.ssort = reinterpret_cast<double*>(cur); cur += al(ns * dim * 8);
@@ -3950,10 +3543,10 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
             tq[1] - tq[0], tq[2] - tq[1], nq > 3 ? tq[3] - tq[2] : 0.0);
   if (getenv("FGT_TREE_TIMING"))
     fprintf(stderr, "device plan: prep %.4f malloc %.4f upload %.4f (%zu bytes); eval tasks: taylor %d "
-            "(conversion %d, max order %d) pw %d; form tasks: hermite %d (shared memory %d, max order %d) pw %d\n",
+            "(conversion %d, max order %d) pw %d; form tasks: hermite %d (max order %d) pw %d\n",
             tm0 - tin, tm1 - tm0, tnow() - tm1, total, D.eval_taylor_n,
             P.dim == 3 ? D.eval3_nsplit : D.eval_taylor_n, D.eval_pmax + 1, D.eval_pw_n, D.form_hermite_n,
-            P.dim == 3 ? D.form3_nsplit : D.form_hermite_n, D.form_pmax + 1, D.form_pw_n);
+            D.form_pmax + 1, D.form_pw_n);
   return cudaSuccess;
 }
 
@@ -4135,7 +3728,7 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
         launches++;
       }
     }
-    if (P.dim == 3 && D.form_hermite_n > 0 && D.form3_smem) {
+    if (P.dim == 3 && D.form_hermite_n > 0) {
       for (size_t gi = 0; gi < D.fchunk_groups.size(); gi++) {
         const OrderGroup& G = D.fchunk_groups[gi];
         const int Pn = G.p + 1, mt = (Pn + 7) / 8;
@@ -4184,58 +3777,6 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
         }
         launches++;
       }
-      // Hermite -> plane wave per order group: tensor-core passes where the
-      // order and node count fit their fragments and shared memory
-      for (const OrderGroup& G : D.form_groups) {
-        if (G.beg >= D.form3_nsplit) break;  // the scratch fallback's orders
-        const int Pn = G.p + 1, ks = (Pn + 7) / 8, mt = (P.npw / 2 + 7) / 8;
-        const H3Dims Z3(Pn, P.npw / 2);
-        const bool pf = Z3.total_pf * 8 <= 227 * 1024;
-        const size_t sh = (pf ? Z3.total_pf : Z3.total_ov) * 8;
-        const int ntk = G.end - G.beg;
-        const dim3 hg(ntk, nd);
-        const FormTask* ft = D.form + G.beg;
-        const int* cb = D.fcbeg + G.beg;
-        // persistent CTAs: as many as fit on the SMs at once
-        const dim3 pg(D.pgrid(ntk, ks * mt <= 4 && 2 * (sh + 1024) <= 228 * 1024 ? 2 : 1), nd);
-        if (ks <= 4 && mt <= 4 && sh <= 227 * 1024) {
-          switch (4 * (ks - 1) + mt - 1) {
-#define H2PW_CASE(KS_, MT_)                                                                        \
-  case 4 * (KS_ - 1) + MT_ - 1:                                                                    \
-    CK(smem_limit(k_form3d_h2pw_mma<KS_, MT_>)); \
-    k_form3d_h2pw_mma<KS_, MT_><<<pg, 256, sh, st>>>(k, ft, ntk, cb, D.fchunks, D.hbuf, pf);       \
-    break;
-            H2PW_CASE(1, 1) H2PW_CASE(1, 2) H2PW_CASE(1, 3) H2PW_CASE(1, 4)
-            H2PW_CASE(2, 1) H2PW_CASE(2, 2) H2PW_CASE(2, 3) H2PW_CASE(2, 4)
-            H2PW_CASE(3, 1) H2PW_CASE(3, 2) H2PW_CASE(3, 3) H2PW_CASE(3, 4)
-            H2PW_CASE(4, 1) H2PW_CASE(4, 2) H2PW_CASE(4, 3) H2PW_CASE(4, 4)
-#undef H2PW_CASE
-            default: return cudaErrorNotSupported;
-          }
-        } else {
-          const size_t shb = form3_simt_smem(Pn, P.npw);
-          CK(smem_limit(k_form3d_h2pw));
-          k_form3d_h2pw<<<hg, 512, shb, st>>>(k, ft, cb, D.fchunks, D.hbuf);
-        }
-        launches++;
-      }
-    }
-    if (P.dim == 3 && D.form3_nsplit < D.form_hermite_n) {
-      // scratch fallback for the orders above the shared-memory kernels
-      const FormTask* ft = D.form + D.form3_nsplit;
-      const int nft = D.form_hermite_n - D.form3_nsplit;
-      int Pn = D.form_pmax + 1;
-      size_t sh = ((size_t)Pn * Pn * Pn + 3 * FORM_CH * Pn) * 8;
-      if (Pn > 32 || sh > 227 * 1024) return cudaErrorNotSupported;
-      int grid = std::min(D.scratch_ctas, 2 * D.psm());
-      if (Pn <= 16) {
-        CK(smem_limit(k_form3d_hermite<16>));
-        k_form3d_hermite<16><<<grid, 256, sh, st>>>(k, ft, nft, D.scratch, D.scratch_per_cta, D.isq);
-      } else {
-        CK(smem_limit(k_form3d_hermite<32>));
-        k_form3d_hermite<32><<<grid, 256, sh, st>>>(k, ft, nft, D.scratch, D.scratch_per_cta, D.isq);
-      }
-      launches++;
     }
     if (P.dim == 3 && D.form_pw_n > 0) {
       size_t sh = ((size_t)FORM_CH * (2 * P.npw + n2) + 8) * 16;
@@ -4251,7 +3792,14 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
       launches++;
     }
     mark(2);
-    // (b) merge, bottom-up
+    // (b) merge, bottom-up (2D); 3D: the leaves to the cut level
+    if (D.up.nboxes > 0) {
+      CK(sep_up(k, D.up, D.hbuf, st, launches));
+      if (D.nupw_groups > 0) {
+        CK(sep_add(k, D.mp, D.up.ph, D.upw_groups, D.nupw_groups, D.upw, st));
+        launches++;
+      }
+    }
     for (int l = P.nlevels - 1; l >= P.nlevstart; l--) {
       int ng = D.merge_end[l] - D.merge_beg[l];
       if (ng <= 0) continue;
@@ -4555,6 +4103,74 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
     cudaEventDestroy(dev1);
   }
   return cudaSuccess;
+}
+
+cudaError_t device_plan_box_expansion(const HostPlan& H, DevicePlan& D, int box, double* out, cudaStream_t st) {
+  const Tree& t = H.tree;
+  const Params& P = H.P;
+  std::vector<SepItem> items, pw;
+  for (const SepItem& s : D.up_items) {
+    int b = s.box;
+    while (t.level[b] > t.level[box]) b = t.parent[b];
+    if (b != box) continue;
+    std::vector<SepItem>& to = H.mp_slot[s.box] >= 0 && t.level[s.box] > std::max(P.npwlevel, 0) ? pw : items;
+    to.push_back(s);
+    to.back().root = 0;
+  }
+  const std::vector<int> roots{box}, slot{0};
+  sep_sort(t, roots, items);
+  sep_sort(t, roots, pw);
+  SepLists L;
+  sep_lists(items, slot, P.npw, L);
+  int dmax = 0;
+  for (const SepItem& s : items) dmax = std::max(dmax, s.d);
+  for (const SepItem& s : pw) dmax = std::max(dmax, s.d);
+  std::vector<double> ph;
+  sep_phases(H, dmax, t.boxsize[t.level[box]], ph);
+  std::vector<SepShift> sh;
+  for (const SepItem& s : pw) {
+    const int r0 = (1 << s.d) - 1;
+    sh.push_back({s.index, {r0 + s.x[0], r0 + s.x[1], r0 + s.x[2]}});
+  }
+  const std::vector<MergeGroup> g{{0, 0, (int)sh.size()}};
+  const size_t nd = P.nd, per = nd * P.nexp * 16;
+  char* mem = nullptr;
+  CK(cudaMallocAsync(reinterpret_cast<void**>(&mem),
+                     bytes_of(L.leaves) + bytes_of(L.cols) + bytes_of(L.slabs) + bytes_of(L.boxes) +
+                         bytes_of(L.box_slabs) + bytes_of(ph) + bytes_of(sh) + bytes_of(g) + al(L.t1 * nd * 8) +
+                         al(L.t2 * nd * 8) + al(per) + 4096,
+                     st));
+  auto run = [&]() -> cudaError_t {
+    char* cur = mem;
+    SepDev S;
+    SepShift* dsh = nullptr;
+    MergeGroup* dg = nullptr;
+    double* dph = nullptr;
+    CK(put(cur, S.leaves, L.leaves, st));
+    CK(put(cur, S.cols, L.cols, st));
+    CK(put(cur, S.slabs, L.slabs, st));
+    CK(put(cur, S.boxes, L.boxes, st));
+    CK(put(cur, S.box_slabs, L.box_slabs, st));
+    CK(put(cur, dph, ph, st));
+    CK(put(cur, dsh, sh, st));
+    CK(put(cur, dg, g, st));
+    S.ph = reinterpret_cast<double2*>(dph);
+    S.nboxes = 1;
+    S.groups = L.groups;
+    S.sms = D.sm_count;
+    S.t1 = reinterpret_cast<double*>(cur); cur += al(L.t1 * nd * 8);
+    S.t2 = reinterpret_cast<double*>(cur); cur += al(L.t2 * nd * 8);
+    KP k = make_kp(D);
+    k.mp = reinterpret_cast<double2*>(cur);
+    long long launches = 0;
+    CK(sep_up(k, S, D.hbuf, st, launches));
+    CK(sep_add(k, D.mp, S.ph, dg, sh.empty() ? 0 : 1, dsh, st));
+    CK(cudaMemcpyAsync(out, k.mp, per, cudaMemcpyDeviceToHost, st));
+    return cudaStreamSynchronize(st);
+  };
+  const cudaError_t e = run();
+  cudaFreeAsync(mem, st);
+  return e;
 }
 
 cudaError_t probe_fp64_mma(double* tflops) {

@@ -271,33 +271,39 @@ static void build_tasks(HostPlan& H) {
     H.merge.reserve(nb);
     H.split.reserve(nb);
     H.eval.reserve((size_t)nb + (size_t)(P.ns + P.nt) / 2048 + 16);
+    // 3D multipole expansions: the cut level's, and those of the leaves below
+    // it that form theirs directly; the Hermite leaves' blocks go straight to
+    // the cut level (fgt_sep3d.cu)
+    auto form_route = [&](int l, int b) {
+      if (D == 2) return (int)ROUTE_HERMITE;
+      const int p = H.nlocal[l];
+      const double r1 = (p + 1.0) / P.npw;  // fgt3d.f:931-940
+      int r = r1 * r1 * r1 >= 3 && t.ns(b) <= 1000000 ? ROUTE_PW : ROUTE_HERMITE;
+      // no Hermite block of more than 29^3 coefficients: the exact
+      // exponential sum replaces it
+      if (p + 1 > 29) r = ROUTE_PW;
+      return r;
+    };
     for (int l = nls; l <= P.nlevels; l++)
       for (int b = t.lfirst[l]; b <= t.llast[l]; b++) {
         bool leaf = t.nchild[b] == 0;
-        if (t.ns(b) > 0 && !(leaf && l == npl)) H.mp_slot[b] = H.nmp++;
+        if (t.ns(b) > 0 && !(leaf && l == npl) &&
+            (D == 2 || l == nls || (leaf && form_route(l, b) == ROUTE_PW)))
+          H.mp_slot[b] = H.nmp++;
         if (relevant(b) > 0 && !(leaf && l == npl && !iflocal(b))) H.loc_slot[b] = H.nloc++;
       }
     // (a) form, levels nlevels .. max(npwlevel+1, 0) (fgt2d.f:871)
     for (int l = P.nlevels; l >= std::max(npl + 1, 0); l--) {
       int p = H.nlocal[l];
-      int route = ROUTE_HERMITE;
-      if (D == 3) {
-        double r1 = (p + 1.0) / P.npw, r3 = r1 * r1 * r1;
-        route = r3 >= 3 ? ROUTE_PW : ROUTE_HERMITE;  // fgt3d.f:931-940
-      }
       for (int b = t.lfirst[l]; b <= t.llast[l]; b++) {
         if (t.nchild[b] != 0 || t.ns(b) <= 0) continue;
-        int r = route;
-        if (D == 3 && route == ROUTE_PW && t.ns(b) > 1000000) r = ROUTE_HERMITE;
-        // a 3D Hermite block of more than 29^3 coefficients does not fit in
-        // shared memory; the exact exponential sum replaces it there
-        if (D == 3 && r == ROUTE_HERMITE && p + 1 > 29) r = ROUTE_PW;
-        H.form.push_back({b, t.s0[b], t.ns(b), H.mp_slot[b], p, r});
+        H.form.push_back({b, t.s0[b], t.ns(b), H.mp_slot[b], p, form_route(l, b)});
         H.form_sources += t.ns(b);
       }
     }
-    // (b) merge, parents at levels nlevels-1 .. nlevstart
-    for (int l = P.nlevels - 1; l >= nls; l--) {
+    // (b) merge, parents at levels nlevels-1 .. nlevstart (2D; in 3D the plan's
+    // device side adds the leaves to the cut level)
+    for (int l = P.nlevels - 1; l >= nls && D == 2; l--) {
       H.merge_beg[l] = (int)H.merge.size();
       for (int b = t.lfirst[l]; b <= t.llast[l]; b++) {
         if (H.mp_slot[b] < 0 || t.nchild[b] == 0) continue;
@@ -440,6 +446,17 @@ static void build_tasks(HostPlan& H) {
     start(H.nmp); for (auto& s : H.merge) see(s.src); ra = c;
     start(H.nmp); for (auto& s : H.merge) see(s.dst); rb = c;
     H.shift_bytes[0] = per * (ra + rb);
+    if (D == 3) {  // the leaves' own expansions and the cut-level expansions they are added to
+      start(H.nmp);
+      for (auto& f : H.form)
+        if (f.route == ROUTE_PW && t.level[f.box] > nls) {
+          see(f.slot);
+          int a = f.box;
+          while (t.level[a] > nls) a = t.parent[a];
+          see(H.mp_slot[a]);
+        }
+      H.shift_bytes[0] = per * c;
+    }
     start(H.nmp); for (auto& m : H.m2l) see(m.self_mp); for (auto& n : H.m2l_nbr) see(n.mp); ra = c;
     start(H.nloc); for (auto& m : H.m2l) see(m.loc); rb = c;
     H.shift_bytes[1] = per * (ra + rb);
