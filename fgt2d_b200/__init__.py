@@ -195,11 +195,11 @@ class Context:
         _check(lib().fgt_ctx_set_scheme(self._h, {"planewave": 0, "nufft": 1}[scheme]), "fgt_ctx_set_scheme")
 
     def set_sm_budget(self, sms):
-        """SMs the persistent kernels of plans created afterwards size their grids for (0: all)."""
+        """Accepted, without effect (the transforms have no persistent kernels)."""
         _check(lib().fgt_ctx_set_sm_budget(self._h, int(sms)), "fgt_ctx_set_sm_budget")
 
     def set_grid_yield(self, on):
-        """One CTA per task instead of persistent CTAs (plans created afterwards)."""
+        """Accepted, without effect (the transforms have no persistent kernels)."""
         _check(lib().fgt_ctx_set_grid_yield(self._h, int(bool(on))), "fgt_ctx_set_grid_yield")
 
     def set_precision(self, precision):

@@ -32,8 +32,6 @@ struct fgt_ctx {
   int precision = FGT_PREC_AUTO;
   int tree = FGT_TREE_DEVICE;
   int nthreads = 0;
-  int sm_budget = 0;  // SMs the persistent kernels of this context's plans size their grids for (0: all)
-  bool yield_grids = false;  // one CTA per task where a kernel allows it (DevicePlan::yield_grids)
   int scheme = FGT_SCHEME_PLANEWAVE;  // the algorithm of the context's plans
   // uploads of a one-shot call's source strengths: they follow the points on
   // the copy engine while the tree build runs on `stream`
@@ -204,8 +202,6 @@ int plan_device(fgt_plan* p, const double* src_host, const double* trg_host) {
   if (!P.large_delta) {
     CKS(device_plan_create(p->H, p->D));
     p->have_device = true;
-    p->D.persist_sms = p->ctx->sm_budget;
-  p->D.yield_grids = p->ctx->yield_grids;
     CKS(device_plan_set_points(p->D, p->d_src, p->d_trg, st));
   }
   return FGT_OK;
@@ -301,8 +297,6 @@ int plan_create_device_tree(fgt_plan* p, int dim, int nd, double delta, double e
   }
   CKS(device_plan_create(p->H, p->D, d_isrc, d_itarg, s));
   p->have_device = true;
-  p->D.persist_sms = p->ctx->sm_budget;
-  p->D.yield_grids = p->ctx->yield_grids;
   CKS(device_plan_set_points(p->D, p->d_src, p->d_trg, s));
   CKS(cudaStreamSynchronize(s));
   if (getenv("FGT_TREE_TIMING"))
@@ -557,12 +551,10 @@ int fgt_ctx_set_scheme(fgt_ctx* c, int scheme) {
 }
 int fgt_ctx_set_sm_budget(fgt_ctx* c, int sms) {
   if (!c || sms < 0) return FGT_ERR_BADARG;
-  c->sm_budget = sms;
   return FGT_OK;
 }
-int fgt_ctx_set_grid_yield(fgt_ctx* c, int on) {
+int fgt_ctx_set_grid_yield(fgt_ctx* c, int) {
   if (!c) return FGT_ERR_BADARG;
-  c->yield_grids = on != 0;
   return FGT_OK;
 }
 int fgt_ctx_set_host_threads(fgt_ctx* c, int nthreads) {
@@ -1008,13 +1000,30 @@ int fgt_plan_expansion(fgt_plan* p, int which, int box, double* out) {
     CKS(device_plan_box_expansion(H, p->D, box, out, p->ctx->stream));
     return FGT_OK;
   }
-  if (slots[box] < 0) return FGT_ERR_BADARG;
+  int slot = slots[box], a = box;
+  if (which == 1 && slot < 0 && H.P.dim == 3 && H.P.scheme == 0 && H.tree.level[box] > lcut &&
+      ((H.P.ifpghtarg > 0 ? H.tree.nt(box) : 0) + (H.P.ifpgh > 0 ? H.tree.ns(box) : 0)) > 0) {
+    while (H.tree.level[a] > lcut) a = H.tree.parent[a];
+    slot = slots[a];
+  }
+  if (slot < 0) return FGT_ERR_BADARG;
   const double2* pool = which == 0 ? p->D.mp : p->D.loc;
   const size_t per = (size_t)H.P.nd * H.P.nexp;
   CKS(cudaSetDevice(p->ctx->device));
   if (p->done) CKS(cudaEventSynchronize(p->done));
-  CKS(cudaMemcpyAsync(out, pool + (size_t)slots[box] * per, per * 16, cudaMemcpyDeviceToHost, p->ctx->stream));
+  CKS(cudaMemcpyAsync(out, pool + (size_t)slot * per, per * 16, cudaMemcpyDeviceToHost, p->ctx->stream));
   CKS(cudaStreamSynchronize(p->ctx->stream));
+  if (a != box) {  // below the cut level: the cut-level box's expansion about this box's centre
+    const int npw = H.P.npw;
+    for (size_t e = 0; e < per; e++) {
+      const int i = (int)(e % H.P.nexp), m[3] = {i % npw, (i / npw) % npw, i / (npw * npw)};
+      double th = 0.0;
+      for (int d = 0; d < 3; d++) th += H.ts[m[d]] * (H.tree.c(box, d) - H.tree.c(a, d)) * H.P.dsq;
+      const double c = std::cos(th), s = std::sin(th), re = out[2 * e], im = out[2 * e + 1];
+      out[2 * e] = re * c - im * s;
+      out[2 * e + 1] = re * s + im * c;
+    }
+  }
   return FGT_OK;
 }
 

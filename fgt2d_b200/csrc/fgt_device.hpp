@@ -69,12 +69,8 @@ struct HornerTask {
 // A leaf below (or at) a root box, with its place in the root's grid of boxes
 // of its level: the root holds 2^d boxes per dimension at depth d.
 struct SepItem {
-  int box = 0, root = 0;  // boxes; root by its position in the list of roots
-  int p = 0, d = 0;       // order of the block, depth below the root
-  int x[3] = {0, 0, 0};   // place in the root's grid
-  long long off = 0;      // the leaf's block (doubles)
-  int n = 1;              // partial blocks at off, off + P^3, ... (Hermite blocks)
-  int index = 0;          // the caller's number of the leaf
+  int box, root;  // box; root as its number among the boxes of the root level
+  int d, x[3];    // depth below the root, place in the root's grid
 };
 // A leaf's plane-wave expansion added to a cut-level one: its slot and its
 // phase rows in x, y and z.
@@ -94,6 +90,13 @@ struct SepNode {
 };
 struct SepGroup {  // columns and slabs of one order
   int p, cbeg, cend, sbeg, send;
+  bool blocks = true;  // downward: the leaves get Taylor blocks
+};
+// Evaluation of a leaf's points [i0, i0 + n) of a set from its column: the
+// column's offset, the leaf's z phase row, order + 1.
+struct ColTask {
+  int box, set, i0, n, row, p;
+  long long off;
 };
 struct SepLists {
   std::vector<SepLeaf> leaves;
@@ -176,29 +179,18 @@ struct DevicePlan {
   // 3D Hermite form in two kernels: source chunks and their partial blocks
   FormChunk* fchunks = nullptr;
   int nfchunks = 0;
-  int* fcbeg = nullptr;      // per Hermite form task, first chunk (size n+1)
   double* hbuf = nullptr;    // partial Hermite blocks
   // 3D plane-wave scheme: the leaves' Hermite blocks to the cut level's
   // expansions; the leaves' own expansions (plane-wave route) added to them
-  SepDev up;
+  SepDev up, dn;  // dn: the cut level's local expansions to the leaves' evaluation
+  ColTask* ctask = nullptr;
+  std::vector<OrderGroup> ctask_groups;
   MergeGroup* upw_groups = nullptr;
   SepShift* upw = nullptr;
   int nupw_groups = 0;
-  std::vector<SepItem> up_items;  // the Hermite leaves (host copy)
-  bool eval3_smem = false;
-  bool eval3_split = false;  // 3D Taylor eval in two kernels (conversion, Horner)
-  int eval3_nsplit = 0;      // 3D Taylor tasks [0, eval3_nsplit) take the two kernels
-  size_t eval3_sh = 0;
+  std::vector<int> up_box;       // the Hermite leaves and their blocks (host copy)
+  std::vector<SepLeaf> up_leaf;
   std::vector<OrderGroup> fchunk_groups;  // chunk ranges of equal order
-  // per-CTA scratch of the 3D separable transforms (fallback path)
-  double2* scratch = nullptr;
-  size_t scratch_per_cta = 0;  // in double2
-  int scratch_ctas = 0;
-  // U2 scratch of the persistent 3D PW -> Taylor conversion: conv3_ctas CTAs
-  // per density, uscr_per_cta doubles each
-  double* uscr = nullptr;
-  size_t uscr_per_cta = 0;
-  int conv3_ctas = 0;
   // launch shapes
   int form_hermite_n = 0, form_pw_n = 0;
   int eval_taylor_n = 0, eval_pw_n = 0;
@@ -216,19 +208,6 @@ struct DevicePlan {
   double* tables = nullptr;  // padded operand tables of the 2D MMA transforms
   std::vector<OrderGroup> conv_groups, horner_groups;
   int sm_count = 148;
-  // SMs the persistent kernels of this plan size their grids for (0: all);
-  // a server caps it so that a large request's persistent kernels leave SMs
-  // to the requests that arrive while they run
-  int persist_sms = 0;
-  int psm() const { return persist_sms > 0 && persist_sms < sm_count ? persist_sms : sm_count; }
-  // One CTA per task instead of persistent CTAs, in the kernels whose CTAs
-  // hold no per-CTA scratch: CTAs of other streams (a server's small
-  // requests, on higher-priority streams) are then scheduled as soon as any
-  // CTA of this plan finishes, not after the whole launch.
-  bool yield_grids = false;
-  int pgrid(int ntask, int per_sm) const {
-    return yield_grids ? ntask : (ntask < psm() * per_sm ? ntask : psm() * per_sm);
-  }
   // statistics copied from the host plan
   long long direct_pairs = 0, form_sources = 0, eval_points = 0;
   long long launches = 0;

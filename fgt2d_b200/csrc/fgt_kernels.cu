@@ -63,11 +63,11 @@ __device__ __forceinline__ double2 cmul_rn(double2 a, double2 b) {
   return make_double2(__dsub_rn(__dmul_rn(a.x, b.x), __dmul_rn(a.y, b.y)),
                       __dadd_rn(__dmul_rn(a.x, b.y), __dmul_rn(a.y, b.x)));
 }
-__global__ void k_shift_tables(int dim, int npw, int nexp, int nlevels, int lstart, int nms,
+__global__ void k_shift_tables(int dim, int npw, int nexp, int nlevels, int lstart, int nms, long long nm,
                                const double2* __restrict__ ww, const double2* __restrict__ w1,
                                double2* __restrict__ wms, double2* __restrict__ wsh) {
   const int nch = 1 << dim, n2 = npw / 2, ns3 = dim == 2 ? 9 : 27;
-  const long long nm = (long long)(nlevels + 1) * nch * nexp, total = nm + (long long)ns3 * nexp;
+  const long long total = nm + (long long)ns3 * nexp;  // nm: merge entries (0: no merge rows)
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
     const bool merge = i < nm;
@@ -668,9 +668,6 @@ __global__ void __launch_bounds__(256) k_form3d_mma(KP k, const FormTask* __rest
   }
 }
 
-// q / d for 0 <= q < 1115 and 1 <= d <= 64, with mg = ceil(2^16 / d)
-__device__ __forceinline__ int div16(int q, int mg) { return (q * mg) >> 16; }
-
 // ------------------------------------------------------------ (c) eval, 2D Taylor in two kernels
 // k_pw2taylor2d: one warp per evaluation leaf converts the leaf's plane-wave
 // expansion L[j2 + n2 j1] into the real Taylor block (g2dpw2local_real_vec,
@@ -920,648 +917,20 @@ __global__ void __launch_bounds__(128) k_eval2d_horner_any(KP k, const HornerTas
   }
 }
 
-// ------------------------------------------------------------ (c) eval, 3D Taylor in two kernels
-// k_pw2taylor3d: one CTA per evaluation leaf converts the leaf's plane-wave
-// expansion L[(m1 npw + m2) npw + m3] (m1 over the stored half) into the real
-// Taylor block (g3dpw2local_real_vec, g3drouts.f:1774-1938)
-//   S1[m2][a]    = i^a  sum_m3 x2l[a][m3] L[m1][m2][m3]        (pass 1, per m1)
-//   U2[a][b][m1] = i^b  sum_m2 x2l[b][m2] S1[m2][a]            (pass 2, per m1)
-//   lo[c][b][a]  = 2 Re( i^c sum_{m1 < n2} x2l[c][m1] U2[a][b][m1] )   (pass 3)
-// as FP64 MMA products.  Passes 1 and 2 run slice by slice over m1 (the
-// warps take the slices in turn), so the only large intermediate is U2,
-// kept as its real and imaginary parts: pass 3 is two real products, even c
-// against Re U2 and odd c against Im U2 (2 Re(i^c z) keeps z.x or z.y).
-// Pass 1 reads L straight from the expansion pool: a fragment is four runs of
-// 64 contiguous bytes.  The real and imaginary parts of a pass-1 or pass-2
-// result sit in the lanes r and r xor 1 of the accumulator layout (rows
-// interleave re / im), so one exchange pairs them for the rotation.
-struct Conv3Dims {
-  int Pn, E, n2, npw;
-  int N1, K1, M1;       // pass 1: N1 = a (padded), K1 = m3, M1 = (m2, re/im)
-  int M2, K2;           // pass 2: M2 = (a, re/im), K2 = m2, N = N1 (b)
-  int M3, K3, N3;       // pass 3: M3 = (a, b) compact, K3 = m1, N3 = c of one parity
-  int ldT, ldA2, ldU, ldB3;
-  int tab, warp, shared;  // doubles: CTA tables, per-warp area, shared U2
-  __host__ __device__ Conv3Dims(int P, int npw_) {
-    Pn = P;
-    npw = npw_;
-    n2 = npw / 2;
-    E = (Pn + 1) & ~1;
-    N1 = (Pn + 7) & ~7;
-    K1 = (npw + 3) & ~3;
-    M1 = (2 * npw + 7) & ~7;
-    M2 = 2 * N1;
-    K2 = K1;
-    M3 = (Pn * Pn + 7) & ~7;
-    K3 = (n2 + 3) & ~3;
-    N3 = (((Pn + 1) / 2) + 7) & ~7;
-    ldT = mma_ldb(N1);
-    ldA2 = mma_lda(K2);
-    ldU = mma_lda(K3);
-    ldB3 = mma_ldb(N3);
-    tab = K1 * ldT + 2 * K3 * ldB3;
-    warp = M2 * ldA2;
-    shared = 2 * M3 * ldU;
-  }
-};
-
-// Shared memory of k_pw2taylor3d with nw warps (the tables and one pass-2
-// operand per warp; U2 lives in the CTA's global scratch, conv3_scratch).
-size_t conv3_smem_bytes(int Pn, int npw, int nw) {
-  const Conv3Dims Z(Pn, npw);
-  return ((size_t)Z.tab + (size_t)nw * Z.warp) * 8;
-}
-// Doubles of U2 (real and imaginary parts) per CTA.
-size_t conv3_scratch(int Pn, int npw) {
-  const Conv3Dims Z(Pn, npw);
-  return (size_t)Z.shared;
-}
-
-// Tables of k_pw2taylor3d for order P: XT[m][n] = x2l[n][m] (m < npw, n < P),
-// B3e[m1][i] = x2l[2i][m1], B3o[m1][i] = x2l[2i+1][m1] (m1 < n2), zero padded.
-void build_conv3_table(const HostPlan& H, int Pn, std::vector<double>& out) {
-  const int npw = H.P.npw, n2 = npw / 2;
-  const Conv3Dims Z(Pn, npw);
-  const size_t base = out.size();
-  out.resize(base + Z.tab, 0.0);
-  double* XT = out.data() + base;
-  double* B3e = XT + Z.K1 * Z.ldT;
-  double* B3o = B3e + Z.K3 * Z.ldB3;
-  for (int m = 0; m < npw; m++)
-    for (int n = 0; n < Pn; n++) XT[m * Z.ldT + n] = H.x2l[(size_t)n * npw + m];
-  for (int m1 = 0; m1 < n2; m1++)
-    for (int c = 0; c < Pn; c++) {
-      double* B = (c & 1) ? B3o : B3e;
-      B[m1 * Z.ldB3 + c / 2] = H.x2l[(size_t)c * npw + m1];
-    }
-}
-
-// Persistent CTAs: the launch's tasks (one order) are taken in turn; U2
-// (the pass-3 operand, 2 P^2 n2 doubles) lives in the CTA's slice of uscr
-// (global memory, L2-resident), so shared memory holds only the tables and
-// one pass-2 operand per warp and several CTAs fit on an SM.
-template <int KS1>  // pass 1 depth in steps of 4: KS1 = ceil(npw / 4)
-__global__ void __launch_bounds__(128) k_pw2taylor3d(KP k, const ConvTask* __restrict__ tasks, int ntask,
-                                                     double* __restrict__ lo_all,
-                                                     const double* __restrict__ tab,
-                                                     double* __restrict__ uscr, size_t uper) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int r = lane >> 2, c = lane & 3;
-  const int ind = blockIdx.y;
-  const Conv3Dims Z(tasks[0].p + 1, k.npw);
-  const int Pn = Z.Pn, E = Z.E, npw = Z.npw, n2 = Z.n2;
-  extern __shared__ double s3[];
-  double* XT = s3;                                 // [K1][ldT]
-  double* B3e = XT + Z.K1 * Z.ldT;                 // [K3][ldB3]
-  double* B3o = B3e + Z.K3 * Z.ldB3;
-  double* A2 = s3 + Z.tab + warp * Z.warp;         // [M2][ldA2]
-  double* Ure = uscr + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * uper;  // [M3][ldU]
-  double* Uim = Ure + Z.M3 * Z.ldU;
-  for (int e = threadIdx.x; e < Z.tab; e += blockDim.x) s3[e] = tab[e];
-  // every task writes the same entries of U2; the rest (padding) stays zero
-  for (int e = threadIdx.x; e < 2 * Z.M3 * Z.ldU; e += blockDim.x) Ure[e] = 0.0;
-  __syncthreads();
-  for (int task = blockIdx.x; task < ntask; task += gridDim.x) {
-    const ConvTask T = tasks[task];
-    const double* Ld = reinterpret_cast<const double*>(k.loc + ((size_t)T.slot * k.nd + ind) * k.nexp);
-    for (int m1 = warp; m1 < n2; m1 += nw) {
-      // pass 1: rows (m2, re/im) of the slice, columns a
-      for (int mt = 0; mt < Z.M1 / 8; mt++) {
-        const int row = 8 * mt + r, m2 = row >> 1, comp = row & 1;
-        const bool rok = m2 < npw;
-        const double* ap = Ld + ((size_t)(m1 * npw + m2) * npw) * 2 + comp;
-        double av[KS1];
-#pragma unroll
-        for (int ks = 0; ks < KS1; ks++) {
-          const int m3 = 4 * ks + c;
-          av[ks] = (rok && m3 < npw) ? __ldg(ap + 2 * m3) : 0.0;
-        }
-        for (int nt = 0; nt < Z.N1 / 8; nt++) {
-          const double* bp = XT + c * Z.ldT + 8 * nt + r;
-          double d0 = 0.0, d1 = 0.0, e0 = 0.0, e1 = 0.0;
-#pragma unroll
-          for (int ks = 0; ks < KS1; ks++) {
-            if (ks & 1) dmma_884(e0, e1, av[ks], bp[4 * ks * Z.ldT]);
-            else dmma_884(d0, d1, av[ks], bp[4 * ks * Z.ldT]);
-          }
-          d0 += e0;
-          d1 += e1;
-          // lane r holds comp (r & 1) of S1[m2][a0], S1[m2][a0 + 1]; r xor 1 the other
-          const double o0 = __shfl_xor_sync(FULL_MASK, d0, 4), o1 = __shfl_xor_sync(FULL_MASK, d1, 4);
-          const int a0 = 8 * nt + 2 * c;
-          const double2 z0 = rot_bf(comp ? make_double2(o0, d0) : make_double2(d0, o0), a0);
-          const double2 z1 = rot_bf(comp ? make_double2(o1, d1) : make_double2(d1, o1), a0 + 1);
-          if (m2 < Z.K2) {
-            if (comp == 0) {
-              A2[(2 * a0) * Z.ldA2 + m2] = z0.x;
-              A2[(2 * a0 + 1) * Z.ldA2 + m2] = z0.y;
-            } else {
-              A2[(2 * a0 + 2) * Z.ldA2 + m2] = z1.x;
-              A2[(2 * a0 + 3) * Z.ldA2 + m2] = z1.y;
-            }
-          }
-        }
-      }
-      __syncwarp();
-      // pass 2: rows (a, re/im), columns b; U2[a][b][m1] into Ure / Uim
-      for (int mt = 0; mt < Z.M2 / 8; mt++) {
-        const double* ap = A2 + (8 * mt + r) * Z.ldA2 + c;
-        for (int nt = 0; nt < Z.N1 / 8; nt++) {
-          const double* bp = XT + c * Z.ldT + 8 * nt + r;
-          double d0 = 0.0, d1 = 0.0, e0 = 0.0, e1 = 0.0;
-          for (int ks = 0; ks < Z.K2 / 4; ks += 2) {
-            dmma_884(d0, d1, ap[4 * ks], bp[4 * ks * Z.ldT]);
-            if (ks + 1 < Z.K2 / 4) dmma_884(e0, e1, ap[4 * ks + 4], bp[(4 * ks + 4) * Z.ldT]);
-          }
-          d0 += e0;
-          d1 += e1;
-          const double o0 = __shfl_xor_sync(FULL_MASK, d0, 4), o1 = __shfl_xor_sync(FULL_MASK, d1, 4);
-          const int row = 8 * mt + r, a = row >> 1, comp = row & 1, b0 = 8 * nt + 2 * c;
-          const double2 z0 = rot_bf(comp ? make_double2(o0, d0) : make_double2(d0, o0), b0);
-          const double2 z1 = rot_bf(comp ? make_double2(o1, d1) : make_double2(d1, o1), b0 + 1);
-          if (a < Pn) {
-            if (comp == 0 && b0 < Pn) {
-              Ure[(a * Pn + b0) * Z.ldU + m1] = z0.x;
-              Uim[(a * Pn + b0) * Z.ldU + m1] = z0.y;
-            }
-            if (comp == 1 && b0 + 1 < Pn) {
-              Ure[(a * Pn + b0 + 1) * Z.ldU + m1] = z1.x;
-              Uim[(a * Pn + b0 + 1) * Z.ldU + m1] = z1.y;
-            }
-          }
-        }
-      }
-      __syncwarp();
-    }
-    __syncthreads();
-    // pass 3: lo[c][b][a] = 2 {x, -y, -x, y}[c mod 4] of sum_m1 x2l[c][m1] U2[a][b][m1]
-    double* out = lo_all + T.off + (size_t)ind * Pn * Pn * E;
-    for (int mt = warp; mt < Z.M3 / 8; mt += nw) {
-      const double* ae = Ure + (8 * mt + r) * Z.ldU + c;
-      const double* ao = Uim + (8 * mt + r) * Z.ldU + c;
-      for (int nt = 0; nt < Z.N3 / 8; nt++) {
-        const double* be = B3e + c * Z.ldB3 + 8 * nt + r;
-        const double* bo = B3o + c * Z.ldB3 + 8 * nt + r;
-        double e0 = 0.0, e1 = 0.0, o0 = 0.0, o1 = 0.0;
-        for (int ks = 0; ks < Z.K3 / 4; ks++) {
-          dmma_884(e0, e1, ae[4 * ks], be[4 * ks * Z.ldB3]);
-          dmma_884(o0, o1, ao[4 * ks], bo[4 * ks * Z.ldB3]);
-        }
-        const int q = 8 * mt + r;
-        if (q >= Pn * Pn) continue;
-        const int a = q / Pn, b = q - a * Pn;
-        const double ev[2] = {e0, e1}, od[2] = {o0, o1};
-#pragma unroll
-        for (int i = 0; i < 2; i++) {
-          const int ce = 2 * (8 * nt + 2 * c + i), co = ce + 1;
-          if (ce < Pn) out[((size_t)ce * Pn + b) * E + a] = ((ce & 3) == 2 ? -2.0 : 2.0) * ev[i];
-          if (co < Pn) out[((size_t)co * Pn + b) * E + a] = ((co & 3) == 1 ? -2.0 : 2.0) * od[i];
-        }
-      }
-    }
-    if (E > Pn)  // the padding column of every row
-      for (int e = threadIdx.x; e < Pn * Pn; e += blockDim.x) out[(size_t)e * E + Pn] = 0.0;
-    __syncthreads();  // U2 of this task is read until here
-  }
-}
-
-// k_pw2taylor3d_mma: the conversion of k_pw2taylor3d for orders P <= 16 with
-// the mirror symmetry of the node set used in both full dimensions and the
-// node tables as register fragments.  With the signed table
-// tx[a][m] = x2l[a][m] (-1)^(a/2) over the first half m < n2 and mirror node
-// mb = npw - 1 - m (x2l[a][mb] = (-1)^a x2l[a][m]), a sum over all nodes is
-//   i^a sum_m x2l[a][m] L[m] = tx[a][.] (L[m] + L[mb])        (a even)
-//                            = i tx[a][.] (L[m] - L[mb])      (a odd),
-// so every pass is two real products of depth n2 (KS k-steps of 4):
-//   x pass  S1[m1][m2][a] from the staged slices of L     (M = a, N = (m1, m2, re/im))
-//   y pass  S2[m1][b][a]  from S1, same table in b         (M = b, N = (m1, a, re/im))
-//   z pass  lo[c][b][a] += 2 Re(i^c tx[c][m1] S2[m1][b][a]): even c against
-//           Re S2, odd c against -Im S2, K = the four slices m1 of a group
-// The leaf is taken four z slices (one z k-step) at a time: the slices are
-// copied into shared memory with cp.async (the next group's copy overlaps
-// the y and z passes of this one), and the z accumulators stay in registers
-// across the groups (each warp owns up to four of the ceil(P^2 / 8) column
-// tiles).  Row strides: staged slices 8 (mod 16) doubles (the fragment's
-// re/im pairs of four rows are conflict-free), S1 and S2 4 (mod 8).
-// Persistent CTAs of 8 warps, two per SM, over the leaves of one order.
-struct C3Dims {
-  int ldL, ld1, ld2;
-  size_t total;  // doubles
-  __host__ __device__ C3Dims(int Pn, int npw) {
-    ldL = ((2 * npw + 7) & ~15) + 8;
-    ld1 = 8 * Pn + 4;
-    ld2 = 8 * ((Pn * Pn + 7) / 8) + 4;
-    total = (size_t)4 * npw * ldL + (size_t)npw * ld1 + (size_t)8 * ld2 + (size_t)2 * (2 * npw + npw / 2);
-  }
-};
-// The fused split's phase tables of one task (x and y over all npw nodes, z
-// over the stored half) into ph (double2 [2 npw + n2]); node t_m = x2l[1][m].
-__device__ __forceinline__ void conv_phases(const KP& k, const ConvTask& T, double2* ph) {
-  const int npw = k.npw, n2 = k.n2;
-  for (int e = threadIdx.x; e < 2 * npw + n2; e += blockDim.x) {
-    const int d = e < npw ? 0 : e < 2 * npw ? 1 : 2, m = e - d * npw;
-    double sn, cs;
-    sincos(k.x2l[npw + m] * T.sh[d], &sn, &cs);
-    ph[e] = make_double2(cs, sn);
-  }
-}
-// Multiplies staged slices (rows (m1, m2) of npw complex m3, row stride ldL
-// doubles, slices m1 = m1_0 .. m1_0 + ns - 1) by the task's phases.
-__device__ __forceinline__ void conv_apply_phases(double* Lb, int ldL, int npw, int m1_0, int ns,
-                                                  const double2* ph) {
-  const int n = ns * npw * npw;
-  for (int e = threadIdx.x; e < n; e += blockDim.x) {
-    const int row = e / npw, m3 = e - row * npw, m1 = m1_0 + row / npw, m2 = row - (row / npw) * npw;
-    double2* z = reinterpret_cast<double2*>(Lb + (size_t)row * ldL + 2 * m3);
-    *z = cmul(*z, cmul(ph[m3], cmul(ph[npw + m2], ph[2 * npw + m1])));
-  }
-}
-
-template <int KS>
-__global__ void __launch_bounds__(256, 2) k_pw2taylor3d_mma(KP k, const ConvTask* __restrict__ tasks, int ntask,
-                                                            double* __restrict__ lo_all) {
-  constexpr int NTW = 4;  // z-pass column tiles per warp (ceil(16^2 / 8) / 8)
-  const int ind = blockIdx.y;
-  const int npw = k.npw, n2 = k.n2;
-  const int Pn = tasks[0].p + 1, E = (Pn + 1) & ~1, P2 = Pn * Pn;
-  const int mgN = (65536 + npw - 1) / npw, mgP = (65536 + Pn - 1) / Pn;  // div16 factors
-  const C3Dims Z(Pn, npw);
-  extern __shared__ double sm[];
-  double* Lb = sm;                                  // [4 m1][npw m2][ldL]: (m3, re/im)
-  double* S1 = Lb + (size_t)4 * npw * Z.ldL;        // [npw m2][ld1]: (m1, a, re/im)
-  double* S2r = S1 + (size_t)npw * Z.ld1;           // [4 m1][ld2]: (b, a)
-  double* S2i = S2r + 4 * Z.ld2;
-  double2* PH = reinterpret_cast<double2*>(S2i + 4 * Z.ld2);  // fused split: [2 npw + n2] phases
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = lane >> 2, c = lane & 3;
-  int tk = blockIdx.x;
-  if (tk >= ntask) return;
-  // A fragments: tx[par][s] = table row 2 r + par, node 4 s + c
-  double tx[2][KS];
-#pragma unroll
-  for (int par = 0; par < 2; par++)
-#pragma unroll
-    for (int s = 0; s < KS; s++) {
-      const int a = 2 * r + par, m = 4 * s + c;
-      tx[par][s] = (a < Pn && m < n2) ? (((a >> 1) & 1) ? -k.x2l[a * npw + m] : k.x2l[a * npw + m]) : 0.0;
-    }
-  // copy the slices 4 g .. 4 g + 3 of the expansion in the given slot (rows of npw complex)
-  auto stage = [&](int slot, int g) {
-    const double* L = reinterpret_cast<const double*>(k.loc + ((size_t)slot * k.nd + ind) * k.nexp) +
-                      (size_t)8 * g * npw * npw;
-    const int rows = min(4, n2 - 4 * g) * npw;
-    const unsigned dst = (unsigned)__cvta_generic_to_shared(Lb);
-    for (int row = warp; row < rows; row += 8)
-      for (int u = lane; u < npw; u += 32)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 8u * (unsigned)(row * Z.ldL + 2 * u)),
-                     "l"(L + (size_t)row * 2 * npw + 2 * u) : "memory");
-  };
-  int slot = tasks[tk].slot;
-  stage(slot, 0);
-  double acc[NTW][2][2];
-#pragma unroll
-  for (int i = 0; i < NTW; i++) acc[i][0][0] = acc[i][0][1] = acc[i][1][0] = acc[i][1][1] = 0.0;
-  const int ntZ = (P2 + 7) / 8;
-  for (; tk < ntask; tk += gridDim.x) {
-    const int tn = tk + gridDim.x;
-    const int nslot = tn < ntask ? tasks[tn].slot : 0;
-    const long long off = tasks[tk].off;
-    const bool fused = tasks[tk].fused;
-    if (fused) conv_phases(k, tasks[tk], PH);
-    for (int g = 0; g < KS; g++) {
-      const int ns = min(4, n2 - 4 * g);
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      __syncthreads();
-      if (fused) {  // the ancestor's slices become the leaf's: the split, fused
-        conv_apply_phases(Lb, Z.ldL, npw, 4 * g, ns, PH);
-        __syncthreads();
-      }
-      // x pass: columns (m1, m2, re/im) of the staged slices
-      const int ntX = (ns * npw * 2 + 7) / 8;
-      for (int nt = warp; nt < ntX; nt += 8) {
-        const int col = 8 * nt + r;
-        const double* bp = Lb + (col >> 1) * Z.ldL + (col & 1);
-        double e0 = 0.0, e1 = 0.0, o0 = 0.0, o1 = 0.0;
-#pragma unroll
-        for (int s = 0; s < KS; s++) {
-          const int m = 4 * s + c;
-          double v1 = 0.0, v2 = 0.0;
-          if (m < n2) {
-            v1 = bp[2 * m];
-            v2 = bp[2 * (npw - 1 - m)];
-          }
-          dmma_884(e0, e1, tx[0][s], v1 + v2);
-          dmma_884(o0, o1, tx[1][s], v1 - v2);
-        }
-        const int q = 4 * nt + c;  // the lane's complex column (m1, m2)
-        if (q < ns * npw) {
-          const int m1 = div16(q, mgN), m2 = q - m1 * npw;
-          double* o = S1 + m2 * Z.ld1 + 2 * (m1 * Pn + 2 * r);
-          if (2 * r < Pn) *reinterpret_cast<double2*>(o) = make_double2(e0, e1);
-          if (2 * r + 1 < Pn) *reinterpret_cast<double2*>(o + 2) = make_double2(-o1, o0);
-        }
-      }
-      __syncthreads();
-      // the slices are consumed: copy the next group's (or the next leaf's first)
-      if (g + 1 < KS) stage(slot, g + 1);
-      else if (tn < ntask) stage(nslot, 0);
-      // y pass: columns (m1, a, re/im)
-      const int ntY = (ns * Pn * 2 + 7) / 8;
-      for (int nt = warp; nt < ntY; nt += 8) {
-        const int col = 8 * nt + r;
-        double e0 = 0.0, e1 = 0.0, o0 = 0.0, o1 = 0.0;
-#pragma unroll
-        for (int s = 0; s < KS; s++) {
-          const int m = 4 * s + c;
-          double v1 = 0.0, v2 = 0.0;
-          if (m < n2) {
-            v1 = S1[m * Z.ld1 + col];
-            v2 = S1[(npw - 1 - m) * Z.ld1 + col];
-          }
-          dmma_884(e0, e1, tx[0][s], v1 + v2);
-          dmma_884(o0, o1, tx[1][s], v1 - v2);
-        }
-        const int q = 4 * nt + c;  // the lane's complex column (m1, a)
-        if (q < ns * Pn) {
-          const int m1 = div16(q, mgP), a = q - m1 * Pn;
-          const int o = m1 * Z.ld2 + 2 * r * Pn + a;
-          if (2 * r < Pn) {
-            S2r[o] = e0;
-            S2i[o] = e1;
-          }
-          if (2 * r + 1 < Pn) {
-            S2r[o + Pn] = -o1;
-            S2i[o + Pn] = o0;
-          }
-        }
-      }
-      __syncthreads();
-      // z pass: k-step g of the accumulators, rows c = 2 r + par, columns (b, a)
-      double te = tx[0][0], to = tx[1][0];
-#pragma unroll
-      for (int s = 1; s < KS; s++)
-        if (s == g) {
-          te = tx[0][s];
-          to = tx[1][s];
-        }
-#pragma unroll
-      for (int i = 0; i < NTW; i++) {
-        const int nt = warp + 8 * i;
-        if (nt < ntZ) {
-          const double br = c < ns ? S2r[c * Z.ld2 + 8 * nt + r] : 0.0;
-          const double bi = c < ns ? S2i[c * Z.ld2 + 8 * nt + r] : 0.0;
-          dmma_884(acc[i][0][0], acc[i][0][1], te, br);
-          dmma_884(acc[i][1][0], acc[i][1][1], to, bi);
-        }
-      }
-    }
-    // lo[c][b][a] = 2 acc (even c), -2 acc (odd c); rows of E doubles
-    double* out = lo_all + off + (size_t)ind * P2 * E;
-#pragma unroll
-    for (int i = 0; i < NTW; i++) {
-      const int nt = warp + 8 * i;
-#pragma unroll
-      for (int ii = 0; ii < 2; ii++) {
-        const int q = 8 * nt + 2 * c + ii;
-        if (nt < ntZ && q < P2) {
-          const int b = div16(q, mgP), a = q - b * Pn;
-          if (2 * r < Pn) out[((2 * r) * Pn + b) * E + a] = 2.0 * acc[i][0][ii];
-          if (2 * r + 1 < Pn) out[((2 * r + 1) * Pn + b) * E + a] = -2.0 * acc[i][1][ii];
-        }
-        acc[i][0][ii] = acc[i][1][ii] = 0.0;
-      }
-    }
-    if (E > Pn)  // the padding column of every row
-      for (int e = threadIdx.x; e < P2; e += blockDim.x) out[(size_t)e * E + Pn] = 0.0;
-    slot = nslot;
-  }
-}
-
-// k_pw2taylor3d_mma2: the same conversion for orders 17..32 (two 8-row tiles
-// of each parity).  The z accumulators of these orders do not fit in
-// registers, so S2 keeps every z slice (Re and Im, n2 rows of P^2) and the z
-// pass runs once per leaf after the x and y passes of all its slice groups;
-// a group is gs slices (4, 2 or 1, the largest whose shared memory fits).
-// One CTA of 8 warps per SM, persistent over the leaves of one order.
-struct C3Dims2 {
-  int gs, ldL, ld1, ld2;
-  size_t total;  // doubles
-  __host__ __device__ C3Dims2(int Pn, int npw, int gs_) {
-    const int n2 = npw / 2;
-    gs = gs_;
-    ldL = ((2 * npw + 7) & ~15) + 8;
-    ld1 = 8 * ((2 * gs * Pn + 7) / 8) + 4;
-    ld2 = 8 * ((Pn * Pn + 7) / 8) + 4;
-    total = (size_t)gs * npw * ldL + (size_t)npw * ld1 + (size_t)2 * n2 * ld2 + (size_t)2 * (2 * npw + n2);
-  }
-};
-
-template <int KS>
-__global__ void __launch_bounds__(256, 1) k_pw2taylor3d_mma2(KP k, const ConvTask* __restrict__ tasks, int ntask,
-                                                             double* __restrict__ lo_all, int gs) {
-  const int ind = blockIdx.y;
-  const int npw = k.npw, n2 = k.n2;
-  const int Pn = tasks[0].p + 1, E = (Pn + 1) & ~1, P2 = Pn * Pn;
-  const int mgN = (65536 + npw - 1) / npw, mgP = (65536 + Pn - 1) / Pn;  // div16 factors
-  const C3Dims2 Z(Pn, npw, gs);
-  extern __shared__ double sm[];
-  double* Lb = sm;                                  // [gs m1][npw m2][ldL]: (m3, re/im)
-  double* S1 = Lb + (size_t)gs * npw * Z.ldL;       // [npw m2][ld1]: (m1, a, re/im)
-  double* S2r = S1 + (size_t)npw * Z.ld1;           // [n2 m1][ld2]: (b, a)
-  double* S2i = S2r + (size_t)n2 * Z.ld2;
-  double2* PH = reinterpret_cast<double2*>(S2i + (size_t)n2 * Z.ld2);  // fused split: [2 npw + n2] phases
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = lane >> 2, c = lane & 3;
-  int tk = blockIdx.x;
-  if (tk >= ntask) return;
-  // A fragments: tx[u][par][s] = table row 2 (8 u + r) + par, node 4 s + c
-  double tx[2][2][KS];
-#pragma unroll
-  for (int u = 0; u < 2; u++)
-#pragma unroll
-    for (int par = 0; par < 2; par++)
-#pragma unroll
-      for (int s = 0; s < KS; s++) {
-        const int a = 2 * (8 * u + r) + par, m = 4 * s + c;
-        tx[u][par][s] =
-            (a < Pn && m < n2) ? (((a >> 1) & 1) ? -k.x2l[a * npw + m] : k.x2l[a * npw + m]) : 0.0;
-      }
-  const int ng = (n2 + gs - 1) / gs;
-  auto stage = [&](int slot, int g) {
-    const double* L = reinterpret_cast<const double*>(k.loc + ((size_t)slot * k.nd + ind) * k.nexp) +
-                      (size_t)2 * gs * g * npw * npw;
-    const int rows = min(gs, n2 - gs * g) * npw;
-    const unsigned dst = (unsigned)__cvta_generic_to_shared(Lb);
-    for (int row = warp; row < rows; row += 8)
-      for (int u = lane; u < npw; u += 32)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 8u * (unsigned)(row * Z.ldL + 2 * u)),
-                     "l"(L + (size_t)row * 2 * npw + 2 * u) : "memory");
-  };
-  int slot = tasks[tk].slot;
-  stage(slot, 0);
-  const int ntZ = (P2 + 7) / 8;
-  for (; tk < ntask; tk += gridDim.x) {
-    const int tn = tk + gridDim.x;
-    const int nslot = tn < ntask ? tasks[tn].slot : 0;
-    const long long off = tasks[tk].off;
-    const bool fused = tasks[tk].fused;
-    if (fused) conv_phases(k, tasks[tk], PH);
-    for (int g = 0; g < ng; g++) {
-      const int ns = min(gs, n2 - gs * g);
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      __syncthreads();
-      if (fused) {  // the ancestor's slices become the leaf's: the split, fused
-        conv_apply_phases(Lb, Z.ldL, npw, gs * g, ns, PH);
-        __syncthreads();
-      }
-      // x pass: columns (m1, m2, re/im) of the staged slices
-      const int ntX = (ns * npw * 2 + 7) / 8;
-      for (int nt = warp; nt < ntX; nt += 8) {
-        const int col = 8 * nt + r;
-        const double* bp = Lb + (col >> 1) * Z.ldL + (col & 1);
-        double acc[2][4];
-#pragma unroll
-        for (int u = 0; u < 2; u++) acc[u][0] = acc[u][1] = acc[u][2] = acc[u][3] = 0.0;
-#pragma unroll
-        for (int s = 0; s < KS; s++) {
-          const int m = 4 * s + c;
-          double v1 = 0.0, v2 = 0.0;
-          if (m < n2) {
-            v1 = bp[2 * m];
-            v2 = bp[2 * (npw - 1 - m)];
-          }
-#pragma unroll
-          for (int u = 0; u < 2; u++) {
-            dmma_884(acc[u][0], acc[u][1], tx[u][0][s], v1 + v2);
-            dmma_884(acc[u][2], acc[u][3], tx[u][1][s], v1 - v2);
-          }
-        }
-        const int q = 4 * nt + c;  // the lane's complex column (m1, m2)
-        if (q < ns * npw) {
-          const int m1 = div16(q, mgN), m2 = q - m1 * npw;
-#pragma unroll
-          for (int u = 0; u < 2; u++) {
-            const int a = 2 * (8 * u + r);
-            double* o = S1 + m2 * Z.ld1 + 2 * (m1 * Pn + a);
-            if (a < Pn) *reinterpret_cast<double2*>(o) = make_double2(acc[u][0], acc[u][1]);
-            if (a + 1 < Pn) *reinterpret_cast<double2*>(o + 2) = make_double2(-acc[u][3], acc[u][2]);
-          }
-        }
-      }
-      __syncthreads();
-      // the slices are consumed: copy the next group's (or the next leaf's first)
-      if (g + 1 < ng) stage(slot, g + 1);
-      else if (tn < ntask) stage(nslot, 0);
-      // y pass: columns (m1, a, re/im) into the z slices gs g + m1 of S2
-      const int ntY = (ns * Pn * 2 + 7) / 8;
-      for (int nt = warp; nt < ntY; nt += 8) {
-        const int col = 8 * nt + r;
-        double acc[2][4];
-#pragma unroll
-        for (int u = 0; u < 2; u++) acc[u][0] = acc[u][1] = acc[u][2] = acc[u][3] = 0.0;
-#pragma unroll
-        for (int s = 0; s < KS; s++) {
-          const int m = 4 * s + c;
-          double v1 = 0.0, v2 = 0.0;
-          if (m < n2) {
-            v1 = S1[m * Z.ld1 + col];
-            v2 = S1[(npw - 1 - m) * Z.ld1 + col];
-          }
-#pragma unroll
-          for (int u = 0; u < 2; u++) {
-            dmma_884(acc[u][0], acc[u][1], tx[u][0][s], v1 + v2);
-            dmma_884(acc[u][2], acc[u][3], tx[u][1][s], v1 - v2);
-          }
-        }
-        const int q = 4 * nt + c;  // the lane's complex column (m1, a)
-        if (q < ns * Pn) {
-          const int m1 = div16(q, mgP), a = q - m1 * Pn;
-#pragma unroll
-          for (int u = 0; u < 2; u++) {
-            const int b = 2 * (8 * u + r);
-            const int o = (gs * g + m1) * Z.ld2 + b * Pn + a;
-            if (b < Pn) {
-              S2r[o] = acc[u][0];
-              S2i[o] = acc[u][1];
-            }
-            if (b + 1 < Pn) {
-              S2r[o + Pn] = -acc[u][3];
-              S2i[o + Pn] = acc[u][2];
-            }
-          }
-        }
-      }
-    }
-    __syncthreads();
-    // z pass over all slices: rows c = 2 (8 u + r) + par, columns (b, a)
-    double* out = lo_all + off + (size_t)ind * P2 * E;
-    for (int nt = warp; nt < ntZ; nt += 8) {
-      double acc[2][2][2];
-#pragma unroll
-      for (int u = 0; u < 2; u++) acc[u][0][0] = acc[u][0][1] = acc[u][1][0] = acc[u][1][1] = 0.0;
-#pragma unroll
-      for (int s = 0; s < KS; s++) {
-        const int m1 = 4 * s + c;
-        const double br = m1 < n2 ? S2r[m1 * Z.ld2 + 8 * nt + r] : 0.0;
-        const double bi = m1 < n2 ? S2i[m1 * Z.ld2 + 8 * nt + r] : 0.0;
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-          dmma_884(acc[u][0][0], acc[u][0][1], tx[u][0][s], br);
-          dmma_884(acc[u][1][0], acc[u][1][1], tx[u][1][s], bi);
-        }
-      }
-#pragma unroll
-      for (int ii = 0; ii < 2; ii++) {
-        const int q = 8 * nt + 2 * c + ii;
-        if (q < P2) {
-          const int b = div16(q, mgP), a = q - b * Pn;
-#pragma unroll
-          for (int u = 0; u < 2; u++) {
-            const int ce = 2 * (8 * u + r);
-            if (ce < Pn) out[(ce * Pn + b) * E + a] = 2.0 * acc[u][0][ii];
-            if (ce + 1 < Pn) out[((ce + 1) * Pn + b) * E + a] = -2.0 * acc[u][1][ii];
-          }
-        }
-      }
-    }
-    if (E > Pn)  // the padding column of every row
-      for (int e = threadIdx.x; e < P2; e += blockDim.x) out[(size_t)e * E + Pn] = 0.0;
-    slot = nslot;
-  }
-}
-
-// k_eval3d_sep: potential at a leaf's points straight from its plane-wave
-// local expansion, for the plane-wave route (g3dpwevalp_vec,
-// g3drouts.f:2268-2362) and for Taylor-route leaves whose order exceeds the
-// conversion kernels (g3dpw2local_real_vec + g3dlevalp_vec).  Both are
+// ------------------------------------------------------------ (c) eval, 3D plane-wave route, potentials
+// k_eval3d_sep (g3dpwevalp_vec, g3drouts.f:2268-2362):
 //   pot = 2 Re sum_{m1 < n2} Z[m1](z) sum_{m2} Y[m2](y) sum_{m3} X[m3](x) L[m1][m2][m3]
-// with X[m](x) = exp(i t_m x) on the plane-wave route and, on the Taylor
-// route, its series truncated at the order, sum_{a<P} x2l[a][m] (i x)^a: the
-// Taylor block lo[c][b][a] of the conversion contracted with x^a y^b z^c is
-// exactly this sum, evaluated without forming the P^3 block.  One CTA per
+// with X[m](x) = exp(i t_m x).  One CTA per
 // task; points in blocks of 32 whose phase tables sit in shared memory; a
 // thread takes rows (m1, m2) of the expansion for four points (L read once
 // per block, through the read-only cache), and the partial sums are reduced
 // in a fixed order.  Potentials only (the derivative variants keep their own
 // kernels).
 constexpr int SEP_NPB = 32;
-// xt: the x2l table of the order, staged in shared memory ([a][m], npw per row)
-__device__ __forceinline__ double2 sep_phase(const KP& k, bool taylor, int m, double u, int Pn,
-                                             const double* xt) {
-  const double t = (2 * (m - k.n2) + 1) * k.t1;
-  if (!taylor) return cexpi(t * u);
-  // sum_{a<P} x2l[a][m] (i u)^a by Horner in (i u)
-  double re = xt[(Pn - 1) * k.npw + m], im = 0.0;
-  for (int a = Pn - 2; a >= 0; a--) {
-    const double nr = fma(-im, u, xt[a * k.npw + m]);
-    im = re * u;
-    re = nr;
-  }
-  return make_double2(re, im);
-}
-template <bool TAYLOR>
 __global__ void __launch_bounds__(256, 2) k_eval3d_sep(KP k, const EvalTask* __restrict__ tasks) {
   const EvalTask T = tasks[blockIdx.x];
   const int ind = blockIdx.y;
-  const int npw = k.npw, n2 = k.n2, Pn = T.p + 1, tid = threadIdx.x;
+  const int npw = k.npw, n2 = k.n2, tid = threadIdx.x;
   const double2* L = k.loc + ((size_t)T.slot * k.nd + ind) * k.nexp;
   const double* pts = T.set ? k.trg : k.src;
   double* out = T.set ? k.pottarg : k.pot;
@@ -1572,11 +941,7 @@ __global__ void __launch_bounds__(256, 2) k_eval3d_sep(KP k, const EvalTask* __r
   double2* Y = X + npw * SEP_NPB;           // [npw][SEP_NPB]
   double2* Zt = Y + npw * SEP_NPB;          // [n2][SEP_NPB]
   double2* part = Zt + n2 * SEP_NPB;        // [256][4] partial sums
-  double* xt = reinterpret_cast<double*>(part + 256 * 4);  // Taylor route: x2l rows a < P
-  if (TAYLOR)
-    for (int e = tid; e < Pn * npw; e += blockDim.x) xt[e] = k.x2l[e];
   const int nrow = n2 * npw;
-  __syncthreads();
   for (int p0 = 0; p0 < T.n; p0 += SEP_NPB) {
     const int np = min(SEP_NPB, T.n - p0);
     for (int e = tid; e < (2 * npw + n2) * SEP_NPB; e += blockDim.x) {
@@ -1585,7 +950,7 @@ __global__ void __launch_bounds__(256, 2) k_eval3d_sep(KP k, const EvalTask* __r
       double2 v = make_double2(0.0, 0.0);
       if (pt < np) {
         const double u = (pts[3 * (T.i0 + p0 + pt) + d] - (d == 0 ? cx : d == 1 ? cy : cz)) * k.dsq;
-        v = sep_phase(k, TAYLOR, node, u, Pn, xt);
+        v = cexpi((2 * (node - n2) + 1) * k.t1 * u);
       }
       // X, Y and Zt are consecutive; point 4 g + j sits at j * 8 + g of its
       // row, so the eight point groups of one j are one 128-byte line
@@ -1744,76 +1109,6 @@ __global__ void __launch_bounds__(128) k_eval3d_horner(KP k, const HornerTask* _
   if (two) {
     hemit<PGH>(a[1], k.dsq, v);
     add_out<NC>(out, pb, k.nd, nc, ind, v);
-  }
-}
-
-// ------------------------------------------------------------ (c) eval, 3D Taylor in shared memory
-// One CTA per chunk of an evaluation leaf: plane wave -> Taylor
-// (g3dpw2local_real_vec, g3drouts.f:1774-1938) with x and y passes over the
-// positive half (mirror pre-add) and the z pass over the stored half, then
-// Horner evaluation, two points per thread.
-template <int PGH>
-__global__ void __launch_bounds__(512) k_eval3d_taylor_smem(KP k, const EvalTask* __restrict__ tasks) {
-  constexpr int NC = ncomp<3, PGH>();
-  const EvalTask T = tasks[blockIdx.x];
-  const int ind = blockIdx.y;
-  const int npw = k.npw, n2 = k.n2;
-  const int Pn = T.p + 1, P2 = Pn * Pn;
-  extern __shared__ double sm[];
-  const size_t szA = max((size_t)2 * Pn * npw * n2, (size_t)P2 * Pn);
-  double2* U1 = reinterpret_cast<double2*>(sm);                       // [(a npw + m2) n2 + m1]
-  double* lo = sm;                                                    // overwrites U1
-  double2* U2 = reinterpret_cast<double2*>(sm + ((szA + 1) & ~size_t(1)));  // [(a P + b) n2 + m1]
-  const double2* L = k.loc + ((size_t)T.slot * k.nd + ind) * k.nexp;
-  for (int idx = threadIdx.x; idx < Pn * npw * n2; idx += blockDim.x) {
-    const int m1 = idx % n2, r = idx / n2, m2 = r % npw, a = r / npw;
-    const double2* row = L + (size_t)npw * (m2 + (size_t)npw * m1);
-    const double sg = (a & 1) ? -1.0 : 1.0;
-    double2 s = make_double2(0.0, 0.0);
-    for (int m = 0; m < n2; m++) {
-      const double h = k.x2l[a * npw + n2 + m];
-      const double2 u = row[n2 + m], v = row[n2 - 1 - m];
-      s.x = fma(h, fma(sg, v.x, u.x), s.x);
-      s.y = fma(h, fma(sg, v.y, u.y), s.y);
-    }
-    U1[idx] = rot(s, a);
-  }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < P2 * n2; idx += blockDim.x) {
-    const int m1 = idx % n2, r = idx / n2, b = r % Pn, a = r / Pn;
-    const double sg = (b & 1) ? -1.0 : 1.0;
-    double2 s = make_double2(0.0, 0.0);
-    for (int m = 0; m < n2; m++) {
-      const double h = k.x2l[b * npw + n2 + m];
-      const double2 u = U1[((size_t)a * npw + n2 + m) * n2 + m1], v = U1[((size_t)a * npw + n2 - 1 - m) * n2 + m1];
-      s.x = fma(h, fma(sg, v.x, u.x), s.x);
-      s.y = fma(h, fma(sg, v.y, u.y), s.y);
-    }
-    U2[idx] = rot(s, b);
-  }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < P2 * Pn; idx += blockDim.x) {
-    const int a = idx % Pn, r = idx / Pn, b = r % Pn, c = r / Pn;
-    double2 s = make_double2(0.0, 0.0);
-    for (int m1 = 0; m1 < n2; m1++) {
-      const double h = k.x2l[c * npw + m1];
-      const double2 v = U2[((size_t)a * Pn + b) * n2 + m1];
-      s.x = fma(h, v.x, s.x);
-      s.y = fma(h, v.y, s.y);
-    }
-    lo[idx] = 2.0 * rot(s, c).x;
-  }
-  __syncthreads();
-  const double* pts = T.set ? k.trg : k.src;
-  double* out = T.set ? k.pottarg : k.pot;
-  const int nc = T.set ? k.nc_t : k.nc_s;
-  const double cx = k.centers[3 * T.box], cy = k.centers[3 * T.box + 1], cz = k.centers[3 * T.box + 2];
-  for (int i = threadIdx.x; i < T.n; i += blockDim.x) {
-    const int ip = T.i0 + i;
-    double v[NC];
-    horner3_rt<PGH>(lo, Pn, Pn, (pts[3 * ip] - cx) * k.dsq, (pts[3 * ip + 1] - cy) * k.dsq,
-                    (pts[3 * ip + 2] - cz) * k.dsq, k.dsq, v);
-    add_out<NC>(out, ip, k.nd, nc, ind, v);
   }
 }
 
@@ -2152,77 +1447,6 @@ __global__ void __launch_bounds__(256) k_eval2d(KP k, const EvalTask* __restrict
 }
 
 // ------------------------------------------------------------ (c) eval, 3D
-// Taylor route, persistent CTAs: plane wave -> Taylor through the scratch
-// slab (x, y passes) and a z pass into shared memory
-// (g3dpw2local_real_vec, g3drouts.f:1774-1938), then Horner evaluation.
-template <int PGH>
-__global__ void __launch_bounds__(256) k_eval3d_taylor(KP k, const EvalTask* __restrict__ tasks, int ntasks,
-                                                       double2* __restrict__ scratch, size_t slab) {
-  constexpr int NC = ncomp<3, PGH>();
-  const int npw = k.npw, n2 = k.n2;
-  double2* U1 = scratch + slab * blockIdx.x;
-  for (int w = blockIdx.x; w < ntasks * k.nd; w += gridDim.x) {
-    const EvalTask T = tasks[w / k.nd];
-    const int ind = w % k.nd;
-    const int Pn = T.p + 1, P2 = Pn * Pn;
-    double2* U2 = U1 + (size_t)Pn * npw * n2;
-    double* lo = reinterpret_cast<double*>(U2 + (size_t)P2 * n2);  // [P^3]
-    const double2* L = k.loc + ((size_t)T.slot * k.nd + ind) * k.nexp;
-    // x pass: U1[(a npw + m2) n2 + m1] = i^a sum_m3 x2l(m3,a) L[m3 + npw (m2 + npw m1)]
-    for (int idx = threadIdx.x; idx < Pn * npw * n2; idx += blockDim.x) {
-      const int m1 = idx % n2, r = idx / n2, m2 = r % npw, a = r / npw;
-      double2 s = make_double2(0.0, 0.0);
-      const double2* row = L + (size_t)npw * (m2 + (size_t)npw * m1);
-      for (int m3 = 0; m3 < npw; m3++) {
-        const double h = k.x2l[a * npw + m3];
-        const double2 v = row[m3];
-        s.x = fma(h, v.x, s.x);
-        s.y = fma(h, v.y, s.y);
-      }
-      U1[idx] = rot(s, a);
-    }
-    __syncthreads();
-    // y pass: U2[(a P + b) n2 + m1] = i^b sum_m2 x2l(m2,b) U1[(a npw + m2) n2 + m1]
-    for (int idx = threadIdx.x; idx < P2 * n2; idx += blockDim.x) {
-      const int m1 = idx % n2, r = idx / n2, b = r % Pn, a = r / Pn;
-      double2 s = make_double2(0.0, 0.0);
-      for (int m2 = 0; m2 < npw; m2++) {
-        const double h = k.x2l[b * npw + m2];
-        const double2 v = U1[((size_t)a * npw + m2) * n2 + m1];
-        s.x = fma(h, v.x, s.x);
-        s.y = fma(h, v.y, s.y);
-      }
-      U2[idx] = rot(s, b);
-    }
-    __syncthreads();
-    // z pass over the half: lo[a + P (b + P c)] = 2 Re(i^c sum_m1 x2l(m1,c) U2[(a P + b) n2 + m1])
-    for (int idx = threadIdx.x; idx < P2 * Pn; idx += blockDim.x) {
-      const int a = idx % Pn, r = idx / Pn, b = r % Pn, c = r / Pn;
-      double2 s = make_double2(0.0, 0.0);
-      for (int m1 = 0; m1 < n2; m1++) {
-        const double h = k.x2l[c * npw + m1];
-        const double2 v = U2[((size_t)a * Pn + b) * n2 + m1];
-        s.x = fma(h, v.x, s.x);
-        s.y = fma(h, v.y, s.y);
-      }
-      lo[idx] = 2.0 * rot(s, c).x;
-    }
-    __syncthreads();
-    const double* pts = T.set ? k.trg : k.src;
-    double* out = T.set ? k.pottarg : k.pot;
-    const int nc = T.set ? k.nc_t : k.nc_s;
-    const double cx = k.centers[3 * T.box], cy = k.centers[3 * T.box + 1], cz = k.centers[3 * T.box + 2];
-    for (int i = threadIdx.x; i < T.n; i += blockDim.x) {
-      const int ip = T.i0 + i;
-      double v[NC];
-      horner3_rt<PGH>(lo, Pn, Pn, (pts[3 * ip] - cx) * k.dsq, (pts[3 * ip + 1] - cy) * k.dsq,
-                      (pts[3 * ip + 2] - cz) * k.dsq, k.dsq, v);
-      add_out<NC>(out, ip, k.nd, nc, ind, v);
-    }
-    __syncthreads();
-  }
-}
-
 // PW route (g3dpwevalp_vec, g3drouts.f:2268-2362): one CTA per task.  x and y
 // run over both signs (PwAcc), z over the stored half, whose nodes are
 // negative: e^{-i t z} has z derivatives -i t and -t^2.  With Y(a,b) the x/y
@@ -3000,7 +2224,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     (f.route == ROUTE_PW ? D.form_pw_n : D.form_hermite_n)++;
     if (f.route == ROUTE_HERMITE) D.form_pmax = std::max(D.form_pmax, f.p);
   }
-  const std::vector<EvalTask> ev = route_order_sort(H.eval);
+  std::vector<EvalTask> ev = route_order_sort(H.eval);
   D.neval = (int)ev.size();
   for (auto& e : ev) {
     (e.route == ROUTE_PW ? D.eval_pw_n : D.eval_taylor_n)++;
@@ -3010,69 +2234,59 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   // slabs of their cut-level boxes, and the leaves with their own expansions
   const int lcut = std::max(P.npwlevel, 0);
   const bool sep = P.dim == 3 && P.scheme == 0 && !P.all_direct;
+  if (sep)  // the plane-wave route evaluates the cut-level box's expansion about its centre
+    for (int t = D.eval_taylor_n; t < D.neval; t++)
+      while (H.tree.level[ev[t].box] > lcut) ev[t].box = H.tree.parent[ev[t].box];
   SepLists up;
   std::vector<MergeGroup> upw_groups;
   std::vector<SepShift> upw;
   std::vector<double> sep_ph;
+  std::vector<SepItem> sep_items;  // every leaf at or below the cut level, in the order of the lists
+  std::vector<int> sep_order_of;   // order by depth below the cut level
   if (sep) {
     const Tree& tr = H.tree;
-    auto cut_box = [&](int b) {
-      while (tr.level[b] > lcut) b = tr.parent[b];
-      return b;
-    };
-    std::vector<int> roots, root_slot, rank(tr.llast[lcut] + 1, -1);
-    auto root_of = [&](int b) {
-      const int a = cut_box(b);
-      if (rank[a] < 0) {
-        rank[a] = (int)roots.size();
-        roots.push_back(a);
-        root_slot.push_back(H.mp_slot[a]);
+    const int nroot = tr.llast[lcut] - tr.lfirst[lcut] + 1;
+    std::vector<int> boxes, task(tr.nboxes, -1);
+    boxes.reserve(tr.nboxes - tr.lfirst[lcut]);
+    for (int b = tr.lfirst[lcut]; b < tr.nboxes; b++)
+      if (tr.nchild[b] == 0) boxes.push_back(b);
+    for (int l = lcut; l <= P.nlevels; l++) sep_order_of.push_back(H.nlocal[l]);
+    sep_order(tr, lcut, boxes, sep_rank(sep_order_of), sep_items);
+    sep_phases(H, P.nlevels - lcut, tr.boxsize[lcut], sep_ph);
+    for (int i = 0; i < D.nform; i++) task[form[i].box] = i;
+    const std::vector<FormTask> in(form.begin(), form.begin() + D.form_hermite_n);
+    std::vector<SepItem> items, pw;
+    items.reserve(D.form_hermite_n);
+    D.up_leaf.reserve(D.form_hermite_n);
+    D.up_box.reserve(D.form_hermite_n);
+    long long hoff = 0;
+    for (const SepItem& s : sep_items) {
+      const int i = task[s.box];
+      if (i < 0) continue;
+      if (i >= D.form_hermite_n) {
+        if (s.d > 0) pw.push_back(s);  // else it forms the cut level's expansion itself
+        continue;
       }
-      return rank[a];
-    };
-    std::vector<SepItem> items(D.form_hermite_n), pw;
-    for (int i = 0; i < D.nform; i++) {
-      const FormTask& f = form[i];
-      if (i >= D.form_hermite_n && tr.level[f.box] == lcut) continue;  // forms the cut level's expansion itself
-      SepItem s;
-      s.box = f.box;
-      s.root = root_of(f.box);
-      s.p = f.p;
-      s.index = i;
-      if (i < D.form_hermite_n) items[i] = s;
-      else pw.push_back(s);
+      const FormTask& f = form[items.size()] = in[i];
+      const int n = (f.n + 4095) / 4096;
+      items.push_back(s);
+      D.up_box.push_back(s.box);
+      D.up_leaf.push_back({hoff, 0, n});
+      hoff += (long long)n * (f.p + 1) * (f.p + 1) * (f.p + 1);
     }
-    sep_sort(tr, roots, items);
-    {
-      const std::vector<FormTask> in(form.begin(), form.begin() + D.form_hermite_n);
-      long long hoff = 0;
-      for (int i = 0; i < D.form_hermite_n; i++) {
-        SepItem& s = items[i];
-        form[i] = in[s.index];
-        s.index = i;
-        s.off = hoff;
-        s.n = (form[i].n + 4095) / 4096;
-        hoff += (long long)s.n * (s.p + 1) * (s.p + 1) * (s.p + 1);
-      }
-    }
-    sep_lists(items, root_slot, P.npw, up);
-    sep_sort(tr, roots, pw);
+    std::vector<int> slot(nroot);
+    std::vector<uint8_t> also(nroot, 0);
+    for (int r = 0; r < nroot; r++) slot[r] = H.mp_slot[tr.lfirst[lcut] + r];
     std::stable_sort(pw.begin(), pw.end(), [](const SepItem& a, const SepItem& b) { return a.root < b.root; });
-    int dmax = 0;
-    for (const SepItem& s : items) dmax = std::max(dmax, s.d);
     for (size_t i = 0; i < pw.size(); i++) {
       const SepItem& s = pw[i];
-      dmax = std::max(dmax, s.d);
-      if (i == 0 || pw[i - 1].root != s.root) upw_groups.push_back({root_slot[s.root], (int)i, 0});
+      if (i == 0 || pw[i - 1].root != s.root) upw_groups.push_back({slot[s.root], (int)i, 0});
       upw_groups.back().cnt++;
+      also[s.root] = 1;
       const int r0 = (1 << s.d) - 1;
-      upw.push_back({form[s.index].slot, {r0 + s.x[0], r0 + s.x[1], r0 + s.x[2]}});
+      upw.push_back({H.mp_slot[s.box], {r0 + s.x[0], r0 + s.x[1], r0 + s.x[2]}});
     }
-    sep_phases(H, dmax, H.tree.boxsize[lcut], sep_ph);
-    D.up_items = items;
-    for (SepItem& s : D.up_items) s.root = 0;
-    D.up_items.insert(D.up_items.end(), pw.begin(), pw.end());  // (their index: the form task)
-    for (size_t i = items.size(); i < D.up_items.size(); i++) D.up_items[i].index = form[D.up_items[i].index].slot;
+    sep_lists(items, D.up_leaf, sep_order_of, slot, also, P.npw, up);
   }
   tq[nq++] = tnow();
   // launch groups of equal order among the Hermite form / Taylor eval tasks
@@ -3101,45 +2315,18 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   std::vector<ConvTask> conv;
   std::vector<HornerTask> horner;
   size_t lo_doubles = 0;
-  // 3D: the same two kernels for the Taylor tasks whose order's shared-memory
-  // needs fit (k_eval3d_horner is instantiated for rows of up to 30
-  // coefficients); the tasks are sorted by order, so these are a prefix and
-  // the higher orders take the direct separable evaluation (k_eval3d_sep) or,
-  // with derivatives, the fallback kernels
-  if (P.dim == 3 && !P.all_direct) {
-    int t = 0;
-    while (t < D.eval_taylor_n && ev[t].p + 1 <= 30 && conv3_smem_bytes(ev[t].p + 1, P.npw, 4) <= 200 * 1024 &&
-           (P.npw + 3) / 4 <= CONV_MAXKS)
-      t++;
-    D.eval3_nsplit = t;
-  }
-  D.eval3_split = D.eval3_nsplit > 0;
-  const int split_pmax = D.eval3_split ? ev[D.eval3_nsplit - 1].p : -1;
-  // The split is fused into the conversion kernels (2D: all; 3D: those that
-  // stage the expansion in shared memory, orders <= 32): they read the
-  // cut-level ancestor's local expansion and apply the leaf's phases
+  // The split is fused into the conversion (k_pw2taylor2d): it reads the
+  // cut-level ancestor's local expansion and applies the leaf's phases
   // (ConvTask.sh)
-  // 2D: every conversion (k_pw2taylor2d) applies the fused split itself
-  auto conv_fusable = [&](int Pn) {
-    if (P.dim == 2) return true;
-    const int ksm = (P.npw / 2 + 3) / 4;
-    if (ksm > 8) return false;
-    if (Pn <= 16) return C3Dims(Pn, P.npw).total * 8 <= 227 * 1024;
-    if (Pn > 32) return false;
-    int gs2 = 4;
-    while (gs2 > 1 && C3Dims2(Pn, P.npw, gs2).total * 8 > 227 * 1024) gs2 >>= 1;
-    return C3Dims2(Pn, P.npw, gs2).total * 8 <= 227 * 1024;
-  };
   std::vector<uint8_t> fused_leaf(H.tree.nboxes, 0);
   tq[nq++] = tnow();
-  if ((P.dim == 2 || D.eval3_split) && !P.all_direct) {
-    const int ntay = P.dim == 2 ? D.eval_taylor_n : D.eval3_nsplit;
+  if (P.dim == 2 && !P.all_direct) {
+    const int ntay = D.eval_taylor_n;
     // the conversion of leaf slot s, made by its first task: (ConvTask, the
     // fused split), the same for either way of filling below
     auto make_conv = [&](const EvalTask& e, long long off) {
-      const long long Pn = e.p + 1;
       ConvTask ct{e.slot, e.p, off};
-      if (conv_fusable((int)Pn) && H.tree.level[e.box] > lcut) {
+      if (H.tree.level[e.box] > lcut) {
         int a = e.box;
         while (H.tree.level[a] > lcut) a = H.tree.parent[a];
         if (a >= 0 && H.loc_slot[a] >= 0) {
@@ -3153,7 +2340,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     };
     auto lo_size = [&](const EvalTask& e) {
       const long long Pn = e.p + 1, E = (Pn + 1) & ~1LL;
-      return (size_t)(P.nd * Pn * E * (P.dim == 3 ? Pn : 1));
+      return (size_t)(P.nd * Pn * E);
     };
     // The tasks of one leaf are consecutive (the builder emits them leaf by
     // leaf and the route sort is stable): then every slot's first task starts
@@ -3222,6 +2409,87 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
       t = u;
     }
   }
+  // 3D: the Taylor leaves in the order of the columns and slabs of their
+  // cut-level boxes (loc slots in sep_lists), each order group either with
+  // Taylor blocks or evaluated from the columns
+  SepLists dn;
+  std::vector<ColTask> ctask;
+  if (sep) {
+    const Tree& tr = H.tree;
+    const int pgh = std::max(1, std::max(P.ifpgh, P.ifpghtarg)), n2 = P.npw / 2;
+    // the tasks [run.first, run.second) of a leaf, by box (they are consecutive)
+    std::vector<std::pair<int, int>> run(tr.nboxes, {0, 0});
+    for (int t = 0; t < D.eval_taylor_n; t++) {
+      std::pair<int, int>& r = run[ev[t].box];
+      if (r.second == 0) r.first = t;
+      r.second = t + 1;
+    }
+    std::vector<SepItem> items;
+    items.reserve(sep_items.size());
+    for (const SepItem& s : sep_items)
+      if (run[s.box].second > 0) items.push_back(s);
+    const int cp = sep_col_points(pgh);
+    std::vector<uint8_t> blocks(D.eval_pmax + 2, 0);
+    for (size_t i = 0; i < items.size();) {
+      // Multiply-adds on the FP64 pipe of the two ways, each with what its
+      // kernels lose beside them (measured, 3D, eps 1e-6 and 1e-9): a leaf's
+      // block costs P^3 (n2 + 44) (44: its two passes over memory) and its
+      // points 2 P^3 per 32 begun; the column way 1.5 * 2 n2 P^2 per 8 points
+      // begun.  Mixed potentials up to order 15 are evaluated on the BF16
+      // tensor cores from the blocks; rows above 30 coefficients have no
+      // block evaluation.
+      const int p = sep_order_of[items[i].d];
+      const double Pn = p + 1, P3 = Pn * Pn * Pn;
+      double cb = 0.0, cc = 0.0;
+      size_t j = i;
+      for (; j < items.size() && sep_order_of[items[j].d] == p; j++) {
+        cb += P3 * (n2 + 44);
+        for (int t = run[items[j].box].first; t < run[items[j].box].second; t++) {
+          cb += 2.0 * P3 * pgh * (32 * ((ev[t].n + 31) / 32));
+          cc += 3.0 * n2 * Pn * Pn * pgh * (8 * ((ev[t].n + 7) / 8));
+        }
+      }
+      blocks[p] = Pn <= 30 && ((Pn <= 16 && pgh == 1 && !P.ifdipole) || cb < cc);
+      i = j;
+    }
+    std::vector<SepLeaf> leaf;
+    leaf.reserve(items.size());
+    for (const SepItem& it : items) {
+      const int p = sep_order_of[it.d];
+      const long long Pn = p + 1, E = (Pn + 1) & ~1LL;
+      leaf.push_back({(long long)lo_doubles, 0, 1});
+      if (blocks[p]) lo_doubles += (size_t)(P.nd * Pn * Pn * E);
+    }
+    std::vector<int> slot(tr.llast[lcut] - tr.lfirst[lcut] + 1);
+    for (size_t r = 0; r < slot.size(); r++) slot[r] = H.loc_slot[tr.lfirst[lcut] + r];
+    sep_lists(items, leaf, sep_order_of, slot, {}, P.npw, dn);
+    size_t nh = 0, nct = 0;
+    for (int t = 0; t < D.eval_taylor_n; t++) {
+      if (blocks[ev[t].p]) nh += (ev[t].n + 255) / 256;
+      else nct += (ev[t].n + cp - 1) / cp;
+    }
+    horner.reserve(nh);
+    ctask.reserve(nct);
+    for (SepGroup& G : dn.groups) {
+      G.blocks = blocks[G.p];
+      const int h0 = (int)horner.size(), c0 = (int)ctask.size();
+      for (int c = G.cbeg; c < G.cend; c++)
+        for (int l = dn.cols[c].beg; l < dn.cols[c].beg + dn.cols[c].cnt; l++) {
+          const std::pair<int, int> r = run[items[l].box];
+          for (int t = r.first; t < r.second; t++) {
+            const EvalTask& e = ev[t];
+            if (G.blocks)
+              for (int q = 0; q < e.n; q += 256)
+                horner.push_back({e.box, e.set, e.i0 + q, std::min(256, e.n - q), e.p, leaf[l].off});
+            else
+              for (int q = 0; q < e.n; q += cp)
+                ctask.push_back({e.box, e.set, e.i0 + q, std::min(cp, e.n - q), dn.leaves[l].row, e.p + 1, dn.cols[c].off});
+          }
+        }
+      if (G.blocks) D.horner_groups.push_back({G.p, h0, (int)horner.size()});
+      else D.ctask_groups.push_back({G.p, c0, (int)ctask.size()});
+    }
+  }
   tp[np_++] = tnow();
   // padded operand tables of the 2D MMA transforms, one per order group
   std::vector<double> tables;
@@ -3236,11 +2504,6 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
       build_conv_table(H, G.p + 1, tables);
     }
   }
-  if (D.eval3_split)
-    for (OrderGroup& G : D.conv_groups) {
-      G.tab = (long long)tables.size();
-      build_conv3_table(H, G.p + 1, tables);
-    }
   tp[np_++] = tnow();
   // merge groups: consecutive tasks with the same destination
   std::vector<MergeGroup> groups;
@@ -3298,7 +2561,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   D.form_sources = H.form_sources;
   D.eval_points = H.eval_points;
   tp[np_++] = tnow();
-  // 3D: shared-memory paths when the largest order fits, else the scratch path
+  // 3D: source chunks and their partial Hermite blocks
   std::vector<FormChunk> fchunks;
   size_t hbuf_doubles = 0;
   // 2D: Hermite blocks of the MMA form (orders <= 31), nd P^2 doubles per leaf
@@ -3313,8 +2576,6 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     }
   }
   if (P.dim == 3 && !P.all_direct) {
-    const size_t lim = 227 * 1024;
-    const int n2 = P.npw / 2;
     if (D.form_hermite_n > 0) {
       long long hoff = 0;
       for (int t = 0; t < D.form_hermite_n; t++) {
@@ -3342,37 +2603,12 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
         t = u;
       }
     }
-    if (D.eval_taylor_n > 0) {
-      const size_t Pn = D.eval_pmax + 1;
-      size_t szA = std::max(2 * Pn * P.npw * n2, Pn * Pn * Pn);
-      D.eval3_sh = (((szA + 1) & ~size_t(1)) + 2 * Pn * Pn * n2) * 8;
-      // the fallback kernels run only on the Taylor tasks beyond the split
-      // kernels' orders, and only with derivatives
-      const bool fallback = D.eval3_nsplit < D.eval_taylor_n && std::max(P.ifpgh, P.ifpghtarg) >= 2;
-      D.eval3_smem = D.eval3_sh <= lim || !fallback;
-    }
-  }
-  // scratch for the 3D separable transforms (fallback path)
-  if (P.dim == 3 && !P.all_direct && !D.eval3_smem) {
-    size_t slab = 0;
-    int n2 = P.npw / 2;
-    for (auto& e : ev)
-        if (e.route == ROUTE_TAYLOR) {
-        size_t Pn = e.p + 1;
-        slab = std::max(slab, Pn * P.npw * n2 + Pn * Pn * n2 + (Pn * Pn * Pn + 1) / 2);
-      }
-    D.scratch_per_cta = (slab + 15) & ~size_t(15);
-    D.scratch_ctas = D.scratch_per_cta ? D.sm_count * 2 : 0;
-  }
-  if (D.eval3_split) {
-    D.uscr_per_cta = (conv3_scratch(split_pmax + 1, P.npw) + 31) & ~size_t(31);
-    D.conv3_ctas = D.sm_count * 4;
   }
   size_t ns = P.ns, nt = P.nt, nd = P.nd, dim = P.dim;
   // FP32 coordinates of the mixed near field (charges only)
   const bool fmix = D.ndir > 0 && !P.ifdipole;
   // diagonal translation tables (formed on the device)
-  const size_t n_wms = P.all_direct ? 0 : (size_t)(P.nlevels + 1) * D.nch * P.nexp;
+  const size_t n_wms = P.all_direct || P.dim == 3 ? 0 : (size_t)(P.nlevels + 1) * D.nch * P.nexp;
   const size_t n_wsh = P.all_direct ? 0 : (size_t)(P.dim == 2 ? 9 : 27) * P.nexp;
   size_t total = bytes_of(H.box_centers) + bytes_of(H.h2x) + bytes_of(H.x2l) + al(n_wms * 16) + al(n_wsh * 16) + al(H.ww.size() * 8) + al(H.w1.size() * 8) + 2 * al((size_t)P.ns * 4) + 2 * al((size_t)P.nt * 4) +
                  al((size_t)(std::max(P.ntermmax, 1) + 2) * 8) + al(32 * 8) +
@@ -3385,11 +2621,11 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
                  (fmix ? al(ns * dim * 8) + al((P.ifpghtarg > 0 ? nt : 0) * dim * 8) : 0) +
                  al(P.ifdipole ? ns * dim * 8 : 0) + al(P.ifdipole ? ns * nd * 8 : 0) +
                  al(nt * nd * out_comps(dim, P.ifpghtarg) * 8) +
-                 al((size_t)D.scratch_ctas * D.scratch_per_cta * 16) + bytes_of(fchunks) +
+                 bytes_of(fchunks) +
                  bytes_of(up.leaves) + bytes_of(up.cols) + bytes_of(up.slabs) + bytes_of(up.boxes) +
-                 bytes_of(up.box_slabs) + bytes_of(upw_groups) + bytes_of(upw) + bytes_of(sep_ph) +
-                 al(up.t1 * nd * 8) + al(up.t2 * nd * 8) +
-                 al((size_t)D.conv3_ctas * nd * D.uscr_per_cta * 8) +
+                 bytes_of(up.box_slabs) + bytes_of(dn.cols) + bytes_of(dn.leaves) + bytes_of(dn.slabs) +
+                 bytes_of(dn.boxes) + bytes_of(dn.box_slabs) + bytes_of(ctask) + bytes_of(upw_groups) + bytes_of(upw) + bytes_of(sep_ph) +
+                 al(std::max(up.t1, dn.t1) * nd * 8) + al(std::max(up.t2, dn.t2) * nd * 8) +
                  al(hbuf_doubles * 8) + bytes_of(form_hoff) + bytes_of(tables) + bytes_of(conv) + bytes_of(horner) +
                  al(lo_doubles * 8) + 4096;
   D.bytes = total;
@@ -3444,6 +2680,12 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     st.add(cur, D.up.slabs, up.slabs);
     st.add(cur, D.up.boxes, up.boxes);
     st.add(cur, D.up.box_slabs, up.box_slabs);
+    st.add(cur, D.dn.leaves, dn.leaves);
+    st.add(cur, D.dn.cols, dn.cols);
+    st.add(cur, D.dn.slabs, dn.slabs);
+    st.add(cur, D.dn.boxes, dn.boxes);
+    st.add(cur, D.dn.box_slabs, dn.box_slabs);
+    st.add(cur, D.ctask, ctask);
     st.add(cur, D.upw_groups, upw_groups);
     st.add(cur, D.upw, upw);
     double* ph = nullptr;
@@ -3451,7 +2693,9 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     D.up.ph = reinterpret_cast<double2*>(ph);
     D.up.nboxes = (int)up.boxes.size();
     D.up.groups = up.groups;
-    D.up.sms = D.psm();
+    D.dn.ph = D.up.ph;
+    D.dn.nboxes = (int)dn.boxes.size();
+    D.dn.groups = dn.groups;
     D.nupw_groups = (int)upw_groups.size();
     st.add(cur, D.form_hoff, form_hoff);
     st.add(cur, D.tables, tables);
@@ -3462,10 +2706,10 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   // translation tables formed on the device from their 1D factors
   D.wms = reinterpret_cast<double2*>(cur); cur += al(n_wms * 16);
   D.wsh = reinterpret_cast<double2*>(cur); cur += al(n_wsh * 16);
-  if (n_wms > 0) {
+  if (n_wms + n_wsh > 0) {
     const long long tot = (long long)(n_wms + n_wsh);
     const int blocks = (int)std::min<long long>((tot + 255) / 256, (long long)D.sm_count * 16);
-    k_shift_tables<<<blocks, 256, 0, s>>>(P.dim, P.npw, P.nexp, P.nlevels, std::max(P.nlevstart, 0), H.nms,
+    k_shift_tables<<<blocks, 256, 0, s>>>(P.dim, P.npw, P.nexp, P.nlevels, std::max(P.nlevstart, 0), H.nms, (long long)n_wms,
                                           d_ww, d_w1, D.wms, D.wsh);
     CK(cudaGetLastError());
   }
@@ -3518,8 +2762,9 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   }
   D.lo = reinterpret_cast<double*>(cur); cur += al(lo_doubles * 8);
   D.hbuf = reinterpret_cast<double*>(cur); cur += al(hbuf_doubles * 8);
-  D.up.t1 = reinterpret_cast<double*>(cur); cur += al(up.t1 * nd * 8);
-  D.up.t2 = reinterpret_cast<double*>(cur); cur += al(up.t2 * nd * 8);
+  // the intermediates of the two directions, one after the other
+  D.up.t1 = D.dn.t1 = reinterpret_cast<double*>(cur); cur += al(std::max(up.t1, dn.t1) * nd * 8);
+  D.up.t2 = D.dn.t2 = reinterpret_cast<double*>(cur); cur += al(std::max(up.t2, dn.t2) * nd * 8);
   D.mp = reinterpret_cast<double2*>(cur); cur += al((size_t)H.nmp * nd * P.nexp * 16);
   D.loc = reinterpret_cast<double2*>(cur); cur += al((size_t)H.nloc * nd * P.nexp * 16);
   D.ssort = reinterpret_cast<double*>(cur); cur += al(ns * dim * 8);
@@ -3533,8 +2778,6 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   }
   D.psort = reinterpret_cast<double*>(cur); cur += al(ns * nd * out_comps(dim, P.ifpgh) * 8);
   D.ptsort = reinterpret_cast<double*>(cur); cur += al(nt * nd * out_comps(dim, P.ifpghtarg) * 8);
-  D.scratch = reinterpret_cast<double2*>(cur); cur += al((size_t)D.scratch_ctas * D.scratch_per_cta * 16);
-  D.uscr = reinterpret_cast<double*>(cur); cur += al((size_t)D.conv3_ctas * nd * D.uscr_per_cta * 8);
   CK(cudaStreamSynchronize(s));
   if (getenv("FGT_TREE_TIMING"))
     fprintf(stderr, "device plan prep parts: sort %.4f conv %.4f tables %.4f merge %.4f split %.4f rest %.4f"
@@ -3543,9 +2786,9 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
             tq[1] - tq[0], tq[2] - tq[1], nq > 3 ? tq[3] - tq[2] : 0.0);
   if (getenv("FGT_TREE_TIMING"))
     fprintf(stderr, "device plan: prep %.4f malloc %.4f upload %.4f (%zu bytes); eval tasks: taylor %d "
-            "(conversion %d, max order %d) pw %d; form tasks: hermite %d (max order %d) pw %d\n",
+            "(max order %d) pw %d; form tasks: hermite %d (max order %d) pw %d\n",
             tm0 - tin, tm1 - tm0, tnow() - tm1, total, D.eval_taylor_n,
-            P.dim == 3 ? D.eval3_nsplit : D.eval_taylor_n, D.eval_pmax + 1, D.eval_pw_n, D.form_hermite_n,
+            D.eval_pmax + 1, D.eval_pw_n, D.form_hermite_n,
             D.form_pmax + 1, D.form_pw_n);
   return cudaSuccess;
 }
@@ -3895,61 +3138,10 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
         launches++;
       }
     }
-    if (P.dim == 3 && D.eval3_split) {
-      for (const OrderGroup& G : D.conv_groups) {
-        const int Pn = G.p + 1, nt = G.end - G.beg;
-        const int nw = 4;
-        const size_t sh = conv3_smem_bytes(Pn, P.npw, nw);
-        const dim3 cg(std::min(nt, std::min(D.conv3_ctas, 4 * D.psm())), nd);
-        const int n2 = P.npw / 2, ksm = (n2 + 3) / 4;
-        const size_t shm = C3Dims(Pn, P.npw).total * 8;
-        if (Pn <= 16 && ksm <= 8 && shm <= 227 * 1024) {
-          const dim3 pg(D.pgrid(nt, 2 * (shm + 1024) <= 228 * 1024 ? 2 : 1), nd);
-          switch (ksm) {
-#define CONV3M_CASE(N)                                                                            \
-  case N:                                                                                         \
-    CK(smem_limit(k_pw2taylor3d_mma<N>)); \
-    k_pw2taylor3d_mma<N><<<pg, 256, shm, st>>>(k, D.conv + G.beg, nt, D.lo);                      \
-    break;
-            CONV3M_CASE(1) CONV3M_CASE(2) CONV3M_CASE(3) CONV3M_CASE(4)
-            CONV3M_CASE(5) CONV3M_CASE(6) CONV3M_CASE(7) CONV3M_CASE(8)
-#undef CONV3M_CASE
-            default: return cudaErrorNotSupported;
-          }
-          launches++;
-          continue;
-        }
-        int gs2 = 4;
-        while (gs2 > 1 && C3Dims2(Pn, P.npw, gs2).total * 8 > 227 * 1024) gs2 >>= 1;
-        const size_t shm2 = C3Dims2(Pn, P.npw, gs2).total * 8;
-        if (Pn > 16 && Pn <= 32 && ksm <= 8 && shm2 <= 227 * 1024) {
-          const dim3 pg(D.pgrid(nt, 1), nd);
-          switch (ksm) {
-#define CONV3M2_CASE(N)                                                                           \
-  case N:                                                                                         \
-    CK(smem_limit(k_pw2taylor3d_mma2<N>)); \
-    k_pw2taylor3d_mma2<N><<<pg, 256, shm2, st>>>(k, D.conv + G.beg, nt, D.lo, gs2);               \
-    break;
-            CONV3M2_CASE(1) CONV3M2_CASE(2) CONV3M2_CASE(3) CONV3M2_CASE(4)
-            CONV3M2_CASE(5) CONV3M2_CASE(6) CONV3M2_CASE(7) CONV3M2_CASE(8)
-#undef CONV3M2_CASE
-            default: return cudaErrorNotSupported;
-          }
-          launches++;
-          continue;
-        }
-        switch ((P.npw + 3) / 4) {
-#define CONV3_CASE(N)                                                                             \
-  case N:                                                                                         \
-    CK(smem_limit(k_pw2taylor3d<N>)); \
-    k_pw2taylor3d<N><<<cg, 32 * nw, sh, st>>>(k, D.conv + G.beg, nt, D.lo, D.tables + G.tab,      \
-                                              D.uscr, D.uscr_per_cta);                            \
-    break;
-          CONV3_CASE(1) CONV3_CASE(2) CONV3_CASE(3) CONV3_CASE(4) CONV3_CASE(5) CONV3_CASE(6)
-          CONV3_CASE(7) CONV3_CASE(8) CONV3_CASE(9) CONV3_CASE(10) CONV3_CASE(11) CONV3_CASE(12)
-#undef CONV3_CASE
-          default: return cudaErrorNotSupported;
-        }
+    if (P.dim == 3 && D.dn.nboxes > 0) {
+      CK(sep_down(k, D.dn, D.lo, st, launches));
+      for (const OrderGroup& G : D.ctask_groups) {
+        CK(sep_eval_cols(k, D.dn, D.ctask + G.beg, G.end - G.beg, G.p + 1, pgh, st));
         launches++;
       }
       for (const OrderGroup& G : D.horner_groups) {
@@ -3986,40 +3178,10 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
         launches++;
       }
     }
-    // 3D Taylor tasks beyond the conversion kernels' orders, and the
-    // plane-wave route: the direct separable evaluation for potentials
-    const int nbig = P.dim == 3 ? D.eval_taylor_n - D.eval3_nsplit : 0;
-    const size_t sh_sep = ((size_t)(2 * P.npw + P.npw / 2) * SEP_NPB + 256 * 4) * 16 +
-                          (size_t)(D.eval_pmax + 1) * P.npw * 8;
-    if (nbig > 0 && pgh == 1) {
-      CK(smem_limit(k_eval3d_sep<true>));
-      k_eval3d_sep<true><<<dim3(nbig, nd), 256, sh_sep, st>>>(k, D.eval + D.eval3_nsplit);
-      launches++;
-    } else if (nbig > 0 && D.eval3_smem) {
-      {
-          const cudaError_t e_pgh = with_pgh(pgh, [&](auto G) -> cudaError_t {
-        constexpr int PG = decltype(G)::value;
-        CK(smem_limit(k_eval3d_taylor_smem<PG>));
-        k_eval3d_taylor_smem<PG><<<dim3(nbig, nd), 512, D.eval3_sh, st>>>(k, D.eval + D.eval3_nsplit);
-        return cudaSuccess;
-      });
-          CK(e_pgh);
-        }
-      launches++;
-    } else if (nbig > 0) {
-      {
-          const cudaError_t e_pgh = with_pgh(pgh, [&](auto G) -> cudaError_t {
-        k_eval3d_taylor<decltype(G)::value><<<std::min(D.scratch_ctas, 2 * D.psm()), 256, 0, st>>>(k, D.eval + D.eval3_nsplit, nbig,
-                                                                           D.scratch, D.scratch_per_cta);
-        return cudaSuccess;
-      });
-          CK(e_pgh);
-        }
-      launches++;
-    }
+    const size_t sh_sep = ((size_t)(2 * P.npw + P.npw / 2) * SEP_NPB + 256 * 4) * 16;
     if (P.dim == 3 && D.eval_pw_n > 0 && pgh == 1) {
-      CK(smem_limit(k_eval3d_sep<false>));
-      k_eval3d_sep<false><<<dim3(D.eval_pw_n, nd), 256, sh_sep, st>>>(k, D.eval + D.eval_taylor_n);
+      CK(smem_limit(k_eval3d_sep));
+      k_eval3d_sep<<<dim3(D.eval_pw_n, nd), 256, sh_sep, st>>>(k, D.eval + D.eval_taylor_n);
       launches++;
     } else if (P.dim == 3 && D.eval_pw_n > 0) {
       {
@@ -4108,29 +3270,38 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
 cudaError_t device_plan_box_expansion(const HostPlan& H, DevicePlan& D, int box, double* out, cudaStream_t st) {
   const Tree& t = H.tree;
   const Params& P = H.P;
+  const int lb = t.level[box], lcut = std::max(P.npwlevel, 0);
+  auto inside = [&](int b) {
+    while (t.level[b] > lb) b = t.parent[b];
+    return b == box;
+  };
+  std::vector<int> boxes, pwb, at(t.nboxes, -1);
+  for (size_t i = 0; i < D.up_box.size(); i++)
+    if (inside(D.up_box[i])) {
+      boxes.push_back(D.up_box[i]);
+      at[D.up_box[i]] = (int)i;
+    }
+  for (const FormTask& f : H.form)
+    if (f.route == ROUTE_PW && t.level[f.box] > lcut && inside(f.box)) pwb.push_back(f.box);
+  std::vector<int> order;
+  for (int l = lb; l <= P.nlevels; l++) order.push_back(H.nlocal[l]);
   std::vector<SepItem> items, pw;
-  for (const SepItem& s : D.up_items) {
-    int b = s.box;
-    while (t.level[b] > t.level[box]) b = t.parent[b];
-    if (b != box) continue;
-    std::vector<SepItem>& to = H.mp_slot[s.box] >= 0 && t.level[s.box] > std::max(P.npwlevel, 0) ? pw : items;
-    to.push_back(s);
-    to.back().root = 0;
-  }
-  const std::vector<int> roots{box}, slot{0};
-  sep_sort(t, roots, items);
-  sep_sort(t, roots, pw);
+  sep_order(t, lb, boxes, sep_rank(order), items);
+  sep_order(t, lb, pwb, sep_rank(order), pw);
+  std::vector<SepLeaf> leaf;
+  for (const SepItem& s : items) leaf.push_back(D.up_leaf[at[s.box]]);
+  std::vector<int> slot(t.llast[lb] - t.lfirst[lb] + 1, -1);
+  std::vector<uint8_t> also(slot.size(), 0);
+  slot[box - t.lfirst[lb]] = 0;
+  also[box - t.lfirst[lb]] = 1;
   SepLists L;
-  sep_lists(items, slot, P.npw, L);
-  int dmax = 0;
-  for (const SepItem& s : items) dmax = std::max(dmax, s.d);
-  for (const SepItem& s : pw) dmax = std::max(dmax, s.d);
+  sep_lists(items, leaf, order, slot, also, P.npw, L);
   std::vector<double> ph;
-  sep_phases(H, dmax, t.boxsize[t.level[box]], ph);
+  sep_phases(H, P.nlevels - lb, t.boxsize[lb], ph);
   std::vector<SepShift> sh;
   for (const SepItem& s : pw) {
     const int r0 = (1 << s.d) - 1;
-    sh.push_back({s.index, {r0 + s.x[0], r0 + s.x[1], r0 + s.x[2]}});
+    sh.push_back({H.mp_slot[s.box], {r0 + s.x[0], r0 + s.x[1], r0 + s.x[2]}});
   }
   const std::vector<MergeGroup> g{{0, 0, (int)sh.size()}};
   const size_t nd = P.nd, per = nd * P.nexp * 16;

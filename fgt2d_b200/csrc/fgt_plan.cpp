@@ -290,7 +290,8 @@ static void build_tasks(HostPlan& H) {
         if (t.ns(b) > 0 && !(leaf && l == npl) &&
             (D == 2 || l == nls || (leaf && form_route(l, b) == ROUTE_PW)))
           H.mp_slot[b] = H.nmp++;
-        if (relevant(b) > 0 && !(leaf && l == npl && !iflocal(b))) H.loc_slot[b] = H.nloc++;
+        // 3D local expansions: the cut level's
+        if (relevant(b) > 0 && !(leaf && l == npl && !iflocal(b)) && (D == 2 || l == nls)) H.loc_slot[b] = H.nloc++;
       }
     // (a) form, levels nlevels .. max(npwlevel+1, 0) (fgt2d.f:871)
     for (int l = P.nlevels; l >= std::max(npl + 1, 0); l--) {
@@ -360,8 +361,8 @@ static void build_tasks(HostPlan& H) {
       }
     }
     tq[nq++] = now();
-    // (b) split, parents at levels nlevstart .. nlevels-1
-    for (int l = nls; l <= P.nlevels - 1; l++) {
+    // (b) split, parents at levels nlevstart .. nlevels-1 (2D)
+    for (int l = nls; l <= P.nlevels - 1 && D == 2; l++) {
       H.split_beg[l] = (int)H.split.size();
       for (int b = t.lfirst[l]; b <= t.llast[l]; b++) {
         if (H.loc_slot[b] < 0 || t.nchild[b] == 0) continue;
@@ -382,8 +383,12 @@ static void build_tasks(HostPlan& H) {
         pw = r3 >= 3;
       }
       for (int b = t.lfirst[l]; b <= t.llast[l]; b++) {
-        if (t.nchild[b] != 0 || H.loc_slot[b] < 0) continue;
+        if (t.nchild[b] != 0 || relevant(b) <= 0) continue;
         if (l == npl && !iflocal(b)) continue;
+        int a = b;  // the box whose local expansion the leaf reads
+        while (D == 3 && t.level[a] > nls) a = t.parent[a];
+        const int slot = H.loc_slot[a];
+        if (slot < 0) continue;
         int route = pw ? ROUTE_PW : ROUTE_TAYLOR;
         if (D == 3 && pw && t.ns(b) + t.nt(b) >= 1000000) route = ROUTE_TAYLOR;
         // big leaves are cut into chunks so that no CTA serialises a
@@ -394,7 +399,7 @@ static void build_tasks(HostPlan& H) {
           if (set == 0 && !(P.ifpgh >= 1 && t.ns(b) > 0)) continue;
           int i0 = set ? t.t0[b] : t.s0[b], n = set ? t.nt(b) : t.ns(b);
           for (int c = 0; c < n; c += evch)
-            H.eval.push_back({b, set, i0 + c, std::min(evch, n - c), H.loc_slot[b], p, route});
+            H.eval.push_back({b, set, i0 + c, std::min(evch, n - c), slot, p, route});
           H.eval_points += n;
         }
       }

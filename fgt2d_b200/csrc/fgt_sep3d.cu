@@ -29,6 +29,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <type_traits>
 
 #include "fgt_kcommon.cuh"
 #include "fgt_sep3d.hpp"
@@ -36,78 +37,89 @@
 namespace fgtb {
 
 // ------------------------------------------------------------ lists
-void sep_sort(const Tree& t, const std::vector<int>& root_box, std::vector<SepItem>& items) {
-  const int n = (int)items.size();
-#pragma omp parallel for schedule(static) if (n > 4096)
-  for (int i = 0; i < n; i++) {
-    SepItem& s = items[i];
-    const int a = root_box[s.root], l = t.level[s.box];
-    s.d = l - t.level[a];
-    for (int q = 0; q < 3; q++)
-      s.x[q] = (int)std::lround((t.c(s.box, q) - t.c(a, q)) / t.boxsize[l] + 0.5 * ((1 << s.d) - 1));
-  }
-  int dmax = 0, pmax = 0;
-  for (const SepItem& s : items) {
-    dmax = std::max(dmax, s.d);
-    pmax = std::max(pmax, s.p);
-  }
-  // one key per item, (p, d, root, x, y, z) from the top, sorted by digits of
-  // 11 bits; the items move once
+std::vector<int> sep_rank(const std::vector<int>& order) {
+  std::vector<int> by(order.size()), rank(order.size());
+  for (size_t d = 0; d < by.size(); d++) by[d] = (int)d;
+  std::stable_sort(by.begin(), by.end(), [&](int a, int b) { return order[a] < order[b]; });
+  for (size_t i = 0; i < by.size(); i++) rank[by[i]] = (int)i;
+  return rank;
+}
+
+void sep_order(const Tree& t, int lroot, const std::vector<int>& boxes, const std::vector<int>& rank,
+               std::vector<SepItem>& items) {
+  const int n = (int)boxes.size(), a0 = t.lfirst[lroot], dmax = (int)rank.size() - 1;
   auto width = [](unsigned long long v) {
     int w = 0;
     while (v >> w) w++;
     return w;
   };
-  const int wr = width(root_box.size()), wd = width(dmax), wp = width(pmax), bits = 3 * dmax + wr + wd + wp;
-  if (bits > 64) {  // a tree deeper than the keys hold
-    std::stable_sort(items.begin(), items.end(), [](const SepItem& a, const SepItem& b) {
-      if (a.p != b.p) return a.p < b.p;
-      if (a.d != b.d) return a.d < b.d;
+  // one key per item, (rank, root, x, y, z, number), sorted by digits of 11
+  // bits; the items are written once, in order
+  const int wn = width(n), wr = width(t.llast[lroot] - a0), wd = width(dmax);
+  const bool packed = 3 * dmax + wr + wd + wn <= 64;
+  std::vector<SepItem> raw(n);
+  std::vector<uint64_t> key(packed ? n : 0), tmp(packed ? n : 0);
+#pragma omp parallel for schedule(static) if (n > 2048)
+  for (int i = 0; i < n; i++) {
+    SepItem& s = raw[i];
+    s.box = boxes[i];
+    const int l = t.level[s.box];
+    int a = s.box;
+    while (t.level[a] > lroot) a = t.parent[a];
+    s.root = a - a0;
+    s.d = l - lroot;
+    for (int q = 0; q < 3; q++)
+      s.x[q] = (int)std::lround((t.c(s.box, q) - t.c(a, q)) / t.boxsize[l] + 0.5 * ((1 << s.d) - 1));
+    if (packed) {
+      uint64_t k = (uint64_t)rank[s.d] << wr | (uint64_t)s.root;
+      for (int q = 0; q < 3; q++) k = k << dmax | (uint64_t)s.x[q];
+      key[i] = k << wn | (uint64_t)i;
+    }
+  }
+  if (!packed) {  // a tree deeper than the keys hold
+    std::stable_sort(raw.begin(), raw.end(), [&](const SepItem& a, const SepItem& b) {
+      if (a.d != b.d) return rank[a.d] < rank[b.d];
       if (a.root != b.root) return a.root < b.root;
       return std::lexicographical_compare(a.x, a.x + 3, b.x, b.x + 3);
     });
+    items.swap(raw);
     return;
   }
-  struct Key {
-    uint64_t k;
-    int i;
-  };
-  std::vector<Key> key(n), tmp(n);
-  for (int i = 0; i < n; i++) {
-    const SepItem& s = items[i];
-    uint64_t k = ((uint64_t)s.p << wd | (uint64_t)s.d) << wr | (uint64_t)s.root;
-    for (int q = 0; q < 3; q++) k = k << dmax | (uint64_t)s.x[q];
-    key[i] = {k, i};
-  }
-  for (int b = 0; b < bits; b += 11) {
+  for (int b = wn; b < wn + 3 * dmax + wr + wd; b += 11) {
     int cnt[2049] = {0};
-    for (const Key& e : key) cnt[((e.k >> b) & 2047) + 1]++;
+    for (uint64_t k : key) cnt[((k >> b) & 2047) + 1]++;
     for (int i = 0; i < 2048; i++) cnt[i + 1] += cnt[i];
-    for (const Key& e : key) tmp[cnt[(e.k >> b) & 2047]++] = e;
+    for (uint64_t k : key) tmp[cnt[(k >> b) & 2047]++] = k;
     key.swap(tmp);
   }
-  std::vector<SepItem> out(n);
-  for (int i = 0; i < n; i++) out[i] = items[key[i].i];
-  items.swap(out);
+  items.resize(n);
+  const uint64_t mask = (uint64_t(1) << wn) - 1;
+#pragma omp parallel for schedule(static) if (n > 2048)
+  for (int i = 0; i < n; i++) items[i] = raw[key[i] & mask];
 }
 
-void sep_lists(const std::vector<SepItem>& items, const std::vector<int>& slot, int npw, SepLists& S) {
+void sep_lists(const std::vector<SepItem>& items, const std::vector<SepLeaf>& leaf, const std::vector<int>& order,
+               const std::vector<int>& slot, const std::vector<uint8_t>& also, int npw, SepLists& S) {
   const int n = (int)items.size(), n2 = npw / 2, nroot = (int)slot.size();
   S = SepLists();
-  S.leaves.reserve(n);
+  S.leaves = leaf;
+  S.cols.reserve(n);
+  S.slabs.reserve(n);
   auto row = [](const SepItem& s, int q) { return (1 << s.d) - 1 + s.x[q]; };
-  std::vector<int> slab_root;
+  std::vector<int> cnt(nroot + 1, 0), slab_root;
+  slab_root.reserve(n);
   for (int i = 0; i < n; i++) {
     const SepItem& s = items[i];
-    const long long Pn = s.p + 1;
+    const int p = order[s.d];
+    const long long Pn = p + 1;
     const SepItem* o = i ? &items[i - 1] : nullptr;
-    const bool group = !o || o->p != s.p;
-    const bool slab = group || o->d != s.d || o->root != s.root || o->x[0] != s.x[0];
-    if (group) S.groups.push_back({s.p, (int)S.cols.size(), 0, (int)S.slabs.size(), 0});
+    const bool slab = !o || o->d != s.d || o->root != s.root || o->x[0] != s.x[0];
+    if (!o || order[o->d] != p) S.groups.push_back({p, (int)S.cols.size(), 0, (int)S.slabs.size(), 0});
     if (slab) {
       S.slabs.push_back({(long long)S.t2, (int)S.cols.size(), 0, row(s, 0), (int)Pn});
       S.t2 += (size_t)(Pn * n2 * npw * 2);
       slab_root.push_back(s.root);
+      cnt[s.root + 1]++;
     }
     if (slab || o->x[1] != s.x[1]) {
       S.cols.push_back({(long long)S.t1, i, 0, row(s, 1), (int)Pn});
@@ -115,14 +127,13 @@ void sep_lists(const std::vector<SepItem>& items, const std::vector<int>& slot, 
       S.slabs.back().cnt++;
     }
     S.cols.back().cnt++;
-    S.leaves.push_back({s.off, row(s, 2), s.n});
+    S.leaves[i].row = row(s, 2);
     S.groups.back().cend = (int)S.cols.size();
     S.groups.back().send = (int)S.slabs.size();
   }
-  std::vector<int> cnt(nroot + 1, 0);
-  for (int r : slab_root) cnt[r + 1]++;
   for (int r = 0; r < nroot; r++) {
-    S.boxes.push_back({(long long)slot[r], cnt[r], cnt[r + 1], 0, 0});
+    const int m = cnt[r + 1];
+    if (m > 0 || (!also.empty() && also[r])) S.boxes.push_back({(long long)slot[r], cnt[r], m, 0, 0});
     cnt[r + 1] += cnt[r];
   }
   S.box_slabs.resize(slab_root.size());
@@ -338,6 +349,415 @@ __global__ void __launch_bounds__(128) k_up_xy(KP k, const SepNode* __restrict__
   }
 }
 
+// ------------------------------------------------------------ downward
+// The mirror image: the cut level's local expansions to the leaves' Taylor
+// blocks (g3dpw2local_real_vec, g3drouts.f:1690-1880, after the split),
+//   U1[a][kz][ky]  = i^a sum_kx x2l[a][kx] px(kx) L[kz][ky][kx]    per slab
+//   U2[b][a][kz]   = i^b sum_ky x2l[b][ky] py(ky) U1[a][kz][ky]    per column
+//   lo[c][b][a]    = 2 Re i^c sum_kz x2l[c][kz] pz(kz) U2[b][a][kz] per leaf
+// with p(i, k) = exp(+i t_k sh_i).  The mirror nodes make every sum two real
+// products of depth n2: with S = L[m] p + L[mb] p* and D = L[m] p - L[mb] p*,
+// even orders take tx . S, odd ones i tx . D, tx[a] = (-1)^(a/2) x2l[a].
+// Measured against a whole conversion per leaf (B200, one execute): 4e6 blob
+// targets, eps 1e-6, 3.33 -> 0.69 ms; 3e5 uniform points, eps 1e-9, delta
+// 1e-3, 7.4 -> 0.78 ms (no blocks: evaluated from the columns below).
+
+// x pass (boxes -> slabs) and, with Y, y pass (slabs -> columns).  A warp owns
+// four complex columns of the parent, held in registers with their mirror
+// sums, and serves the children in turn: four multiply-adds per element turn
+// it to the child's phase, 2 U products of KS steps give the child's 16 U
+// orders from 16 u0 on.  X: columns (kz, ky) -> U1[(kz, ky)][a]; Y: columns
+// (kz, a) -> U2[kz][b][a].  GEN: node halves beyond 4 KS in blocks, with the
+// parent read again for every child.
+template <int KS, int U, bool Y, bool GEN>
+__global__ void __launch_bounds__(128) k_down_xy(KP k, const SepNode* __restrict__ nodes,
+                                                 const SepNode* __restrict__ kids, const int* __restrict__ idx,
+                                                 int Pm, int u0, const double* __restrict__ Tin,
+                                                 double* __restrict__ Tout, const double2* __restrict__ ph) {
+  const SepNode N = nodes[blockIdx.x];
+  const int ind = blockIdx.z, npw = k.npw, n2 = k.n2, nkb = GEN ? (n2 + 4 * KS - 1) / (4 * KS) : 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = lane >> 2, c = lane & 3;
+  const int ncol = Y ? n2 * N.p : n2 * npw, kst = Y ? N.p : 1;
+  const double sg = (r & 1) ? 1.0 : -1.0;
+  const double2* src = Y ? reinterpret_cast<const double2*>(Tin + (size_t)N.off * k.nd) + (size_t)ind * N.p * n2 * npw
+                         : k.loc + ((size_t)N.off * k.nd + ind) * k.nexp;
+  double tx[U][2][KS];
+  auto table = [&](int kb) {
+#pragma unroll
+    for (int u = 0; u < U; u++)
+#pragma unroll
+      for (int par = 0; par < 2; par++)
+#pragma unroll
+        for (int s = 0; s < KS; s++) {
+          const int a = 2 * (8 * (u0 + u) + r) + par, m = 4 * (KS * kb + s) + c;
+          tx[u][par][s] = (a < Pm && m < n2) ? ((a & 2) ? -k.x2l[a * npw + m] : k.x2l[a * npw + m]) : 0.0;
+        }
+  };
+  double os[KS], od[KS], ts[KS], td[KS];
+  auto load = [&](const double2* L, int kb) {
+#pragma unroll
+    for (int s = 0; s < KS; s++) {
+      const int m = min(4 * (KS * kb + s) + c, n2 - 1);
+      const double2 a = L[(size_t)m * kst], b = L[(size_t)(npw - 1 - m) * kst];
+      const double o1 = (r & 1) ? a.y : a.x, o2 = (r & 1) ? b.y : b.x;
+      const double t1 = sg * ((r & 1) ? a.x : a.y), t2 = sg * ((r & 1) ? b.x : b.y);
+      os[s] = o1 + o2;
+      od[s] = o1 - o2;
+      ts[s] = t1 + t2;
+      td[s] = t1 - t2;
+    }
+  };
+  if (!GEN) table(0);
+  const int ntiles = (ncol + 3) / 4;
+  for (int nt = blockIdx.y * 4 + warp; nt < ntiles; nt += gridDim.y * 4) {
+    const int qb = min(4 * nt + (r >> 1), ncol - 1);  // the column of the lane's operand
+    const double2* L = src + (Y ? (size_t)(qb / N.p) * npw * N.p + qb % N.p : (size_t)qb * npw);
+    if (!GEN) load(L, 0);
+    for (int i = N.beg; i < N.beg + N.cnt; i++) {
+      const SepNode K = kids[idx ? idx[i] : i];
+      if (!Y && K.p <= 16 * u0) continue;
+      double acc[U][4];
+#pragma unroll
+      for (int u = 0; u < U; u++) acc[u][0] = acc[u][1] = acc[u][2] = acc[u][3] = 0.0;
+      for (int kb = 0; kb < nkb; kb++) {
+        if (GEN) {
+          table(kb);
+          load(L, kb);
+        }
+#pragma unroll
+        for (int s = 0; s < KS; s++) {
+          const double2 p = __ldg(ph + K.row * npw + min(4 * (KS * kb + s) + c, n2 - 1));
+          const double S = fma(p.y, td[s], p.x * os[s]), D = fma(p.y, ts[s], p.x * od[s]);
+#pragma unroll
+          for (int u = 0; u < U; u++)
+            if (u == 0 || 16 * (u0 + u) < K.p) {
+              dmma_884(acc[u][0], acc[u][1], tx[u][0][s], S);
+              dmma_884(acc[u][2], acc[u][3], tx[u][1][s], D);
+            }
+        }
+      }
+      const int q = 4 * nt + c;  // the lane's complex column
+      if (q < ncol) {
+        double2* o;
+        int st;
+        if (Y) {
+          const int P = N.p, kz = q / P;
+          st = P;
+          o = reinterpret_cast<double2*>(Tout + (size_t)K.off * k.nd) + ((size_t)ind * n2 + kz) * P * P + (q - kz * P);
+        } else {
+          st = 1;
+          o = reinterpret_cast<double2*>(Tout + (size_t)K.off * k.nd) + ((size_t)ind * n2 * npw + q) * K.p;
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          const int a = 2 * (8 * (u0 + u) + r);
+          if (a < K.p) o[(size_t)a * st] = make_double2(acc[u][0], acc[u][1]);
+          if (a + 1 < K.p) o[(size_t)(a + 1) * st] = make_double2(-acc[u][3], acc[u][2]);
+        }
+      }
+    }
+  }
+}
+
+// z pass: a column's U2 to its leaves' Taylor blocks, rows of E = P rounded up
+// to even doubles (the padding zero), orders P <= 32 (16 U).  A warp owns
+// eight (b, a) and keeps their n2 values in registers for all the leaves.
+template <int KS, int U, bool GEN>
+__global__ void __launch_bounds__(128) k_down_z(KP k, const SepNode* __restrict__ cols,
+                                                const SepLeaf* __restrict__ leaves, int Pn,
+                                                const double* __restrict__ Tin, double* __restrict__ lo_all,
+                                                const double2* __restrict__ ph) {
+  const SepNode C = cols[blockIdx.x];
+  const int ind = blockIdx.z, npw = k.npw, n2 = k.n2, P2 = Pn * Pn, E = (Pn + 1) & ~1;
+  const int nkb = GEN ? (n2 + 4 * KS - 1) / (4 * KS) : 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = lane >> 2, c = lane & 3;
+  const double2* src = reinterpret_cast<const double2*>(Tin + (size_t)C.off * k.nd) + (size_t)ind * P2 * n2;
+  double tx[U][2][KS];
+  auto table = [&](int kb) {
+#pragma unroll
+    for (int u = 0; u < U; u++)
+#pragma unroll
+      for (int par = 0; par < 2; par++)
+#pragma unroll
+        for (int s = 0; s < KS; s++) {
+          const int a = 2 * (8 * u + r) + par, m = 4 * (KS * kb + s) + c;
+          tx[u][par][s] = (a < Pn && m < n2) ? ((a & 2) ? -k.x2l[a * npw + m] : k.x2l[a * npw + m]) : 0.0;
+        }
+  };
+  double2 z[KS];
+  auto load = [&](const double2* L, int kb) {
+#pragma unroll
+    for (int s = 0; s < KS; s++) z[s] = L[(size_t)min(4 * (KS * kb + s) + c, n2 - 1) * P2];
+  };
+  if (!GEN) table(0);
+  const int ntiles = (P2 + 7) / 8;
+  for (int nt = blockIdx.y * 4 + warp; nt < ntiles; nt += gridDim.y * 4) {
+    const double2* L = src + min(8 * nt + r, P2 - 1);
+    if (!GEN) load(L, 0);
+    for (int i = C.beg; i < C.beg + C.cnt; i++) {
+      const SepLeaf F = leaves[i];
+      double acc[U][4];
+#pragma unroll
+      for (int u = 0; u < U; u++) acc[u][0] = acc[u][1] = acc[u][2] = acc[u][3] = 0.0;
+      for (int kb = 0; kb < nkb; kb++) {
+        if (GEN) {
+          table(kb);
+          load(L, kb);
+        }
+#pragma unroll
+        for (int s = 0; s < KS; s++) {
+          const double2 p = __ldg(ph + F.row * npw + min(4 * (KS * kb + s) + c, n2 - 1));
+          const double re = fma(-z[s].y, p.y, z[s].x * p.x), im = fma(z[s].y, p.x, z[s].x * p.y);
+#pragma unroll
+          for (int u = 0; u < U; u++) {
+            dmma_884(acc[u][0], acc[u][1], tx[u][0][s], re);
+            dmma_884(acc[u][2], acc[u][3], tx[u][1][s], im);
+          }
+        }
+      }
+      double* out = lo_all + F.off + (size_t)ind * P2 * E;
+#pragma unroll
+      for (int ii = 0; ii < 2; ii++) {
+        const int q = 8 * nt + 2 * c + ii;
+        if (q < P2) {
+          const int b = q / Pn, a = q - b * Pn;
+          const bool pad = a == Pn - 1 && E > Pn;
+#pragma unroll
+          for (int u = 0; u < U; u++) {
+            const int ce = 2 * (8 * u + r);
+            double* o = out + ((size_t)ce * Pn + b) * E + a;
+            if (ce < Pn) {
+              o[0] = 2.0 * acc[u][ii];
+              if (pad) o[1] = 0.0;
+            }
+            if (ce + 1 < Pn) {
+              o[Pn * E] = -2.0 * acc[u][2 + ii];
+              if (pad) o[Pn * E + 1] = 0.0;
+            }
+          }
+        }
+      }
+    }
+  }
+}
+
+// ------------------------------------------------------------ evaluation from a column
+// The Taylor block of a leaf costs P^3 n2 multiply-adds and two passes over
+// memory, whatever its number of points; a leaf of few points is evaluated
+// from its column's U2 instead:
+//   pot(x, y, z) = sum_b,a y^b x^a sum_kz Re(Z(kz) U2[kz][b][a]),
+//   Z(kz) = 2 pz(kz) sum_{c<P} x2l[c][kz] (i z)^c,
+// the same truncated sum with the z contraction taken at the points.  One CTA
+// of four warps per chunk of at most 8 MT points: the rows (Re Z, -Im Z) of
+// the points (and of their z derivatives: PGH products) in shared memory,
+// U2[kz][q = (b, a)] read from global memory straight into the B fragments
+// (each element once per chunk), the warps taking the tiles of q in turn, two
+// at a time; the lane's sums of W[point][q] x^a y^b (and with the derivative
+// powers) are added over the lanes and warps at the end in a fixed order.
+// Bound by the tensor pipe and the operand loads.  Measured: 1e5 uniform
+// points, eps 1e-6 (24 points a leaf, order 21), 1.02 ms with blocks and
+// Horner -> 0.18 ms; 3e5 points, eps 1e-9, 3.2 -> 1.0 ms (orders 20 and 31);
+// gradients of 1e5 points at eps 1e-9, 37.5 -> 0.94 ms.
+template <int PGH>
+__host__ __device__ constexpr int colev_tiles() { return PGH == 1 ? 4 : PGH == 2 ? 3 : 2; }
+
+struct ColevDims {
+  int K, lda, ldx;
+  size_t total;  // doubles
+  __host__ __device__ ColevDims(int Pn, int n2, int MT, int pgh) {
+    K = (2 * n2 + 3) & ~3;
+    lda = (K & 15) <= 4 ? (K & ~15) + 4 : (K & ~15) + 20;  // 4 (mod 16): conflict-free A fragments
+    ldx = Pn | 1;
+    const int rows = 8 * MT, nc = pgh == 1 ? 1 : pgh == 2 ? 4 : 10;
+    total = (size_t)pgh * rows * lda + (size_t)2 * pgh * rows * ldx + (size_t)4 * rows * nc + rows;
+  }
+};
+
+template <int MT, int PGH>
+__device__ __forceinline__ void colev_body(const double2* __restrict__ U2, const double* Zs, const double* Xs,
+                                           const double* Ys, const ColevDims& Z, int rows, int Pn, int n2,
+                                           double (*sum)[ncomp<3, PGH>()]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = lane >> 2, c = lane & 3;
+  const int P2 = Pn * Pn, ks = Z.K >> 2, ntp = (P2 + 15) / 16;
+  const double* Ud = reinterpret_cast<const double*>(U2) + (c & 1);
+#pragma unroll
+  for (int i = 0; i < MT; i++)
+#pragma unroll
+    for (int v = 0; v < ncomp<3, PGH>(); v++) sum[i][v] = 0.0;
+  for (int np = warp; np < ntp; np += 4) {
+    double acc[2][MT][PGH][2];
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+      for (int i = 0; i < MT; i++)
+#pragma unroll
+        for (int g = 0; g < PGH; g++) acc[h][i][g][0] = acc[h][i][g][1] = 0.0;
+    const double* B0 = Ud + (size_t)2 * min(16 * np + r, P2 - 1);
+    const double* B1 = Ud + (size_t)2 * min(16 * np + 8 + r, P2 - 1);
+    auto fetch = [&](int s, double (&b)[4][2]) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const size_t o = (size_t)2 * min(2 * (s + j) + (c >> 1), n2 - 1) * P2;
+        b[j][0] = B0[o];
+        b[j][1] = B1[o];
+      }
+    };
+    double bn[4][2];
+    fetch(0, bn);
+    for (int s = 0; s < ks; s += 4) {
+      double b[4][2];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        b[j][0] = bn[j][0];
+        b[j][1] = bn[j][1];
+      }
+      if (s + 4 < ks) fetch(s + 4, bn);
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (s + j < ks) {
+#pragma unroll
+          for (int i = 0; i < MT; i++)
+#pragma unroll
+            for (int g = 0; g < PGH; g++) {
+              const double a = Zs[((size_t)g * rows + 8 * i + r) * Z.lda + 4 * (s + j) + c];
+              dmma_884(acc[0][i][g][0], acc[0][i][g][1], a, b[j][0]);
+              dmma_884(acc[1][i][g][0], acc[1][i][g][1], a, b[j][1]);
+            }
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int q = 16 * np + 8 * h + 2 * c + e;
+        if (q < P2) {
+          const int bq = q / Pn, aq = q - bq * Pn;
+#pragma unroll
+          for (int i = 0; i < MT; i++) {
+            const int xo = (8 * i + r) * Z.ldx + aq, yo = (8 * i + r) * Z.ldx + bq, sz = rows * Z.ldx;
+            const double x0 = Xs[xo], y0 = Ys[yo], xy = x0 * y0;
+            const double w0 = acc[h][i][0][e];
+            sum[i][0] = fma(w0, xy, sum[i][0]);
+            if constexpr (PGH >= 2) {
+              const double x1 = Xs[sz + xo], y1 = Ys[sz + yo], w1 = acc[h][i][1][e];
+              sum[i][1] = fma(w0, x1 * y0, sum[i][1]);
+              sum[i][2] = fma(w0, x0 * y1, sum[i][2]);
+              sum[i][3] = fma(w1, xy, sum[i][3]);
+              if constexpr (PGH >= 3) {
+                const double x2 = Xs[2 * sz + xo], y2 = Ys[2 * sz + yo], w2 = acc[h][i][2][e];
+                sum[i][4] = fma(w0, x2 * y0, sum[i][4]);
+                sum[i][5] = fma(w0, x0 * y2, sum[i][5]);
+                sum[i][6] = fma(w2, xy, sum[i][6]);
+                sum[i][7] = fma(w0, x1 * y1, sum[i][7]);
+                sum[i][8] = fma(w1, x1 * y0, sum[i][8]);
+                sum[i][9] = fma(w1, x0 * y1, sum[i][9]);
+              }
+            }
+          }
+        }
+      }
+  }
+}
+
+template <int PGH>
+__global__ void __launch_bounds__(128) k_eval3d_col(KP k, const ColTask* __restrict__ tasks,
+                                                    const double* __restrict__ Tin,
+                                                    const double2* __restrict__ ph) {
+  constexpr int MT = colev_tiles<PGH>(), ROWS = 8 * MT, NC = ncomp<3, PGH>();
+  const ColTask T = tasks[blockIdx.x];
+  const int ind = blockIdx.y, Pn = T.p, P2 = Pn * Pn, npw = k.npw, n2 = k.n2, tid = threadIdx.x;
+  const ColevDims Z(Pn, n2, MT, PGH);
+  extern __shared__ double sm[];
+  double* Zs = sm;                                  // [PGH][ROWS][lda]
+  double* Xs = Zs + (size_t)PGH * ROWS * Z.lda;     // [PGH][ROWS][ldx]: x^a and its derivatives
+  double* Ys = Xs + (size_t)PGH * ROWS * Z.ldx;
+  double* red = Ys + (size_t)PGH * ROWS * Z.ldx;    // [4][ROWS][NC]
+  double* zc = red + (size_t)4 * ROWS * NC;         // [ROWS]
+  const double* pts = T.set ? k.trg : k.src;
+  if (tid < ROWS) {
+    const int i = T.i0 + min(tid, T.n - 1);
+    double v[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) v[d] = (pts[(size_t)3 * i + d] - k.centers[3 * T.box + d]) * k.dsq;
+    zc[tid] = v[2];
+#pragma unroll
+    for (int d = 0; d < 2; d++) {
+      double* X = (d ? Ys : Xs) + tid * Z.ldx;
+      double p0 = 1.0, p1 = 0.0, p2 = 0.0;  // x^a, a x^(a-1), a (a-1) x^(a-2)
+      for (int a = 0; a < Pn; a++) {
+        X[a] = p0;
+        if (PGH >= 2) X[ROWS * Z.ldx + a] = p1;
+        if (PGH >= 3) X[2 * ROWS * Z.ldx + a] = p2;
+        if (PGH >= 3) p2 = fma(p2, v[d], 2.0 * p1);
+        if (PGH >= 2) p1 = fma(p1, v[d], p0);
+        p0 *= v[d];
+      }
+    }
+  }
+  __syncthreads();
+  // Z rows: Horner in i z with the derivative chains s' <- s' (i z) + i s
+  for (int e = tid; e < ROWS * (Z.K >> 1); e += 128) {
+    const int pt = e / (Z.K >> 1), kz = e - pt * (Z.K >> 1);
+    double2 f[3];
+    f[0] = f[1] = f[2] = make_double2(0.0, 0.0);
+    if (kz < n2 && pt < T.n) {
+      const double u = zc[pt];
+      double2 s0 = make_double2(0.0, 0.0), s1 = s0, s2 = s0;
+      for (int j = Pn - 1; j >= 0; j--) {
+        if (PGH >= 3) s2 = make_double2(fma(-s2.y, u, -2.0 * s1.y), fma(s2.x, u, 2.0 * s1.x));
+        if (PGH >= 2) s1 = make_double2(fma(-s1.y, u, -s0.y), fma(s1.x, u, s0.x));
+        s0 = make_double2(fma(-s0.y, u, __ldg(k.x2l + j * npw + kz)), s0.x * u);
+      }
+      const double2 p = __ldg(ph + T.row * npw + kz), p2 = make_double2(2.0 * p.x, 2.0 * p.y);
+      f[0] = cmul(s0, p2);
+      if (PGH >= 2) f[1] = cmul(s1, p2);
+      if (PGH >= 3) f[2] = cmul(s2, p2);
+    }
+#pragma unroll
+    for (int g = 0; g < PGH; g++) {
+      double* a = Zs + ((size_t)g * ROWS + pt) * Z.lda + 2 * kz;
+      a[0] = f[g].x;
+      a[1] = -f[g].y;
+    }
+  }
+  __syncthreads();
+  const double2* U2 = reinterpret_cast<const double2*>(Tin + (size_t)T.off * k.nd) + (size_t)ind * P2 * n2;
+  double sum[MT][NC];
+  const int nmt = (T.n + 7) / 8;
+#pragma unroll
+  for (int i = 0; i < MT; i++)
+#pragma unroll
+    for (int v = 0; v < NC; v++) sum[i][v] = 0.0;
+  if (nmt == 1) colev_body<1, PGH>(U2, Zs, Xs, Ys, Z, ROWS, Pn, n2, sum);
+  else if (nmt == 2) colev_body<2, PGH>(U2, Zs, Xs, Ys, Z, ROWS, Pn, n2, sum);
+  else if constexpr (MT >= 3) {
+    if (MT == 3 || nmt == 3) colev_body<3, PGH>(U2, Zs, Xs, Ys, Z, ROWS, Pn, n2, sum);
+    else colev_body<MT, PGH>(U2, Zs, Xs, Ys, Z, ROWS, Pn, n2, sum);
+  }
+  const int lane = tid & 31, warp = tid >> 5, r = lane >> 2, c = lane & 3;
+#pragma unroll
+  for (int i = 0; i < MT; i++)
+#pragma unroll
+    for (int v = 0; v < NC; v++) {
+      double a = sum[i][v];
+      a += __shfl_xor_sync(FULL_MASK, a, 1);
+      a += __shfl_xor_sync(FULL_MASK, a, 2);
+      if (c == 0) red[((size_t)warp * ROWS + 8 * i + r) * NC + v] = a;
+    }
+  __syncthreads();
+  double* out = T.set ? k.pottarg : k.pot;
+  const int nc = T.set ? k.nc_t : k.nc_s;
+  for (int e = tid; e < T.n * NC; e += 128) {
+    const int pt = e / NC, v = e - pt * NC;
+    if (v >= nc) continue;
+    double a = 0.0;
+#pragma unroll
+    for (int w = 0; w < 4; w++) a += red[((size_t)w * ROWS + pt) * NC + v];
+    const double sc = v == 0 ? 1.0 : v < 4 ? k.dsq : k.dsq * k.dsq;
+    out[((size_t)(T.i0 + pt) * nc + v) * k.nd + ind] += a * sc;
+  }
+}
+
 // A leaf's expansion times the phases from its centre to the box's, summed
 // over the leaves of a box; one coefficient per thread (memory-bound).
 __global__ void __launch_bounds__(256) k_up_add(KP k, const double2* __restrict__ src,
@@ -430,6 +850,68 @@ cudaError_t sep_up(const KP& k, const SepDev& S, const double* hbuf, cudaStream_
       launches++;
     }
   }
+  return cudaGetLastError();
+}
+
+cudaError_t sep_down(const KP& k, const SepDev& S, double* lo, cudaStream_t st, long long& launches) {
+  const int n2 = k.n2, ksm = (n2 + 3) / 4;
+  int pmax = 0;
+  for (const SepGroup& G : S.groups) pmax = std::max(pmax, G.p + 1);
+  if (S.nboxes <= 0 || pmax == 0) return cudaSuccess;
+  auto cases = [&](int U, auto launch) {
+    const int v = ksm > 8 ? 0 : ksm;
+    switch (2 * v + U - 1) {
+#define DOWN_CASE(N)                                                                            \
+  case 2 * N: launch(std::integral_constant<int, N>(), std::integral_constant<int, 1>(), std::false_type()); break; \
+  case 2 * N + 1: launch(std::integral_constant<int, N>(), std::integral_constant<int, 2>(), std::false_type()); break;
+      DOWN_CASE(1) DOWN_CASE(2) DOWN_CASE(3) DOWN_CASE(4) DOWN_CASE(5) DOWN_CASE(6) DOWN_CASE(7) DOWN_CASE(8)
+#undef DOWN_CASE
+      default: launch(std::integral_constant<int, 8>(), std::integral_constant<int, 2>(), std::true_type()); break;
+    }
+    launches++;
+  };
+  const dim3 gx(S.nboxes, split_for(S.nboxes, k.nd, (n2 * k.npw + 3) / 4, S.sms), k.nd);
+  for (int u0 = 0; 16 * u0 < pmax; u0 += 2)
+    cases(pmax - 16 * u0 <= 16 ? 1 : 2, [&](auto N, auto U, auto G) {
+      k_down_xy<decltype(N)::value, decltype(U)::value, false, decltype(G)::value>
+          <<<gx, 128, 0, st>>>(k, S.boxes, S.slabs, S.box_slabs, pmax, u0, nullptr, S.t2, S.ph);
+    });
+  for (const SepGroup& G : S.groups) {
+    const int Pn = G.p + 1, nslab = G.send - G.sbeg, ncol = G.cend - G.cbeg;
+    const dim3 gy(nslab, split_for(nslab, k.nd, (n2 * Pn + 3) / 4, S.sms), k.nd);
+    for (int u0 = 0; 16 * u0 < Pn; u0 += 2)
+      cases(Pn - 16 * u0 <= 16 ? 1 : 2, [&](auto N, auto U, auto F) {
+        k_down_xy<decltype(N)::value, decltype(U)::value, true, decltype(F)::value>
+            <<<gy, 128, 0, st>>>(k, S.slabs + G.sbeg, S.cols, nullptr, Pn, u0, S.t2, S.t1, S.ph);
+      });
+    if (!G.blocks) continue;  // evaluated from the columns
+    if (Pn > 32) return cudaErrorNotSupported;
+    const dim3 gz(ncol, split_for(ncol, k.nd, (Pn * Pn + 7) / 8, S.sms), k.nd);
+    cases(Pn <= 16 ? 1 : 2, [&](auto N, auto U, auto F) {
+      k_down_z<decltype(N)::value, decltype(U)::value, decltype(F)::value>
+          <<<gz, 128, 0, st>>>(k, S.cols + G.cbeg, S.leaves, Pn, S.t1, lo, S.ph);
+    });
+  }
+  return cudaGetLastError();
+}
+
+int sep_col_points(int pgh) { return 8 * (pgh <= 1 ? colev_tiles<1>() : pgh == 2 ? colev_tiles<2>() : colev_tiles<3>()); }
+
+cudaError_t sep_eval_cols(const KP& k, const SepDev& S, const ColTask* tasks, int ntask, int Pn, int pgh,
+                          cudaStream_t st) {
+  if (ntask <= 0) return cudaSuccess;
+  const dim3 g(ntask, k.nd);
+  const size_t sh = ColevDims(Pn, k.n2, sep_col_points(pgh) / 8, pgh).total * 8;
+  if (sh > 227 * 1024) return cudaErrorNotSupported;
+#define COLEV_CASE(PG)                                            \
+  {                                                               \
+    CK(smem_limit(k_eval3d_col<PG>));                             \
+    k_eval3d_col<PG><<<g, 128, sh, st>>>(k, tasks, S.t1, S.ph);   \
+  }
+  if (pgh <= 1) COLEV_CASE(1)
+  else if (pgh == 2) COLEV_CASE(2)
+  else COLEV_CASE(3)
+#undef COLEV_CASE
   return cudaGetLastError();
 }
 

@@ -4,6 +4,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cstdint>
 #include <vector>
 
 #include "fgt_device.hpp"
@@ -13,14 +14,21 @@ namespace fgtb {
 
 struct KP;
 
-// Fills d and x of every item from the tree (root_box[item.root]) and sorts
-// the items by (p, d, root, x, y, z).
-void sep_sort(const Tree& t, const std::vector<int>& root_box, std::vector<SepItem>& items);
+// The boxes as items, sorted by (rank[depth], root, x, y, z); roots are the
+// boxes of level lroot, numbered from its first.  rank: by depth, equal orders
+// next to one another.
+void sep_order(const Tree& t, int lroot, const std::vector<int>& boxes, const std::vector<int>& rank,
+               std::vector<SepItem>& items);
+// rank of sep_order from the orders by depth (increasing order, then depth)
+std::vector<int> sep_rank(const std::vector<int>& order_of_depth);
 
 // Columns (equal root, depth, x, y), slabs (equal root, depth, x) and boxes
-// of sorted items; offsets and sizes per density.  Every root gets a box,
-// with no slabs where it has no leaf; slot: the root's expansion slot.
-void sep_lists(const std::vector<SepItem>& items, const std::vector<int>& slot, int npw, SepLists& S);
+// of sorted items with their blocks (leaf.off, leaf.n; the rows are filled
+// here); offsets and sizes per density.  slot: the expansion slots by root; a
+// root in `also` gets a box even without leaves.
+void sep_lists(const std::vector<SepItem>& items, const std::vector<SepLeaf>& leaf,
+               const std::vector<int>& order_of_depth, const std::vector<int>& slot,
+               const std::vector<uint8_t>& also, int npw, SepLists& S);
 
 // Phase rows of depths 0..dmax: row 2^d - 1 + i holds exp(i t_m sh) of the
 // npw nodes, sh the offset of box i of 2^d from its root's centre over
@@ -34,5 +42,15 @@ cudaError_t sep_add(const KP& k, const double2* src, const double2* ph, const Me
 
 // Upward: Hermite blocks in hbuf -> the expansions k.mp of the boxes' slots.
 cudaError_t sep_up(const KP& k, const SepDev& S, const double* hbuf, cudaStream_t st, long long& launches);
+
+// Downward: the expansions k.loc of the boxes' slots -> the columns (t1) of
+// every order and the Taylor blocks (lo) of the groups with blocks.
+cudaError_t sep_down(const KP& k, const SepDev& S, double* lo, cudaStream_t st, long long& launches);
+
+// Evaluation from the columns: the most points of a task, and the tasks of
+// one order (Pn: order + 1).
+int sep_col_points(int pgh);
+cudaError_t sep_eval_cols(const KP& k, const SepDev& S, const ColTask* tasks, int ntask, int Pn, int pgh,
+                          cudaStream_t st);
 
 }  // namespace fgtb

@@ -104,16 +104,10 @@ int fgt_ctx_set_host_threads(fgt_ctx* ctx, int nthreads);
  * FGT_TREE_HOST); both give the same tree.  No counterpart in the reference,
  * whose tree is built on the host (pts_tree_build, pts_tree2d4.f:363-590). */
 int fgt_ctx_set_tree(fgt_ctx* ctx, int where);
-/* how many SMs the persistent kernels of the context's plans (created after
- * the call) size their grids for; 0 (the default) uses every SM.  A smaller
- * budget leaves SMs free for work that arrives while a large transform runs
- * (fgt_server_set_sm_budget).  No counterpart in the reference. */
+/* Accepted for older callers, without effect: the transforms have no
+ * persistent kernels, so work that arrives on other streams gets SMs as soon
+ * as any CTA finishes. */
 int fgt_ctx_set_sm_budget(fgt_ctx* ctx, int sms);
-/* on != 0: the context's plans (created after the call) launch one CTA per
- * task, instead of persistent CTAs, in the kernels that allow it, so that a
- * large transform's launches let work on other (higher-priority) streams
- * onto the SMs as soon as any of their CTAs finish.  Default off.  No
- * counterpart in the reference. */
 int fgt_ctx_set_grid_yield(fgt_ctx* ctx, int on);
 /* the algorithm of the plans created after the call (FGT_SCHEME_*): the
  * reference selects it by building 2d/planewave or 2d/nufft (3D likewise),
@@ -255,7 +249,7 @@ int fgt_plan_get_info(const fgt_plan* plan, fgt_plan_info* info);
  * orders, fgt2d.f:1518-1610 / fgt3d.f).  box is 0-based in the tree's
  * numbering (the reference's box - 1).  FGT_ERR_BADARG when the box holds
  * no such expansion (this library allocates them only where the transform
- * reads them).  For checking intermediate stages against the reference. */
+ * reads them; below the cut level in 3D they are formed by this call).  For checking intermediate stages against the reference. */
 int fgt_plan_expansion(fgt_plan* plan, int which, int box, double* out);
 /* One execute with CUDA events around the plan's dominant tensor-core launch
  * (the Hermite-block MMA kernel of the form order group with the most
@@ -377,10 +371,8 @@ typedef struct fgt_server_stats {
 } fgt_server_stats;
 int fgt_server_create(int device, long long max_device_bytes, int nworkers, fgt_server** out);
 int fgt_server_set_precision(fgt_server* server, int precision);
-/* SMs the persistent kernels of the requests planned afterwards size their
- * grids for (0, the default: every SM); see fgt_ctx_set_sm_budget. */
+/* accepted, without effect (see fgt_ctx_set_sm_budget) */
 int fgt_server_set_sm_budget(fgt_server* server, int sms);
-/* fgt_ctx_set_grid_yield for the requests planned afterwards */
 int fgt_server_set_grid_yield(fgt_server* server, int on);
 int fgt_server_submit(fgt_server* server, const fgt_request* request, long long* id);
 /* blocks until request id completes; returns its status (and frees its id) */

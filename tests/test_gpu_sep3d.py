@@ -56,6 +56,37 @@ def test_sep3d_matches_oracle(fgt, oracle, case):
         assert e <= TOL, (k, e)
 
 
+# evaluation of few points per leaf (from the columns) and of many (from the
+# Taylor blocks), with derivatives, at one point and at odd remainders; node
+# halves beyond 32 (eps 1e-18).  Bars of the derivative routes: 1e-12 for the
+# potential, a digit more per derivative.
+EVAL_CASES = [  # kind, ns, nt, delta, eps, nd, pgh
+    ("uniform", 4000, 1, 2e-2, 1e-6, 1, 3),
+    ("uniform", 4001, 7000, 2e-2, 1e-6, 1, 2),
+    ("uniform", 2500, 777, 2e-2, 1e-9, 2, 3),
+    ("cluster", 9001, 12007, 2e-2, 1e-6, 1, 2),
+    ("cluster", 9001, 4003, 2e-2, 1e-12, 1, 1),
+    ("uniform", 1200, 901, 5e-2, 1e-18, 1, 2),
+]
+
+
+@pytest.mark.parametrize("case", EVAL_CASES, ids=[f"{c[0]}_{c[4]:g}_{c[2]}_{c[6]}" for c in EVAL_CASES])
+def test_sep3d_evaluation(fgt, oracle, case):
+    kind, ns, nt, delta, eps, nd, pgh = case
+    rng = np.random.default_rng(ns + nt)
+    src, trg = _points(kind, ns, rng), _points(kind, nt, rng)
+    q = rng.standard_normal((ns, nd))
+    ctx = fgt.Context(0, precision="fp64")
+    got = fgt.transform_pgh(3, nd, delta, eps, src, q, trg, 1, pgh, ctx=ctx)
+    ref = oracle.fgt_pgh(3, nd, delta, eps, src, q, trg, 1, pgh)
+    for k, tol in (("pot", 1e-12), ("pottarg", 1e-12), ("gradtarg", 1e-11), ("hesstarg", 1e-10)):
+        if got[k] is None:
+            continue
+        e = oracle.derr(ref[k], got[k])
+        print(f"{case}: {k} {e:.2e}")
+        assert e <= tol, (k, e)
+
+
 @pytest.mark.parametrize("eps", [1e-3, 1e-6, 1e-12])
 def test_expansions_below_the_cut(fgt, oracle, eps):
     rng = np.random.default_rng(5)
