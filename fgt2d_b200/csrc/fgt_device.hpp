@@ -179,6 +179,7 @@ struct DevicePlan {
   // 3D Hermite form in two kernels: source chunks and their partial blocks
   FormChunk* fchunks = nullptr;
   int nfchunks = 0;
+  int form3_chunk = 4096;    // most sources of a chunk
   double* hbuf = nullptr;    // partial Hermite blocks
   // 3D plane-wave scheme: the leaves' Hermite blocks to the cut level's
   // expansions; the leaves' own expansions (plane-wave route) added to them

@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(128) k_h2pw2d(KP k, const FormTask* __restrict
 }
 
 // ------------------------------------------------------------ (a) form, 3D
-// One CTA per chunk of <= 4096 sources of a leaf accumulates the chunk's
+// One CTA per chunk of at most form3_chunk sources of a leaf accumulates the chunk's
 // Hermite block H[j + P (k + P l)] (g3dformhc_vec, g3drouts.f:109-192) and
 // writes it to its slot of the partial buffer; fgt_sep3d.cu sums a leaf's
 // blocks in chunk order and takes them to the cut level's expansions.
@@ -566,67 +566,95 @@ __global__ void __launch_bounds__(128) k_h2pw2d(KP k, const FormTask* __restrict
 // The chunk's Hermite block on the FP64 tensor cores: H[j][(k, l)] =
 // sum_t x_t^j (q_t y_t^k z_t^l) (with the 1/sqrt(j!) factors, g3dformhc_vec,
 // g3drouts.f:109-192) is one product with M = j (MT tiles of 8), N = the
-// P^2 pairs (k, l) and K = the sources, four per mma.m8n8k4 step.  Sources
-// are staged 64 at a time as power rows in shared memory (row stride 68: the
-// A fragments are conflict-free); a B element is y^k q z^l, one multiply of
-// two staged powers, with (k, l) of the lane's column fixed per tile.  The
-// eight warps split the N tiles (up to four each per pass over the sources).
-// The partial block goes to the chunk's slot of the Hermite buffer, laid out
-// H[j + P (k + P l)] as k_up_z reads it.
-// With dipoles (DIP) every source stages three columns (dip3_coef), 21
-// sources (63 columns) per batch.
-template <int MT, bool DIP>
-__global__ void __launch_bounds__(256) k_form3d_mma(KP k, const FormTask* __restrict__ tasks,
+// P^2 pairs (k, l) and K = the sources, four per mma.m8n8k4 step.  A column
+// tile is four k by two l: its B fragment is y^k q z^l, one multiply of a y
+// fragment that serves every l of the warp and a z fragment that serves every
+// k, so a step of KQ x NLP tiles loads KQ + NLP + MT operands for MT KQ NLP
+// products, each load one or two wavefronts (rows of 44 doubles; tiles of
+// eight consecutive (k, l) straddled rows and conflicted at every order that
+// is no multiple of four).  The warps take the l pairs in turn, starting with
+// another one in every CTA (warp w always runs on sub-partition w mod 4);
+// KQ quads of k per pass over the sources.  Sources are staged 40 at a time
+// as power rows (one thread per source and dimension, the next batch's
+// coordinates loaded while this one is summed).  The partial block goes to
+// the chunk's slot of the Hermite buffer, laid out H[j + P (k + P l)] as
+// k_up_z reads it.  Bound by the tensor pipe (16 cycles per product and
+// sub-partition).
+// Measured (order 13, eps 1e-6): 4e6 sources in leaves of 115, 1.56 ms with
+// eight consecutive columns per tile and eight warps, 1.37 ms; 2e6 in leaves
+// of 1157, 0.68 -> 0.66 (65% of the pipe, the rest mostly the tail of three
+// waves of CTAs); 1.5e5 of order 15, 0.24 -> 0.09; 3e5 of order 19 at eps
+// 1e-9, 0.51 -> 0.38.  Orders above 15 take fewer quads per pass: with three,
+// 176 registers left eight warps on an SM and cost more than the passes.
+// With dipoles (DIP) every source stages three columns (dip3_coef), 13
+// sources (39 columns) per batch.
+constexpr int FORM3_SB = 40, FORM3_SW = 44;
+// quads of k per pass and pairs of l per warp at MT row tiles
+__host__ __device__ constexpr int form3_kq(int P) { return P <= 8 ? 2 : P <= 12 ? 3 : P <= 16 ? 4 : P <= 24 ? 2 : 1; }
+__host__ __device__ constexpr int form3_nlp(int P) { return P <= 8 ? 1 : P <= 16 ? 2 : P <= 24 ? 3 : 4; }
+size_t form3_smem(int Pn) {
+  return (size_t)(8 * ((Pn + 7) / 8) + 4 * ((Pn + 3) / 4) + 2 * ((Pn + 1) / 2)) * FORM3_SW * 8;
+}
+
+template <int MT, int KQ, int NLP, bool DIP>
+__global__ void __launch_bounds__(128) k_form3d_mma(KP k, const FormTask* __restrict__ tasks,
                                                     const FormChunk* __restrict__ chunks,
                                                     double* __restrict__ hbuf, const double* __restrict__ isq) {
-  constexpr int SB = 64, SW = 68, NTW = 4;
+  constexpr int SB = FORM3_SB, SW = FORM3_SW;
   constexpr int VC = DIP ? 3 : 1, SBS = SB / VC;  // columns per source, sources per batch
   const FormChunk C = chunks[blockIdx.x];
   const FormTask T = tasks[C.task];
   const int ind = blockIdx.y;
-  const int Pn = T.p + 1, P2 = Pn * Pn, P3 = P2 * Pn, ntiles = (P2 + 7) / 8;
+  const int Pn = T.p + 1, P2 = Pn * Pn, P3 = P2 * Pn, nkq = (Pn + 3) / 4, nlp = (Pn + 1) / 2;
   extern __shared__ double sm[];
   double* X = sm;                // [8 MT][SW]
-  double* Y = X + 8 * MT * SW;   // [Pn][SW]
-  double* Z = Y + Pn * SW;       // [Pn][SW], times q
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = lane >> 2, c = lane & 3;
-  const double cx = k.centers[3 * T.box], cy = k.centers[3 * T.box + 1], cz = k.centers[3 * T.box + 2];
-  for (int e = threadIdx.x; e < (8 * MT - Pn) * SW; e += blockDim.x) X[Pn * SW + e] = 0.0;
-  double* out = hbuf + ((size_t)C.hoff * k.nd + (size_t)ind * P3);
-  for (int base = 0; base < ntiles; base += 8 * NTW) {
-    double acc[MT][NTW][2];
-    int ko[NTW], lo_[NTW];
-#pragma unroll
-    for (int i = 0; i < NTW; i++) {
-      const int n = 8 * (base + warp + 8 * i) + r;
-      ko[i] = n < P2 ? (n % Pn) * SW : -1;
-      lo_[i] = n < P2 ? (n / Pn) * SW : 0;
-#pragma unroll
-      for (int mt = 0; mt < MT; mt++) acc[mt][i][0] = acc[mt][i][1] = 0.0;
+  double* Y = X + 8 * MT * SW;   // [4 nkq][SW]
+  double* Z = Y + 4 * nkq * SW;  // [2 nlp][SW], times q
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = lane >> 2, c = lane & 3;
+  const int lp0 = (warp + blockIdx.x) & 3;  // the warp's l pairs: lp0 + 4 i
+  for (int e = tid; e < (8 * MT + 4 * nkq + 2 * nlp) * SW; e += 128) sm[e] = 0.0;  // rows past the order stay zero
+  const int d = tid / SB, t = tid - SB * d;  // staging job
+  const bool job = tid < 3 * SB;
+  double* const row = (d == 0 ? X : d == 1 ? Y : Z) + t;
+  const double cen = k.centers[3 * T.box + (job ? d : 0)];
+  auto fetch = [&](int c0, double& u, double& q) {
+    u = cen;
+    q = 0.0;
+    if (job && c0 + t < C.n && !DIP) {
+      const size_t i = (size_t)C.s0 + c0 + t;
+      u = k.src[3 * i + d];
+      q = d == 2 ? k.chg[i * k.nd + ind] : 1.0;
     }
+  };
+  double* out = hbuf + ((size_t)C.hoff * k.nd + (size_t)ind * P3);
+  for (int kq0 = 0; kq0 < nkq; kq0 += KQ) {
+    double acc[KQ][NLP][MT][2];
+#pragma unroll
+    for (int g = 0; g < KQ; g++)
+#pragma unroll
+      for (int i = 0; i < NLP; i++)
+#pragma unroll
+        for (int mt = 0; mt < MT; mt++) acc[g][i][mt][0] = acc[g][i][mt][1] = 0.0;
+    double un, qn;
+    fetch(0, un, qn);
     for (int c0 = 0; c0 < C.n; c0 += SBS) {
       const int m = VC * min(SBS, C.n - c0);
       __syncthreads();
-      for (int job = threadIdx.x; job < 3 * SB; job += blockDim.x) {
-        const int t = job / 3, d = job - 3 * t;
-        double* row = (d == 0 ? X : d == 1 ? Y : Z) + t;
+      if (job) {
         if (!DIP) {
-          double v = 0.0, w = 0.0;
-          if (t < m) {
-            const int i = C.s0 + c0 + t;
-            v = (k.src[3 * i + d] - (d == 0 ? cx : d == 1 ? cy : cz)) * k.dsq;
-            w = d == 2 ? k.chg[(size_t)i * k.nd + ind] : 1.0;
-          }
+          const double v = (un - cen) * k.dsq;
+          double w = qn;
           row[0] = w;
+#pragma unroll 4
           for (int j = 1; j < Pn; j++) {
-            w = w * v * isq[j];
+            w *= v * __ldg(isq + j);
             row[j * SW] = w;
           }
         } else {
           double v = 0.0, a = 0.0, b = 0.0;
           if (t < m) {
             const int i = C.s0 + c0 + t / VC;
-            v = (k.src[3 * i + d] - (d == 0 ? cx : d == 1 ? cy : cz)) * k.dsq;
+            v = (k.src[(size_t)3 * i + d] - cen) * k.dsq;
             double dv[3];
             src_dipole<3>(k, i, ind, dv);
             dip3_coef(t % VC, d, src_charge(k, i, ind), dv, a, b);
@@ -634,37 +662,48 @@ __global__ void __launch_bounds__(256) k_form3d_mma(KP k, const FormTask* __rest
           dip_row(row, SW, Pn, v, a, b, k.dsq, isq);
         }
       }
+      fetch(c0 + SBS, un, qn);
       __syncthreads();
       const int nst = (m + 3) >> 2;
+      const double* xp = X + r * SW + c;
+      const double* yp = Y + (4 * kq0 + (r & 3)) * SW + c;
+      const double* zp = Z + (2 * lp0 + (r >> 2)) * SW + c;
       for (int st = 0; st < nst; st++) {
-        const int s = 4 * st + c;
-        double a[MT];
+        double a[MT], y[KQ], z[NLP];
 #pragma unroll
-        for (int mt = 0; mt < MT; mt++) a[mt] = X[(8 * mt + r) * SW + s];
+        for (int mt = 0; mt < MT; mt++) a[mt] = xp[8 * mt * SW + 4 * st];
 #pragma unroll
-        for (int i = 0; i < NTW; i++) {
-          if (base + warp + 8 * i < ntiles) {
-            const double b = ko[i] >= 0 ? Y[ko[i] + s] * Z[lo_[i] + s] : 0.0;
+        for (int g = 0; g < KQ; g++) y[g] = kq0 + g < nkq ? yp[4 * g * SW + 4 * st] : 0.0;
 #pragma unroll
-            for (int mt = 0; mt < MT; mt++) dmma_884(acc[mt][i][0], acc[mt][i][1], a[mt], b);
+        for (int i = 0; i < NLP; i++) {
+          if (lp0 + 4 * i < nlp) {
+            z[i] = zp[8 * i * SW + 4 * st];
+#pragma unroll
+            for (int g = 0; g < KQ; g++)
+              if (kq0 + g < nkq) {
+                const double b = y[g] * z[i];
+#pragma unroll
+                for (int mt = 0; mt < MT; mt++) dmma_884(acc[g][i][mt][0], acc[g][i][mt][1], a[mt], b);
+              }
           }
         }
       }
     }
+    // the lane's columns 2 c, 2 c + 1 of a tile: k = 4 (kq0 + g) + (2 c & 3) + {0, 1}, l = 2 (lp0 + 4 i) + c / 2
 #pragma unroll
-    for (int i = 0; i < NTW; i++) {
-      const int nt = base + warp + 8 * i;
-      if (nt >= ntiles) continue;
+    for (int g = 0; g < KQ; g++)
 #pragma unroll
-      for (int mt = 0; mt < MT; mt++) {
-        const int j = 8 * mt + r;
+      for (int i = 0; i < NLP; i++) {
+        const int kk = 4 * (kq0 + g) + ((2 * c) & 3), l = 2 * (lp0 + 4 * i) + (c >> 1);
 #pragma unroll
-        for (int ii = 0; ii < 2; ii++) {
-          const int n = 8 * nt + 2 * c + ii;
-          if (j < Pn && n < P2) out[j + Pn * n] = acc[mt][i][ii];
+        for (int mt = 0; mt < MT; mt++) {
+          const int j = 8 * mt + r;
+          if (j < Pn && l < Pn) {
+            if (kk < Pn) out[j + Pn * (kk + Pn * l)] = acc[g][i][mt][0];
+            if (kk + 1 < Pn) out[j + Pn * (kk + 1 + Pn * l)] = acc[g][i][mt][1];
+          }
         }
       }
-    }
   }
 }
 
@@ -2259,7 +2298,12 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     items.reserve(D.form_hermite_n);
     D.up_leaf.reserve(D.form_hermite_n);
     D.up_box.reserve(D.form_hermite_n);
-    long long hoff = 0;
+    // Sources per partial block: at most 4096, fewer (whole batches of the
+    // kernel) where that leaves SMs without a CTA
+    long long nsrc = 0, hoff = 0;
+    for (int i = 0; i < D.form_hermite_n; i++) nsrc += form[i].n;
+    const int batch = P.ifdipole ? FORM3_SB / 3 : FORM3_SB;
+    D.form3_chunk = (int)std::min<long long>(4096 / batch, std::max<long long>(6, nsrc / (8LL * D.sm_count * batch))) * batch;
     for (const SepItem& s : sep_items) {
       const int i = task[s.box];
       if (i < 0) continue;
@@ -2268,7 +2312,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
         continue;
       }
       const FormTask& f = form[items.size()] = in[i];
-      const int n = (f.n + 4095) / 4096;
+      const int n = (f.n + D.form3_chunk - 1) / D.form3_chunk;
       items.push_back(s);
       D.up_box.push_back(s.box);
       D.up_leaf.push_back({hoff, 0, n});
@@ -2581,8 +2625,8 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
       for (int t = 0; t < D.form_hermite_n; t++) {
         const FormTask& f = form[t];
         long long p3 = (long long)(f.p + 1) * (f.p + 1) * (f.p + 1);
-        for (int c = 0; c < f.n; c += 4096) {
-          fchunks.push_back({t, f.s0 + c, std::min(4096, f.n - c), hoff});
+        for (int c = 0; c < f.n; c += D.form3_chunk) {
+          fchunks.push_back({t, f.s0 + c, std::min(D.form3_chunk, f.n - c), hoff});
           hoff += p3;
         }
       }
@@ -2977,7 +3021,7 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
         const int Pn = G.p + 1, mt = (Pn + 7) / 8;
         const bool dom = times && (int)gi == D.dom_fchunk_group;
         if (dom) cudaEventRecord(dev0, st);
-        const size_t sh = ((size_t)8 * mt + 2 * Pn) * 68 * 8;
+        const size_t sh = form3_smem(Pn);
         const dim3 fg(G.end - G.beg, nd);
         const FormChunk* ch = D.fchunks + G.beg;
         // The tcgen05 Hermite blocks (BF16 x 3) only on request: building
@@ -2997,21 +3041,20 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
           launches++;
           continue;
         }
-        switch (mt) {
-#define FORM3_CASE(N)                                                                             \
-  case N:                                                                                         \
+#define FORM3_CASE(PMAX)                                                                          \
+  else if (Pn <= PMAX) {                                                                          \
+    constexpr int MT = (PMAX + 7) / 8, KQ = form3_kq(PMAX), NL = form3_nlp(PMAX);                 \
     if (P.ifdipole) {                                                                             \
-      CK(smem_limit(k_form3d_mma<N, true>)); \
-      k_form3d_mma<N, true><<<fg, 256, sh, st>>>(k, D.form, ch, D.hbuf, D.isq);                   \
+      CK(smem_limit(k_form3d_mma<MT, KQ, NL, true>));                                             \
+      k_form3d_mma<MT, KQ, NL, true><<<fg, 128, sh, st>>>(k, D.form, ch, D.hbuf, D.isq);          \
     } else {                                                                                      \
-      CK(smem_limit(k_form3d_mma<N, false>)); \
-      k_form3d_mma<N, false><<<fg, 256, sh, st>>>(k, D.form, ch, D.hbuf, D.isq);                  \
+      CK(smem_limit(k_form3d_mma<MT, KQ, NL, false>));                                            \
+      k_form3d_mma<MT, KQ, NL, false><<<fg, 128, sh, st>>>(k, D.form, ch, D.hbuf, D.isq);         \
     }                                                                                             \
-    break;
-          FORM3_CASE(1) FORM3_CASE(2) FORM3_CASE(3) FORM3_CASE(4)
+  }
+        if (Pn > 32) return cudaErrorNotSupported;
+        FORM3_CASE(8) FORM3_CASE(12) FORM3_CASE(16) FORM3_CASE(24) FORM3_CASE(32)
 #undef FORM3_CASE
-          default: return cudaErrorNotSupported;
-        }
         if (dom) {
           cudaEventRecord(dev1, st);
           snprintf(times->dom_name, sizeof(times->dom_name), "k_form3d_mma<%d>", mt);
