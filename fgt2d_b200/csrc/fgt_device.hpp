@@ -195,6 +195,7 @@ struct DevicePlan {
   // launch shapes
   int form_hermite_n = 0, form_pw_n = 0;
   int eval_taylor_n = 0, eval_pw_n = 0;
+  int eval_pw_max = 0;  // most points of a plane-wave evaluation task
   int form_pmax = 0, eval_pmax = 0;  // largest order among Hermite form / Taylor eval tasks
   std::vector<OrderGroup> form_groups;
   int dom_form_group = -1;        // 2D: form group with the most sources (MMA kernels)

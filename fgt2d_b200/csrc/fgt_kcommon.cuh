@@ -371,6 +371,10 @@ cudaError_t launch_direct_mixed_x2(const KP& k, const DirTask* tasks, int ntask,
 cudaError_t launch_eval2d_horner_f32(const KP& k, const HornerTask* tasks, int ntask, int nd, int Pn,
                                      const double* lo, cudaStream_t st);
 
+// 3D plane-wave route (fgt_pw3d.cu): potentials, gradients and Hessians of the
+// tasks' points, at most nmax each, from their expansions.
+cudaError_t launch_eval3d_pw(const KP& k, const EvalTask* tasks, int ntask, int nmax, int pgh, cudaStream_t st);
+
 // Tensor-core kernels (fgt_tc.cu).  3D Taylor evaluation of potentials as
 // BF16 x 3 tcgen05 products for the point chunks of one order group.
 bool eval3d_tc_supported(int Pn);

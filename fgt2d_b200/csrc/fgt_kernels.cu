@@ -956,107 +956,7 @@ __global__ void __launch_bounds__(128) k_eval2d_horner_any(KP k, const HornerTas
   }
 }
 
-// ------------------------------------------------------------ (c) eval, 3D plane-wave route, potentials
-// k_eval3d_sep (g3dpwevalp_vec, g3drouts.f:2268-2362):
-//   pot = 2 Re sum_{m1 < n2} Z[m1](z) sum_{m2} Y[m2](y) sum_{m3} X[m3](x) L[m1][m2][m3]
-// with X[m](x) = exp(i t_m x).  One CTA per
-// task; points in blocks of 32 whose phase tables sit in shared memory; a
-// thread takes rows (m1, m2) of the expansion for four points (L read once
-// per block, through the read-only cache), and the partial sums are reduced
-// in a fixed order.  Potentials only (the derivative variants keep their own
-// kernels).
-constexpr int SEP_NPB = 32;
-__global__ void __launch_bounds__(256, 2) k_eval3d_sep(KP k, const EvalTask* __restrict__ tasks) {
-  const EvalTask T = tasks[blockIdx.x];
-  const int ind = blockIdx.y;
-  const int npw = k.npw, n2 = k.n2, tid = threadIdx.x;
-  const double2* L = k.loc + ((size_t)T.slot * k.nd + ind) * k.nexp;
-  const double* pts = T.set ? k.trg : k.src;
-  double* out = T.set ? k.pottarg : k.pot;
-  const int nc = T.set ? k.nc_t : k.nc_s;
-  const double cx = k.centers[3 * T.box], cy = k.centers[3 * T.box + 1], cz = k.centers[3 * T.box + 2];
-  extern __shared__ double2 sep_sh[];
-  double2* X = sep_sh;                      // [npw][SEP_NPB]
-  double2* Y = X + npw * SEP_NPB;           // [npw][SEP_NPB]
-  double2* Zt = Y + npw * SEP_NPB;          // [n2][SEP_NPB]
-  double2* part = Zt + n2 * SEP_NPB;        // [256][4] partial sums
-  const int nrow = n2 * npw;
-  for (int p0 = 0; p0 < T.n; p0 += SEP_NPB) {
-    const int np = min(SEP_NPB, T.n - p0);
-    for (int e = tid; e < (2 * npw + n2) * SEP_NPB; e += blockDim.x) {
-      const int m = e / SEP_NPB, pt = e % SEP_NPB;
-      const int d = m < npw ? 0 : m < 2 * npw ? 1 : 2, node = d == 0 ? m : d == 1 ? m - npw : m - 2 * npw;
-      double2 v = make_double2(0.0, 0.0);
-      if (pt < np) {
-        const double u = (pts[3 * (T.i0 + p0 + pt) + d] - (d == 0 ? cx : d == 1 ? cy : cz)) * k.dsq;
-        v = cexpi((2 * (node - n2) + 1) * k.t1 * u);
-      }
-      // X, Y and Zt are consecutive; point 4 g + j sits at j * 8 + g of its
-      // row, so the eight point groups of one j are one 128-byte line
-      X[m * SEP_NPB + (pt & 3) * 8 + (pt >> 2)] = v;
-    }
-    __syncthreads();
-    const int npg = (np + 3) / 4, rstep = blockDim.x / npg;
-    const int pg = tid % npg, rs = tid / npg;
-    double2 acc[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) acc[j] = make_double2(0.0, 0.0);
-    if (rs < rstep) {
-      int m1 = 0, m2 = rs;
-      while (m2 >= npw) {
-        m2 -= npw;
-        m1++;
-      }
-      for (int row = rs; row < nrow; row += rstep) {
-        const double2* Lr = L + (size_t)row * npw;
-        double2 s[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) s[j] = make_double2(0.0, 0.0);
-        // eight coefficients loaded before their products (loads in flight)
-        int m3 = 0;
-        for (; m3 + 8 <= npw; m3 += 8) {
-          double2 l[8];
-#pragma unroll
-          for (int u = 0; u < 8; u++) l[u] = __ldg(Lr + m3 + u);
-#pragma unroll
-          for (int u = 0; u < 8; u++) {
-            const double2* xp = X + (m3 + u) * SEP_NPB + pg;
-#pragma unroll
-            for (int j = 0; j < 4; j++) s[j] = cfma(l[u], xp[8 * j], s[j]);
-          }
-        }
-        for (; m3 < npw; m3++) {
-          const double2 l = __ldg(Lr + m3);
-          const double2* xp = X + m3 * SEP_NPB + pg;
-#pragma unroll
-          for (int j = 0; j < 4; j++) s[j] = cfma(l, xp[8 * j], s[j]);
-        }
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          const double2 yz = cmul(Y[m2 * SEP_NPB + 8 * j + pg], Zt[m1 * SEP_NPB + 8 * j + pg]);
-          acc[j] = cfma(s[j], yz, acc[j]);
-        }
-        m2 += rstep;
-        while (m2 >= npw) {
-          m2 -= npw;
-          m1++;
-        }
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 4; j++) part[tid * 4 + j] = acc[j];
-    __syncthreads();
-    if (tid < np) {
-      const int g = tid >> 2, j = tid & 3;
-      double re = 0.0;
-      for (int r = 0; r < rstep; r++) re += part[(r * npg + g) * 4 + j].x;
-      const double v = 2.0 * re;
-      add_out<1>(out, T.i0 + p0 + tid, k.nd, nc, ind, &v);
-    }
-    __syncthreads();
-  }
-}
-
+// ------------------------------------------------------------ (c) eval, 3D Taylor blocks
 // k_eval3d_horner: one CTA (128 threads) per chunk of <= 256 points of an
 // evaluation leaf; the leaf's Taylor block lo[c][b][a] (rows of E = 2 NP2)
 // is staged in shared memory and each thread evaluates two points by Horner
@@ -1480,101 +1380,6 @@ __global__ void __launch_bounds__(256) k_eval2d(KP k, const EvalTask* __restrict
       v[3] = -2.0 * z[3].x * d2;
       v[4] = -2.0 * z[4].x * d2;
       v[5] = -2.0 * z[5].x * d2;
-    }
-    add_out<NC>(out, ip, k.nd, nc, ind, v);
-  }
-}
-
-// ------------------------------------------------------------ (c) eval, 3D
-// PW route (g3dpwevalp_vec, g3drouts.f:2268-2362): one CTA per task.  x and y
-// run over both signs (PwAcc), z over the stored half, whose nodes are
-// negative: e^{-i t z} has z derivatives -i t and -t^2.  With Y(a,b) the x/y
-// sums of derivative orders a, b and F(a,b) = sum_z Y(a,b) e^{-itz},
-// G(a,b) = sum_z t Y(a,b) e^{-itz}, Gz2 = sum_z t^2 Y(0,0) e^{-itz}:
-//   pot = 2 Re F00, g = (-2 Im F10, -2 Im F01, 2 Im G00),
-//   h_xx, h_yy, h_zz = -2 Re F20, -2 Re F02, -2 Re Gz2,
-//   h_xy, h_xz, h_yz = -2 Re F11, 2 Re G10, 2 Re G01   (times dsq per derivative).
-template <int PGH>
-__global__ void __launch_bounds__(256) k_eval3d_pw(KP k, const EvalTask* __restrict__ tasks) {
-  constexpr int NC = ncomp<3, PGH>(), ORD = PGH - 1;
-  const EvalTask T = tasks[blockIdx.x];
-  const int ind = blockIdx.y;
-  const int npw = k.npw, n2 = k.n2;
-  const double2* L = k.loc + ((size_t)T.slot * k.nd + ind) * k.nexp;
-  const double* pts = T.set ? k.trg : k.src;
-  double* out = T.set ? k.pottarg : k.pot;
-  const int nc = T.set ? k.nc_t : k.nc_s;
-  const double cx = k.centers[3 * T.box], cy = k.centers[3 * T.box + 1], cz = k.centers[3 * T.box + 2];
-  for (int i = threadIdx.x; i < T.n; i += blockDim.x) {
-    const int ip = T.i0 + i;
-    const double x = (pts[3 * ip] - cx) * k.dsq, y = (pts[3 * ip + 1] - cy) * k.dsq,
-                 z = (pts[3 * ip + 2] - cz) * k.dsq;
-    const double2 ex = cexpi(k.t1 * x), ey = cexpi(k.t1 * y), ez = cexpi(k.t1 * z);
-    const double2 exx = cmul(ex, ex), eyy = cmul(ey, ey), ezz = cmul(ez, ez);
-    // acc: [0] F00, [1] F10, [2] F01, [3] G00, [4] F20, [5] F02, [6] Gz2, [7] F11, [8] G10, [9] G01
-    double2 acc[NC];
-#pragma unroll
-    for (int c = 0; c < NC; c++) acc[c] = make_double2(0.0, 0.0);
-    double2 w3 = ez;
-    for (int mz = 0; mz < n2; mz++) {
-      // z index n2-1-mz holds node -(2 mz + 1) t1
-      const double tz = (2 * mz + 1) * k.t1;
-      // Y[b][a]: y order b of the x order a sums
-      PwAcc<ORD> Y[ORD + 1];
-      double2 w2 = ey;
-      for (int my = 0; my < n2; my++) {
-        const double ty = (2 * my + 1) * k.t1;
-        const double2* rp = L + (size_t)npw * ((n2 + my) + (size_t)npw * (n2 - 1 - mz));
-        const double2* rm = L + (size_t)npw * ((n2 - 1 - my) + (size_t)npw * (n2 - 1 - mz));
-        PwAcc<ORD> sp, sn;
-        double2 w1 = ex;
-        for (int mx = 0; mx < n2; mx++) {
-          const double tx = (2 * mx + 1) * k.t1;
-          sp.add(rp[n2 + mx], rp[n2 - 1 - mx], w1, tx);
-          sn.add(rm[n2 + mx], rm[n2 - 1 - mx], w1, tx);
-          w1 = cmul(w1, exx);
-        }
-#pragma unroll
-        for (int a = 0; a <= ORD; a++) Y[a].add(sp.s[a], sn.s[a], w2, ty);
-        w2 = cmul(w2, eyy);
-      }
-      // conj(w3) factors
-      const double2 f00 = cmulc(Y[0].s[0], w3);
-      acc[0].x += f00.x;
-      acc[0].y += f00.y;
-      if (PGH >= 2) {
-        const double2 f10 = cmulc(Y[ORD >= 1 ? 1 : 0].s[0], w3), f01 = cmulc(Y[0].s[ORD >= 1 ? 1 : 0], w3);
-        acc[1].y += f10.y;
-        acc[2].y += f01.y;
-        acc[3].y = fma(tz, f00.y, acc[3].y);
-        if (PGH >= 3) {
-          const double2 f20 = cmulc(Y[ORD >= 2 ? 2 : 0].s[0], w3), f02 = cmulc(Y[0].s[ORD >= 2 ? 2 : 0], w3);
-          const double2 f11 = cmulc(Y[ORD >= 1 ? 1 : 0].s[ORD >= 1 ? 1 : 0], w3);
-          acc[4].x += f20.x;
-          acc[5].x += f02.x;
-          acc[6].x = fma(tz * tz, f00.x, acc[6].x);
-          acc[7].x += f11.x;
-          acc[8].x = fma(tz, f10.x, acc[8].x);
-          acc[9].x = fma(tz, f01.x, acc[9].x);
-        }
-      }
-      w3 = cmul(w3, ezz);
-    }
-    double v[NC];
-    v[0] = 2.0 * acc[0].x;
-    if (PGH >= 2) {
-      v[1] = -2.0 * acc[1].y * k.dsq;
-      v[2] = -2.0 * acc[2].y * k.dsq;
-      v[3] = 2.0 * acc[3].y * k.dsq;
-    }
-    if (PGH >= 3) {
-      const double d2 = k.dsq * k.dsq;
-      v[4] = -2.0 * acc[4].x * d2;
-      v[5] = -2.0 * acc[5].x * d2;
-      v[6] = -2.0 * acc[6].x * d2;
-      v[7] = -2.0 * acc[7].x * d2;
-      v[8] = 2.0 * acc[8].x * d2;
-      v[9] = 2.0 * acc[9].x * d2;
     }
     add_out<NC>(out, ip, k.nd, nc, ind, v);
   }
@@ -2268,6 +2073,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   for (auto& e : ev) {
     (e.route == ROUTE_PW ? D.eval_pw_n : D.eval_taylor_n)++;
     if (e.route == ROUTE_TAYLOR) D.eval_pmax = std::max(D.eval_pmax, e.p);
+    else D.eval_pw_max = std::max(D.eval_pw_max, e.n);
   }
   // 3D plane-wave scheme: the Hermite leaves in the order of the columns and
   // slabs of their cut-level boxes, and the leaves with their own expansions
@@ -3221,19 +3027,8 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
         launches++;
       }
     }
-    const size_t sh_sep = ((size_t)(2 * P.npw + P.npw / 2) * SEP_NPB + 256 * 4) * 16;
-    if (P.dim == 3 && D.eval_pw_n > 0 && pgh == 1) {
-      CK(smem_limit(k_eval3d_sep));
-      k_eval3d_sep<<<dim3(D.eval_pw_n, nd), 256, sh_sep, st>>>(k, D.eval + D.eval_taylor_n);
-      launches++;
-    } else if (P.dim == 3 && D.eval_pw_n > 0) {
-      {
-          const cudaError_t e_pgh = with_pgh(pgh, [&](auto G) -> cudaError_t {
-        k_eval3d_pw<decltype(G)::value><<<dim3(D.eval_pw_n, nd), 256, 0, st>>>(k, D.eval + D.eval_taylor_n);
-        return cudaSuccess;
-      });
-          CK(e_pgh);
-        }
+    if (P.dim == 3 && D.eval_pw_n > 0) {  // the plane-wave route
+      CK(launch_eval3d_pw(k, D.eval + D.eval_taylor_n, D.eval_pw_n, D.eval_pw_max, pgh, st));
       launches++;
     }
    }  // phase 2
