@@ -72,10 +72,10 @@ struct SepItem {
   int box, root;  // box; root as its number among the boxes of the root level
   int d, x[3];    // depth below the root, place in the root's grid
 };
-// A leaf's plane-wave expansion added to a cut-level one: its slot and its
-// phase rows in x, y and z.
-struct SepShift {
-  int src, row[3];
+// 3D plane-wave form: a box's expansion (slot) about its centre from the
+// source ranges [beg, beg + cnt), added (add) to what sep_up put there.
+struct PwFormTask {
+  int box, slot, beg, cnt, add;
 };
 // Separable 3D transforms (fgt_sep3d.hpp).  A leaf's block with its z phase
 // row; a node of the levels above: a column (x, y) of leaves, a slab (x) of
@@ -181,14 +181,13 @@ struct DevicePlan {
   int nfchunks = 0;
   int form3_chunk = 4096;    // most sources of a chunk
   double* hbuf = nullptr;    // partial Hermite blocks
-  // 3D plane-wave scheme: the leaves' Hermite blocks to the cut level's
-  // expansions; the leaves' own expansions (plane-wave route) added to them
+  // 3D plane-wave scheme: the leaves' Hermite blocks to the cut level's expansions
   SepDev up, dn;  // dn: the cut level's local expansions to the leaves' evaluation
   ColTask* ctask = nullptr;
   std::vector<OrderGroup> ctask_groups;
-  MergeGroup* upw_groups = nullptr;
-  SepShift* upw = nullptr;
-  int nupw_groups = 0;
+  PwFormTask* pwf = nullptr;  // boxes formed from exponential sums, and their sources
+  SrcRange* pwf_src = nullptr;
+  int npwf = 0;
   std::vector<int> up_box;       // the Hermite leaves and their blocks (host copy)
   std::vector<SepLeaf> up_leaf;
   std::vector<OrderGroup> fchunk_groups;  // chunk ranges of equal order

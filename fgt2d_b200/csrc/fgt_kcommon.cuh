@@ -371,8 +371,11 @@ cudaError_t launch_direct_mixed_x2(const KP& k, const DirTask* tasks, int ntask,
 cudaError_t launch_eval2d_horner_f32(const KP& k, const HornerTask* tasks, int ntask, int nd, int Pn,
                                      const double* lo, cudaStream_t st);
 
-// 3D plane-wave route (fgt_pw3d.cu): potentials, gradients and Hessians of the
+// 3D plane-wave route (fgt_pw3d.cu): the expansions k.mp of the tasks' boxes
+// from their source ranges, added to what is there or stored; potentials, gradients and Hessians of the
 // tasks' points, at most nmax each, from their expansions.
+cudaError_t launch_form3d_pw(const KP& k, const PwFormTask* tasks, int ntask, const SrcRange* ranges,
+                             cudaStream_t st, long long& launches);
 cudaError_t launch_eval3d_pw(const KP& k, const EvalTask* tasks, int ntask, int nmax, int pgh, cudaStream_t st);
 
 // Tensor-core kernels (fgt_tc.cu).  3D Taylor evaluation of potentials as

@@ -1051,109 +1051,6 @@ __global__ void __launch_bounds__(128) k_eval3d_horner(KP k, const HornerTask* _
   }
 }
 
-// ------------------------------------------------------------ (a) form, 3D direct
-// pw[k3,k2,k1] = sum_i q_i w(k3) e^{-i t x} w(k2) e^{-i t y} w(k1) e^{-i t z}
-// (g3dformpwc_vec, g3drouts.f:1950-2038).  One CTA per (leaf, density);
-// sources in chunks of FORM_CH, each with its three factor rows built once
-// in shared memory; a thread owns expansion rows (k1, k2) for one block of 8
-// consecutive k3 (its block fixed, its rows strided), so each source costs
-// one row product and 8 complex FMAs per item, and the chunks' sums are added
-// to the slot in chunk order.
-__global__ void __launch_bounds__(256) k_form3d_pw(KP k, const FormTask* __restrict__ tasks) {
-  const FormTask T = tasks[blockIdx.x];
-  const int ind = blockIdx.y;
-  const int npw = k.npw, n2 = k.n2;
-  extern __shared__ double sm[];
-  double2* F1 = reinterpret_cast<double2*>(sm);      // [FORM_CH][npw] (+ 8 padding)
-  double2* F2 = F1 + FORM_CH * npw + 8;                // [FORM_CH][npw]
-  double2* F3 = F2 + FORM_CH * npw;                    // [FORM_CH][n2], charge folded in
-  const double cx = k.centers[3 * T.box], cy = k.centers[3 * T.box + 1], cz = k.centers[3 * T.box + 2];
-  double2* out = k.mp + ((size_t)T.slot * k.nd + ind) * k.nexp;
-  // this thread's k3 block and first row; rows advance by rstep.  The block
-  // is the slow index, so a warp's lanes share it (the k3 factors are
-  // broadcast loads) and take consecutive rows
-  const int nmb = (npw + 7) / 8, rstep = blockDim.x / nmb, mb = threadIdx.x / rstep;
-  const int row0 = threadIdx.x - mb * rstep, nrow = n2 * npw;
-  // dipoles (g3dformpwd_vec / g3dformpwcd_vec, g3drouts.f:2042-2262): three
-  // columns per source, the factor of one dimension times v_d (-i t dsq)
-  // in each (as dip3_coef), 10 sources per chunk
-  const int vc = k.ifdipole ? 3 : 1, chs = FORM_CH / vc;
-  for (int c0 = 0; c0 < T.n; c0 += chs) {
-    const int m = vc * min(chs, T.n - c0);
-    __syncthreads();
-    if (threadIdx.x < m) {
-      const int i = T.s0 + c0 + threadIdx.x / vc, col = threadIdx.x % vc;
-      const double x = (k.src[3 * i] - cx) * k.dsq, y = (k.src[3 * i + 1] - cy) * k.dsq,
-                   z = (k.src[3 * i + 2] - cz) * k.dsq;
-      double dv[3] = {0.0, 0.0, 0.0}, ca[3], cb[3];
-      if (k.ifdipole) src_dipole<3>(k, i, ind, dv);
-      const double q = k.ifdipole ? src_charge(k, i, ind) : k.chg[(size_t)i * k.nd + ind];
-      for (int d = 0; d < 3; d++) dip3_coef(col, d, q, dv, ca[d], cb[d]);
-      // positive node m: t = (2m+1) t1 at index n2+m; its mirror n2-1-m
-      double2 ex = cexpi(-k.t1 * x), ey = cexpi(-k.t1 * y), ez = cexpi(-k.t1 * z);
-      const double2 exx = cmul(ex, ex), eyy = cmul(ey, ey), ezz = cmul(ez, ez);
-      double2* f1 = F1 + threadIdx.x * npw;
-      double2* f2 = F2 + threadIdx.x * npw;
-      double2* f3 = F3 + threadIdx.x * n2;
-      for (int mm = 0; mm < n2; mm++) {
-        const double w = k.ws[n2 + mm];
-        double2 a = make_double2(ex.x * w, ex.y * w), b = make_double2(ey.x * w, ey.y * w),
-                c = make_double2(ez.x * w * q, ez.y * w * q);
-        if (k.ifdipole) {
-          // ca f + cb f (-i t dsq) per dimension, f = w e^{-i t x}
-          const double td = (2 * mm + 1) * k.t1 * k.dsq;
-          auto mix = [td](double2 f, double p0, double p1) {
-            return make_double2(fma(p0, f.x, p1 * td * f.y), fma(p0, f.y, -p1 * td * f.x));
-          };
-          a = mix(a, ca[0], cb[0]);
-          b = mix(b, ca[1], cb[1]);
-          c = mix(make_double2(ez.x * w, ez.y * w), ca[2], cb[2]);
-        }
-        f1[n2 + mm] = a; f1[n2 - 1 - mm] = make_double2(a.x, -a.y);
-        f2[n2 + mm] = b; f2[n2 - 1 - mm] = make_double2(b.x, -b.y);
-        f3[n2 - 1 - mm] = make_double2(c.x, -c.y);
-        ex = cmul(ex, exx); ey = cmul(ey, eyy); ez = cmul(ez, ezz);
-      }
-    }
-    __syncthreads();
-    if (mb >= nmb) continue;
-    int i1 = 0, i2 = row0;
-    while (i2 >= npw) {
-      i2 -= npw;
-      i1++;
-    }
-    for (int row = row0; row < nrow; row += rstep) {
-      double2 acc[8];
-#pragma unroll
-      for (int j = 0; j < 8; j++) acc[j] = make_double2(0.0, 0.0);
-      for (int t = 0; t < m; t++) {
-        const double2 yz = cmul(F2[t * npw + i2], F3[t * n2 + i1]);
-        const double2* f1 = F1 + t * npw + 8 * mb;
-#pragma unroll
-        for (int j = 0; j < 8; j++) acc[j] = cfma(f1[j], yz, acc[j]);
-      }
-      double2* o = out + (size_t)row * npw + 8 * mb;
-#pragma unroll
-      for (int j = 0; j < 8; j++)
-        if (8 * mb + j < npw) {
-          if (c0 == 0) {
-            o[j] = acc[j];
-          } else {
-            const double2 p = o[j];
-            o[j] = make_double2(p.x + acc[j].x, p.y + acc[j].y);
-          }
-        }
-      i2 += rstep;
-      while (i2 >= npw) {
-        i2 -= npw;
-        i1++;
-      }
-    }
-  }
-  if (T.n == 0)  // no sources: a zero expansion
-    for (int e = threadIdx.x; e < k.nexp; e += blockDim.x) out[e] = make_double2(0.0, 0.0);
-}
-
 // 2D plane-wave expansion of a box formed directly from its sources: the
 // exact sum that the NUFFT scheme computes with a type-1 NUFFT
 // (g2dformpwc_vec, 2d/nufft/src/g2drouts.f:1234-1307),
@@ -2083,8 +1980,8 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     for (int t = D.eval_taylor_n; t < D.neval; t++)
       while (H.tree.level[ev[t].box] > lcut) ev[t].box = H.tree.parent[ev[t].box];
   SepLists up;
-  std::vector<MergeGroup> upw_groups;
-  std::vector<SepShift> upw;
+  std::vector<PwFormTask> pwf;  // 3D boxes formed from exponential sums
+  std::vector<SrcRange> pwf_src;
   std::vector<double> sep_ph;
   std::vector<SepItem> sep_items;  // every leaf at or below the cut level, in the order of the lists
   std::vector<int> sep_order_of;   // order by depth below the cut level
@@ -2114,7 +2011,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
       const int i = task[s.box];
       if (i < 0) continue;
       if (i >= D.form_hermite_n) {
-        if (s.d > 0) pw.push_back(s);  // else it forms the cut level's expansion itself
+        pw.push_back(s);
         continue;
       }
       const FormTask& f = form[items.size()] = in[i];
@@ -2125,19 +2022,24 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
       hoff += (long long)n * (f.p + 1) * (f.p + 1) * (f.p + 1);
     }
     std::vector<int> slot(nroot);
-    std::vector<uint8_t> also(nroot, 0);
+    std::vector<uint8_t> has(nroot, 0);
     for (int r = 0; r < nroot; r++) slot[r] = H.mp_slot[tr.lfirst[lcut] + r];
+    for (const SepItem& s : items) has[s.root] = 1;
     std::stable_sort(pw.begin(), pw.end(), [](const SepItem& a, const SepItem& b) { return a.root < b.root; });
     for (size_t i = 0; i < pw.size(); i++) {
-      const SepItem& s = pw[i];
-      if (i == 0 || pw[i - 1].root != s.root) upw_groups.push_back({slot[s.root], (int)i, 0});
-      upw_groups.back().cnt++;
-      also[s.root] = 1;
-      const int r0 = (1 << s.d) - 1;
-      upw.push_back({H.mp_slot[s.box], {r0 + s.x[0], r0 + s.x[1], r0 + s.x[2]}});
+      const FormTask& f = form[task[pw[i].box]];
+      const int r = pw[i].root;
+      if (i == 0 || pw[i - 1].root != r) pwf.push_back({tr.lfirst[lcut] + r, slot[r], (int)pwf_src.size(), 0, has[r]});
+      pwf_src.push_back({f.s0, f.n});
+      pwf.back().cnt++;
     }
-    sep_lists(items, D.up_leaf, sep_order_of, slot, also, P.npw, up);
+    sep_lists(items, D.up_leaf, sep_order_of, slot, -1, P.npw, up);
   }
+  if (P.dim == 3 && P.scheme == 1)  // the NUFFT scheme: every box by itself
+    for (const FormTask& f : form) {
+      pwf.push_back({f.box, f.slot, (int)pwf_src.size(), 1, 0});
+      pwf_src.push_back({f.s0, f.n});
+    }
   tq[nq++] = tnow();
   // launch groups of equal order among the Hermite form / Taylor eval tasks
   for (int t = 0; t < D.form_hermite_n;) {
@@ -2312,7 +2214,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     }
     std::vector<int> slot(tr.llast[lcut] - tr.lfirst[lcut] + 1);
     for (size_t r = 0; r < slot.size(); r++) slot[r] = H.loc_slot[tr.lfirst[lcut] + r];
-    sep_lists(items, leaf, sep_order_of, slot, {}, P.npw, dn);
+    sep_lists(items, leaf, sep_order_of, slot, -1, P.npw, dn);
     size_t nh = 0, nct = 0;
     for (int t = 0; t < D.eval_taylor_n; t++) {
       if (blocks[ev[t].p]) nh += (ev[t].n + 255) / 256;
@@ -2474,7 +2376,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
                  bytes_of(fchunks) +
                  bytes_of(up.leaves) + bytes_of(up.cols) + bytes_of(up.slabs) + bytes_of(up.boxes) +
                  bytes_of(up.box_slabs) + bytes_of(dn.cols) + bytes_of(dn.leaves) + bytes_of(dn.slabs) +
-                 bytes_of(dn.boxes) + bytes_of(dn.box_slabs) + bytes_of(ctask) + bytes_of(upw_groups) + bytes_of(upw) + bytes_of(sep_ph) +
+                 bytes_of(dn.boxes) + bytes_of(dn.box_slabs) + bytes_of(ctask) + bytes_of(pwf) + bytes_of(pwf_src) + bytes_of(sep_ph) +
                  al(std::max(up.t1, dn.t1) * nd * 8) + al(std::max(up.t2, dn.t2) * nd * 8) +
                  al(hbuf_doubles * 8) + bytes_of(form_hoff) + bytes_of(tables) + bytes_of(conv) + bytes_of(horner) +
                  al(lo_doubles * 8) + 4096;
@@ -2536,8 +2438,8 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     st.add(cur, D.dn.boxes, dn.boxes);
     st.add(cur, D.dn.box_slabs, dn.box_slabs);
     st.add(cur, D.ctask, ctask);
-    st.add(cur, D.upw_groups, upw_groups);
-    st.add(cur, D.upw, upw);
+    st.add(cur, D.pwf, pwf);
+    st.add(cur, D.pwf_src, pwf_src);
     double* ph = nullptr;
     st.add(cur, ph, sep_ph);
     D.up.ph = reinterpret_cast<double2*>(ph);
@@ -2546,7 +2448,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     D.dn.ph = D.up.ph;
     D.dn.nboxes = (int)dn.boxes.size();
     D.dn.groups = dn.groups;
-    D.nupw_groups = (int)upw_groups.size();
+    D.npwf = (int)pwf.size();
     st.add(cur, D.form_hoff, form_hoff);
     st.add(cur, D.tables, tables);
     st.add(cur, D.conv, conv);
@@ -2870,12 +2772,6 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
         launches++;
       }
     }
-    if (P.dim == 3 && D.form_pw_n > 0) {
-      size_t sh = ((size_t)FORM_CH * (2 * P.npw + n2) + 8) * 16;
-      CK(smem_limit(k_form3d_pw));
-      k_form3d_pw<<<dim3(D.form_pw_n, nd), 256, sh, st>>>(k, D.form + D.form_hermite_n);
-      launches++;
-    }
     if (P.dim == 2 && D.form_pw_n > 0) {  // the NUFFT scheme's direct form
       const size_t sh = (size_t)FORM_CH * (P.npw + n2) * 16;
       if (sh > 227 * 1024) return cudaErrorNotSupported;
@@ -2887,11 +2783,8 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
     // (b) merge, bottom-up (2D); 3D: the leaves to the cut level
     if (D.up.nboxes > 0) {
       CK(sep_up(k, D.up, D.hbuf, st, launches));
-      if (D.nupw_groups > 0) {
-        CK(sep_add(k, D.mp, D.up.ph, D.upw_groups, D.nupw_groups, D.upw, st));
-        launches++;
-      }
     }
+    if (D.npwf > 0) CK(launch_form3d_pw(k, D.pwf, D.npwf, D.pwf_src, st, launches));
     for (int l = P.nlevels - 1; l >= P.nlevstart; l--) {
       int ng = D.merge_end[l] - D.merge_beg[l];
       if (ng <= 0) continue;
@@ -3108,52 +3001,49 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
 cudaError_t device_plan_box_expansion(const HostPlan& H, DevicePlan& D, int box, double* out, cudaStream_t st) {
   const Tree& t = H.tree;
   const Params& P = H.P;
-  const int lb = t.level[box], lcut = std::max(P.npwlevel, 0);
+  const int lb = t.level[box];
   auto inside = [&](int b) {
     while (t.level[b] > lb) b = t.parent[b];
     return b == box;
   };
-  std::vector<int> boxes, pwb, at(t.nboxes, -1);
+  std::vector<int> boxes, at(t.nboxes, -1);
   for (size_t i = 0; i < D.up_box.size(); i++)
     if (inside(D.up_box[i])) {
       boxes.push_back(D.up_box[i]);
       at[D.up_box[i]] = (int)i;
     }
+  PwFormTask pw{box, 0, 0, 0, 1};
+  std::vector<SrcRange> pw_src;
   for (const FormTask& f : H.form)
-    if (f.route == ROUTE_PW && t.level[f.box] > lcut && inside(f.box)) pwb.push_back(f.box);
+    if (f.route == ROUTE_PW && inside(f.box)) {
+      pw_src.push_back({f.s0, f.n});
+      pw.cnt++;
+    }
   std::vector<int> order;
   for (int l = lb; l <= P.nlevels; l++) order.push_back(H.nlocal[l]);
-  std::vector<SepItem> items, pw;
+  std::vector<SepItem> items;
   sep_order(t, lb, boxes, sep_rank(order), items);
-  sep_order(t, lb, pwb, sep_rank(order), pw);
   std::vector<SepLeaf> leaf;
   for (const SepItem& s : items) leaf.push_back(D.up_leaf[at[s.box]]);
   std::vector<int> slot(t.llast[lb] - t.lfirst[lb] + 1, -1);
-  std::vector<uint8_t> also(slot.size(), 0);
   slot[box - t.lfirst[lb]] = 0;
-  also[box - t.lfirst[lb]] = 1;
   SepLists L;
-  sep_lists(items, leaf, order, slot, also, P.npw, L);
+  sep_lists(items, leaf, order, slot, box - t.lfirst[lb], P.npw, L);
   std::vector<double> ph;
   sep_phases(H, P.nlevels - lb, t.boxsize[lb], ph);
-  std::vector<SepShift> sh;
-  for (const SepItem& s : pw) {
-    const int r0 = (1 << s.d) - 1;
-    sh.push_back({H.mp_slot[s.box], {r0 + s.x[0], r0 + s.x[1], r0 + s.x[2]}});
-  }
-  const std::vector<MergeGroup> g{{0, 0, (int)sh.size()}};
+  const std::vector<PwFormTask> pwt(1, pw);
   const size_t nd = P.nd, per = nd * P.nexp * 16;
   char* mem = nullptr;
   CK(cudaMallocAsync(reinterpret_cast<void**>(&mem),
                      bytes_of(L.leaves) + bytes_of(L.cols) + bytes_of(L.slabs) + bytes_of(L.boxes) +
-                         bytes_of(L.box_slabs) + bytes_of(ph) + bytes_of(sh) + bytes_of(g) + al(L.t1 * nd * 8) +
+                         bytes_of(L.box_slabs) + bytes_of(ph) + bytes_of(pwt) + bytes_of(pw_src) + al(L.t1 * nd * 8) +
                          al(L.t2 * nd * 8) + al(per) + 4096,
                      st));
   auto run = [&]() -> cudaError_t {
     char* cur = mem;
     SepDev S;
-    SepShift* dsh = nullptr;
-    MergeGroup* dg = nullptr;
+    PwFormTask* dpw = nullptr;
+    SrcRange* dsrc = nullptr;
     double* dph = nullptr;
     CK(put(cur, S.leaves, L.leaves, st));
     CK(put(cur, S.cols, L.cols, st));
@@ -3161,8 +3051,8 @@ cudaError_t device_plan_box_expansion(const HostPlan& H, DevicePlan& D, int box,
     CK(put(cur, S.boxes, L.boxes, st));
     CK(put(cur, S.box_slabs, L.box_slabs, st));
     CK(put(cur, dph, ph, st));
-    CK(put(cur, dsh, sh, st));
-    CK(put(cur, dg, g, st));
+    CK(put(cur, dpw, pwt, st));
+    CK(put(cur, dsrc, pw_src, st));
     S.ph = reinterpret_cast<double2*>(dph);
     S.nboxes = 1;
     S.groups = L.groups;
@@ -3170,10 +3060,11 @@ cudaError_t device_plan_box_expansion(const HostPlan& H, DevicePlan& D, int box,
     S.t1 = reinterpret_cast<double*>(cur); cur += al(L.t1 * nd * 8);
     S.t2 = reinterpret_cast<double*>(cur); cur += al(L.t2 * nd * 8);
     KP k = make_kp(D);
+    k.ws = D.h2x;  // row j = 0
     k.mp = reinterpret_cast<double2*>(cur);
     long long launches = 0;
     CK(sep_up(k, S, D.hbuf, st, launches));
-    CK(sep_add(k, D.mp, S.ph, dg, sh.empty() ? 0 : 1, dsh, st));
+    CK(launch_form3d_pw(k, dpw, pw.cnt > 0 ? 1 : 0, dsrc, st, launches));
     CK(cudaMemcpyAsync(out, k.mp, per, cudaMemcpyDeviceToHost, st));
     return cudaStreamSynchronize(st);
   };

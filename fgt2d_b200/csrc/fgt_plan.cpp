@@ -271,9 +271,7 @@ static void build_tasks(HostPlan& H) {
     H.merge.reserve(nb);
     H.split.reserve(nb);
     H.eval.reserve((size_t)nb + (size_t)(P.ns + P.nt) / 2048 + 16);
-    // 3D multipole expansions: the cut level's, and those of the leaves below
-    // it that form theirs directly; the Hermite leaves' blocks go straight to
-    // the cut level (fgt_sep3d.cu)
+    // 3D multipole expansions: the cut level's only (fgt_sep3d.cu, fgt_pw3d.cu)
     auto form_route = [&](int l, int b) {
       if (D == 2) return (int)ROUTE_HERMITE;
       const int p = H.nlocal[l];
@@ -288,7 +286,7 @@ static void build_tasks(HostPlan& H) {
       for (int b = t.lfirst[l]; b <= t.llast[l]; b++) {
         bool leaf = t.nchild[b] == 0;
         if (t.ns(b) > 0 && !(leaf && l == npl) &&
-            (D == 2 || l == nls || (leaf && form_route(l, b) == ROUTE_PW)))
+            (D == 2 || l == nls))
           H.mp_slot[b] = H.nmp++;
         // 3D local expansions: the cut level's
         if (relevant(b) > 0 && !(leaf && l == npl && !iflocal(b)) && (D == 2 || l == nls)) H.loc_slot[b] = H.nloc++;
@@ -451,17 +449,6 @@ static void build_tasks(HostPlan& H) {
     start(H.nmp); for (auto& s : H.merge) see(s.src); ra = c;
     start(H.nmp); for (auto& s : H.merge) see(s.dst); rb = c;
     H.shift_bytes[0] = per * (ra + rb);
-    if (D == 3) {  // the leaves' own expansions and the cut-level expansions they are added to
-      start(H.nmp);
-      for (auto& f : H.form)
-        if (f.route == ROUTE_PW && t.level[f.box] > nls) {
-          see(f.slot);
-          int a = f.box;
-          while (t.level[a] > nls) a = t.parent[a];
-          see(H.mp_slot[a]);
-        }
-      H.shift_bytes[0] = per * c;
-    }
     start(H.nmp); for (auto& m : H.m2l) see(m.self_mp); for (auto& n : H.m2l_nbr) see(n.mp); ra = c;
     start(H.nloc); for (auto& m : H.m2l) see(m.loc); rb = c;
     H.shift_bytes[1] = per * (ra + rb);

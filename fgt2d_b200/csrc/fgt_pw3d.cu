@@ -223,6 +223,152 @@ __global__ void __launch_bounds__(128) k_eval3d_pw(KP k, const EvalTask* __restr
   }
 }
 
+// ------------------------------------------------------------ formation
+//   mp[q][kx] (+)= sum_s X_s(kx) b_s(q),  b_s = q_s Y_s(ky) Z_s(kz), q = (kz, ky)
+// with X_s(kx) = w_kx e^{-i t_kx x_s} (and Y, Z likewise), conjugate at the
+// mirror node: E = sum Re X b and O = sum Im X b over the positive nodes m are
+// two real products with the sources as depth, and node m gets E + i O, its
+// mirror E - i O.  A task is a box with the source ranges whose expansion it
+// takes about the box's centre.  A warp keeps NP column pairs (eight complex
+// columns each) of the box in registers for all its sources; those come 32 at
+// a time, their factors formed once per CTA (a thread per source and
+// dimension, by recurrence) into shared memory, where a B fragment is one
+// complex product of two of them.  With dipoles a source stages three columns
+// (dip3_coef, the factor of one dimension times v_d (-i t dsq)), ten sources
+// at a time.
+template <int MT>
+__host__ __device__ constexpr int pwform_pairs() { return MT == 1 ? 4 : MT == 2 ? 3 : MT == 3 ? 2 : 1; }
+constexpr int PWF_SC = 32;  // source columns per batch
+
+struct PwformDims {
+  int lda, ldy;
+  size_t total;
+  __host__ __device__ PwformDims(int npw, int MT) {
+    lda = PWF_SC + 4;
+    ldy = ((npw + 3) & ~7) + 4;
+    total = (size_t)2 * 8 * MT * lda + (size_t)2 * PWF_SC * (ldy + npw / 2);
+  }
+};
+
+template <int MT>
+__global__ void __launch_bounds__(128) k_form3d_pw(KP k, const PwFormTask* __restrict__ tasks,
+                                                   const SrcRange* __restrict__ ranges, int t0) {
+  constexpr int NP = pwform_pairs<MT>();
+  const PwFormTask T = tasks[blockIdx.x];
+  const int ind = blockIdx.z, npw = k.npw, n2 = k.n2, ncol = n2 * npw, tid = threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5, r = lane >> 2, c = lane & 3;
+  const PwformDims Z(npw, MT);
+  extern __shared__ double sm[];
+  double* A = sm;                                                        // [2][8 MT][lda]: Re, Im X[m][s]
+  double2* Y = reinterpret_cast<double2*>(A + (size_t)2 * 8 * MT * Z.lda);  // [s][ldy]
+  double2* Zf = Y + (size_t)PWF_SC * Z.ldy;                              // [s][n2]
+  const int vc = k.ifdipole ? 3 : 1, chs = PWF_SC / vc;
+  const int pair0 = (blockIdx.y * 4 + warp) * NP;
+  double acc[NP][2][MT][4];
+  int yo[NP][2], zo[NP][2];
+#pragma unroll
+  for (int p = 0; p < NP; p++)
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int q = min(8 * (pair0 + p) + 4 * h + (r >> 1), ncol - 1);
+      zo[p][h] = q / npw;
+      yo[p][h] = q - zo[p][h] * npw;
+#pragma unroll
+      for (int t = 0; t < MT; t++) acc[p][h][t][0] = acc[p][h][t][1] = acc[p][h][t][2] = acc[p][h][t][3] = 0.0;
+    }
+  for (int e = T.beg; e < T.beg + T.cnt; e++) {
+    const SrcRange R = ranges[e];
+    for (int c0 = 0; c0 < R.n; c0 += chs) {
+      const int m = vc * min(chs, R.n - c0), mp = (m + 3) & ~3;
+      __syncthreads();
+      if (tid < 3 * PWF_SC) {
+        const int d = tid / PWF_SC, s = tid - d * PWF_SC;
+        if (s < mp) {
+          double u = 0.0, q = 0.0, dv[3] = {0.0, 0.0, 0.0}, ca = 0.0, cb = 0.0;
+          if (s < m) {
+            const int i = R.s0 + c0 + s / vc;
+            u = (k.src[(size_t)3 * i + d] - k.centers[3 * T.box + d]) * k.dsq;
+            q = src_charge(k, i, ind);
+            if (k.ifdipole) src_dipole<3>(k, i, ind, dv);
+            dip3_coef(s % vc, d, q, dv, ca, cb);
+          }
+          double2 f = cexpi(-k.t1 * u);
+          const double2 ff = cmul(f, f);
+          for (int j = 0; j < n2; j++) {  // positive node j: t = (2j+1) t1 at n2 + j, its mirror at n2 - 1 - j
+            const double w = k.ws[n2 + j], td = (2 * j + 1) * k.t1 * k.dsq * cb;
+            // (ca - i t dsq cb) w e^{-i t u}
+            const double2 g = make_double2(w * fma(ca, f.x, td * f.y), w * fma(ca, f.y, -td * f.x));
+            if (d == 0) {
+              const int mr = j - 8 * t0;
+              if (mr >= 0 && mr < 8 * MT) {
+                A[mr * Z.lda + s] = g.x;
+                A[(8 * MT + mr) * Z.lda + s] = g.y;
+              }
+            } else if (d == 1) {
+              Y[s * Z.ldy + n2 + j] = g;
+              Y[s * Z.ldy + n2 - 1 - j] = make_double2(g.x, -g.y);
+            } else {
+              Zf[s * n2 + n2 - 1 - j] = make_double2(g.x, -g.y);
+            }
+            f = cmul(f, ff);
+          }
+          if (d == 0)
+            for (int mr = max(0, n2 - 8 * t0); mr < 8 * MT; mr++) A[mr * Z.lda + s] = A[(8 * MT + mr) * Z.lda + s] = 0.0;
+        }
+      }
+      __syncthreads();
+      for (int st = 0; st < mp; st += 4) {
+        double a[MT][2];
+#pragma unroll
+        for (int t = 0; t < MT; t++) {
+          a[t][0] = A[(8 * t + r) * Z.lda + st + c];
+          a[t][1] = A[(8 * MT + 8 * t + r) * Z.lda + st + c];
+        }
+        const double2* Ys = Y + (st + c) * Z.ldy;
+        const double2* Zs = Zf + (st + c) * n2;
+#pragma unroll
+        for (int p = 0; p < NP; p++)
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const double2 y = Ys[yo[p][h]], z = Zs[zo[p][h]];
+            const double b = (r & 1) ? fma(y.x, z.y, y.y * z.x) : fma(y.x, z.x, -y.y * z.y);
+#pragma unroll
+            for (int t = 0; t < MT; t++) {
+              dmma_884(acc[p][h][t][0], acc[p][h][t][1], a[t][0], b);
+              dmma_884(acc[p][h][t][2], acc[p][h][t][3], a[t][1], b);
+            }
+          }
+      }
+    }
+  }
+  double2* out = k.mp + ((size_t)T.slot * k.nd + ind) * k.nexp;
+#pragma unroll
+  for (int p = 0; p < NP; p++)
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int q = 8 * (pair0 + p) + 4 * h + c;  // the lane's column
+      if (q < ncol) {
+#pragma unroll
+        for (int t = 0; t < MT; t++) {
+          const int m = 8 * (t0 + t) + r;
+          if (m < n2) {
+            const double* v = acc[p][h][t];
+            double2* op = out + (size_t)q * npw + n2 + m;
+            double2* om = out + (size_t)q * npw + n2 - 1 - m;
+            double2 vp = make_double2(v[0] - v[3], v[1] + v[2]), vm = make_double2(v[0] + v[3], v[1] - v[2]);
+            if (T.add) {
+              const double2 a = *op, b = *om;
+              vp = make_double2(vp.x + a.x, vp.y + a.y);
+              vm = make_double2(vm.x + b.x, vm.y + b.y);
+            }
+            *op = vp;
+            *om = vm;
+          }
+        }
+      }
+    }
+}
+
 }  // namespace
 
 #define CK(x)                               \
@@ -246,6 +392,29 @@ cudaError_t launch_eval3d_pw(const KP& k, const EvalTask* tasks, int ntask, int 
   else if (pgh == 2) PWEV_CASE(2)
   else PWEV_CASE(3)
 #undef PWEV_CASE
+  return cudaGetLastError();
+}
+
+cudaError_t launch_form3d_pw(const KP& k, const PwFormTask* tasks, int ntask, const SrcRange* ranges,
+                             cudaStream_t st, long long& launches) {
+  if (ntask <= 0) return cudaSuccess;
+  const int tiles = (k.n2 + 7) / 8, pairs = (k.n2 * k.npw + 7) / 8;
+  for (int t0 = 0; t0 < tiles; t0 += 4) {
+    switch (std::min(4, tiles - t0)) {
+#define PWF_CASE(MT)                                                                                    \
+  case MT: {                                                                                            \
+    const size_t sh = PwformDims(k.npw, MT).total * 8;                                                  \
+    if (sh > 227 * 1024) return cudaErrorNotSupported;                                                  \
+    CK(smem_limit(k_form3d_pw<MT>));                                                                    \
+    const dim3 g(ntask, (pairs + 4 * pwform_pairs<MT>() - 1) / (4 * pwform_pairs<MT>()), k.nd);         \
+    k_form3d_pw<MT><<<g, 128, sh, st>>>(k, tasks, ranges, t0);                                          \
+    break;                                                                                              \
+  }
+      PWF_CASE(1) PWF_CASE(2) PWF_CASE(3) PWF_CASE(4)
+#undef PWF_CASE
+    }
+    launches++;
+  }
   return cudaGetLastError();
 }
 

@@ -99,7 +99,7 @@ void sep_order(const Tree& t, int lroot, const std::vector<int>& boxes, const st
 }
 
 void sep_lists(const std::vector<SepItem>& items, const std::vector<SepLeaf>& leaf, const std::vector<int>& order,
-               const std::vector<int>& slot, const std::vector<uint8_t>& also, int npw, SepLists& S) {
+               const std::vector<int>& slot, int also, int npw, SepLists& S) {
   const int n = (int)items.size(), n2 = npw / 2, nroot = (int)slot.size();
   S = SepLists();
   S.leaves = leaf;
@@ -133,7 +133,7 @@ void sep_lists(const std::vector<SepItem>& items, const std::vector<SepLeaf>& le
   }
   for (int r = 0; r < nroot; r++) {
     const int m = cnt[r + 1];
-    if (m > 0 || (!also.empty() && also[r])) S.boxes.push_back({(long long)slot[r], cnt[r], m, 0, 0});
+    if (m > 0 || r == also) S.boxes.push_back({(long long)slot[r], cnt[r], m, 0, 0});
     cnt[r + 1] += cnt[r];
   }
   S.box_slabs.resize(slab_root.size());
@@ -758,26 +758,6 @@ __global__ void __launch_bounds__(128) k_eval3d_col(KP k, const ColTask* __restr
   }
 }
 
-// A leaf's expansion times the phases from its centre to the box's, summed
-// over the leaves of a box; one coefficient per thread (memory-bound).
-__global__ void __launch_bounds__(256) k_up_add(KP k, const double2* __restrict__ src,
-                                                const double2* __restrict__ ph,
-                                                const MergeGroup* __restrict__ groups,
-                                                const SepShift* __restrict__ shifts) {
-  const MergeGroup G = groups[blockIdx.x];
-  const int ind = blockIdx.z, npw = k.npw, e = blockIdx.y * blockDim.x + threadIdx.x;
-  if (e >= k.nexp) return;
-  const int kx = e % npw, ky = (e / npw) % npw, kz = e / (npw * npw);
-  double2* dst = k.mp + ((size_t)G.dst * k.nd + ind) * k.nexp + e;
-  double2 a = *dst;
-  for (int t = G.beg; t < G.beg + G.cnt; t++) {
-    const SepShift S = shifts[t];
-    const double2 f = cmul(ph[S.row[0] * npw + kx], cmul(ph[S.row[1] * npw + ky], ph[S.row[2] * npw + kz]));
-    a = cfmac(src[((size_t)S.src * k.nd + ind) * k.nexp + e], f, a);
-  }
-  *dst = a;
-}
-
 // CTAs per node so that the launch fills the SMs several times over
 int split_for(int nodes, int nd, int tiles, int sms) {
   const long long have = (long long)nodes * nd, want = (long long)sms * 12;
@@ -792,13 +772,6 @@ int split_for(int nodes, int nd, int tiles, int sms) {
     cudaError_t e_ = (x);                   \
     if (e_ != cudaSuccess) return e_;       \
   } while (0)
-
-cudaError_t sep_add(const KP& k, const double2* src, const double2* ph, const MergeGroup* groups, int ngroups,
-                    const SepShift* shifts, cudaStream_t st) {
-  if (ngroups <= 0) return cudaSuccess;
-  k_up_add<<<dim3(ngroups, (k.nexp + 255) / 256, k.nd), 256, 0, st>>>(k, src, ph, groups, shifts);
-  return cudaGetLastError();
-}
 
 cudaError_t sep_up(const KP& k, const SepDev& S, const double* hbuf, cudaStream_t st, long long& launches) {
   const int n2 = k.n2, tiles = (n2 + 7) / 8;

@@ -24,21 +24,16 @@ std::vector<int> sep_rank(const std::vector<int>& order_of_depth);
 
 // Columns (equal root, depth, x, y), slabs (equal root, depth, x) and boxes
 // of sorted items with their blocks (leaf.off, leaf.n; the rows are filled
-// here); offsets and sizes per density.  slot: the expansion slots by root; a
-// root in `also` gets a box even without leaves.
+// here); offsets and sizes per density.  slot: the expansion slots by root;
+// the roots with leaves get a box, and root `also` (-1: none) without any.
 void sep_lists(const std::vector<SepItem>& items, const std::vector<SepLeaf>& leaf,
                const std::vector<int>& order_of_depth, const std::vector<int>& slot,
-               const std::vector<uint8_t>& also, int npw, SepLists& S);
+               int also, int npw, SepLists& S);
 
 // Phase rows of depths 0..dmax: row 2^d - 1 + i holds exp(i t_m sh) of the
 // npw nodes, sh the offset of box i of 2^d from its root's centre over
 // sqrt(delta) (bs0: the root's size).
 void sep_phases(const HostPlan& H, int dmax, double bs0, std::vector<double>& ph);
-
-// The leaves' own expansions (pool src) added to the expansions k.mp of the
-// groups' slots (after sep_up).
-cudaError_t sep_add(const KP& k, const double2* src, const double2* ph, const MergeGroup* groups, int ngroups,
-                    const SepShift* shifts, cudaStream_t st);
 
 // Upward: Hermite blocks in hbuf -> the expansions k.mp of the boxes' slots.
 cudaError_t sep_up(const KP& k, const SepDev& S, const double* hbuf, cudaStream_t st, long long& launches);
