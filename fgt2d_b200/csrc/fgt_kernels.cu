@@ -137,13 +137,28 @@ __global__ void k_invperm(const int* __restrict__ perm, int n, int* __restrict__
   if (i < n) inv[perm[i]] = i;
 }
 // Caller order: out row j = in row iperm[j] (dreorderi / dreorderiv,
-// fmmcommon2d.f:29-90), written as a gather so the stores stay coalesced.
-// A sorted row is `stride` doubles; out takes the w doubles from `off`.
-__global__ void k_unsort(const double* __restrict__ in, double* __restrict__ out,
-                         const int* __restrict__ iperm, int n, int stride, int off, int w) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-    const long long p = iperm[j];
-    for (int c = 0; c < w; c++) out[(long long)j * w + c] = in[p * stride + off + c];
+// fmmcommon2d.f:29-90), written as a gather so the stores stay coalesced.  A
+// sorted row holds the potentials, gradients and Hessians of a point (w0, w1,
+// w2 values); each goes to its own array (null: skipped).  A thread per value,
+// so a row's random read is one access for all three (an array at a time, the
+// rows of 3e5 + 1e5 points with Hessians took 27 us, 15 us this way).
+__global__ void __launch_bounds__(256) k_unsort(const double* __restrict__ in, const int* __restrict__ iperm, int n,
+                                                int w0, int w1, int w2, double* __restrict__ o0,
+                                                double* __restrict__ o1, double* __restrict__ o2) {
+  const unsigned w = w0 + w1 + w2;
+  const long long total = (long long)n * w;
+  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
+       t += (long long)gridDim.x * blockDim.x) {
+    const long long j = total < (1LL << 31) ? (unsigned)t / w : t / w;
+    const int e = (int)(t - j * w);
+    const double v = in[(long long)iperm[j] * w + e];
+    if (e < w0) {
+      if (o0) o0[j * w0 + e] = v;
+    } else if (e < w0 + w1) {
+      if (o1) o1[j * w1 + e - w0] = v;
+    } else if (o2) {
+      o2[j * w2 + e - w0 - w1] = v;
+    }
   }
 }
 
@@ -2963,20 +2978,13 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
   const int nh = P.dim == 2 ? 3 : 6;
   auto unsort = [&](const double* in, const int* inv, int n, int nc, double* pot, double* grad,
                     double* hess) {
-    if (pot) {
-      // one density, one component per point: the same random gather
-      if (nd == 1 && nc == 1) k_gather1<<<gb, 256, 0, st>>>(in, inv, n, pot);
-      else k_unsort<<<gb, 256, 0, st>>>(in, pot, inv, n, nc * nd, 0, nd);
-      launches++;
-    }
-    if (nc > 1 && grad) {
-      k_unsort<<<gb, 256, 0, st>>>(in, grad, inv, n, nc * nd, nd, P.dim * nd);
-      launches++;
-    }
-    if (nc > 1 + P.dim && hess) {
-      k_unsort<<<gb, 256, 0, st>>>(in, hess, inv, n, nc * nd, (1 + P.dim) * nd, nh * nd);
-      launches++;
-    }
+    // one density, one component per point: the random gather of the charges
+    if (!pot && (nc == 1 || (!grad && !hess))) return;
+    if (nd == 1 && nc == 1) k_gather1<<<gb, 256, 0, st>>>(in, inv, n, pot);
+    else
+      k_unsort<<<8 * D.sm_count, 256, 0, st>>>(in, inv, n, nd, nc > 1 ? P.dim * nd : 0, nc > 1 + P.dim ? nh * nd : 0,
+                                               pot, grad, hess);
+    launches++;
   };
   if (ph2 && P.ifpgh > 0 && P.ns > 0) unsort(D.psort, D.isrc_inv, P.ns, k.nc_s, outs.pot, outs.grad, outs.hess);
   if (ph2 && P.ifpghtarg > 0 && P.nt > 0)
