@@ -42,8 +42,18 @@ struct MergeGroup {
   int dst, beg, cnt;
 };
 
+// n partial blocks of len doubles per density from off on (2D form)
+struct BlockSum {
+  long long off;
+  int len, n;
+};
+
 struct OrderGroup {
   int p, beg, end;     // tasks [beg, end) of expansion order p
+  // 2D form: the group's source chunks and the leaves of several; a chunk per
+  // warp instead of per CTA
+  int cbeg = 0, cend = 0, sbeg = 0, send = 0;
+  bool warp = false;
   long long tab = -1;  // offset of the group's operand tables in DevicePlan::tables (doubles)
 };
 
@@ -202,6 +212,9 @@ struct DevicePlan {
   std::vector<double> group_flops;      // 2 n P^dim per form group (2D) / chunk group (3D)
   std::vector<double> group_alg_flops;  // 4 n npw^dim per form group (2D) / chunk group (3D)
   // 2D Taylor evaluation (conversion per leaf, then Horner per point chunk)
+  FormTask* form2_chunks = nullptr;  // 2D MMA form: source chunks, the offsets of their blocks, the sums
+  long long* form2_choff = nullptr;
+  BlockSum* form2_sums = nullptr;
   long long* form_hoff = nullptr;  // 2D MMA form: per form task, offset of its Hermite block in hbuf
   ConvTask* conv = nullptr;
   HornerTask* horner = nullptr;

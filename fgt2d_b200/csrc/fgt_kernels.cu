@@ -338,12 +338,19 @@ __device__ __forceinline__ void warp_gemm(const double* A, int lda, const double
 //   column 0: X = x^j,               Y = q y^k + v2 k dsq y^(k-1)
 //   column 1: X = v1 j dsq x^(j-1),  Y = y^k
 // (v = dipstr * n), so a block of 32 columns holds 16 sources.
-template <int NT, bool DIP>
-__global__ void __launch_bounds__(128) k_form2d_mma(KP k, const FormTask* __restrict__ tasks,
+// WARP: a task per warp instead of per CTA, for leaves of few sources (two
+// blocks of columns or less per leaf left half of the CTA's warps idle and the
+// other half waiting for the final sum): 3e5 sources, 19 a leaf, order 21, 69 ->
+// 25 us; 1e5, 52 a leaf, order 30, 47 -> 16; dipoles of two densities, 2e5
+// sources, 26 a leaf, 133 -> 57.
+template <int NT, bool DIP, bool WARP>
+__global__ void __launch_bounds__(128) k_form2d_mma(KP k, const FormTask* __restrict__ tasks, int ntask,
                                                     const long long* __restrict__ hoff,
                                                     double* __restrict__ hbuf) {
   constexpr int PP = 8 * NT, SW = 36, WS = 2 * PP * SW;  // per-warp staging [2][PP][SW]
-  const FormTask T = tasks[blockIdx.x];
+  const int task = WARP ? blockIdx.x * 4 + (threadIdx.x >> 5) : blockIdx.x;
+  if (WARP && task >= ntask) return;  // no CTA-wide barrier on this path
+  const FormTask T = tasks[task];
   const int ind = blockIdx.y;
   const int Pn = T.p + 1;
   extern __shared__ double smf[];
@@ -365,7 +372,7 @@ __global__ void __launch_bounds__(128) k_form2d_mma(KP k, const FormTask* __rest
   // K = 4 steps of the FP64 MMA over the block, alternating two accumulator
   // sets so consecutive steps are independent
   constexpr int SPB = DIP ? 16 : 32;  // sources per 32-column block
-  for (int base = SPB * warp; base < T.n; base += 4 * SPB) {
+  for (int base = WARP ? 0 : SPB * warp; base < T.n; base += WARP ? SPB : 4 * SPB) {
     const int sl = DIP ? lane >> 1 : lane;
     double x = 0.0, y = 0.0, q = 0.0, v[2] = {0.0, 0.0};
     if (base + sl < T.n) {
@@ -431,6 +438,19 @@ __global__ void __launch_bounds__(128) k_form2d_mma(KP k, const FormTask* __rest
   // tile (a, b) holds H'[j = 8a + lane/4][k = 8b + 2 (lane%4) + i]; each warp
   // writes its sum into its own staging area, then the four are added and
   // the leaf's P x P block is stored row-major (x power j, y power k)
+  double* hb = hbuf + hoff[task] + (size_t)ind * Pn * Pn;
+  if (WARP) {
+#pragma unroll
+    for (int a = 0; a < NT; a++)
+#pragma unroll
+      for (int b = 0; b < NT; b++)
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          const int j = 8 * a + j0, kk = 8 * b + 2 * tl + i;
+          if (j < Pn && kk < Pn) hb[j * Pn + kk] = c[0][a][b][i] + c[1][a][b][i];
+        }
+    return;
+  }
   double* part = X;
 #pragma unroll
   for (int a = 0; a < NT; a++)
@@ -440,10 +460,36 @@ __global__ void __launch_bounds__(128) k_form2d_mma(KP k, const FormTask* __rest
       for (int i = 0; i < 2; i++)
         part[(8 * a + j0) + PP * (8 * b + 2 * tl + i)] = c[0][a][b][i] + c[1][a][b][i];
   __syncthreads();
-  double* hb = hbuf + hoff[blockIdx.x] + (size_t)ind * Pn * Pn;
   for (int e = threadIdx.x; e < Pn * Pn; e += 128) {
     const int j = e / Pn, kk = e - j * Pn, f = j + PP * kk;
     hb[e] = stg[f] + stg[WS + f] + stg[2 * WS + f] + stg[3 * WS + f];
+  }
+}
+
+// A leaf's partial Hermite blocks (one after the other, n of them) added into
+// the first: 32 coefficients per CTA, eight threads each with every eighth
+// block (a thread alone waits for hundreds of loads in a row: 37 us instead of
+// 5 at 586 blocks), added in a fixed order.
+__global__ void __launch_bounds__(256) k_sum_blocks2d(const BlockSum* __restrict__ sums, int nd,
+                                                      double* __restrict__ hbuf) {
+  __shared__ double part[8][32];
+  const BlockSum S = sums[blockIdx.x];
+  const int len = S.len * nd, x = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double* h = hbuf + S.off;
+  for (int e0 = 32 * blockIdx.y; e0 < len; e0 += 32 * gridDim.y) {
+    double a = 0.0;
+    if (e0 + x < len) {
+#pragma unroll 4
+      for (int b = w; b < S.n; b += 8) a += h[(size_t)b * len + e0 + x];
+    }
+    part[w][x] = a;
+    __syncthreads();
+    if (w == 0 && e0 + x < len) {
+#pragma unroll
+      for (int i = 1; i < 8; i++) a += part[i][x];
+      h[e0 + x] = a;
+    }
+    __syncthreads();
   }
 }
 
@@ -2331,15 +2377,49 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   // 3D: source chunks and their partial Hermite blocks
   std::vector<FormChunk> fchunks;
   size_t hbuf_doubles = 0;
-  // 2D: Hermite blocks of the MMA form (orders <= 31), nd P^2 doubles per leaf
-  std::vector<long long> form_hoff;
+  // 2D: Hermite blocks of the MMA form (orders <= 31), nd P^2 doubles per
+  // source chunk of a leaf, a leaf's chunks one after the other: about eight
+  // chunks per SM of at least 512 sources, whole passes of the kernels' four
+  // warps (four leaves of 75000 sources in four CTAs took 0.76 ms of a 0.80 ms
+  // execute, 0.02 of 0.08 cut up)
+  std::vector<long long> form_hoff, choff;
+  std::vector<FormTask> chunks2;
+  std::vector<BlockSum> sums2;
   if (P.dim == 2 && !P.all_direct) {
-    form_hoff.assign(form.size(), 0);
+    long long nsrc = 0;
+    int most = 0;
     for (int t = 0; t < D.form_hermite_n; t++) {
-      const long long Pn = form[t].p + 1;
-      if (Pn > 32) continue;
-      form_hoff[t] = (long long)hbuf_doubles;
-      hbuf_doubles += (size_t)(P.nd * Pn * Pn);
+      nsrc += form[t].n;
+      most = std::max(most, form[t].n);
+    }
+    const int step = (int)std::max<long long>(512, (nsrc / (8LL * D.sm_count) + 255) / 256 * 256);
+    const bool cut = most > step;  // otherwise the leaves are the chunks
+    form_hoff.assign(form.size(), 0);
+    for (OrderGroup& G : D.form_groups) {
+      const long long Pn = G.p + 1;
+      G.cbeg = cut ? (int)chunks2.size() : G.beg;
+      G.sbeg = (int)sums2.size();
+      long long n = 0;
+      for (int t = G.beg; t < G.end && Pn <= 32; t++) {
+        const FormTask& f = form[t];
+        const size_t len = (size_t)(P.nd * Pn * Pn);
+        const int nc = cut ? std::max(1, (f.n + step - 1) / step) : 1;
+        form_hoff[t] = (long long)hbuf_doubles;
+        if (nc > 1) sums2.push_back({form_hoff[t], (int)(Pn * Pn), nc});
+        for (int c = 0; c < nc && cut; c++) {
+          FormTask g = f;
+          g.s0 = f.s0 + c * step;
+          g.n = std::min(step, f.n - c * step);
+          chunks2.push_back(g);
+          choff.push_back(form_hoff[t] + (long long)(c * len));
+        }
+        hbuf_doubles += nc * len;
+        n += f.n;
+      }
+      G.cend = cut ? (int)chunks2.size() : G.end;
+      G.send = (int)sums2.size();
+      // leaves of about two blocks of source columns or less: a warp each
+      G.warp = n * (P.ifdipole ? 2 : 1) <= 80LL * (G.cend - G.cbeg);
     }
   }
   if (P.dim == 3 && !P.all_direct) {
@@ -2393,7 +2473,8 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
                  bytes_of(up.box_slabs) + bytes_of(dn.cols) + bytes_of(dn.leaves) + bytes_of(dn.slabs) +
                  bytes_of(dn.boxes) + bytes_of(dn.box_slabs) + bytes_of(ctask) + bytes_of(pwf) + bytes_of(pwf_src) + bytes_of(sep_ph) +
                  al(std::max(up.t1, dn.t1) * nd * 8) + al(std::max(up.t2, dn.t2) * nd * 8) +
-                 al(hbuf_doubles * 8) + bytes_of(form_hoff) + bytes_of(tables) + bytes_of(conv) + bytes_of(horner) +
+                 al(hbuf_doubles * 8) + bytes_of(form_hoff) + bytes_of(choff) +
+                 bytes_of(chunks2) + bytes_of(sums2) + bytes_of(tables) + bytes_of(conv) + bytes_of(horner) +
                  al(lo_doubles * 8) + 4096;
   D.bytes = total;
   if (size_only) {
@@ -2465,6 +2546,13 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     D.dn.groups = dn.groups;
     D.npwf = (int)pwf.size();
     st.add(cur, D.form_hoff, form_hoff);
+    st.add(cur, D.form2_choff, choff);
+    st.add(cur, D.form2_chunks, chunks2);
+    st.add(cur, D.form2_sums, sums2);
+    if (chunks2.empty()) {
+      D.form2_chunks = D.form;
+      D.form2_choff = D.form_hoff;
+    }
     st.add(cur, D.tables, tables);
     st.add(cur, D.conv, conv);
     st.add(cur, D.horner, horner);
@@ -2681,23 +2769,27 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
       for (size_t gi = 0; gi < D.form_groups.size(); gi++) {
         const OrderGroup& G = D.form_groups[gi];
         const int Pn = G.p + 1;
-        dim3 g(G.end - G.beg, nd);
+        // the group's leaves and their source chunks (with the partial blocks)
+        const int ntk = G.cend - G.cbeg;
         const FormTask* tk = D.form + G.beg;
+        const FormTask* ck = D.form2_chunks + G.cbeg;
+        const long long* choff = D.form2_choff + G.cbeg;
         const bool dom = times && (int)gi == D.dom_form_group;
         if (dom) cudaEventRecord(dev0, st);
         if (Pn <= 32) {
-#define FORM_MMA(NT)                                                                              \
-  do {                                                                                            \
-    const size_t sh = (size_t)4 * 2 * (8 * NT) * 36 * 8;                                          \
-    if (P.ifdipole) {                                                                             \
-      CK(smem_limit(k_form2d_mma<NT, true>)); \
-      k_form2d_mma<NT, true><<<g, 128, sh, st>>>(k, tk, D.form_hoff + G.beg, D.hbuf);             \
-    } else {                                                                                      \
-      CK(smem_limit(k_form2d_mma<NT, false>)); \
-      k_form2d_mma<NT, false><<<g, 128, sh, st>>>(k, tk, D.form_hoff + G.beg, D.hbuf);            \
-    }                                                                                             \
+#define FORM_MMA(NT)                                                                                         \
+  do {                                                                                                       \
+    const size_t sh = (size_t)4 * 2 * (8 * NT) * 36 * 8;                                                     \
+    const dim3 g(G.warp ? (ntk + 3) / 4 : ntk, nd);                                                          \
+    auto run = [&](auto kernel) -> cudaError_t {                                                             \
+      CK(smem_limit(kernel));                                                                                \
+      kernel<<<g, 128, sh, st>>>(k, ck, ntk, choff, D.hbuf);                                                 \
+      return cudaSuccess;                                                                                    \
+    };                                                                                                       \
+    if (P.ifdipole) CK(G.warp ? run(k_form2d_mma<NT, true, true>) : run(k_form2d_mma<NT, true, false>));     \
+    else CK(G.warp ? run(k_form2d_mma<NT, false, true>) : run(k_form2d_mma<NT, false, false>));              \
   } while (0)
-          if (mixed_ac && Pn <= 16) CK(launch_form2d_f32(k, tk, G.end - G.beg, nd, D.form_hoff + G.beg, D.hbuf, Pn, st));
+          if (mixed_ac && Pn <= 16) CK(launch_form2d_f32(k, ck, ntk, nd, choff, D.hbuf, Pn, st));
           else if (Pn <= 8) FORM_MMA(1);
           else if (Pn <= 16) FORM_MMA(2);
           else if (Pn <= 24) FORM_MMA(3);
@@ -2709,6 +2801,10 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
             else snprintf(times->dom_name, sizeof(times->dom_name), "k_form2d_mma<%d>", (Pn + 7) / 8);
             times->dom_flops = D.group_flops[gi];
             times->dom_alg_flops = D.group_alg_flops[gi];
+          }
+          if (G.send > G.sbeg) {
+            k_sum_blocks2d<<<dim3(G.send - G.sbeg, std::min(32, (Pn * Pn * nd + 31) / 32)), 256, 0, st>>>(D.form2_sums + G.sbeg, nd, D.hbuf);
+            launches++;
           }
           const int nt = G.end - G.beg;
           const H2pwDims Z(Pn, P.npw);
@@ -2733,7 +2829,7 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
           const int ch = Pp <= 32 ? 128 : 64;
           size_t sh = ((size_t)2 * ch * Pp + 4096 + 2 * (size_t)Pn * n2) * 8;
           CK(smem_limit(k_form2d));
-          k_form2d<<<g, 256, sh, st>>>(k, tk, D.isq, ch);
+          k_form2d<<<dim3(G.end - G.beg, nd), 256, sh, st>>>(k, tk, D.isq, ch);
         }
         launches++;
       }

@@ -1,5 +1,10 @@
-"""2D calls on either side of 3000 points, whose trees are built on the host
-and on the device, against the oracle.
+"""The 2D form and evaluation kernels against the oracle, where their tiles
+and the rules of their dispatch end: orders on either side of the tiles of
+eight powers and of 32 (eps 1e-3 to 1e-15), leaves of a few sources (a warp
+each) and of hundreds (a CTA each), leaves cut into several partial blocks,
+evaluation at one point, at remainders of sixteen and with derivatives, several
+densities, dipoles; and calls on either side of 3000 points, whose trees are
+built on the host and on the device.
 
 FP64, other orders of summation than the oracle's: relative l2 <= 1e-12 for
 the potential, a digit more per derivative, as for every FP64 route.
@@ -12,6 +17,17 @@ pytestmark = pytest.mark.gpu
 TOLS = (("pot", 1e-12), ("pottarg", 1e-12), ("gradtarg", 1e-11), ("hesstarg", 1e-10))
 
 CASES = [  # kind, ns, nt, delta, eps, nd, dipoles, pgh
+    ("uniform", 4000, 1, 2e-3, 1e-3, 1, 0, 3),
+    ("uniform", 4001, 5003, 2e-3, 1e-6, 1, 0, 2),
+    ("uniform", 4001, 3001, 2e-3, 1e-6, 2, 1, 1),
+    ("uniform", 6007, 2017, 2e-3, 1e-9, 1, 0, 3),
+    ("uniform", 6007, 9001, 2e-3, 1e-12, 1, 1, 2),
+    ("uniform", 5000, 1777, 2e-3, 1e-15, 1, 0, 3),
+    ("cluster", 8009, 3005, 2e-3, 1e-6, 1, 0, 1),
+    ("cluster", 8009, 3005, 2e-3, 1e-12, 2, 0, 2),
+    ("uniform", 9001, 2003, 0.1, 1e-6, 2, 0, 2),  # leaves of several partial blocks
+    ("uniform", 9001, 2003, 0.1, 1e-9, 1, 1, 1),
+    ("uniform", 2048, 513, 0.1, 1e-6, 1, 0, 1),   # a leaf of exactly one block
     ("uniform", 2000, 1000, 2e-3, 1e-6, 1, 0, 1),  # 3000 points: host tree
     ("uniform", 2000, 1001, 2e-3, 1e-6, 1, 0, 1),
 ]
