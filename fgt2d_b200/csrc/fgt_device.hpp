@@ -50,6 +50,7 @@ struct BlockSum {
 
 struct OrderGroup {
   int p, beg, end;     // tasks [beg, end) of expansion order p
+  int per = 0;         // 2D evaluation by k_eval2d_mma: warps per task, 0: Horner
   // 2D form: the group's source chunks and the leaves of several; a chunk per
   // warp instead of per CTA
   int cbeg = 0, cend = 0, sbeg = 0, send = 0;

@@ -933,6 +933,131 @@ __global__ void __launch_bounds__(128) k_pw2taylor2d(KP k, const ConvTask* __res
                   });
 }
 
+// ------------------------------------------------------------ (c) eval, 2D Taylor blocks
+// FP64 evaluation of a leaf's Taylor block lo[b][a] (P rows of E = P rounded up
+// to even, y^b x^a; g2dlevalp/g/h_vec, g2drouts.f:847-1085), orders 24 to 39:
+//   pot = sum_b y^b C[b],  C[b] = sum_a x^a lo[b][a],
+// the inner sum as a product on the FP64 tensor cores, eight points as rows
+// (x^a and, for derivatives, a x^(a-1) and a (a-1) x^(a-2): PGH row sets on
+// the same columns), K = a in KS steps of four, the columns b; the lane then
+// folds its two columns of its point into the sums with y^b and its
+// derivatives.  A warp owns 8 MT points and keeps their row sets in
+// registers, the block comes from global memory (L1) straight into the
+// fragments; a task has one, two or four warps by its points.
+// MMA and FMA have the same FP64 rate and the MMA pads P to 4 and 8; what it
+// saves against Horner (below, a thread per point) is the idle threads of
+// leaves of a few dozen points and the block's passes through shared memory.
+// Both, potentials (with gradients; with Hessians), 1e5 uniform points, eps
+// 1e-9, order 30-33, 52 points a task: 21 (41; 70) us here, 35 (65; 98) Horner;
+// order 24, 35 points: 45 and 56; but order 18-21, 52 points: 49 (102; 147)
+// and 41 (84; 125); 26 points: 38 (85; 112) and 38 (65; 94).  So Horner keeps
+// the orders below 24, and the tasks of more than 72 points on average
+// (order 24, 67 points: 78 and 82; order 19, 237 points: 45 and 25).
+template <int KS, int PGH>
+__global__ void __launch_bounds__(128) k_eval2d_mma(KP k, const HornerTask* __restrict__ tasks, int ntask, int per,
+                                                    const double* __restrict__ lo_all) {
+  constexpr int NC = ncomp<2, PGH>(), MT = PGH == 1 ? 2 : 1;
+  const int w = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (w >= ntask * per) return;  // no CTA-wide barrier in this kernel
+  const int warp = w & (per - 1);
+  const HornerTask T = tasks[w / per];
+  const int ind = blockIdx.y, Pn = T.p + 1, E = (Pn + 1) & ~1;
+  const int lane = threadIdx.x & 31, r = lane >> 2, c = lane & 3;
+  const double* lo = lo_all + T.off + (size_t)ind * Pn * E;
+  const double2* pts = reinterpret_cast<const double2*>(T.set ? k.trg : k.src);
+  double* out = T.set ? k.pottarg : k.pot;
+  const int nc = T.set ? k.nc_t : k.nc_s;
+  const double cx = k.centers[2 * T.box], cy = k.centers[2 * T.box + 1];
+  for (int p0 = 8 * MT * warp; p0 < T.n; p0 += 8 * MT * per) {
+    double x[PGH][MT][KS];  // the lane's row entries a = 4 s + c
+    double yb[MT], ym[MT], yl[MT], y8[MT], y1[MT];
+#pragma unroll
+    for (int i = 0; i < MT; i++) {
+      const double2 p = pts[T.i0 + min(p0 + 8 * i + r, T.n - 1)];
+      const double u = (p.x - cx) * k.dsq, v = (p.y - cy) * k.dsq;
+      const double u2 = u * u, u4 = u2 * u2;
+      double q0 = c == 0 ? 1.0 : c == 1 ? u : c == 2 ? u2 : u2 * u;  // u^a
+      double q1 = c == 0 ? 0.0 : c == 1 ? 1.0 : c == 2 ? u : u2;     // u^(a-1)
+      double q2 = c < 2 ? 0.0 : c == 2 ? 1.0 : u;                    // u^(a-2)
+#pragma unroll
+      for (int s = 0; s < KS; s++) {
+        const int a = 4 * s + c;
+        const bool in = a < Pn;
+        x[0][i][s] = in ? q0 : 0.0;
+        if (PGH >= 2) x[PGH >= 2 ? 1 : 0][i][s] = in ? a * q1 : 0.0;
+        if (PGH >= 3) x[PGH >= 3 ? 2 : 0][i][s] = in ? a * (a - 1) * q2 : 0.0;
+        q1 = s == 0 && c == 0 ? u2 * u : q1 * u4;
+        q2 = s == 0 && c < 2 ? (c == 0 ? u2 : u2 * u) : q2 * u4;
+        q0 *= u4;
+      }
+      // the columns b = 8 nt + 2 c and b + 1: y^b, y^(b-1), y^(b-2)
+      const double v2 = v * v, v4 = v2 * v2;
+      y1[i] = v;
+      y8[i] = v4 * v4;
+      yb[i] = c == 0 ? 1.0 : c == 1 ? v2 : c == 2 ? v4 : v4 * v2;
+      ym[i] = c == 0 ? 0.0 : c == 1 ? v : c == 2 ? v2 * v : v4 * v;
+      yl[i] = c == 0 ? 0.0 : c == 1 ? 1.0 : c == 2 ? v2 : v4;
+    }
+    double sum[MT][NC];
+#pragma unroll
+    for (int i = 0; i < MT; i++)
+#pragma unroll
+      for (int v = 0; v < NC; v++) sum[i][v] = 0.0;
+    for (int nt = 0; 8 * nt < Pn; nt++) {
+      const double* row = lo + min(8 * nt + r, Pn - 1) * E;
+      double b[KS];
+#pragma unroll
+      for (int s = 0; s < KS; s++) b[s] = row[min(4 * s + c, E - 1)];
+      double acc[PGH][MT][2];
+#pragma unroll
+      for (int g = 0; g < PGH; g++)
+#pragma unroll
+        for (int i = 0; i < MT; i++) acc[g][i][0] = acc[g][i][1] = 0.0;
+#pragma unroll
+      for (int s = 0; s < KS; s++)
+#pragma unroll
+        for (int g = 0; g < PGH; g++)
+#pragma unroll
+          for (int i = 0; i < MT; i++) dmma_884(acc[g][i][0], acc[g][i][1], x[g][i][s], b[s]);
+      const int bb = 8 * nt + 2 * c;
+      const double f0 = bb < Pn ? 1.0 : 0.0, f1 = bb + 1 < Pn ? 1.0 : 0.0;  // columns past the block
+#pragma unroll
+      for (int i = 0; i < MT; i++) {
+        const double w0 = f0 * yb[i], w1 = f1 * yb[i] * y1[i];
+        sum[i][0] = fma(acc[0][i][0], w0, fma(acc[0][i][1], w1, sum[i][0]));
+        if constexpr (PGH >= 2) {
+          const double d0 = f0 * bb * ym[i], d1 = f1 * (bb + 1) * yb[i];
+          sum[i][1] = fma(acc[1][i][0], w0, fma(acc[1][i][1], w1, sum[i][1]));
+          sum[i][2] = fma(acc[0][i][0], d0, fma(acc[0][i][1], d1, sum[i][2]));
+          if constexpr (PGH >= 3) {
+            const double h0 = f0 * bb * (bb - 1) * yl[i], h1 = f1 * (bb + 1) * bb * ym[i];
+            sum[i][3] = fma(acc[2][i][0], w0, fma(acc[2][i][1], w1, sum[i][3]));
+            sum[i][4] = fma(acc[1][i][0], d0, fma(acc[1][i][1], d1, sum[i][4]));
+            sum[i][5] = fma(acc[0][i][0], h0, fma(acc[0][i][1], h1, sum[i][5]));
+          }
+        }
+        // the next eight columns
+        const double v = y1[i], v2 = v * v, v4 = v2 * v2;
+        yl[i] = nt == 0 && c == 0 ? v4 * v2 : yl[i] * y8[i];
+        ym[i] = nt == 0 && c == 0 ? v4 * v2 * v : ym[i] * y8[i];
+        yb[i] *= y8[i];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < MT; i++) {
+      const int pt = p0 + 8 * i + r;
+#pragma unroll
+      for (int v = 0; v < NC; v++) {
+        double a = sum[i][v];
+        a += __shfl_xor_sync(FULL_MASK, a, 1);
+        a += __shfl_xor_sync(FULL_MASK, a, 2);
+        if ((v & 3) == c && pt < T.n && v < nc)
+          out[((size_t)(T.i0 + pt) * nc + v) * k.nd + ind] += a * (v == 0 ? 1.0 : v < 3 ? k.dsq : k.dsq * k.dsq);
+      }
+    }
+  }
+}
+
 // k_eval2d_horner: one CTA (128 threads) per chunk of <= 256 points of an
 // evaluation leaf; the leaf's Taylor block (P rows of E = 2 NP2) is staged in
 // shared memory and each thread evaluates two points (g2dlevalp_vec,
@@ -2219,6 +2344,13 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
       size_t u = t;
       while (u < horner.size() && horner[u].p == horner[t].p) u++;
       D.horner_groups.push_back({horner[t].p, (int)t, (int)u});
+      // k_eval2d_mma where it is the faster one (its comment), with as many
+      // warps per task as have points
+      long long n = 0;
+      for (size_t i = t; i < u; i++) n += horner[i].n;
+      const long long cnt = u - t, tile = std::max(P.ifpgh, P.ifpghtarg) <= 1 ? 16 : 8;
+      if (P.dim == 2 && horner[t].p >= 24 && horner[t].p < 40 && n <= 72 * cnt)
+        D.horner_groups.back().per = n > 3 * tile * cnt ? 4 : n > tile * cnt ? 2 : 1;
       t = u;
     }
   }
@@ -2951,6 +3083,22 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
         if (sh > 227 * 1024) return cudaErrorNotSupported;
         if (mixed_ac && pgh == 1 && np2 <= 16) {
           CK(launch_eval2d_horner_f32(k, tk, G.end - G.beg, nd, Pn, D.lo, st));
+          launches++;
+          continue;
+        }
+        if (G.per > 0) {
+          const dim3 gw((unsigned)(((long long)(G.end - G.beg) * G.per + 3) / 4), nd);
+          const cudaError_t e2 = with_pgh(pgh, [&](auto PG) -> cudaError_t {
+            switch ((Pn + 3) / 4) {
+#define EVAL2_CASE(N) \
+  case N: k_eval2d_mma<N, decltype(PG)::value><<<gw, 128, 0, st>>>(k, tk, G.end - G.beg, G.per, D.lo); break;
+              EVAL2_CASE(7) EVAL2_CASE(8) EVAL2_CASE(9) EVAL2_CASE(10)
+#undef EVAL2_CASE
+              default: return cudaErrorNotSupported;
+            }
+            return cudaSuccess;
+          });
+          CK(e2);
           launches++;
           continue;
         }
