@@ -461,15 +461,16 @@ def ours_arm(args, w, rank, world, local_rank):
     else:
         roof = {"bound": "tensor", "kernel": None, "achieved": None, "peak": tf, "unit": "TFLOP/s",
                 "frac": None, "traffic": None, "note": "no tensor-core launch in this plan"}
-    sb = info["shift_bytes"]
-    t_b = (stage.get("merge", 0) + stage.get("m2l", 0) + stage.get("split", 0)) / 1e3
+    # mp -> loc; merge and split are parts of the transforms around it
+    sb = info["shift_bytes"][1]
+    t_b = stage.get("m2l", 0) / 1e3
     roof_b = None
     if t_b > 0:
-        gbs = (sb[0] + sb[1] + sb[2]) / t_b / 1e9
-        roof_b = {"bound": "hbm", "stage": "shifts (merge + mp->loc + split)", "achieved": gbs,
+        gbs = sb / t_b / 1e9
+        roof_b = {"bound": "hbm", "stage": "shifts (mp->loc)", "achieved": gbs,
                   "peak": hbm, "unit": "GB/s", "frac": gbs / hbm,
-                  "work": f"{sb[0] + sb[1] + sb[2]:.4g} bytes per step: 16 B per complex "
-                          f"coefficient, each distinct expansion read or written once per stage",
+                  "work": f"{sb:.4g} bytes per step: 16 B per complex "
+                          f"coefficient, each distinct expansion read or written once",
                   "stage_ms": t_b * 1e3}
     stage_rates = {
         "form_tflops_algorithmic": info["form_flops"] / (stage["form"] / 1e3) / 1e12 if stage.get("form") else None,

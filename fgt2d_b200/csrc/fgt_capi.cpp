@@ -864,7 +864,7 @@ int fgt_plan_mp_unpack(fgt_plan* p, int peer, const double* d_buf, void* stream)
 struct fgt_host_shard {
   HostPlan H;
   ShardInfo S;
-  long long nform = 0, neval = 0, ndir = 0, nm2l = 0, nmerge = 0, nsplit = 0;
+  long long nform = 0, neval = 0, ndir = 0, nm2l = 0;
   int nmp = 0;
 };
 
@@ -888,8 +888,6 @@ int fgt_host_shard_create(int dim, int nd, double delta, double eps, int ns, con
   h->neval = (long long)h->H.eval.size();
   h->ndir = (long long)h->H.dir.size();
   h->nm2l = (long long)h->H.m2l.size();
-  h->nmerge = (long long)h->H.merge.size();
-  h->nsplit = (long long)h->H.split.size();
   h->nmp = h->H.nmp;
   *out = h.release();
   return FGT_OK;
@@ -915,7 +913,7 @@ int fgt_host_shard_stats(fgt_host_shard* h, long long* out8) {
   out8[3] = h->neval;
   out8[4] = h->ndir;
   out8[5] = h->nm2l;
-  out8[6] = h->nmerge + h->nsplit;
+  out8[6] = 0;  // merge and split run with formation and evaluation
   out8[7] = h->nmp;
   return FGT_OK;
 }
@@ -1012,7 +1010,7 @@ int fgt_plan_expansion(fgt_plan* p, int which, int box, double* out) {
   const std::vector<int>& slots = which == 0 ? H.mp_slot : H.loc_slot;
   if ((int)slots.size() <= box) return FGT_ERR_BADARG;
   const int lcut = std::max(H.P.npwlevel, 0);
-  if (which == 0 && slots[box] < 0 && H.P.dim == 3 && H.P.scheme == 0 && H.tree.level[box] > lcut &&
+  if (which == 0 && slots[box] < 0 && H.P.scheme == 0 && H.tree.level[box] > lcut &&
       H.tree.ns(box) > 0) {
     // below the cut level the transform forms none: formed here on request
     CKS(cudaSetDevice(p->ctx->device));
@@ -1021,7 +1019,7 @@ int fgt_plan_expansion(fgt_plan* p, int which, int box, double* out) {
     return FGT_OK;
   }
   int slot = slots[box], a = box;
-  if (which == 1 && slot < 0 && H.P.dim == 3 && H.P.scheme == 0 && H.tree.level[box] > lcut &&
+  if (which == 1 && slot < 0 && H.P.scheme == 0 && H.tree.level[box] > lcut &&
       ((H.P.ifpghtarg > 0 ? H.tree.nt(box) : 0) + (H.P.ifpgh > 0 ? H.tree.ns(box) : 0)) > 0) {
     while (H.tree.level[a] > lcut) a = H.tree.parent[a];
     slot = slots[a];
@@ -1036,9 +1034,10 @@ int fgt_plan_expansion(fgt_plan* p, int which, int box, double* out) {
   if (a != box) {  // below the cut level: the cut-level box's expansion about this box's centre
     const int npw = H.P.npw;
     for (size_t e = 0; e < per; e++) {
-      const int i = (int)(e % H.P.nexp), m[3] = {i % npw, (i / npw) % npw, i / (npw * npw)};
+      const int i = (int)(e % H.P.nexp), n2 = npw / 2;
+      const int m[3] = {H.P.dim == 2 ? i % n2 : i % npw, H.P.dim == 2 ? i / n2 : (i / npw) % npw, i / (npw * npw)};
       double th = 0.0;
-      for (int d = 0; d < 3; d++) th += H.ts[m[d]] * (H.tree.c(box, d) - H.tree.c(a, d)) * H.P.dsq;
+      for (int d = 0; d < H.P.dim; d++) th += H.ts[m[d]] * (H.tree.c(box, d) - H.tree.c(a, d)) * H.P.dsq;
       const double c = std::cos(th), s = std::sin(th), re = out[2 * e], im = out[2 * e + 1];
       out[2 * e] = re * c - im * s;
       out[2 * e + 1] = re * s + im * c;
@@ -1064,7 +1063,6 @@ int fgt_plan_get_info(const fgt_plan* p, fgt_plan_info* o) {
   o->large_delta = P.large_delta; o->all_direct = P.all_direct;
   o->kernel_launches = p->last_launches;
   for (int i = 0; i < 3; i++) o->shift_bytes[i] = p->H.shift_bytes[i];
-  if (p->have_device) o->shift_bytes[2] = p->D.split_bytes;  // the splits that run
   o->form_route_flops = p->H.form_route_flops;
   o->eval_route_flops = p->H.eval_route_flops;
   double npwd = std::pow((double)P.npw, P.dim);

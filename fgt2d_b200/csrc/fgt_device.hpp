@@ -38,10 +38,6 @@ struct Outputs {
   double* hesstarg = nullptr;
 };
 
-struct MergeGroup {
-  int dst, beg, cnt;
-};
-
 // n partial blocks of len doubles per density from off on (2D form)
 struct BlockSum {
   long long off;
@@ -51,27 +47,10 @@ struct BlockSum {
 struct OrderGroup {
   int p, beg, end;     // tasks [beg, end) of expansion order p
   int per = 0;         // 2D evaluation by k_eval2d_mma: warps per task, 0: Horner
-  // 2D form: the group's source chunks and the leaves of several; a chunk per
-  // warp instead of per CTA
-  int cbeg = 0, cend = 0, sbeg = 0, send = 0;
-  bool warp = false;
-  long long tab = -1;  // offset of the group's operand tables in DevicePlan::tables (doubles)
+  bool warp = false;   // 2D form: a leaf (or chunk) per warp instead of per CTA
 };
 
-// 2D Taylor evaluation in two kernels: one plane wave -> Taylor conversion per
-// evaluation leaf (its block of nd * P * E doubles at `off`, E = P rounded up
-// to even), then point chunks of <= 256 that read the block.
-struct ConvTask {
-  int slot, p;
-  long long off;
-  // split fused into the conversion: slot is then the cut-level ancestor's
-  // local expansion and sh the leaf centre minus the ancestor's, scaled by
-  // 1/sqrt(delta); the conversion multiplies the ancestor's coefficients by
-  // exp(i t . sh) (3D: t_m3 sh0 + t_m2 sh1 + t_m1 sh2; 2D: t_j2 sh0 + t_J
-  // sh1), the product of the split factors from the ancestor to the leaf
-  int fused = 0;
-  double sh[3] = {0, 0, 0};
-};
+// Taylor evaluation: a chunk of <= 256 points and its leaf's block.
 struct HornerTask {
   int box, set, i0, n, p;
   long long off;
@@ -82,13 +61,14 @@ struct HornerTask {
 struct SepItem {
   int box, root;  // box; root as its number among the boxes of the root level
   int d, x[3];    // depth below the root, place in the root's grid
+  int num;        // number in the list that was sorted
 };
 // 3D plane-wave form: a box's expansion (slot) about its centre from the
 // source ranges [beg, beg + cnt), added (add) to what sep_up put there.
 struct PwFormTask {
   int box, slot, beg, cnt, add;
 };
-// Separable 3D transforms (fgt_sep3d.hpp).  A leaf's block with its z phase
+// Separable transforms (fgt_sep.hpp).  A leaf's block with its z phase
 // row; a node of the levels above: a column (x, y) of leaves, a slab (x) of
 // columns, a cut-level box of slabs.
 struct SepLeaf {
@@ -100,7 +80,8 @@ struct SepNode {
   int beg, cnt, row, p;  // children [beg, beg + cnt), own phase row, order + 1
 };
 struct SepGroup {  // columns and slabs of one order
-  int p, cbeg, cend, sbeg, send;
+  int p, cbeg, cend, sbeg, send;  // columns, slabs
+  int lbeg, lend;                 // leaves
   bool blocks = true;  // downward: the leaves get Taylor blocks
 };
 // Evaluation of a leaf's points [i0, i0 + n) of a set from its column: the
@@ -112,14 +93,17 @@ struct ColTask {
 struct SepLists {
   std::vector<SepLeaf> leaves;
   std::vector<SepNode> cols, slabs, boxes;
-  std::vector<int> box_slabs;  // the boxes' slabs (a box has slabs of several orders)
+  std::vector<int> box_kids;  // the boxes' slabs (2D: columns), of several orders
   std::vector<SepGroup> groups;
+  std::vector<int> col_slot, leaf_col;  // 2D: the columns' boxes' slots, the leaves' columns
   size_t t1 = 0, t2 = 0;  // doubles per density of all columns and all slabs
 };
 struct SepDev {
   SepLeaf* leaves = nullptr;
   SepNode *cols = nullptr, *slabs = nullptr, *boxes = nullptr;
-  int* box_slabs = nullptr;
+  int* box_kids = nullptr;
+  int *col_slot = nullptr, *leaf_col = nullptr;
+  const double* hx = nullptr;  // Hermite -> plane wave table of the blocks' normalisation
   int nboxes = 0;
   std::vector<SepGroup> groups;
   double2* ph = nullptr;
@@ -128,7 +112,7 @@ struct SepDev {
 };
 
 struct StageTimes {
-  float ms[8];  // gather, form, merge, m2l, split, eval, direct, scatter
+  float ms[8];  // gather, form, merge, m2l, split (none), eval, direct, scatter
   // the dominant tensor-core launch: the Hermite-block MMA kernel of the
   // form group with the most sources (k_form2d_mma / k_form3d_mma)
   float dom_ms = 0;
@@ -147,21 +131,15 @@ struct DevicePlan {
   double* centers = nullptr;
   double* h2x = nullptr;
   double* x2l = nullptr;
-  double2* wms = nullptr;
   double2* wsh = nullptr;
   int* isrc = nullptr;       // sorted position -> caller index
   int* itarg = nullptr;
   int* isrc_inv = nullptr;   // caller index -> sorted position
   int* itarg_inv = nullptr;
   double* isq = nullptr;     // 1/sqrt(j), j = 0..ntermmax+1
-  double* cfac = nullptr;    // 1/sqrt(j!), j < 32
+  double* hx = nullptr;      // 2D: h2x of the unnormalised Hermite blocks (HostPlan::hx)
   FormTask* form = nullptr;
   int nform = 0;
-  std::vector<int> merge_beg, merge_end;  // host copies of group ranges per level
-  MergeGroup* mgroups = nullptr;
-  ShiftTask* merge = nullptr;
-  ShiftTask* split = nullptr;
-  std::vector<int> split_beg, split_end;
   M2LTask* m2l = nullptr;
   int nm2l = 0;
   M2LNbr* m2l_nbr = nullptr;
@@ -190,7 +168,7 @@ struct DevicePlan {
   // 3D Hermite form in two kernels: source chunks and their partial blocks
   FormChunk* fchunks = nullptr;
   int nfchunks = 0;
-  int form3_chunk = 4096;    // most sources of a chunk
+  int form_chunk = 1 << 30;  // most sources of a chunk
   double* hbuf = nullptr;    // partial Hermite blocks
   // 3D plane-wave scheme: the leaves' Hermite blocks to the cut level's expansions
   SepDev up, dn;  // dn: the cut level's local expansions to the leaves' evaluation
@@ -212,24 +190,17 @@ struct DevicePlan {
   int dom_fchunk_group = -1;      // 3D: chunk group with the most sources
   std::vector<double> group_flops;      // 2 n P^dim per form group (2D) / chunk group (3D)
   std::vector<double> group_alg_flops;  // 4 n npw^dim per form group (2D) / chunk group (3D)
-  // 2D Taylor evaluation (conversion per leaf, then Horner per point chunk)
-  FormTask* form2_chunks = nullptr;  // 2D MMA form: source chunks, the offsets of their blocks, the sums
-  long long* form2_choff = nullptr;
-  BlockSum* form2_sums = nullptr;
+  // Taylor evaluation from the leaves' blocks
+  BlockSum* form2_sums = nullptr;  // 2D: leaves of several partial blocks
+  int form2_nsums = 0;
   long long* form_hoff = nullptr;  // 2D MMA form: per form task, offset of its Hermite block in hbuf
-  ConvTask* conv = nullptr;
   HornerTask* horner = nullptr;
   double* lo = nullptr;
-  double* tables = nullptr;  // padded operand tables of the 2D MMA transforms
-  std::vector<OrderGroup> conv_groups, horner_groups;
+  std::vector<OrderGroup> horner_groups;
   int sm_count = 148;
   // statistics copied from the host plan
   long long direct_pairs = 0, form_sources = 0, eval_points = 0;
   long long launches = 0;
-  // algorithmic bytes of the split tasks that run (the others are fused into
-  // the conversion): each distinct expansion read or written once, 16 B per
-  // complex coefficient
-  long long split_bytes = 0;
 };
 
 // Makes freed stream-ordered allocations stay in the current device's default
@@ -276,14 +247,14 @@ cudaError_t device_plan_set_points(DevicePlan& D, const double* src, const doubl
 // Runs charge gather -> stages -> scatter on `stream`.  Device pointers in
 // the caller's order: charge (ns, nd) and the outputs.
 // times (optional) receives per-stage milliseconds (synchronises).
-// phase: 0 everything; 1 through the merge (every mp expansion up to the
+// phase: 0 everything; 1 through the merge (the mp expansions of the
 // cut level), 2 from mp -> loc on (the caller may replace mp expansions of
 // the cut level between the two).
 cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& out,
                                 int precision, cudaStream_t stream, StageTimes* times, int phase = 0);
 
 // The multipole expansion of a box below the cut level after the last
-// execute (3D plane-wave scheme, which forms none there): its leaves' blocks
+// execute (plane-wave scheme, which forms none there): its leaves' blocks
 // and expansions taken to the box instead of the cut level, nd * nexp complex
 // in out (host); synchronous on st.
 cudaError_t device_plan_box_expansion(const HostPlan& H, DevicePlan& D, int box, double* out, cudaStream_t st);

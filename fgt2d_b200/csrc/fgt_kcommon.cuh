@@ -19,7 +19,6 @@ struct KP {
   const double* h2x;
   const double* x2l;
   const double* ws;
-  const double2* wms;
   const double2* wsh;
   double2* mp;
   double2* loc;
@@ -367,7 +366,7 @@ cudaError_t launch_direct_mixed_x2(const KP& k, const DirTask* tasks, int ntask,
                                    const SrcRange* ranges, float amax, cudaStream_t st);
 // 2D Taylor evaluation of potentials in FP32 (Pn <= 32) for the point chunks
 // of one order group, added into the sorted outputs; the group's Taylor
-// blocks must have been written in FP32 pairs (k_pw2taylor2d with f32).
+// blocks must have been written in FP32 pairs (k_down2d_x with f32).
 cudaError_t launch_eval2d_horner_f32(const KP& k, const HornerTask* tasks, int ntask, int nd, int Pn,
                                      const double* lo, cudaStream_t st);
 

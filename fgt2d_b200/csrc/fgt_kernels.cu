@@ -5,8 +5,9 @@
 //                g3dformhc_vec + g3dh2pw_real_vec), or the direct tensor-product
 //                exponential sum (g3dformpwc_vec) where the reference uses it.
 // (b) shifts   : diagonal plane-wave translations (g2dshiftpw_vec,
-//                g2dcopypwexp_vec): merge up to the cut level, mp -> loc over the
-//                plane-wave list, split down to the leaves.  HBM-bound.
+//                g2dcopypwexp_vec): mp -> loc over the plane-wave list here; merge
+//                up to the cut level and split down to the leaves are parts of
+//                the transforms (fgt_sep.cu, fgt_sep3d.cu).
 // (c) eval     : per leaf, plane wave -> Taylor (g2dpw2local_real_vec) and
 //                Taylor evaluation (g2dlevalp_vec), or direct plane-wave
 //                evaluation (g2dpwevalp_vec) on the levels the reference picks.
@@ -19,6 +20,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <exception>
 #include <cstdio>
 #include <cstdlib>
 #include <cmath>
@@ -29,7 +31,7 @@
 
 #include "fgt_device.hpp"
 #include "fgt_kcommon.cuh"
-#include "fgt_sep3d.hpp"
+#include "fgt_sep.hpp"
 
 namespace fgtb {
 
@@ -53,59 +55,28 @@ __global__ void k_gather_pts(const double* __restrict__ x, const double* __restr
       for (int c = 0; c < nd; c++) qs[(long long)i * nd + c] = q[p * nd + c];
   }
 }
-// Diagonal translation tables from their 1D factors (merge_split_pw_matrices,
-// pw_translation_matrices): merge row (l nch + jc) for parents at level l,
-// entry e = prod_d (child jc on the + side along d ? conj(v) : v) with
-// v = ww[node_d(e)][nlevels - l]; mp->loc row s = (ox+1) + 3 (oy+1) [+ 9 (oz+1)],
-// entry prod_d (o_d = 0 ? 1 : o_d > 0 ? w1 : conj(w1)).  Products are formed
-// left to right without contraction, (ac - bd, ad + bc).
+// mp -> loc translation rows from their 1D factors (pw_translation_matrices):
+// row s = (ox+1) + 3 (oy+1) [+ 9 (oz+1)], entry e = prod_d (o_d = 0 ? 1 :
+// o_d > 0 ? w1 : conj(w1)) at e's node along d.  Products are formed left to
+// right without contraction, (ac - bd, ad + bc).
 __device__ __forceinline__ double2 cmul_rn(double2 a, double2 b) {
   return make_double2(__dsub_rn(__dmul_rn(a.x, b.x), __dmul_rn(a.y, b.y)),
                       __dadd_rn(__dmul_rn(a.x, b.y), __dmul_rn(a.y, b.x)));
 }
-__global__ void k_shift_tables(int dim, int npw, int nexp, int nlevels, int lstart, int nms, long long nm,
-                               const double2* __restrict__ ww, const double2* __restrict__ w1,
-                               double2* __restrict__ wms, double2* __restrict__ wsh) {
-  const int nch = 1 << dim, n2 = npw / 2, ns3 = dim == 2 ? 9 : 27;
-  const long long total = nm + (long long)ns3 * nexp;  // nm: merge entries (0: no merge rows)
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const bool merge = i < nm;
-    const long long r = merge ? i / nexp : (i - nm) / nexp;
-    const int e = (int)((merge ? i : i - nm) % nexp);
-    int node[3];
-    if (dim == 2) {
-      node[0] = e % n2;
-      node[1] = e / n2;
-    } else {
-      node[0] = e % npw;
-      node[1] = (e / npw) % npw;
-      node[2] = e / (npw * npw);
-    }
+__global__ void k_shift_tables(int dim, int npw, int nexp, const double2* __restrict__ w1,
+                               double2* __restrict__ wsh) {
+  const int n2 = npw / 2, total = (dim == 2 ? 9 : 27) * nexp;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const int s = i / nexp, e = i - s * nexp;
+    const int node[3] = {dim == 2 ? e % n2 : e % npw, dim == 2 ? e / n2 : (e / npw) % npw, e / (npw * npw)};
+    const int o[3] = {s % 3 - 1, (s / 3) % 3 - 1, s / 9 - 1};
     double2 f = make_double2(1.0, 0.0);
-    if (merge) {
-      const int l = (int)(r / nch), jc = (int)(r % nch);
-      if (l < lstart || l > nlevels - 1) {
-        wms[i] = make_double2(0.0, 0.0);
-        continue;
-      }
-      const int klev = nlevels - l;
-      for (int d = 0; d < dim; d++) {
-        double2 v = ww[node[d] * (nms + 1) + klev];
-        if ((jc >> d) & 1) v.y = -v.y;
-        f = cmul_rn(f, v);
-      }
-      wms[i] = f;
-    } else {
-      const int s = (int)r;
-      const int o[3] = {s % 3 - 1, (s / 3) % 3 - 1, s / 9 - 1};
-      for (int d = 0; d < dim; d++) {
-        double2 v = o[d] == 0 ? make_double2(1.0, 0.0) : w1[node[d]];
-        if (o[d] < 0) v.y = -v.y;
-        f = cmul_rn(f, v);
-      }
-      wsh[i - nm] = f;
+    for (int d = 0; d < dim; d++) {
+      double2 v = o[d] == 0 ? make_double2(1.0, 0.0) : w1[node[d]];
+      if (o[d] < 0) v.y = -v.y;
+      f = cmul_rn(f, v);
     }
+    wsh[i] = f;
   }
 }
 
@@ -162,129 +133,10 @@ __global__ void __launch_bounds__(256) k_unsort(const double* __restrict__ in, c
   }
 }
 
-// ------------------------------------------------------------ (a) form, 2D
-// One CTA (256 threads) per (leaf, density).
-//   H[j + Pp k] = sum_i q_i x_i^j y_i^k / sqrt(j! k!)      (g2dformhc_vec)
-// is a small (P x n) * (n x P) product: the rows x^j/sqrt(j!) and
-// q y^k/sqrt(k!) of a chunk of sources are built in shared memory with the
-// 1/sqrt(j) table, each thread keeps a 4x4 register tile of H and the chunk's
-// sources are split over G thread groups (split-K), reduced at the end.  Then
-// the two 1D Hermite -> plane-wave passes (g2dh2pw_real_vec,
-// g2drouts.f:1276-1326) run in shared memory.
-// With dipoles each source contributes two columns (as k_form2d_mma):
-// (hx, q hy + v2 dhy) and (v1 dhx, hy), dh_j = sqrt(j) dsq h_(j-1).
-__global__ void __launch_bounds__(256) k_form2d(KP k, const FormTask* __restrict__ tasks,
-                                                const double* __restrict__ isq, int ch) {
-  const FormTask T = tasks[blockIdx.x];
-  const int ind = blockIdx.y;
-  const int Pn = T.p + 1, n2 = k.n2, npw = k.npw;
-  const int tpd = (Pn + 3) >> 2, Pp = tpd * 4, ntiles = tpd * tpd;
-  const int G = 256 / ntiles;
-  extern __shared__ double sm[];
-  double* xs = sm;                     // [ch][Pp]
-  double* ys = xs + ch * Pp;           // [ch][Pp]
-  double* part = ys + ch * Pp;         // [G][Pp*Pp]
-  double* H = part;                    // reduced H overwrites group 0
-  double2* px = reinterpret_cast<double2*>(part + G * Pp * Pp);  // [Pn][n2]
-  const double cx = k.centers[2 * T.box], cy = k.centers[2 * T.box + 1];
-  const int tid = threadIdx.x, tile = tid % ntiles, g = tid / ntiles;
-  const int jb = (tile % tpd) * 4, kb = (tile / tpd) * 4;
-  double acc[4][4];
-#pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int b = 0; b < 4; b++) acc[a][b] = 0.0;
-  const int vc = k.ifdipole ? 2 : 1;     // columns per source
-  const int chs = k.ifdipole ? ch / 2 : ch;  // sources per chunk
-  for (int s0c = 0; s0c < T.n; s0c += chs) {
-    const int ms = min(chs, T.n - s0c), m = vc * ms;
-    for (int r = tid; r < 2 * m; r += 256) {
-      const int t = r >> 1, kind = r & 1;
-      const int i = T.s0 + s0c + t / vc;
-      const double v = kind == 0 ? (k.src[2 * i] - cx) * k.dsq : (k.src[2 * i + 1] - cy) * k.dsq;
-      double* row = (kind ? ys : xs) + t * Pp;
-      if (!k.ifdipole) {
-        double w = kind == 0 ? 1.0 : k.chg[(size_t)i * k.nd + ind];
-        row[0] = w;
-        for (int j = 1; j < Pn; j++) {
-          w = w * v * isq[j];
-          row[j] = w;
-        }
-      } else {
-        // a h_j + b dh_j for the column's factor
-        double dv[2];
-        src_dipole<2>(k, i, ind, dv);
-        const bool c1 = t & 1;
-        double a, b;
-        if (kind == 0) { a = c1 ? 0.0 : 1.0; b = c1 ? dv[0] : 0.0; }
-        else { a = c1 ? 1.0 : src_charge(k, i, ind); b = c1 ? 0.0 : dv[1]; }
-        double h = 1.0;
-        row[0] = a;
-        for (int j = 1; j < Pn; j++) {
-          const double dh = j * isq[j] * k.dsq * h;
-          h = h * v * isq[j];
-          row[j] = fma(a, h, b * dh);
-        }
-      }
-      for (int j = Pn; j < Pp; j++) row[j] = 0.0;
-    }
-    __syncthreads();
-    if (g < G) {
-      for (int t = g; t < m; t += G) {
-        const double2 x01 = *reinterpret_cast<const double2*>(xs + t * Pp + jb);
-        const double2 x23 = *reinterpret_cast<const double2*>(xs + t * Pp + jb + 2);
-        const double2 y01 = *reinterpret_cast<const double2*>(ys + t * Pp + kb);
-        const double2 y23 = *reinterpret_cast<const double2*>(ys + t * Pp + kb + 2);
-        const double xa[4] = {x01.x, x01.y, x23.x, x23.y};
-        const double ya[4] = {y01.x, y01.y, y23.x, y23.y};
-#pragma unroll
-        for (int b = 0; b < 4; b++)
-#pragma unroll
-          for (int a = 0; a < 4; a++) acc[a][b] = fma(ya[b], xa[a], acc[a][b]);
-      }
-    }
-    __syncthreads();
-  }
-  if (g < G) {
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-      for (int b = 0; b < 4; b++) part[g * Pp * Pp + (jb + a) + Pp * (kb + b)] = acc[a][b];
-  }
-  __syncthreads();
-  for (int e = tid; e < Pp * Pp; e += 256) {
-    double v = 0.0;
-    for (int q = 0; q < G; q++) v += part[q * Pp * Pp + e];
-    H[e] = v;  // element e is read and written by this thread only
-  }
-  __syncthreads();
-  // x pass: px[j2][k2] = sum_j1 h2x(j1,k2) i^j1 H[j1][j2], k2 over the positive half
-  for (int idx = tid; idx < Pn * n2; idx += 256) {
-    const int j2 = idx / n2, k2 = idx - j2 * n2;
-    double2 a = make_double2(0.0, 0.0);
-    for (int j1 = 0; j1 < Pn; j1++) addrot(a, k.h2x[j1 * npw + k2] * H[j1 + Pp * j2], j1);
-    px[idx] = a;
-  }
-  __syncthreads();
-  // y pass over the full node set, written to the leaf's multipole slot
-  double2* out = k.mp + ((size_t)T.slot * k.nd + ind) * k.nexp;
-  for (int e = tid; e < k.nexp; e += 256) {
-    const int k1 = e / n2, k2 = e - k1 * n2;
-    double2 a = make_double2(0.0, 0.0);
-    for (int j2 = 0; j2 < Pn; j2++) {
-      const double h = k.h2x[j2 * npw + k1];
-      const double2 z = rot(px[j2 * n2 + k2], j2);
-      a.x = fma(h, z.x, a.x);
-      a.y = fma(h, z.y, a.y);
-    }
-    out[e] = a;
-  }
-}
-
 // ------------------------------------------------------------ (a) form, 2D on FP64 MMA
 // Hermite block of a leaf, H[j][k] = sum_t q_t x_t^j y_t^k (g2dformhc_vec,
-// g2drouts.f:100-168, without the 1/sqrt(j! k!) factors, which k_h2pw2d
-// folds into its tables), on the FP64 tensor cores: mma.sync.m8n8k4.f64 takes
+// g2drouts.f:100-168, without the 1/sqrt(j! k!) factors, which the
+// Hermite -> plane-wave table carries), on the FP64 tensor cores: mma.sync.m8n8k4.f64 takes
 // four sources per step (K = 4) into NT x NT tiles of 8 x 8 (P <= 8 NT).
 // Fragment layout (PTX ISA, m8n8k4 .f64): A element (row = lane/4, col =
 // lane%4), B element (row = lane%4, col = lane/4), accumulator pair (row =
@@ -294,44 +146,6 @@ __global__ void __launch_bounds__(256) k_form2d(KP k, const FormTask* __restrict
 // each fragment load is two conflict-free wavefronts.  Four warps split the
 // leaf's sources; their tiles are summed in shared memory and the P x P block
 // goes to the leaf's slot of the Hermite buffer.
-// Leading dimensions (in doubles) of zero-padded shared-memory operands of
-// the m8n8k4 FP64 MMA: an A operand with K columns is stored with a stride of
-// 4 (mod 16) and a B operand with N columns with a stride of 8 (mod 16), so
-// the eight rows (A) or four rows (B) that a fragment load touches fall in
-// distinct bank pairs: two wavefronts per load, the minimum for 256 bytes.
-__host__ __device__ __forceinline__ int mma_lda(int K) { return K <= 4 ? 4 : ((K + 11) & ~15) + 4; }
-__host__ __device__ __forceinline__ int mma_ldb(int N) { return ((N + 7) & ~15) + 8; }
-
-// Warp-level C = A B (+ C2 = A2 B2 on the same tiles when TWO) on the FP64
-// MMA with row-major, zero-padded operands in shared memory: A is
-// (8 Mt) x (4 Ks), B is (4 Ks) x (8 Nt).  out(i, j, c0, c1 [, d0, d1])
-// receives row i, columns j and j + 1 (j even) of C (and C2).  Two
-// accumulator sets alternate over the K steps.
-template <bool TWO, class Out>
-__device__ __forceinline__ void warp_gemm(const double* A, int lda, const double* B, int ldb,
-                                          const double* A2, const double* B2, int Mt, int Nt, int Ks,
-                                          Out out) {
-  const int lane = threadIdx.x & 31, r = lane >> 2, c = lane & 3;
-  for (int mt = 0; mt < Mt; mt++)
-  for (int nt = 0; nt < Nt; nt++) {
-    const int ao = (8 * mt + r) * lda + c, bo = c * ldb + 8 * nt + r;
-    double d0 = 0.0, d1 = 0.0, e0 = 0.0, e1 = 0.0;
-    double f0 = 0.0, f1 = 0.0, g0 = 0.0, g1 = 0.0;
-    for (int ks = 0; ks < Ks; ks++) {
-      const int ak = ao + 4 * ks, bk = bo + 4 * ks * ldb;
-      if (ks & 1) {
-        dmma_884(e0, e1, A[ak], B[bk]);
-        if (TWO) dmma_884(g0, g1, A2[ak], B2[bk]);
-      } else {
-        dmma_884(d0, d1, A[ak], B[bk]);
-        if (TWO) dmma_884(f0, f1, A2[ak], B2[bk]);
-      }
-    }
-    if (TWO) out(8 * mt + r, 8 * nt + 2 * c, d0 + e0, d1 + e1, f0 + g0, f1 + g1);
-    else out(8 * mt + r, 8 * nt + 2 * c, d0 + e0, d1 + e1, 0.0, 0.0);
-  }
-}
-
 // With dipoles (DIP) the source derivative enters as a second column per
 // source (g2dformhd_vec / g2dformhcd_vec, g2drouts.f:173-338; in the
 // unnormalised powers here d/dX x^j = j dsq x^(j-1)):
@@ -353,6 +167,8 @@ __global__ void __launch_bounds__(128) k_form2d_mma(KP k, const FormTask* __rest
   const FormTask T = tasks[task];
   const int ind = blockIdx.y;
   const int Pn = T.p + 1;
+  // the CTA's PP x PP block of H (orders beyond PP take several)
+  const int nb = (Pn + PP - 1) / PP, jb = PP * (blockIdx.z / nb), kb = PP * (blockIdx.z % nb);
   extern __shared__ double smf[];
   double* stg = smf;                                          // [4][WS]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -389,6 +205,8 @@ __global__ void __launch_bounds__(128) k_form2d_mma(KP k, const FormTask* __rest
     }
     if (!DIP) {
       double xp = 1.0, yp = q;
+      for (int j = 0; j < jb; j++) xp *= x;
+      for (int j = 0; j < kb; j++) yp *= y;
 #pragma unroll
       for (int j = 0; j < PP; j++) {
         X[j * SW + lane] = xp;
@@ -402,6 +220,14 @@ __global__ void __launch_bounds__(128) k_form2d_mma(KP k, const FormTask* __rest
       const double ax = c1 ? 0.0 : 1.0, bx = c1 ? v[0] * k.dsq : 0.0;
       const double ay = c1 ? 1.0 : q, by = c1 ? 0.0 : v[1] * k.dsq;
       double xp = 1.0, yp = 1.0, xm = 0.0, ym = 0.0;  // x^j, j x^(j-1)
+      for (int j = 0; j < jb; j++) {
+        xm = fma(xm, x, xp);
+        xp *= x;
+      }
+      for (int j = 0; j < kb; j++) {
+        ym = fma(ym, y, yp);
+        yp *= y;
+      }
 #pragma unroll
       for (int j = 0; j < PP; j++) {
         X[j * SW + lane] = fma(ax, xp, bx * xm);
@@ -446,7 +272,7 @@ __global__ void __launch_bounds__(128) k_form2d_mma(KP k, const FormTask* __rest
       for (int b = 0; b < NT; b++)
 #pragma unroll
         for (int i = 0; i < 2; i++) {
-          const int j = 8 * a + j0, kk = 8 * b + 2 * tl + i;
+          const int j = jb + 8 * a + j0, kk = kb + 8 * b + 2 * tl + i;
           if (j < Pn && kk < Pn) hb[j * Pn + kk] = c[0][a][b][i] + c[1][a][b][i];
         }
     return;
@@ -460,9 +286,10 @@ __global__ void __launch_bounds__(128) k_form2d_mma(KP k, const FormTask* __rest
       for (int i = 0; i < 2; i++)
         part[(8 * a + j0) + PP * (8 * b + 2 * tl + i)] = c[0][a][b][i] + c[1][a][b][i];
   __syncthreads();
-  for (int e = threadIdx.x; e < Pn * Pn; e += 128) {
-    const int j = e / Pn, kk = e - j * Pn, f = j + PP * kk;
-    hb[e] = stg[f] + stg[WS + f] + stg[2 * WS + f] + stg[3 * WS + f];
+  const int nj = min(PP, Pn - jb), nk = min(PP, Pn - kb);
+  for (int e = threadIdx.x; e < nj * nk; e += 128) {
+    const int j = e / nk, kk = e - j * nk, f = j + PP * kk;
+    hb[(jb + j) * Pn + kb + kk] = stg[f] + stg[WS + f] + stg[2 * WS + f] + stg[3 * WS + f];
   }
 }
 
@@ -493,133 +320,8 @@ __global__ void __launch_bounds__(256) k_sum_blocks2d(const BlockSum* __restrict
   }
 }
 
-// Hermite -> plane wave (g2dh2pw_real_vec, g2drouts.f:1242-1329), one warp
-// per leaf, the two 1D passes on the leaf's P x P block H[j1][j2] as FP64 MMA
-// products:
-//   px[k2][j2]  = sum_j1 i^j1 hx[j1][k2] H[j1][j2]           (pass 1)
-//   pw[k1][k2]  = sum_j2 hx[j2][k1] (i^j2 px[k2][j2])         (pass 2)
-// with hx[j][k] = h2x[j][k] / sqrt(j!).  Pass 1 splits i^j1 by parity: the even
-// rows of H give Re px and the odd rows Im px, through the table signed by
-// (j mod 4 < 2 ? + : -), so it is two real products on the same tiles.  Pass 2
-// is one real product with B[j2][2 k2 + c] = component c of i^j2 px[k2][j2].
-// The tables are shared by the CTA's warps (all leaves of a launch have one
-// order); operands are zero padded to whole tiles.
-struct H2pwDims {
-  int Pn, Ph, Mp, Kp, Np, Kq, Nq, Mq;  // see k_h2pw2d
-  int ldS, ldH, ldP, ldU;
-  int tab, warp;  // doubles: CTA tables, per-warp area
-  __host__ __device__ H2pwDims(int P, int npw) {
-    const int n2 = npw / 2;
-    Pn = P;
-    Ph = (Pn + 1) / 2;
-    Mp = (n2 + 7) & ~7;     // pass 1 rows: k2
-    Kp = (Ph + 3) & ~3;     // pass 1 depth: j1 of one parity
-    Np = (Pn + 7) & ~7;     // pass 1 columns: j2 (also the rows of the pass 2 operand)
-    Kq = (Pn + 3) & ~3;     // pass 2 depth: j2
-    Nq = (npw + 7) & ~7;    // pass 2 columns: (k2, re/im)
-    Mq = (npw + 7) & ~7;    // pass 2 rows: k1
-    ldS = mma_lda(Kp);
-    ldH = mma_ldb(Np);
-    ldP = mma_ldb(Nq > 2 * Mp ? Nq : 2 * Mp);
-    ldU = mma_lda(Kq);
-    tab = 2 * Mp * ldS + Mq * ldU;
-    warp = Np * ldP;
-  }
-};
-
-// Tables of k_h2pw2d for order P (built on the host, copied to shared
-// memory): HSe[k2][i] = s(2i) hx[2i][k2], HSo[k2][i] = s(2i+1) hx[2i+1][k2]
-// with s(j) = (j mod 4 < 2 ? 1 : -1), and HUT[k1][j2] = hx[j2][k1].
-void build_h2pw_table(const HostPlan& H, int Pn, std::vector<double>& out) {
-  const int npw = H.P.npw, n2 = npw / 2;
-  const H2pwDims Z(Pn, npw);
-  std::vector<double> cf(Pn + 1, 1.0);
-  for (int j = 1; j <= Pn; j++) cf[j] = cf[j - 1] / std::sqrt((double)j);
-  auto hx = [&](int j, int kk) { return H.h2x[(size_t)j * npw + kk] * cf[j]; };
-  const size_t base = out.size();
-  out.resize(base + Z.tab, 0.0);
-  double* HSe = out.data() + base;
-  double* HSo = HSe + Z.Mp * Z.ldS;
-  double* HUT = HSo + Z.Mp * Z.ldS;
-  for (int k2 = 0; k2 < n2; k2++)
-    for (int i = 0; 2 * i < Pn; i++) {
-      const int je = 2 * i, jo = 2 * i + 1;
-      HSe[k2 * Z.ldS + i] = (je & 2) ? -hx(je, k2) : hx(je, k2);
-      if (jo < Pn) HSo[k2 * Z.ldS + i] = (jo & 2) ? -hx(jo, k2) : hx(jo, k2);
-    }
-  for (int k1 = 0; k1 < npw; k1++)
-    for (int j2 = 0; j2 < Pn; j2++) HUT[k1 * Z.ldU + j2] = hx(j2, k1);
-}
-
-template <int KQ>  // pass 2 depth in steps of 4: KQ = ceil(P / 4)
-__global__ void __launch_bounds__(128) k_h2pw2d(KP k, const FormTask* __restrict__ tasks, int ntask,
-                                                const long long* __restrict__ hoff,
-                                                const double* __restrict__ hbuf,
-                                                const double* __restrict__ tab) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int t = blockIdx.x * 4 + warp;
-  if (t >= ntask) return;  // no CTA-wide barrier in this kernel
-  const FormTask T = tasks[t];
-  const int npw = k.npw, n2 = k.n2;
-  const H2pwDims Z(T.p + 1, npw);
-  const int Pn = Z.Pn;
-  extern __shared__ double sh2[];
-  double* PB = sh2 + warp * Z.Np * Z.ldP;    // [Np][ldP]
-  const double* HSe = tab;                   // [Mp][ldS], read through L1
-  const double* HSo = HSe + Z.Mp * Z.ldS;    // [Mp][ldS]
-  const double* HUT = HSo + Z.Mp * Z.ldS;    // [Mq][ldU]
-  const int ind = blockIdx.y;
-  const double* H = hbuf + hoff[t] + (size_t)ind * Pn * Pn;
-  const int r = lane >> 2, c = lane & 3;
-  // pass 1: (Re, Im) px[k2][j2] on the same tiles, B operands He[i][j2] =
-  // H[2i][j2] and Ho[i][j2] = H[2i+1][j2] read straight from the block;
-  // PB[j2][2 k2 + c] = i^j2 px (padded rows and columns come out zero)
-  for (int nt = 0; nt < Z.Np / 8; nt++) {
-    const int j2b = 8 * nt + r;
-    for (int mt = 0; mt < Z.Mp / 8; mt++) {
-      const double* ae = HSe + (8 * mt + r) * Z.ldS + c;
-      const double* ao = HSo + (8 * mt + r) * Z.ldS + c;
-      double re0 = 0.0, re1 = 0.0, im0 = 0.0, im1 = 0.0;
-      for (int ks = 0; ks < Z.Kp / 4; ks++) {
-        const int i = 4 * ks + c, je = 2 * i, jo = 2 * i + 1;
-        const double be = (je < Pn && j2b < Pn) ? __ldg(H + je * Pn + j2b) : 0.0;
-        const double bo = (jo < Pn && j2b < Pn) ? __ldg(H + jo * Pn + j2b) : 0.0;
-        dmma_884(re0, re1, __ldg(ae + 4 * ks), be);
-        dmma_884(im0, im1, __ldg(ao + 4 * ks), bo);
-      }
-      const int k2 = 8 * mt + r, j2 = 8 * nt + 2 * c;
-      const double2 z0 = rot_bf(make_double2(re0, im0), j2);
-      const double2 z1 = rot_bf(make_double2(re1, im1), j2 + 1);
-      PB[j2 * Z.ldP + 2 * k2] = z0.x;
-      PB[j2 * Z.ldP + 2 * k2 + 1] = z0.y;
-      PB[(j2 + 1) * Z.ldP + 2 * k2] = z1.x;
-      PB[(j2 + 1) * Z.ldP + 2 * k2 + 1] = z1.y;
-    }
-  }
-  __syncwarp();
-  // pass 2: pw[k1][k2] = sum_j2 hx[j2][k1] PB[j2][(k2, c)]
-  double2* out = k.mp + ((size_t)T.slot * k.nd + ind) * k.nexp;
-  for (int mt = 0; mt < Z.Mq / 8; mt++) {
-    const double* ap = HUT + (8 * mt + r) * Z.ldU + c;
-    double a[KQ];
-#pragma unroll
-    for (int ks = 0; ks < KQ; ks++) a[ks] = __ldg(ap + 4 * ks);
-    for (int nt = 0; nt < Z.Nq / 8; nt++) {
-      const double* bp = PB + c * Z.ldP + 8 * nt + r;
-      double d0 = 0.0, d1 = 0.0, e0 = 0.0, e1 = 0.0;
-#pragma unroll
-      for (int ks = 0; ks < KQ; ks++) {
-        if (ks & 1) dmma_884(e0, e1, a[ks], bp[4 * ks * Z.ldP]);
-        else dmma_884(d0, d1, a[ks], bp[4 * ks * Z.ldP]);
-      }
-      const int k1 = 8 * mt + r, n = 8 * nt + 2 * c;
-      if (k1 < npw && n < npw) out[k1 * n2 + (n >> 1)] = make_double2(d0 + e0, d1 + e1);
-    }
-  }
-}
-
 // ------------------------------------------------------------ (a) form, 3D
-// One CTA per chunk of at most form3_chunk sources of a leaf accumulates the chunk's
+// One CTA per chunk of at most form_chunk sources of a leaf accumulates the chunk's
 // Hermite block H[j + P (k + P l)] (g3dformhc_vec, g3drouts.f:109-192) and
 // writes it to its slot of the partial buffer; fgt_sep3d.cu sums a leaf's
 // blocks in chunk order and takes them to the cut level's expansions.
@@ -766,171 +468,6 @@ __global__ void __launch_bounds__(128) k_form3d_mma(KP k, const FormTask* __rest
         }
       }
   }
-}
-
-// ------------------------------------------------------------ (c) eval, 2D Taylor in two kernels
-// k_pw2taylor2d: one warp per evaluation leaf converts the leaf's plane-wave
-// expansion L[j2 + n2 j1] into the real Taylor block (g2dpw2local_real_vec,
-// g2drouts.f:1417-1540)
-//     lx[k2][j1] = i^k2 sum_j2 x2l[k2][j2] L[j2 + n2 j1]                     (pass A)
-//     lo[k1][k2] = 2 Re( i^k1 sum_{j1 < n2} x2l[k1][j1] (lx[k2][j1] + (-1)^k1 lx[k2][j1 + n2]) )
-// once per leaf, as FP64 MMA products, and stores it row-major with the even
-// row length E >= P (zero padded) for k_eval2d_horner.  Pass A is one real
-// product with B[j2][2 j1 + c] = component c of L[j2 + n2 j1].  2 Re(i^k1 a)
-// keeps a.x (even k1) or a.y (odd k1), so pass B is two real products: even
-// k1 against be[j1][k2] = Re(lx[k2][j1] + lx[k2][j1+n2]), odd k1 against
-// bo[j1][k2] = Im(lx[k2][j1] - lx[k2][j1+n2]).  Operands are zero padded to
-// whole tiles; the x2l tables are shared by the CTA's warps (all leaves of a
-// launch have one order).
-struct ConvDims {
-  int Pn, E, Ph, M1, K1, N1, M2, N2;
-  int ldX, ldA2, ldB2;
-  int tab, warp;  // doubles: CTA tables, per-warp area
-  __host__ __device__ ConvDims(int P, int npw) {
-    const int n2 = npw / 2;
-    Pn = P;
-    E = (Pn + 1) & ~1;
-    Ph = (Pn + 1) / 2;
-    M1 = (Pn + 7) & ~7;        // pass A rows: k2
-    K1 = (n2 + 3) & ~3;        // pass A depth j2, pass B depth j1
-    N1 = (4 * n2 + 7) & ~7;    // pass A columns: (j1, {re, im} of j1 and of j1 + n2)
-    M2 = (Ph + 7) & ~7;        // pass B rows: k1 of one parity
-    N2 = M1;                   // pass B columns: k2
-    ldX = mma_lda(K1);
-    ldA2 = mma_lda(K1);
-    ldB2 = mma_ldb(N2);
-    tab = M1 * ldX + 2 * M2 * ldA2;
-    warp = 2 * K1 * ldB2 + 2 * (n2 + npw);  // be, bo, the fused split's phases (double2 [n2 + npw])
-  }
-};
-constexpr int CONV_MAXKS = 12;  // largest pass A depth in steps of 4: n2 <= 48
-
-// Tables of k_pw2taylor2d for order P: XA[k2][j2] = x2l[k2][j2],
-// AE[i][j1] = x2l[2i][j1], AO[i][j1] = x2l[2i+1][j1], zero padded.
-void build_conv_table(const HostPlan& H, int Pn, std::vector<double>& out) {
-  const int npw = H.P.npw, n2 = npw / 2;
-  const ConvDims Z(Pn, npw);
-  const size_t base = out.size();
-  out.resize(base + Z.tab, 0.0);
-  double* XA = out.data() + base;
-  double* AE = XA + Z.M1 * Z.ldX;
-  double* AO = AE + Z.M2 * Z.ldA2;
-  for (int r = 0; r < Pn; r++)
-    for (int c = 0; c < n2; c++) {
-      XA[r * Z.ldX + c] = H.x2l[(size_t)r * npw + c];
-      if (r % 2 == 0) AE[(r / 2) * Z.ldA2 + c] = H.x2l[(size_t)r * npw + c];
-      else AO[(r / 2) * Z.ldA2 + c] = H.x2l[(size_t)r * npw + c];
-    }
-}
-
-// With f32, each coefficient is stored as the FP32 pair (c, c) in its FP64
-// slot instead (the layout k_eval2d_horner_f32 reads: a row's float4 m holds
-// (c_2m, c_2m, c_2m+1, c_2m+1)), so the mixed evaluation needs no
-// conversion pass of its own.
-template <int KS>  // pass A depth in steps of 4: KS = ceil(n2 / 4)
-__global__ void __launch_bounds__(128) k_pw2taylor2d(KP k, const ConvTask* __restrict__ tasks, int ntask,
-                                                     double* __restrict__ lo_all,
-                                                     const double* __restrict__ tab, int f32) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int t = blockIdx.x * nw + warp;
-  if (t >= ntask) return;  // no CTA-wide barrier in this kernel
-  const ConvTask T = tasks[t];
-  const int n2 = k.n2;
-  const ConvDims Z(T.p + 1, k.npw);
-  const int Pn = Z.Pn, E = Z.E;
-  extern __shared__ double s1[];
-  const double* XA = tab;                 // [M1][ldX], read through L1
-  const double* AE = XA + Z.M1 * Z.ldX;   // [M2][ldA2]
-  const double* AO = AE + Z.M2 * Z.ldA2;  // [M2][ldA2]
-  double* BE = s1 + warp * Z.warp;        // [K1][ldB2]: be[j1][k2]
-  double* BO = BE + Z.K1 * Z.ldB2;        // [K1][ldB2]: bo[j1][k2]
-  double2* PHX = reinterpret_cast<double2*>(BO + Z.K1 * Z.ldB2);  // fused split: [n2] x phases, then
-  double2* PHY = PHX + n2;                                         // [npw] y phases
-  // rows of be / bo that pass A does not write
-  for (int rr = Z.N1 / 4; rr < Z.K1; rr++)
-    for (int c = lane; c < Z.ldB2; c += 32) {
-      BE[rr * Z.ldB2 + c] = 0.0;
-      BO[rr * Z.ldB2 + c] = 0.0;
-    }
-  const int ind = blockIdx.y;
-  const double* Ld = reinterpret_cast<const double*>(k.loc + ((size_t)T.slot * k.nd + ind) * k.nexp);
-  const int r = lane >> 2, c = lane & 3;
-  // the split fused (T.fused: T.slot is the cut-level ancestor's expansion):
-  // the leaf's coefficient (j2, J) is the ancestor's times
-  // exp(i (t_j2 sh0 + t_J sh1)), t_m = x2l[1][m] the nodes, sh the leaf
-  // centre minus the ancestor's over sqrt(delta)
-  if (T.fused) {
-    for (int m = lane; m < n2 + k.npw; m += 32) {
-      double sn, cs;
-      sincos(k.x2l[k.npw + (m < n2 ? m : m - n2)] * T.sh[m < n2 ? 0 : 1], &sn, &cs);
-      PHX[m] = make_double2(cs, sn);
-    }
-    __syncwarp();
-  }
-  // pass A: B[j2][n], n = 4 j1 + {re, im of L[.][j1], re, im of L[.][j1 + n2]},
-  // read straight from the leaf's expansion (it stays in L1 across the tiles).
-  // The accumulator pair of lane (r, c) in tile (mt, nt) is row k2 = 8 mt + r,
-  // j1 = 2 nt + c/2: lx[k2][j1] for even c, lx[k2][j1 + n2] for odd c; the
-  // partner lane (c xor 1) holds the other, so one exchange forms be and bo.
-  for (int nt = 0; nt < Z.N1 / 8; nt++) {
-    double bk[KS];
-    {
-      const int j1 = 2 * nt + (r >> 2), q = r & 3;
-      const bool ok = j1 < n2;
-      const int J = j1 + (q >> 1) * n2;  // the y node of this lane's column
-      const double* bp = Ld + 2 * (c + n2 * J) + (q & 1);
-      if (T.fused) {
-#pragma unroll
-        for (int ks = 0; ks < KS; ks++) {
-          const int j2 = 4 * ks + c;
-          bk[ks] = 0.0;
-          if (ok && j2 < n2) {
-            const double2 L = __ldg(reinterpret_cast<const double2*>(Ld) + j2 + n2 * J);
-            const double2 v = cmul_rn(L, cmul_rn(PHX[j2], PHY[J]));
-            bk[ks] = (q & 1) ? v.y : v.x;
-          }
-        }
-      } else {
-#pragma unroll
-        for (int ks = 0; ks < KS; ks++) bk[ks] = (ok && 4 * ks + c < n2) ? __ldg(bp + 8 * ks) : 0.0;
-      }
-    }
-    for (int mt = 0; mt < Z.M1 / 8; mt++) {
-      const double* ap = XA + (8 * mt + r) * Z.ldX + c;
-      double d0 = 0.0, d1 = 0.0, e0 = 0.0, e1 = 0.0;
-#pragma unroll
-      for (int ks = 0; ks < KS; ks++) {
-        if (ks & 1) dmma_884(e0, e1, __ldg(ap + 4 * ks), bk[ks]);
-        else dmma_884(d0, d1, __ldg(ap + 4 * ks), bk[ks]);
-      }
-      const int k2 = 8 * mt + r, j1 = 2 * nt + (c >> 1);
-      const double2 z = rot_bf(make_double2(d0 + e0, d1 + e1), k2);
-      const double px = __shfl_xor_sync(FULL_MASK, z.x, 1), py = __shfl_xor_sync(FULL_MASK, z.y, 1);
-      if ((c & 1) == 0) BE[j1 * Z.ldB2 + k2] = z.x + px;  // Re(lx[j1] + lx[j1 + n2])
-      else BO[j1 * Z.ldB2 + k2] = py - z.y;               // Im(lx[j1] - lx[j1 + n2])
-    }
-  }
-  __syncwarp();
-  // pass B: 2 Re(i^k1 ...) = 2 {x, -y, -x, y}[k1 mod 4]
-  double* out = lo_all + T.off + (size_t)ind * Pn * E;
-  float2* out2 = reinterpret_cast<float2*>(out);
-  auto put = [&](int e, double v) {
-    if (f32) out2[e] = make_float2((float)v, (float)v);
-    else out[e] = v;
-  };
-  warp_gemm<true>(AE, Z.ldA2, BE, Z.ldB2, AO, BO, Z.M2 / 8, Z.N2 / 8, KS,  // A through L1
-                  [&](int i, int k2, double e0, double e1, double o0, double o1) {
-                    const double se = (i & 1) ? -2.0 : 2.0, so = -se;
-                    const int ke = 2 * i, ko = 2 * i + 1;
-                    if (ke < Pn) {
-                      if (k2 < E) put(ke * E + k2, se * e0);
-                      if (k2 + 1 < E) put(ke * E + k2 + 1, se * e1);
-                    }
-                    if (ko < Pn) {
-                      if (k2 < E) put(ko * E + k2, so * o0);
-                      if (k2 + 1 < E) put(ko * E + k2 + 1, so * o1);
-                    }
-                  });
 }
 
 // ------------------------------------------------------------ (c) eval, 2D Taylor blocks
@@ -1295,20 +832,6 @@ __global__ void __launch_bounds__(256) k_form2d_pw(KP k, const FormTask* __restr
 }
 
 // ------------------------------------------------------------ (b) shifts
-// merge: parent = sum over its children of child * W (g2dshiftpw_vec)
-__global__ void k_merge(KP k, const MergeGroup* __restrict__ groups, const ShiftTask* __restrict__ tasks) {
-  const MergeGroup G = groups[blockIdx.x];
-  const size_t per = (size_t)k.nd * k.nexp;
-  for (size_t e = (size_t)blockIdx.y * blockDim.x + threadIdx.x; e < per; e += (size_t)gridDim.y * blockDim.x) {
-    const int ee = (int)(e % k.nexp);
-    double2 a = make_double2(0.0, 0.0);
-    for (int t = G.beg; t < G.beg + G.cnt; t++) {
-      const ShiftTask S = tasks[t];
-      a = cfma(k.mp[(size_t)S.src * per + e], k.wms[(size_t)S.table * k.nexp + ee], a);
-    }
-    k.mp[(size_t)G.dst * per + e] = a;
-  }
-}
 // mp -> loc at the cut level: sum over the plane-wave list plus the box's own
 // multipole (g2dshiftpw_vec + g2dcopypwexp_vec, fgt2d.f:1048-1060)
 __global__ void k_m2l(KP k, const M2LTask* __restrict__ tasks, const M2LNbr* __restrict__ nbr) {
@@ -1329,36 +852,6 @@ __global__ void k_m2l(KP k, const M2LTask* __restrict__ tasks, const M2LNbr* __r
     k.loc[(size_t)T.loc * per + e] = a;
   }
 }
-// One CTA per (task, block of SHU * 256 coefficients), every density in
-// turn; a thread's SHU loads of the parent and of the table are issued
-// before the first product.
-constexpr int SHU = 4;
-// split: child = parent * conj(W), W the merge factor of that child
-__global__ void __launch_bounds__(256) k_split(KP k, const ShiftTask* __restrict__ tasks) {
-  const ShiftTask S = tasks[blockIdx.x];
-  const size_t per = (size_t)k.nd * k.nexp;
-  const int e0 = blockIdx.y * 256 * SHU + threadIdx.x;
-  const double2* w = k.wms + (size_t)S.table * k.nexp;
-  for (int ind = 0; ind < k.nd; ind++) {
-    const double2* src = k.loc + (size_t)S.src * per + (size_t)ind * k.nexp;
-    double2* dst = k.loc + (size_t)S.dst * per + (size_t)ind * k.nexp;
-    double2 a[SHU], b[SHU];
-#pragma unroll
-    for (int u = 0; u < SHU; u++) {
-      const int e = e0 + 256 * u;
-      if (e < k.nexp) {
-        a[u] = src[e];
-        b[u] = __ldg(w + e);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < SHU; u++) {
-      const int e = e0 + 256 * u;
-      if (e < k.nexp) dst[e] = cmulc(a[u], b[u]);
-    }
-  }
-}
-
 // ------------------------------------------------------------ (c) eval, plane-wave route derivatives
 // A pair of nodes +t, -t with coefficients A (of e^{itx}) and B (of e^{-itx})
 // contributes A w + B conj(w), w = e^{itx}; its x derivatives are
@@ -2105,6 +1598,22 @@ std::vector<Task> route_order_sort(const std::vector<Task>& in) {
   }
   return out;
 }
+// Two pieces of host work, on two threads of the team where `par`.
+template <typename F, typename G>
+void beside(bool par, F&& f, G&& g) {
+  std::exception_ptr err[2];
+#pragma omp parallel for schedule(static, 1) if (par)
+  for (int i = 0; i < 2; i++) {
+    try {
+      if (i == 0) f();
+      else g();
+    } catch (...) {
+      err[i] = std::current_exception();
+    }
+  }
+  for (const std::exception_ptr& e : err)
+    if (e) std::rethrow_exception(e);
+}
 cudaError_t device_pool_setup() {
   // keep freed stream-ordered allocations in the device's default pool
   // instead of returning them at every synchronisation (process-local
@@ -2130,7 +1639,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
   };
   const double tin = tnow();
-  double tp[8];
+  double tp[4];
   int np_ = 0;
   D = DevicePlan();
   D.P = H.P;
@@ -2140,242 +1649,171 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   int dev = 0;
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&D.sm_count, cudaDevAttrMultiProcessorCount, dev));
-  double tq[8];
+  double tq[4];
   int nq = 0;
   tq[nq++] = tnow();
   // order form and eval tasks by route so each kernel gets a contiguous range
   // (then by order; stable)
-  std::vector<FormTask> form = route_order_sort(H.form);
+  std::vector<FormTask> form;
+  std::vector<EvalTask> ev;
+  beside(H.form.size() > 2048, [&] { form = route_order_sort(H.form); }, [&] { ev = route_order_sort(H.eval); });
   D.nform = (int)form.size();
   for (auto& f : form) {
     (f.route == ROUTE_PW ? D.form_pw_n : D.form_hermite_n)++;
     if (f.route == ROUTE_HERMITE) D.form_pmax = std::max(D.form_pmax, f.p);
   }
-  std::vector<EvalTask> ev = route_order_sort(H.eval);
   D.neval = (int)ev.size();
   for (auto& e : ev) {
     (e.route == ROUTE_PW ? D.eval_pw_n : D.eval_taylor_n)++;
     if (e.route == ROUTE_TAYLOR) D.eval_pmax = std::max(D.eval_pmax, e.p);
     else D.eval_pw_max = std::max(D.eval_pw_max, e.n);
   }
-  // 3D plane-wave scheme: the Hermite leaves in the order of the columns and
-  // slabs of their cut-level boxes, and the leaves with their own expansions
+  // Plane-wave scheme: the Hermite leaves in the order of the columns (and
+  // slabs) of their cut-level boxes, and the leaves formed from exponential sums
   const int lcut = std::max(P.npwlevel, 0);
-  const bool sep = P.dim == 3 && P.scheme == 0 && !P.all_direct;
+  const bool sep = P.scheme == 0 && !P.all_direct;
   if (sep)  // the plane-wave route evaluates the cut-level box's expansion about its centre
     for (int t = D.eval_taylor_n; t < D.neval; t++)
       while (H.tree.level[ev[t].box] > lcut) ev[t].box = H.tree.parent[ev[t].box];
   SepLists up;
+  std::vector<BlockSum> sums2;  // 2D: the leaves of several partial blocks
   std::vector<PwFormTask> pwf;  // 3D boxes formed from exponential sums
   std::vector<SrcRange> pwf_src;
   std::vector<double> sep_ph;
-  std::vector<SepItem> sep_items;  // every leaf at or below the cut level, in the order of the lists
+  size_t hbuf_doubles = 0;  // the leaves' (partial) Hermite blocks
+  std::vector<std::pair<int, int>> run;  // a leaf's Taylor tasks, by its number in the list below
+  uvector<SepItem> sep_items;  // every leaf at or below the cut level, in the order of the lists
   std::vector<int> sep_order_of;   // order by depth below the cut level
   if (sep) {
     const Tree& tr = H.tree;
-    const int nroot = tr.llast[lcut] - tr.lfirst[lcut] + 1;
-    std::vector<int> boxes, task(tr.nboxes, -1);
-    boxes.reserve(tr.nboxes - tr.lfirst[lcut]);
-    for (int b = tr.lfirst[lcut]; b < tr.nboxes; b++)
-      if (tr.nchild[b] == 0) boxes.push_back(b);
+    // the leaves that a form or a Taylor task needs, those of the form tasks
+    // first, with their Taylor tasks [run.first, run.second) (a leaf's are
+    // consecutive)
+    uvector<int> num(tr.nboxes);
+#pragma omp parallel for schedule(static) if (tr.nboxes > 16384)
+    for (int b = 0; b < tr.nboxes; b++) num[b] = -1;
+    std::vector<int> boxes(D.nform);
+    boxes.reserve(D.nform + D.eval_taylor_n);
+    for (int i = 0; i < D.nform; i++) {
+      num[form[i].box] = i;
+      boxes[i] = form[i].box;
+    }
+    run.resize(D.nform + D.eval_taylor_n, {0, 0});
+    for (int t = 0, u; t < D.eval_taylor_n; t = u) {
+      const int b = ev[t].box;
+      for (u = t + 1; u < D.eval_taylor_n && ev[u].box == b;) u++;
+      if (num[b] < 0) {
+        num[b] = (int)boxes.size();
+        boxes.push_back(b);
+      }
+      run[num[b]] = {t, u};
+    }
     for (int l = lcut; l <= P.nlevels; l++) sep_order_of.push_back(H.nlocal[l]);
     sep_order(tr, lcut, boxes, sep_rank(sep_order_of), sep_items);
     sep_phases(H, P.nlevels - lcut, tr.boxsize[lcut], sep_ph);
-    for (int i = 0; i < D.nform; i++) task[form[i].box] = i;
+  }
+  std::vector<long long> form_hoff;
+  // Taylor evaluation: point chunks of <= 256 that read a leaf's block
+  std::vector<HornerTask> horner;
+  size_t lo_doubles = 0;
+  // The Taylor leaves in the order of the columns (and slabs) of their
+  // cut-level boxes, in 3D each order group either with Taylor blocks or
+  // evaluated from the columns
+  SepLists dn;
+  std::vector<ColTask> ctask;
+  uvector<SepItem> dn_items;
+  std::vector<long long> first;   // first task of every item
+  std::vector<uint8_t> blocks;    // by order: evaluated from Taylor blocks
+  long long nh = 0, nct = 0;
+  const int pgh = std::max(1, std::max(P.ifpgh, P.ifpghtarg)), cp = sep_col_points(pgh);
+  auto build_up = [&] {
+    const int* mp_slot = H.mp_slot.data() + H.tree.lfirst[lcut];
     const std::vector<FormTask> in(form.begin(), form.begin() + D.form_hermite_n);
-    std::vector<SepItem> items, pw;
-    items.reserve(D.form_hermite_n);
-    D.up_leaf.reserve(D.form_hermite_n);
-    D.up_box.reserve(D.form_hermite_n);
+    uvector<SepItem> items(D.form_hermite_n), pw;
+    std::vector<SepLeaf> leaf(D.form_hermite_n);
+    std::vector<int> box(D.form_hermite_n);
+    int ni = 0;
     // Sources per partial block: at most 4096, fewer (whole batches of the
     // kernel) where that leaves SMs without a CTA
     long long nsrc = 0, hoff = 0;
     for (int i = 0; i < D.form_hermite_n; i++) nsrc += form[i].n;
-    const int batch = P.ifdipole ? FORM3_SB / 3 : FORM3_SB;
-    D.form3_chunk = (int)std::min<long long>(4096 / batch, std::max<long long>(6, nsrc / (8LL * D.sm_count * batch))) * batch;
+    if (P.dim == 3) {
+      const int batch = P.ifdipole ? FORM3_SB / 3 : FORM3_SB;
+      D.form_chunk = (int)std::min<long long>(4096 / batch, std::max<long long>(6, nsrc / (8LL * D.sm_count * batch))) * batch;
+    } else {
+      // 2D: about eight chunks per SM of at least 512 sources, whole passes of
+      // the kernels' four warps (four leaves of 75000 sources in four CTAs took
+      // 0.76 ms of a 0.80 ms execute, 0.02 of 0.08 cut up)
+      D.form_chunk = (int)std::max<long long>(512, (nsrc / (8LL * D.sm_count) + 255) / 256 * 256);
+    }
+    const int chunk = D.form_chunk;
     for (const SepItem& s : sep_items) {
-      const int i = task[s.box];
-      if (i < 0) continue;
+      const int i = s.num;
+      if (i >= D.nform) continue;
       if (i >= D.form_hermite_n) {
         pw.push_back(s);
         continue;
       }
-      const FormTask& f = form[items.size()] = in[i];
-      const int n = (f.n + D.form3_chunk - 1) / D.form3_chunk;
-      items.push_back(s);
-      D.up_box.push_back(s.box);
-      D.up_leaf.push_back({hoff, 0, n});
-      hoff += (long long)n * (f.p + 1) * (f.p + 1) * (f.p + 1);
+      const FormTask& f = form[ni] = in[i];
+      const int n = f.n <= chunk ? 1 : (f.n + chunk - 1) / chunk;
+      items[ni] = s;
+      box[ni] = s.box;
+      leaf[ni++] = {hoff, 0, n};
+      if (P.dim == 2 && n > 1) sums2.push_back({hoff * P.nd, (f.p + 1) * (f.p + 1), n});
+      hoff += (long long)n * (f.p + 1) * (f.p + 1) * (P.dim == 3 ? f.p + 1 : 1);
     }
-    std::vector<int> slot(nroot);
-    std::vector<uint8_t> has(nroot, 0);
-    for (int r = 0; r < nroot; r++) slot[r] = H.mp_slot[tr.lfirst[lcut] + r];
-    for (const SepItem& s : items) has[s.root] = 1;
+    hbuf_doubles = (size_t)hoff * P.nd;
+    // the boxes formed from exponential sums; `add` where leaves below add to them
     std::stable_sort(pw.begin(), pw.end(), [](const SepItem& a, const SepItem& b) { return a.root < b.root; });
+    std::vector<int> has;  // the roots of the other leaves
+    if (!pw.empty()) {
+      for (const SepItem& s : items) has.push_back(s.root);
+      std::sort(has.begin(), has.end());
+    }
     for (size_t i = 0; i < pw.size(); i++) {
-      const FormTask& f = form[task[pw[i].box]];
+      const FormTask& f = form[pw[i].num];
       const int r = pw[i].root;
-      if (i == 0 || pw[i - 1].root != r) pwf.push_back({tr.lfirst[lcut] + r, slot[r], (int)pwf_src.size(), 0, has[r]});
+      if (i == 0 || pw[i - 1].root != r)
+        pwf.push_back({H.tree.lfirst[lcut] + r, mp_slot[r], (int)pwf_src.size(), 0,
+                       std::binary_search(has.begin(), has.end(), r)});
       pwf_src.push_back({f.s0, f.n});
       pwf.back().cnt++;
     }
-    sep_lists(items, D.up_leaf, sep_order_of, slot, -1, P.npw, up);
-  }
-  if (P.dim == 3 && P.scheme == 1)  // the NUFFT scheme: every box by itself
-    for (const FormTask& f : form) {
-      pwf.push_back({f.box, f.slot, (int)pwf_src.size(), 1, 0});
-      pwf_src.push_back({f.s0, f.n});
-    }
-  tq[nq++] = tnow();
-  // launch groups of equal order among the Hermite form / Taylor eval tasks
-  for (int t = 0; t < D.form_hermite_n;) {
-    int u = t;
-    while (u < D.form_hermite_n && form[u].p == form[t].p) u++;
-    D.form_groups.push_back({form[t].p, t, u});
-    t = u;
-  }
-
-  // dominant form group (most sources) for the per-kernel roofline of the bench
-  if (P.dim == 2) {
-    long long best = -1;
-    for (size_t gi = 0; gi < D.form_groups.size(); gi++) {
-      const OrderGroup& G = D.form_groups[gi];
-      long long n = 0;
-      for (int t = G.beg; t < G.end; t++) n += form[t].n;
-      const double Pn = G.p + 1;
-      D.group_flops.push_back(2.0 * (double)n * Pn * Pn * P.nd);
-      D.group_alg_flops.push_back(4.0 * (double)n * P.npw * P.npw * P.nd);
-      if (G.p + 1 <= 32 && n > best) { best = n; D.dom_form_group = (int)gi; }
-    }
-  }
-  tp[np_++] = tnow();
-  // 2D Taylor evaluation: one conversion per leaf slot, point chunks of <= 256
-  std::vector<ConvTask> conv;
-  std::vector<HornerTask> horner;
-  size_t lo_doubles = 0;
-  // The split is fused into the conversion (k_pw2taylor2d): it reads the
-  // cut-level ancestor's local expansion and applies the leaf's phases
-  // (ConvTask.sh)
-  std::vector<uint8_t> fused_leaf(H.tree.nboxes, 0);
-  tq[nq++] = tnow();
-  if (P.dim == 2 && !P.all_direct) {
-    const int ntay = D.eval_taylor_n;
-    // the conversion of leaf slot s, made by its first task: (ConvTask, the
-    // fused split), the same for either way of filling below
-    auto make_conv = [&](const EvalTask& e, long long off) {
-      ConvTask ct{e.slot, e.p, off};
-      if (H.tree.level[e.box] > lcut) {
-        int a = e.box;
-        while (H.tree.level[a] > lcut) a = H.tree.parent[a];
-        if (a >= 0 && H.loc_slot[a] >= 0) {
-          ct.slot = H.loc_slot[a];
-          ct.fused = 1;
-          for (int d = 0; d < P.dim; d++) ct.sh[d] = (H.tree.c(e.box, d) - H.tree.c(a, d)) * P.dsq;
-          fused_leaf[e.box] = 1;
+    D.up_box.swap(box);
+    D.up_leaf = leaf;
+    sep_lists(P.dim, items, leaf, sep_order_of, mp_slot, -1, P.npw, up);
+    // 2D: the source chunks as tasks of their own, each with its partial block
+    if (P.dim == 2 && sums2.empty()) {
+      std::vector<long long> off(form.size());
+      for (size_t t = 0; t < off.size(); t++) off[t] = D.up_leaf[t].off * P.nd;
+      form_hoff.swap(off);
+    } else if (P.dim == 2) {
+      std::vector<FormTask> ch;
+      ch.reserve(form.size());
+      for (int t = 0; t < D.form_hermite_n; t++) {
+        const FormTask& f = form[t];
+        const long long P2 = (long long)(f.p + 1) * (f.p + 1);
+        for (int c = 0, b = 0; c < f.n; c += D.form_chunk, b++) {
+          FormTask g = f;
+          g.s0 = f.s0 + c;
+          g.n = std::min(D.form_chunk, f.n - c);
+          ch.push_back(g);
+          form_hoff.push_back((D.up_leaf[t].off + b * P2) * P.nd);
         }
       }
-      return ct;
-    };
-    auto lo_size = [&](const EvalTask& e) {
-      const long long Pn = e.p + 1, E = (Pn + 1) & ~1LL;
-      return (size_t)(P.nd * Pn * E);
-    };
-    // The tasks of one leaf are consecutive (the builder emits them leaf by
-    // leaf and the route sort is stable): then every slot's first task starts
-    // a run, the conversions and chunk lists are laid out by prefix sums and
-    // filled in parallel.  Otherwise the serial loop below does the same.
-    std::vector<int> cidx(ntay + 1, 0);
-    std::vector<long long> hidx(ntay + 1, 0);
-    bool runs = true;
-    {
-      std::vector<uint8_t> seen(std::max(H.nloc, 1), 0);
-      for (int t = 0; t < ntay; t++) {
-        const bool first = t == 0 || ev[t].slot != ev[t - 1].slot;
-        if (first) {
-          if (seen[ev[t].slot]) runs = false;
-          seen[ev[t].slot] = 1;
-        }
-        cidx[t + 1] = cidx[t] + first;
-        hidx[t + 1] = hidx[t] + (ev[t].n + 255) / 256;
-      }
+      form.swap(ch);
+      D.form_hermite_n = (int)form.size();
     }
-    if (runs) {
-      const int ncv = cidx[ntay];
-      std::vector<long long> coff(ncv + 1, 0);
-      for (int t = 0; t < ntay; t++)
-        if (cidx[t + 1] != cidx[t]) coff[cidx[t] + 1] = (long long)lo_size(ev[t]);
-      for (int c = 0; c < ncv; c++) coff[c + 1] += coff[c];
-      lo_doubles = (size_t)coff[ncv];
-      conv.resize(ncv);
-      horner.resize(hidx[ntay]);
-#pragma omp parallel for schedule(static) if (ntay > 4096)
-      for (int t = 0; t < ntay; t++) {
-        const EvalTask& e = ev[t];
-        const int c = cidx[t + 1] - 1;  // this task's slot's conversion
-        if (cidx[t + 1] != cidx[t]) conv[c] = make_conv(e, coff[c]);
-        long long h = hidx[t];
-        for (int k = 0; k < e.n; k += 256) horner[h++] = {e.box, e.set, e.i0 + k, std::min(256, e.n - k), e.p, coff[c]};
-      }
-    }
-    std::vector<long long> slot_off(runs ? 1 : std::max(H.nloc, 1), -1);
-    if (!runs) {
-      conv.reserve(ntay);
-      horner.reserve(hidx[ntay]);
-    }
-    for (int t = 0; t < ntay && !runs; t++) {
-      const EvalTask& e = ev[t];
-      if (slot_off[e.slot] < 0) {
-        slot_off[e.slot] = (long long)lo_doubles;
-        conv.push_back(make_conv(e, (long long)lo_doubles));
-        lo_doubles += lo_size(e);
-      }
-      for (int c = 0; c < e.n; c += 256)
-        horner.push_back({e.box, e.set, e.i0 + c, std::min(256, e.n - c), e.p, slot_off[e.slot]});
-    }
-    tq[nq++] = tnow();
-    // conv and horner are in order of p (the Taylor tasks are sorted by p)
-    for (size_t t = 0; t < conv.size();) {
-      size_t u = t;
-      while (u < conv.size() && conv[u].p == conv[t].p) u++;
-      D.conv_groups.push_back({conv[t].p, (int)t, (int)u});
-      t = u;
-    }
-    for (size_t t = 0; t < horner.size();) {
-      size_t u = t;
-      while (u < horner.size() && horner[u].p == horner[t].p) u++;
-      D.horner_groups.push_back({horner[t].p, (int)t, (int)u});
-      // k_eval2d_mma where it is the faster one (its comment), with as many
-      // warps per task as have points
-      long long n = 0;
-      for (size_t i = t; i < u; i++) n += horner[i].n;
-      const long long cnt = u - t, tile = std::max(P.ifpgh, P.ifpghtarg) <= 1 ? 16 : 8;
-      if (P.dim == 2 && horner[t].p >= 24 && horner[t].p < 40 && n <= 72 * cnt)
-        D.horner_groups.back().per = n > 3 * tile * cnt ? 4 : n > tile * cnt ? 2 : 1;
-      t = u;
-    }
-  }
-  // 3D: the Taylor leaves in the order of the columns and slabs of their
-  // cut-level boxes (loc slots in sep_lists), each order group either with
-  // Taylor blocks or evaluated from the columns
-  SepLists dn;
-  std::vector<ColTask> ctask;
-  if (sep) {
-    const Tree& tr = H.tree;
-    const int pgh = std::max(1, std::max(P.ifpgh, P.ifpghtarg)), n2 = P.npw / 2;
-    // the tasks [run.first, run.second) of a leaf, by box (they are consecutive)
-    std::vector<std::pair<int, int>> run(tr.nboxes, {0, 0});
-    for (int t = 0; t < D.eval_taylor_n; t++) {
-      std::pair<int, int>& r = run[ev[t].box];
-      if (r.second == 0) r.first = t;
-      r.second = t + 1;
-    }
-    std::vector<SepItem> items;
-    items.reserve(sep_items.size());
+  };
+  auto build_down = [&] {
+    const int n2 = P.npw / 2;
+    uvector<SepItem> items(sep_items.size());
+    int ni = 0;
     for (const SepItem& s : sep_items)
-      if (run[s.box].second > 0) items.push_back(s);
-    const int cp = sep_col_points(pgh);
-    std::vector<uint8_t> blocks(D.eval_pmax + 2, 0);
-    for (size_t i = 0; i < items.size();) {
+      if (run[s.num].second > 0) items[ni++] = s;
+    items.resize(ni);
+    blocks.assign(D.eval_pmax + 2, P.dim == 2);
+    for (size_t i = 0; i < items.size() && P.dim == 3;) {
       // Multiply-adds on the FP64 pipe of the two ways, each with what its
       // kernels lose beside them (measured, 3D, eps 1e-6 and 1e-9): a leaf's
       // block costs P^3 (n2 + 44) (44: its two passes over memory) and its
@@ -2389,7 +1827,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
       size_t j = i;
       for (; j < items.size() && sep_order_of[items[j].d] == p; j++) {
         cb += P3 * (n2 + 44);
-        for (int t = run[items[j].box].first; t < run[items[j].box].second; t++) {
+        for (int t = run[items[j].num].first; t < run[items[j].num].second; t++) {
           cb += 2.0 * P3 * pgh * (32 * ((ev[t].n + 31) / 32));
           cc += 3.0 * n2 * Pn * Pn * pgh * (8 * ((ev[t].n + 7) / 8));
         }
@@ -2397,107 +1835,100 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
       blocks[p] = Pn <= 30 && ((Pn <= 16 && pgh == 1 && !P.ifdipole) || cb < cc);
       i = j;
     }
-    std::vector<SepLeaf> leaf;
-    leaf.reserve(items.size());
-    for (const SepItem& it : items) {
-      const int p = sep_order_of[it.d];
-      const long long Pn = p + 1, E = (Pn + 1) & ~1LL;
-      leaf.push_back({(long long)lo_doubles, 0, 1});
-      if (blocks[p]) lo_doubles += (size_t)(P.nd * Pn * Pn * E);
+    std::vector<long long> len(sep_order_of.size());  // doubles of a block, by depth
+    for (size_t d = 0; d < len.size(); d++) {
+      const long long p = sep_order_of[d], Pn = p + 1, E = (Pn + 1) & ~1LL;
+      len[d] = p < (int)blocks.size() && blocks[p] ? P.nd * Pn * E * (P.dim == 3 ? Pn : 1) : 0;
     }
-    std::vector<int> slot(tr.llast[lcut] - tr.lfirst[lcut] + 1);
-    for (size_t r = 0; r < slot.size(); r++) slot[r] = H.loc_slot[tr.lfirst[lcut] + r];
-    sep_lists(items, leaf, sep_order_of, slot, -1, P.npw, dn);
-    size_t nh = 0, nct = 0;
-    for (int t = 0; t < D.eval_taylor_n; t++) {
-      if (blocks[ev[t].p]) nh += (ev[t].n + 255) / 256;
-      else nct += (ev[t].n + cp - 1) / cp;
+    std::vector<SepLeaf> leaf(ni);
+    long long lo = 0;
+    for (int i = 0; i < ni; i++) {
+      leaf[i] = {lo, 0, 1};
+      lo += len[items[i].d];
     }
-    horner.reserve(nh);
-    ctask.reserve(nct);
+    lo_doubles = (size_t)lo;
+    sep_lists(P.dim, items, leaf, sep_order_of, H.loc_slot.data() + H.tree.lfirst[lcut], -1, P.npw, dn);
+    // first task of every item, the groups' ranges; the tasks below
+    std::vector<long long> at0(ni);
     for (SepGroup& G : dn.groups) {
       G.blocks = blocks[G.p];
-      const int h0 = (int)horner.size(), c0 = (int)ctask.size();
-      for (int c = G.cbeg; c < G.cend; c++)
-        for (int l = dn.cols[c].beg; l < dn.cols[c].beg + dn.cols[c].cnt; l++) {
-          const std::pair<int, int> r = run[items[l].box];
-          for (int t = r.first; t < r.second; t++) {
-            const EvalTask& e = ev[t];
-            if (G.blocks)
-              for (int q = 0; q < e.n; q += 256)
-                horner.push_back({e.box, e.set, e.i0 + q, std::min(256, e.n - q), e.p, leaf[l].off});
-            else
-              for (int q = 0; q < e.n; q += cp)
-                ctask.push_back({e.box, e.set, e.i0 + q, std::min(cp, e.n - q), dn.leaves[l].row, e.p + 1, dn.cols[c].off});
-          }
+      const int step = G.blocks ? 256 : cp;
+      const long long t0 = G.blocks ? nh : nct;
+      long long n = 0, at = t0;
+      const int i0 = dn.cols[G.cbeg].beg, i1 = dn.cols[G.cend - 1].beg + dn.cols[G.cend - 1].cnt;
+      for (int i = i0; i < i1; i++) {
+        const std::pair<int, int> r = run[items[i].num];
+        at0[i] = at;
+        for (int t = r.first; t < r.second; t++) {
+          at += ev[t].n <= step ? 1 : (ev[t].n + step - 1) / step;
+          n += ev[t].n;
         }
-      if (G.blocks) D.horner_groups.push_back({G.p, h0, (int)horner.size()});
-      else D.ctask_groups.push_back({G.p, c0, (int)ctask.size()});
-    }
-  }
-  tp[np_++] = tnow();
-  // padded operand tables of the 2D MMA transforms, one per order group
-  std::vector<double> tables;
-  if (P.dim == 2 && !P.all_direct) {
-    for (OrderGroup& G : D.form_groups)
-      if (G.p + 1 <= 32) {
-        G.tab = (long long)tables.size();
-        build_h2pw_table(H, G.p + 1, tables);
       }
-    for (OrderGroup& G : D.conv_groups) {
-      G.tab = (long long)tables.size();
-      build_conv_table(H, G.p + 1, tables);
+      (G.blocks ? nh : nct) = at;
+      (G.blocks ? D.horner_groups : D.ctask_groups).push_back({G.p, (int)t0, (int)at});
+      // k_eval2d_mma where it is the faster one (its comment), with as many
+      // warps per task as have points
+      const long long cnt = at - t0, tile = pgh <= 1 ? 16 : 8;
+      if (P.dim == 2 && G.p >= 24 && G.p < 40 && n <= 72 * cnt)
+        D.horner_groups.back().per = n > 3 * tile * cnt ? 4 : n > tile * cnt ? 2 : 1;
+    }
+    dn_items.swap(items);
+    first.swap(at0);
+  };
+  if (sep) beside(sep_items.size() > 2048, build_up, build_down);
+  if (P.dim == 3 && P.scheme == 1)  // the NUFFT scheme: every box by itself
+    for (const FormTask& f : form) {
+      pwf.push_back({f.box, f.slot, (int)pwf_src.size(), 1, 0});
+      pwf_src.push_back({f.s0, f.n});
+    }
+  tq[nq++] = tnow();
+  // launch groups of equal order among the Hermite form tasks
+  for (int t = 0; t < D.form_hermite_n;) {
+    int u = t;
+    long long n = 0;
+    for (; u < D.form_hermite_n && form[u].p == form[t].p; u++) n += form[u].n;
+    D.form_groups.push_back({form[t].p, t, u});
+    // 2D: leaves of about two blocks of source columns or less, a warp each
+    D.form_groups.back().warp = n * (P.ifdipole ? 2 : 1) <= 80LL * (u - t);
+    t = u;
+  }
+
+  // dominant form group (most sources) for the per-kernel roofline of the bench
+  if (P.dim == 2) {
+    long long best = -1;
+    for (size_t gi = 0; gi < D.form_groups.size(); gi++) {
+      const OrderGroup& G = D.form_groups[gi];
+      long long n = 0;
+      for (int t = G.beg; t < G.end; t++) n += form[t].n;
+      const double Pn = G.p + 1;
+      D.group_flops.push_back(2.0 * (double)n * Pn * Pn * P.nd);
+      D.group_alg_flops.push_back(4.0 * (double)n * P.npw * P.npw * P.nd);
+      if (n > best) { best = n; D.dom_form_group = (int)gi; }
     }
   }
   tp[np_++] = tnow();
-  // merge groups: consecutive tasks with the same destination
-  std::vector<MergeGroup> groups;
-  D.merge_beg.assign(P.nlevels + 1, 0);
-  D.merge_end.assign(P.nlevels + 1, 0);
-  for (int l = 0; l <= P.nlevels && !H.merge_beg.empty(); l++) {
-    D.merge_beg[l] = (int)groups.size();
-    for (int t = H.merge_beg[l]; t < H.merge_end[l];) {
-      int u = t;
-      while (u < H.merge_end[l] && H.merge[u].dst == H.merge[t].dst) u++;
-      groups.push_back({H.merge[t].dst, t, u - t});
-      t = u;
-    }
-    D.merge_end[l] = (int)groups.size();
-  }
-  tp[np_++] = tnow();
-  // the split tasks still needed: the boxes on the path from the cut level
-  // to every evaluation leaf whose conversion does not fuse the split
-  std::vector<ShiftTask> split_kept;
-  {
-    const Tree& tr = H.tree;
-    std::vector<uint8_t> need(tr.nboxes, 0);
-    for (int t = 0; t < (int)H.eval.size(); t++) {
-      int b = H.eval[t].box;
-      if (fused_leaf[b]) continue;
-      while (b >= 0 && tr.level[b] > lcut && !need[b]) {
-        need[b] = 1;
-        b = tr.parent[b];
+  if (sep) {
+    const uvector<SepItem>& items = dn_items;
+    horner.resize(nh);
+    ctask.resize(nct);
+    const int ncol = (int)dn.cols.size();
+#pragma omp parallel for schedule(static) if (ncol > 1024)
+    for (int c = 0; c < ncol; c++)
+      for (int l = dn.cols[c].beg; l < dn.cols[c].beg + dn.cols[c].cnt; l++) {
+        const std::pair<int, int> r = run[items[l].num];
+        long long at = first[l];
+        for (int t = r.first; t < r.second; t++) {
+          const EvalTask& e = ev[t];
+          if (blocks[e.p])
+            for (int q = 0; q < e.n; q += 256)
+              horner[at++] = {e.box, e.set, e.i0 + q, std::min(256, e.n - q), e.p, dn.leaves[l].off};
+          else
+            for (int q = 0; q < e.n; q += cp)
+              ctask[at++] = {e.box, e.set, e.i0 + q, std::min(cp, e.n - q), dn.leaves[l].row, e.p + 1, dn.cols[c].off};
+        }
       }
-    }
-    std::vector<int> loc_box(std::max(H.nloc, 1), -1);
-    for (int b = 0; b < tr.nboxes; b++)
-      if (H.loc_slot[b] >= 0) loc_box[H.loc_slot[b]] = b;
-    D.split_beg.assign(H.split_beg.size(), 0);
-    D.split_end.assign(H.split_end.size(), 0);
-    for (size_t l = 0; l < H.split_beg.size(); l++) {
-      D.split_beg[l] = (int)split_kept.size();
-      for (int i = H.split_beg[l]; i < H.split_end[l]; i++)
-        if (need[loc_box[H.split[i].dst]]) split_kept.push_back(H.split[i]);
-      D.split_end[l] = (int)split_kept.size();
-    }
-    std::vector<uint8_t> rd(std::max(H.nloc, 1), 0), wr(std::max(H.nloc, 1), 0);
-    long long nrw = 0;
-    for (const ShiftTask& x : split_kept) {
-      nrw += !rd[x.src] + !wr[x.dst];
-      rd[x.src] = wr[x.dst] = 1;
-    }
-    D.split_bytes = 16LL * P.nexp * P.nd * nrw;
   }
+  tp[np_++] = tnow();
   D.nm2l = (int)H.m2l.size();
   D.ndir = (int)(H.dnear.mem ? H.dnear.ndir : (long long)H.dir.size());
   D.nmp = H.nmp;
@@ -2508,64 +1939,17 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   tp[np_++] = tnow();
   // 3D: source chunks and their partial Hermite blocks
   std::vector<FormChunk> fchunks;
-  size_t hbuf_doubles = 0;
-  // 2D: Hermite blocks of the MMA form (orders <= 31), nd P^2 doubles per
-  // source chunk of a leaf, a leaf's chunks one after the other: about eight
-  // chunks per SM of at least 512 sources, whole passes of the kernels' four
-  // warps (four leaves of 75000 sources in four CTAs took 0.76 ms of a 0.80 ms
-  // execute, 0.02 of 0.08 cut up)
-  std::vector<long long> form_hoff, choff;
-  std::vector<FormTask> chunks2;
-  std::vector<BlockSum> sums2;
-  if (P.dim == 2 && !P.all_direct) {
-    long long nsrc = 0;
-    int most = 0;
-    for (int t = 0; t < D.form_hermite_n; t++) {
-      nsrc += form[t].n;
-      most = std::max(most, form[t].n);
-    }
-    const int step = (int)std::max<long long>(512, (nsrc / (8LL * D.sm_count) + 255) / 256 * 256);
-    const bool cut = most > step;  // otherwise the leaves are the chunks
-    form_hoff.assign(form.size(), 0);
-    for (OrderGroup& G : D.form_groups) {
-      const long long Pn = G.p + 1;
-      G.cbeg = cut ? (int)chunks2.size() : G.beg;
-      G.sbeg = (int)sums2.size();
-      long long n = 0;
-      for (int t = G.beg; t < G.end && Pn <= 32; t++) {
-        const FormTask& f = form[t];
-        const size_t len = (size_t)(P.nd * Pn * Pn);
-        const int nc = cut ? std::max(1, (f.n + step - 1) / step) : 1;
-        form_hoff[t] = (long long)hbuf_doubles;
-        if (nc > 1) sums2.push_back({form_hoff[t], (int)(Pn * Pn), nc});
-        for (int c = 0; c < nc && cut; c++) {
-          FormTask g = f;
-          g.s0 = f.s0 + c * step;
-          g.n = std::min(step, f.n - c * step);
-          chunks2.push_back(g);
-          choff.push_back(form_hoff[t] + (long long)(c * len));
-        }
-        hbuf_doubles += nc * len;
-        n += f.n;
-      }
-      G.cend = cut ? (int)chunks2.size() : G.end;
-      G.send = (int)sums2.size();
-      // leaves of about two blocks of source columns or less: a warp each
-      G.warp = n * (P.ifdipole ? 2 : 1) <= 80LL * (G.cend - G.cbeg);
-    }
-  }
   if (P.dim == 3 && !P.all_direct) {
     if (D.form_hermite_n > 0) {
       long long hoff = 0;
       for (int t = 0; t < D.form_hermite_n; t++) {
         const FormTask& f = form[t];
         long long p3 = (long long)(f.p + 1) * (f.p + 1) * (f.p + 1);
-        for (int c = 0; c < f.n; c += D.form3_chunk) {
-          fchunks.push_back({t, f.s0 + c, std::min(D.form3_chunk, f.n - c), hoff});
+        for (int c = 0; c < f.n; c += D.form_chunk) {
+          fchunks.push_back({t, f.s0 + c, std::min(D.form_chunk, f.n - c), hoff});
           hoff += p3;
         }
       }
-      hbuf_doubles = (size_t)hoff * P.nd;
       D.nfchunks = (int)fchunks.size();
       // chunk ranges of equal order (the tasks are sorted by order)
       long long best = -1;
@@ -2586,12 +1970,11 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   size_t ns = P.ns, nt = P.nt, nd = P.nd, dim = P.dim;
   // FP32 coordinates of the mixed near field (charges only)
   const bool fmix = D.ndir > 0 && !P.ifdipole;
-  // diagonal translation tables (formed on the device)
-  const size_t n_wms = P.all_direct || P.dim == 3 ? 0 : (size_t)(P.nlevels + 1) * D.nch * P.nexp;
+  // mp -> loc rows (formed on the device)
   const size_t n_wsh = P.all_direct ? 0 : (size_t)(P.dim == 2 ? 9 : 27) * P.nexp;
-  size_t total = bytes_of(H.box_centers) + bytes_of(H.h2x) + bytes_of(H.x2l) + al(n_wms * 16) + al(n_wsh * 16) + al(H.ww.size() * 8) + al(H.w1.size() * 8) + 2 * al((size_t)P.ns * 4) + 2 * al((size_t)P.nt * 4) +
-                 al((size_t)(std::max(P.ntermmax, 1) + 2) * 8) + al(32 * 8) +
-                 bytes_of(form) + bytes_of(groups) + bytes_of(H.merge) + bytes_of(split_kept) +
+  size_t total = bytes_of(H.box_centers) + bytes_of(H.h2x) + bytes_of(H.x2l) + bytes_of(H.hx) + al(n_wsh * 16) + al(H.w1.size() * 8) + 2 * al((size_t)P.ns * 4) + 2 * al((size_t)P.nt * 4) +
+                 al((size_t)(std::max(P.ntermmax, 1) + 2) * 8) +
+                 bytes_of(form) +
                  bytes_of(H.m2l) + bytes_of(H.m2l_nbr) + bytes_of(ev) + bytes_of(H.dir) +
                  al((size_t)H.dnear.ndir * sizeof(DirTask)) + al((size_t)H.dnear.nsrc * sizeof(SrcRange)) +
                  bytes_of(H.dir_src) + al((size_t)H.nmp * nd * P.nexp * 16) +
@@ -2602,11 +1985,10 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
                  al(nt * nd * out_comps(dim, P.ifpghtarg) * 8) +
                  bytes_of(fchunks) +
                  bytes_of(up.leaves) + bytes_of(up.cols) + bytes_of(up.slabs) + bytes_of(up.boxes) +
-                 bytes_of(up.box_slabs) + bytes_of(dn.cols) + bytes_of(dn.leaves) + bytes_of(dn.slabs) +
-                 bytes_of(dn.boxes) + bytes_of(dn.box_slabs) + bytes_of(ctask) + bytes_of(pwf) + bytes_of(pwf_src) + bytes_of(sep_ph) +
+                 bytes_of(up.box_kids) + bytes_of(dn.cols) + bytes_of(dn.leaves) + bytes_of(dn.slabs) +
+                 bytes_of(dn.boxes) + bytes_of(dn.box_kids) + bytes_of(dn.col_slot) + bytes_of(dn.leaf_col) + bytes_of(sums2) + bytes_of(ctask) + bytes_of(pwf) + bytes_of(pwf_src) + bytes_of(sep_ph) +
                  al(std::max(up.t1, dn.t1) * nd * 8) + al(std::max(up.t2, dn.t2) * nd * 8) +
-                 al(hbuf_doubles * 8) + bytes_of(form_hoff) + bytes_of(choff) +
-                 bytes_of(chunks2) + bytes_of(sums2) + bytes_of(tables) + bytes_of(conv) + bytes_of(horner) +
+                 al(hbuf_doubles * 8) + bytes_of(form_hoff) + bytes_of(horner) +
                  al(lo_doubles * 8) + 4096;
   D.bytes = total;
   if (size_only) {
@@ -2624,29 +2006,21 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   // comes, goes in one copy from a pinned mirror of that range (filled by the
   // host threads); no pageable copy (each would wait for the stream) and no
   // synchronisation here: the kernels below follow the copy on the stream.
-  std::vector<double2> ww(H.ww.size() / 2), w1(H.w1.size() / 2);
-  memcpy(ww.data(), H.ww.data(), H.ww.size() * 8);
+  std::vector<double2> w1(H.w1.size() / 2);
   memcpy(w1.data(), H.w1.data(), H.w1.size() * 8);
   std::vector<double> isq(std::max(P.ntermmax, 1) + 2, 0.0);
   for (size_t j = 1; j < isq.size(); j++) isq[j] = 1.0 / std::sqrt((double)j);
-  std::vector<double> cfac(32);
-  cfac[0] = 1.0;
-  for (int j = 1; j < 32; j++) cfac[j] = cfac[j - 1] / std::sqrt((double)j);
-  double2 *d_ww = nullptr, *d_w1 = nullptr;
+  double2* d_w1 = nullptr;
   {
     char* const b0 = cur;
     Staged st;
     st.add(cur, D.centers, H.box_centers);
     st.add(cur, D.h2x, H.h2x);
     st.add(cur, D.x2l, H.x2l);
-    st.add(cur, d_ww, ww);
+    st.add(cur, D.hx, H.hx);
     st.add(cur, d_w1, w1);
     st.add(cur, D.isq, isq);
-    st.add(cur, D.cfac, cfac);
     st.add(cur, D.form, form);
-    st.add(cur, D.mgroups, groups);
-    st.add(cur, D.merge, H.merge);
-    st.add(cur, D.split, split_kept);
     st.add(cur, D.m2l, H.m2l);
     st.add(cur, D.m2l_nbr, H.m2l_nbr);
     st.add(cur, D.eval, ev);
@@ -2659,12 +2033,16 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     st.add(cur, D.up.cols, up.cols);
     st.add(cur, D.up.slabs, up.slabs);
     st.add(cur, D.up.boxes, up.boxes);
-    st.add(cur, D.up.box_slabs, up.box_slabs);
+    st.add(cur, D.up.box_kids, up.box_kids);
     st.add(cur, D.dn.leaves, dn.leaves);
     st.add(cur, D.dn.cols, dn.cols);
     st.add(cur, D.dn.slabs, dn.slabs);
     st.add(cur, D.dn.boxes, dn.boxes);
-    st.add(cur, D.dn.box_slabs, dn.box_slabs);
+    st.add(cur, D.dn.box_kids, dn.box_kids);
+    st.add(cur, D.dn.col_slot, dn.col_slot);
+    st.add(cur, D.dn.leaf_col, dn.leaf_col);
+    st.add(cur, D.form2_sums, sums2);
+    D.form2_nsums = (int)sums2.size();
     st.add(cur, D.ctask, ctask);
     st.add(cur, D.pwf, pwf);
     st.add(cur, D.pwf_src, pwf_src);
@@ -2674,30 +2052,20 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     D.up.nboxes = (int)up.boxes.size();
     D.up.groups = up.groups;
     D.dn.ph = D.up.ph;
+    D.up.hx = P.dim == 3 ? D.h2x : D.hx;
+    D.up.sms = D.dn.sms = D.sm_count;
     D.dn.nboxes = (int)dn.boxes.size();
     D.dn.groups = dn.groups;
     D.npwf = (int)pwf.size();
     st.add(cur, D.form_hoff, form_hoff);
-    st.add(cur, D.form2_choff, choff);
-    st.add(cur, D.form2_chunks, chunks2);
-    st.add(cur, D.form2_sums, sums2);
-    if (chunks2.empty()) {
-      D.form2_chunks = D.form;
-      D.form2_choff = D.form_hoff;
-    }
-    st.add(cur, D.tables, tables);
-    st.add(cur, D.conv, conv);
     st.add(cur, D.horner, horner);
     CK(st.upload(b0, s));
   }
-  // translation tables formed on the device from their 1D factors
-  D.wms = reinterpret_cast<double2*>(cur); cur += al(n_wms * 16);
+  // mp -> loc rows formed on the device from their 1D factors
   D.wsh = reinterpret_cast<double2*>(cur); cur += al(n_wsh * 16);
-  if (n_wms + n_wsh > 0) {
-    const long long tot = (long long)(n_wms + n_wsh);
-    const int blocks = (int)std::min<long long>((tot + 255) / 256, (long long)D.sm_count * 16);
-    k_shift_tables<<<blocks, 256, 0, s>>>(P.dim, P.npw, P.nexp, P.nlevels, std::max(P.nlevstart, 0), H.nms, (long long)n_wms,
-                                          d_ww, d_w1, D.wms, D.wsh);
+  if (n_wsh > 0) {
+    const int blocks = (int)std::min<size_t>((n_wsh + 255) / 256, (size_t)D.sm_count * 16);
+    k_shift_tables<<<blocks, 256, 0, s>>>(P.dim, P.npw, P.nexp, d_w1, D.wsh);
     CK(cudaGetLastError());
   }
   if (d_isrc) {
@@ -2767,10 +2135,8 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   D.ptsort = reinterpret_cast<double*>(cur); cur += al(nt * nd * out_comps(dim, P.ifpghtarg) * 8);
   CK(cudaStreamSynchronize(s));
   if (getenv("FGT_TREE_TIMING"))
-    fprintf(stderr, "device plan prep parts: sort %.4f conv %.4f tables %.4f merge %.4f split %.4f rest %.4f"
-            " (device %.4f route sorts %.4f groups %.4f conv loop %.4f)\n",
-            tp[0] - tin, tp[1] - tp[0], tp[2] - tp[1], tp[3] - tp[2], tp[4] - tp[3], tm0 - tp[4], tq[0] - tin,
-            tq[1] - tq[0], tq[2] - tq[1], nq > 3 ? tq[3] - tq[2] : 0.0);
+    fprintf(stderr, "device plan prep parts: route sort %.4f up lists %.4f down lists and tasks %.4f rest %.4f\n",
+            tq[1] - tin, tp[0] - tq[1], tp[1] - tp[0], tm0 - tp[1]);
   if (getenv("FGT_TREE_TIMING"))
     fprintf(stderr, "device plan: prep %.4f malloc %.4f upload %.4f (%zu bytes); eval tasks: taylor %d "
             "(max order %d) pw %d; form tasks: hermite %d (max order %d) pw %d\n",
@@ -2792,7 +2158,7 @@ static KP make_kp(const DevicePlan& D) {
   k.dsq = P.dsq; k.delta = P.delta; k.dmax = P.dmax;
   k.t1 = P.npw > 0 ? 0.5 * P.pmax / (P.npw / 2) : 0.0;
   k.centers = D.centers; k.h2x = D.h2x; k.x2l = D.x2l; k.ws = nullptr;
-  k.wms = D.wms; k.wsh = D.wsh; k.mp = D.mp; k.loc = D.loc;
+  k.wsh = D.wsh; k.mp = D.mp; k.loc = D.loc;
   k.src = D.ssort; k.chg = D.csort; k.trg = D.tsort; k.pot = D.psort; k.pottarg = D.ptsort;
   k.nc_s = out_comps(P.dim, P.ifpgh);
   k.nc_t = out_comps(P.dim, P.ifpghtarg);
@@ -2853,7 +2219,7 @@ cudaError_t with_pgh(int pgh, F&& launch) {
 cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& outs,
                                 int precision, cudaStream_t st, StageTimes* times, int phase) {
   const Params& P = D.P;
-  // phase 1: gather, form, merge (every mp expansion up to the cut level);
+  // phase 1: gather, form, merge (the cut level's mp expansions);
   // phase 2: mp -> loc, split, eval, near field, scatter; 0: both
   const bool ph1 = phase != 2, ph2 = phase != 1;
   KP k = make_kp(D);
@@ -2893,7 +2259,6 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
   mark(1);
   const int n2 = P.npw / 2;
   const int echunks = (int)std::min<long long>(65535, ((long long)nd * P.nexp + 255) / 256);
-  const int schunks = (P.nexp + 256 * SHU - 1) / (256 * SHU);  // k_split: every density per block
   if (!P.all_direct) {
    if (ph1) {
     // (a) form
@@ -2901,68 +2266,42 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
       for (size_t gi = 0; gi < D.form_groups.size(); gi++) {
         const OrderGroup& G = D.form_groups[gi];
         const int Pn = G.p + 1;
-        // the group's leaves and their source chunks (with the partial blocks)
-        const int ntk = G.cend - G.cbeg;
         const FormTask* tk = D.form + G.beg;
-        const FormTask* ck = D.form2_chunks + G.cbeg;
-        const long long* choff = D.form2_choff + G.cbeg;
+        const int ntk = G.end - G.beg;
         const bool dom = times && (int)gi == D.dom_form_group;
         if (dom) cudaEventRecord(dev0, st);
-        if (Pn <= 32) {
+        // one block of P <= 32 rows and columns, of 24 beyond (order 41: four
+        // blocks of 24 hold 48, of 32 would hold 64)
 #define FORM_MMA(NT)                                                                                         \
   do {                                                                                                       \
     const size_t sh = (size_t)4 * 2 * (8 * NT) * 36 * 8;                                                     \
-    const dim3 g(G.warp ? (ntk + 3) / 4 : ntk, nd);                                                          \
+    const int nb = (Pn + 8 * NT - 1) / (8 * NT);                                                             \
+    const dim3 g(G.warp ? (ntk + 3) / 4 : ntk, nd, nb * nb);                                                 \
     auto run = [&](auto kernel) -> cudaError_t {                                                             \
       CK(smem_limit(kernel));                                                                                \
-      kernel<<<g, 128, sh, st>>>(k, ck, ntk, choff, D.hbuf);                                                 \
+      kernel<<<g, 128, sh, st>>>(k, tk, ntk, D.form_hoff + G.beg, D.hbuf);                                   \
       return cudaSuccess;                                                                                    \
     };                                                                                                       \
     if (P.ifdipole) CK(G.warp ? run(k_form2d_mma<NT, true, true>) : run(k_form2d_mma<NT, true, false>));     \
     else CK(G.warp ? run(k_form2d_mma<NT, false, true>) : run(k_form2d_mma<NT, false, false>));              \
   } while (0)
-          if (mixed_ac && Pn <= 16) CK(launch_form2d_f32(k, ck, ntk, nd, choff, D.hbuf, Pn, st));
-          else if (Pn <= 8) FORM_MMA(1);
-          else if (Pn <= 16) FORM_MMA(2);
-          else if (Pn <= 24) FORM_MMA(3);
-          else FORM_MMA(4);
+        if (mixed_ac && Pn <= 16) CK(launch_form2d_f32(k, tk, G.end - G.beg, nd, D.form_hoff + G.beg, D.hbuf, Pn, st));
+        else if (Pn <= 8) FORM_MMA(1);
+        else if (Pn <= 16) FORM_MMA(2);
+        else if (Pn <= 24 || Pn > 32) FORM_MMA(3);
+        else FORM_MMA(4);
 #undef FORM_MMA
-          if (dom) {
-            cudaEventRecord(dev1, st);
-            if (mixed_ac && Pn <= 16) snprintf(times->dom_name, sizeof(times->dom_name), "k_form2d_f32");
-            else snprintf(times->dom_name, sizeof(times->dom_name), "k_form2d_mma<%d>", (Pn + 7) / 8);
-            times->dom_flops = D.group_flops[gi];
-            times->dom_alg_flops = D.group_alg_flops[gi];
-          }
-          if (G.send > G.sbeg) {
-            k_sum_blocks2d<<<dim3(G.send - G.sbeg, std::min(32, (Pn * Pn * nd + 31) / 32)), 256, 0, st>>>(D.form2_sums + G.sbeg, nd, D.hbuf);
-            launches++;
-          }
-          const int nt = G.end - G.beg;
-          const H2pwDims Z(Pn, P.npw);
-          const size_t sh2 = 4 * (size_t)Z.warp * 8;
-          if (sh2 > 227 * 1024) return cudaErrorNotSupported;
-          const dim3 hg((nt + 3) / 4, nd);
-          switch (Z.Kq / 4) {
-#define H2PW_CASE(N)                                                                              \
-  case N:                                                                                         \
-    CK(smem_limit(k_h2pw2d<N>)); \
-    k_h2pw2d<N><<<hg, 128, sh2, st>>>(k, tk, nt, D.form_hoff + G.beg, D.hbuf, D.tables + G.tab);  \
-    break;
-            H2PW_CASE(1) H2PW_CASE(2) H2PW_CASE(3) H2PW_CASE(4) H2PW_CASE(5) H2PW_CASE(6)
-            H2PW_CASE(7) H2PW_CASE(8)
-#undef H2PW_CASE
-            default: return cudaErrorNotSupported;
-          }
-          launches++;
-        } else {
-          const int tpd = (Pn + 3) / 4, Pp = 4 * tpd;
-          if (tpd * tpd > 256) return cudaErrorNotSupported;
-          const int ch = Pp <= 32 ? 128 : 64;
-          size_t sh = ((size_t)2 * ch * Pp + 4096 + 2 * (size_t)Pn * n2) * 8;
-          CK(smem_limit(k_form2d));
-          k_form2d<<<dim3(G.end - G.beg, nd), 256, sh, st>>>(k, tk, D.isq, ch);
+        if (dom) {
+          cudaEventRecord(dev1, st);
+          if (mixed_ac && Pn <= 16) snprintf(times->dom_name, sizeof(times->dom_name), "k_form2d_f32");
+          else snprintf(times->dom_name, sizeof(times->dom_name), "k_form2d_mma<%d>", Pn > 32 ? 3 : (Pn + 7) / 8);
+          times->dom_flops = D.group_flops[gi];
+          times->dom_alg_flops = D.group_alg_flops[gi];
         }
+        launches++;
+      }
+      if (D.form2_nsums > 0) {
+        k_sum_blocks2d<<<dim3(D.form2_nsums, 32), 256, 0, st>>>(D.form2_sums, nd, D.hbuf);
         launches++;
       }
     }
@@ -3023,17 +2362,11 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
       launches++;
     }
     mark(2);
-    // (b) merge, bottom-up (2D); 3D: the leaves to the cut level
+    // (b) the leaves' blocks to the cut level's expansions
     if (D.up.nboxes > 0) {
       CK(sep_up(k, D.up, D.hbuf, st, launches));
     }
     if (D.npwf > 0) CK(launch_form3d_pw(k, D.pwf, D.npwf, D.pwf_src, st, launches));
-    for (int l = P.nlevels - 1; l >= P.nlevstart; l--) {
-      int ng = D.merge_end[l] - D.merge_beg[l];
-      if (ng <= 0) continue;
-      k_merge<<<dim3(ng, echunks), 256, 0, st>>>(k, D.mgroups + D.merge_beg[l], D.merge);
-      launches++;
-    }
    }  // phase 1
     mark(3);
    if (ph2) {
@@ -3042,39 +2375,12 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
       launches++;
     }
     mark(4);
-    for (int l = P.nlevstart; l <= P.nlevels - 1; l++) {
-      int nsp = D.split_end[l] - D.split_beg[l];
-      if (nsp <= 0) continue;
-      k_split<<<dim3(nsp, schunks), 256, 0, st>>>(k, D.split + D.split_beg[l]);
-      launches++;
-    }
     mark(5);
     // (c) eval
+    // the blocks that the mixed 2D evaluation reads are written as FP32 pairs
+    // (the condition of its launch below)
+    if (D.dn.nboxes > 0) CK(sep_down(k, D.dn, D.lo, mixed_ac && pgh == 1 ? 32 : 0, st, launches));
     if (P.dim == 2 && D.neval > 0) {
-      for (const OrderGroup& G : D.conv_groups) {
-        const int Pn = G.p + 1, nt = G.end - G.beg;
-        const ConvDims Z(Pn, P.npw);
-        if (Z.K1 / 4 > CONV_MAXKS) return cudaErrorNotSupported;
-        int nw = 4;
-        while (nw > 1 && (size_t)nw * Z.warp * 8 > 100 * 1024) nw >>= 1;
-        const size_t sh = (size_t)nw * Z.warp * 8;
-        if (sh > 227 * 1024) return cudaErrorNotSupported;
-        const dim3 cg((nt + nw - 1) / nw, nd);
-        // the blocks the mixed evaluation reads (the condition of its launch below)
-        const int f32 = mixed_ac && pgh == 1 && (Pn + 1) / 2 <= 16;
-        switch (Z.K1 / 4) {
-#define CONV_CASE(N)                                                                              \
-  case N:                                                                                         \
-    CK(smem_limit(k_pw2taylor2d<N>)); \
-    k_pw2taylor2d<N><<<cg, 32 * nw, sh, st>>>(k, D.conv + G.beg, nt, D.lo, D.tables + G.tab, f32);  \
-    break;
-          CONV_CASE(1) CONV_CASE(2) CONV_CASE(3) CONV_CASE(4) CONV_CASE(5) CONV_CASE(6)
-          CONV_CASE(7) CONV_CASE(8) CONV_CASE(9) CONV_CASE(10) CONV_CASE(11) CONV_CASE(12)
-#undef CONV_CASE
-          default: return cudaErrorNotSupported;
-        }
-        launches++;
-      }
       for (const OrderGroup& G : D.horner_groups) {
         const int Pn = G.p + 1, np2 = (Pn + 1) / 2;
         const dim3 g(G.end - G.beg, nd);
@@ -3140,7 +2446,6 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
       }
     }
     if (P.dim == 3 && D.dn.nboxes > 0) {
-      CK(sep_down(k, D.dn, D.lo, st, launches));
       for (const OrderGroup& G : D.ctask_groups) {
         CK(sep_eval_cols(k, D.dn, D.ctask + G.beg, G.end - G.beg, G.p + 1, pgh, st));
         launches++;
@@ -3273,14 +2578,14 @@ cudaError_t device_plan_box_expansion(const HostPlan& H, DevicePlan& D, int box,
     }
   std::vector<int> order;
   for (int l = lb; l <= P.nlevels; l++) order.push_back(H.nlocal[l]);
-  std::vector<SepItem> items;
+  uvector<SepItem> items;
   sep_order(t, lb, boxes, sep_rank(order), items);
   std::vector<SepLeaf> leaf;
   for (const SepItem& s : items) leaf.push_back(D.up_leaf[at[s.box]]);
   std::vector<int> slot(t.llast[lb] - t.lfirst[lb] + 1, -1);
   slot[box - t.lfirst[lb]] = 0;
   SepLists L;
-  sep_lists(items, leaf, order, slot, box - t.lfirst[lb], P.npw, L);
+  sep_lists(P.dim, items, leaf, order, slot.data(), box - t.lfirst[lb], P.npw, L);
   std::vector<double> ph;
   sep_phases(H, P.nlevels - lb, t.boxsize[lb], ph);
   const std::vector<PwFormTask> pwt(1, pw);
@@ -3288,7 +2593,7 @@ cudaError_t device_plan_box_expansion(const HostPlan& H, DevicePlan& D, int box,
   char* mem = nullptr;
   CK(cudaMallocAsync(reinterpret_cast<void**>(&mem),
                      bytes_of(L.leaves) + bytes_of(L.cols) + bytes_of(L.slabs) + bytes_of(L.boxes) +
-                         bytes_of(L.box_slabs) + bytes_of(ph) + bytes_of(pwt) + bytes_of(pw_src) + al(L.t1 * nd * 8) +
+                         bytes_of(L.box_kids) + bytes_of(ph) + bytes_of(pwt) + bytes_of(pw_src) + al(L.t1 * nd * 8) +
                          al(L.t2 * nd * 8) + al(per) + 4096,
                      st));
   auto run = [&]() -> cudaError_t {
@@ -3301,7 +2606,7 @@ cudaError_t device_plan_box_expansion(const HostPlan& H, DevicePlan& D, int box,
     CK(put(cur, S.cols, L.cols, st));
     CK(put(cur, S.slabs, L.slabs, st));
     CK(put(cur, S.boxes, L.boxes, st));
-    CK(put(cur, S.box_slabs, L.box_slabs, st));
+    CK(put(cur, S.box_kids, L.box_kids, st));
     CK(put(cur, dph, ph, st));
     CK(put(cur, dpw, pwt, st));
     CK(put(cur, dsrc, pw_src, st));
@@ -3309,6 +2614,7 @@ cudaError_t device_plan_box_expansion(const HostPlan& H, DevicePlan& D, int box,
     S.nboxes = 1;
     S.groups = L.groups;
     S.sms = D.sm_count;
+    S.hx = D.up.hx;
     S.t1 = reinterpret_cast<double*>(cur); cur += al(L.t1 * nd * 8);
     S.t2 = reinterpret_cast<double*>(cur); cur += al(L.t2 * nd * 8);
     KP k = make_kp(D);

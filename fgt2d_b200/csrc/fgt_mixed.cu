@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(128) k_form2d_f32(KP k, const FormTask* __rest
 // ------------------------------------------------------------ (c) eval, 2D Taylor, FP32
 // pot += sum_k y^k sum_j L[k][j] x^j (g2dlevalp_vec, g2drouts.f:847-900) for
 // a chunk of <= 256 points of one leaf, two points per thread.  The leaf's
-// Taylor block comes from k_pw2taylor2d already in FP32, each coefficient as
+// Taylor block comes from k_down2d_x already in FP32, each coefficient as
 // the pair (c, c) (row k: float4 m = (c_2m, c_2m, c_2m+1, c_2m+1)), and is
 // copied to shared memory as it is (no conversion).  Each row's polynomial
 // in x runs in FP32 (Pn FMAs), the outer polynomial in y and the output in

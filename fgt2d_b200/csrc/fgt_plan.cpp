@@ -32,7 +32,7 @@ double now() {
 static void build_tables(HostPlan& H) {
   Params& P = H.P;
   const Tree& t = H.tree;
-  int D = P.dim, npw = P.npw, n2 = npw / 2, nch = 1 << D;
+  int D = P.dim, npw = P.npw, n2 = npw / 2;
   double pi = 4.0 * std::atan(1.0);
   // get_pwnodes: 2D +half then -half (g2drouts.f:2205); 3D ascending (g3drouts.f:2669)
   H.ts.assign(npw, 0.0);
@@ -59,24 +59,18 @@ static void build_tables(HostPlan& H) {
         H.x2l[(size_t)j * npw + k] = __builtin_powi(H.ts[k], j) / fac2[j];
       }
   }
-  // 1D factors of the diagonal translation tables; the tables themselves
-  // (nexp entries per row) are formed on the device (device_plan_create).
-  // Merge factors: child slot j merged into its parent, the parent-child
-  // offset at level l being boxsize(l+1)/2; ww(k) = exp(i t xmin2)^(2^(k-1))
-  // as in merge_split_pw_matrices (g2drouts.f:2326-2332).
-  cplx I(0, 1);
-  int nms = std::max(P.nlevels - std::max(P.npwlevel, 0), 1);
-  H.nms = nms;
-  double xmin2 = t.boxsize[P.nlevels] / std::sqrt(P.delta) / 2;
-  H.ww.assign((size_t)npw * (nms + 1) * 2, 0.0);
-  for (int j = 0; j < npw; j++) {
-    cplx z = std::exp(I * H.ts[j] * xmin2);
-    for (int k = 1; k <= nms; k++) {
-      H.ww[2 * ((size_t)j * (nms + 1) + k)] = z.real();
-      H.ww[2 * ((size_t)j * (nms + 1) + k) + 1] = z.imag();
-      z = z * z;
+  if (D == 2) {
+    // the 2D Hermite blocks hold sums of x^j y^k: both 1/sqrt(j!) here
+    H.hx.resize(H.h2x.size());
+    double cf = 1.0;
+    for (int j = 0; j <= tm; j++) {
+      if (j) cf /= std::sqrt((double)j);
+      for (int k = 0; k < npw; k++) H.hx[(size_t)j * npw + k] = H.h2x[(size_t)j * npw + k] * cf;
     }
   }
+  // 1D factors of the mp -> loc rows; the rows themselves (nexp entries) are
+  // formed on the device (device_plan_create).
+  const cplx I(0, 1);
   // mp->loc factors (pw_translation_matrices): exp(i t xmin), xmin = boxsize(cut)
   double xmin = (P.npwlevel >= 0 ? t.boxsize[P.npwlevel] : 0.0) / std::sqrt(P.delta);
   H.w1.assign((size_t)npw * 2, 0.0);
@@ -85,7 +79,6 @@ static void build_tables(HostPlan& H) {
     H.w1[2 * j] = v.real();
     H.w1[2 * j + 1] = v.imag();
   }
-  (void)nch;
 }
 
 // (d) near field, target-centric: for every leaf, the ifhung source boxes
@@ -258,20 +251,14 @@ static void build_tasks(HostPlan& H) {
   H.mp_slot.assign(nb, -1);
   H.loc_slot.assign(nb, -1);
   H.nmp = H.nloc = 0;
-  H.form.clear(); H.merge.clear(); H.split.clear(); H.m2l.clear(); H.m2l_nbr.clear();
+  H.form.clear(); H.m2l.clear(); H.m2l_nbr.clear();
   H.eval.clear();
-  H.merge_beg.assign(P.nlevels + 1, 0);
-  H.merge_end.assign(P.nlevels + 1, 0);
-  H.split_beg.assign(P.nlevels + 1, 0);
-  H.split_end.assign(P.nlevels + 1, 0);
   H.form_sources = H.eval_points = 0;
   if (!P.all_direct) {
     // capacities from the box count (untouched until filled)
     H.form.reserve(nb);
-    H.merge.reserve(nb);
-    H.split.reserve(nb);
     H.eval.reserve((size_t)nb + (size_t)(P.ns + P.nt) / 2048 + 16);
-    // 3D multipole expansions: the cut level's only (fgt_sep3d.cu, fgt_pw3d.cu)
+    // multipole and local expansions: the cut level's only (fgt_sep.cu, fgt_pw3d.cu)
     auto form_route = [&](int l, int b) {
       if (D == 2) return (int)ROUTE_HERMITE;
       const int p = H.nlocal[l];
@@ -286,10 +273,9 @@ static void build_tasks(HostPlan& H) {
       for (int b = t.lfirst[l]; b <= t.llast[l]; b++) {
         bool leaf = t.nchild[b] == 0;
         if (t.ns(b) > 0 && !(leaf && l == npl) &&
-            (D == 2 || l == nls))
+            l == nls)
           H.mp_slot[b] = H.nmp++;
-        // 3D local expansions: the cut level's
-        if (relevant(b) > 0 && !(leaf && l == npl && !iflocal(b)) && (D == 2 || l == nls)) H.loc_slot[b] = H.nloc++;
+        if (relevant(b) > 0 && !(leaf && l == npl && !iflocal(b)) && l == nls) H.loc_slot[b] = H.nloc++;
       }
     // (a) form, levels nlevels .. max(npwlevel+1, 0) (fgt2d.f:871)
     for (int l = P.nlevels; l >= std::max(npl + 1, 0); l--) {
@@ -299,19 +285,6 @@ static void build_tasks(HostPlan& H) {
         H.form.push_back({b, t.s0[b], t.ns(b), H.mp_slot[b], p, form_route(l, b)});
         H.form_sources += t.ns(b);
       }
-    }
-    // (b) merge, parents at levels nlevels-1 .. nlevstart (2D; in 3D the plan's
-    // device side adds the leaves to the cut level)
-    for (int l = P.nlevels - 1; l >= nls && D == 2; l--) {
-      H.merge_beg[l] = (int)H.merge.size();
-      for (int b = t.lfirst[l]; b <= t.llast[l]; b++) {
-        if (H.mp_slot[b] < 0 || t.nchild[b] == 0) continue;
-        for (int j = 0; j < nch; j++) {
-          int c = t.ch(b, j);
-          if (c >= 0 && H.mp_slot[c] >= 0) H.merge.push_back({H.mp_slot[b], H.mp_slot[c], l * nch + j});
-        }
-      }
-      H.merge_end[l] = (int)H.merge.size();
     }
     tq[nq++] = now();
     // (b) mp -> loc at the cut level
@@ -359,18 +332,6 @@ static void build_tasks(HostPlan& H) {
       }
     }
     tq[nq++] = now();
-    // (b) split, parents at levels nlevstart .. nlevels-1 (2D)
-    for (int l = nls; l <= P.nlevels - 1 && D == 2; l++) {
-      H.split_beg[l] = (int)H.split.size();
-      for (int b = t.lfirst[l]; b <= t.llast[l]; b++) {
-        if (H.loc_slot[b] < 0 || t.nchild[b] == 0) continue;
-        for (int j = 0; j < nch; j++) {
-          int c = t.ch(b, j);
-          if (c >= 0 && H.loc_slot[c] >= 0) H.split.push_back({H.loc_slot[c], H.loc_slot[b], l * nch + j});
-        }
-      }
-      H.split_end[l] = (int)H.split.size();
-    }
     // (c) evaluation leaves (fgt2d.f:1141-1271 / fgt3d.f:1283-1446)
     for (int l = nls; l <= P.nlevels; l++) {
       int p = H.nlocal[l];
@@ -384,7 +345,7 @@ static void build_tasks(HostPlan& H) {
         if (t.nchild[b] != 0 || relevant(b) <= 0) continue;
         if (l == npl && !iflocal(b)) continue;
         int a = b;  // the box whose local expansion the leaf reads
-        while (D == 3 && t.level[a] > nls) a = t.parent[a];
+        while (t.level[a] > nls) a = t.parent[a];
         const int slot = H.loc_slot[a];
         if (slot < 0) continue;
         int route = pw ? ROUTE_PW : ROUTE_TAYLOR;
@@ -446,15 +407,10 @@ static void build_tasks(HostPlan& H) {
       if (v >= 0 && !seen[v]) { seen[v] = 1; c++; }
     };
     long long ra, rb;
-    start(H.nmp); for (auto& s : H.merge) see(s.src); ra = c;
-    start(H.nmp); for (auto& s : H.merge) see(s.dst); rb = c;
-    H.shift_bytes[0] = per * (ra + rb);
+    H.shift_bytes[0] = H.shift_bytes[2] = 0;  // no merge, no split (fgt_sep.cu)
     start(H.nmp); for (auto& m : H.m2l) see(m.self_mp); for (auto& n : H.m2l_nbr) see(n.mp); ra = c;
     start(H.nloc); for (auto& m : H.m2l) see(m.loc); rb = c;
     H.shift_bytes[1] = per * (ra + rb);
-    start(H.nloc); for (auto& s : H.split) see(s.src); ra = c;
-    start(H.nloc); for (auto& s : H.split) see(s.dst); rb = c;
-    H.shift_bytes[2] = per * (ra + rb);
   }
   tq[nq++] = now();
   if (getenv("FGT_TREE_TIMING")) {
@@ -484,12 +440,8 @@ static void build_tasks_nufft(HostPlan& H) {
   H.mp_slot.assign(nb, -1);
   H.loc_slot.assign(nb, -1);
   H.nmp = H.nloc = 0;
-  H.form.clear(); H.merge.clear(); H.split.clear(); H.m2l.clear(); H.m2l_nbr.clear();
+  H.form.clear(); H.m2l.clear(); H.m2l_nbr.clear();
   H.eval.clear();
-  H.merge_beg.assign(P.nlevels + 1, 0);
-  H.merge_end.assign(P.nlevels + 1, 0);
-  H.split_beg.assign(P.nlevels + 1, 0);
-  H.split_end.assign(P.nlevels + 1, 0);
   H.form_sources = H.eval_points = 0;
   H.form_route_flops = H.eval_route_flops = 0;
   H.shift_bytes[0] = H.shift_bytes[1] = H.shift_bytes[2] = 0;

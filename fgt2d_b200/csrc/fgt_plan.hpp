@@ -28,10 +28,6 @@ struct FormChunk {
   int task, s0, n;
   long long hoff;
 };
-// stage (b) merge / split: one (parent, child) shift
-struct ShiftTask {
-  int dst, src, table;  // dst slot, src slot, table row (level * nch + child slot)
-};
 // stage (b) mp->loc: one cut-level box, its sources in [off, off+cnt) of the
 // neighbour array
 struct M2LTask {
@@ -79,21 +75,15 @@ struct HostPlan {
   std::vector<double> ts, ws;     // reference node order for the dimension
   std::vector<double> h2x;        // [j * npw + k] = ws_k (-ts_k)^j / sqrt(j!)
   std::vector<double> x2l;        // [j * npw + k] = ts_k^j / j!
-  // 1D factors of the diagonal translation tables (re, im): ww[j][k] =
-  // exp(i t_j xmin2)^(2^(k-1)) for the merge / split rows of nms levels,
-  // w1[j] = exp(i t_j xmin) for mp->loc; the device forms the nexp-long rows
-  std::vector<double> ww, w1;
-  int nms = 1;
+  std::vector<double> hx;         // 2D: h2x[j][k] / sqrt(j!), for Hermite blocks without their 1/sqrt(j! k!)
+  // 1D factors of the mp -> loc rows (re, im): w1[j] = exp(i t_j xmin); the
+  // device forms the nexp-long rows
+  std::vector<double> w1;
   int nmp = 0, nloc = 0;
   std::vector<int> mp_slot, loc_slot;  // per box, -1 when absent
   uvector<double> box_centers;         // dim per box
   // tasks
   std::vector<FormTask> form;
-  // merge / split tasks of parents at level l: [beg[l], end[l])
-  std::vector<int> merge_beg, merge_end;
-  std::vector<ShiftTask> merge;
-  std::vector<int> split_beg, split_end;
-  std::vector<ShiftTask> split;
   std::vector<M2LTask> m2l;
   std::vector<M2LNbr> m2l_nbr;
   std::vector<EvalTask> eval;
@@ -124,7 +114,7 @@ struct HostPlan {
   // statistics
   long long direct_pairs = 0;
   long long form_sources = 0, eval_points = 0;
-  long long shift_bytes[3] = {0, 0, 0};  // algorithmic bytes of merge, mp->loc, split
+  long long shift_bytes[3] = {0, 0, 0};  // algorithmic bytes of merge (none), mp->loc, split (none)
   double form_route_flops = 0, eval_route_flops = 0;
   double host_tree_s = 0, host_lists_s = 0, host_plan_s = 0;
 };

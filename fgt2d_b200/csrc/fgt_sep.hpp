@@ -1,6 +1,6 @@
-// 3D transforms between the leaves' Hermite / Taylor blocks and the cut
-// level's plane-wave expansions, one dimension at a time over the subtree of
-// each cut-level box (fgt_sep3d.cu).
+// Transforms between the leaves' Hermite / Taylor blocks and the cut level's
+// plane-wave expansions, one dimension at a time over the subtree of each
+// cut-level box (fgt_sep.cu; the 3D kernels: fgt_sep3d.cu).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -14,33 +14,39 @@ namespace fgtb {
 
 struct KP;
 
-// The boxes as items, sorted by (rank[depth], root, x, y, z); roots are the
+// The boxes as items, sorted by (rank[depth], root, x, y, z),
+// in 2D (rank[depth], root, y, x); roots are the
 // boxes of level lroot, numbered from its first.  rank: by depth, equal orders
 // next to one another.
 void sep_order(const Tree& t, int lroot, const std::vector<int>& boxes, const std::vector<int>& rank,
-               std::vector<SepItem>& items);
+               uvector<SepItem>& items);
 // rank of sep_order from the orders by depth (increasing order, then depth)
 std::vector<int> sep_rank(const std::vector<int>& order_of_depth);
 
-// Columns (equal root, depth, x, y), slabs (equal root, depth, x) and boxes
-// of sorted items with their blocks (leaf.off, leaf.n; the rows are filled
-// here); offsets and sizes per density.  slot: the expansion slots by root;
-// the roots with leaves get a box, and root `also` (-1: none) without any.
-void sep_lists(const std::vector<SepItem>& items, const std::vector<SepLeaf>& leaf,
-               const std::vector<int>& order_of_depth, const std::vector<int>& slot,
-               int also, int npw, SepLists& S);
+// Columns (equal root, depth, x, y; 2D: y), slabs (3D: equal root, depth, x)
+// and boxes of sorted items with their blocks (leaf.off, leaf.n, taken over;
+// the rows are filled here); offsets and sizes per density.  slot: the
+// expansion slots by root; without any item root `also` (-1: none) gets an
+// empty box.
+void sep_lists(int dim, const uvector<SepItem>& items, std::vector<SepLeaf>& leaf,
+               const std::vector<int>& order_of_depth, const int* slot, int also, int npw, SepLists& S);
 
 // Phase rows of depths 0..dmax: row 2^d - 1 + i holds exp(i t_m sh) of the
 // npw nodes, sh the offset of box i of 2^d from its root's centre over
 // sqrt(delta) (bs0: the root's size).
 void sep_phases(const HostPlan& H, int dmax, double bs0, std::vector<double>& ph);
 
+// 3D (fgt_sep3d.cu)
+cudaError_t sep_up_3d(const KP& k, const SepDev& S, const double* hbuf, cudaStream_t st, long long& launches);
+cudaError_t sep_down_3d(const KP& k, const SepDev& S, double* lo, cudaStream_t st, long long& launches);
+
 // Upward: Hermite blocks in hbuf -> the expansions k.mp of the boxes' slots.
 cudaError_t sep_up(const KP& k, const SepDev& S, const double* hbuf, cudaStream_t st, long long& launches);
 
 // Downward: the expansions k.loc of the boxes' slots -> the columns (t1) of
-// every order and the Taylor blocks (lo) of the groups with blocks.
-cudaError_t sep_down(const KP& k, const SepDev& S, double* lo, cudaStream_t st, long long& launches);
+// every order and the Taylor blocks (lo) of the groups with blocks; 2D blocks
+// of at most f32 rows as FP32 pairs.
+cudaError_t sep_down(const KP& k, const SepDev& S, double* lo, int f32, cudaStream_t st, long long& launches);
 
 // Evaluation from the columns: the most points of a task, and the tasks of
 // one order (Pn: order + 1).

@@ -32,127 +32,9 @@
 #include <type_traits>
 
 #include "fgt_kcommon.cuh"
-#include "fgt_sep3d.hpp"
+#include "fgt_sep.hpp"
 
 namespace fgtb {
-
-// ------------------------------------------------------------ lists
-std::vector<int> sep_rank(const std::vector<int>& order) {
-  std::vector<int> by(order.size()), rank(order.size());
-  for (size_t d = 0; d < by.size(); d++) by[d] = (int)d;
-  std::stable_sort(by.begin(), by.end(), [&](int a, int b) { return order[a] < order[b]; });
-  for (size_t i = 0; i < by.size(); i++) rank[by[i]] = (int)i;
-  return rank;
-}
-
-void sep_order(const Tree& t, int lroot, const std::vector<int>& boxes, const std::vector<int>& rank,
-               std::vector<SepItem>& items) {
-  const int n = (int)boxes.size(), a0 = t.lfirst[lroot], dmax = (int)rank.size() - 1;
-  auto width = [](unsigned long long v) {
-    int w = 0;
-    while (v >> w) w++;
-    return w;
-  };
-  // one key per item, (rank, root, x, y, z, number), sorted by digits of 11
-  // bits; the items are written once, in order
-  const int wn = width(n), wr = width(t.llast[lroot] - a0), wd = width(dmax);
-  const bool packed = 3 * dmax + wr + wd + wn <= 64;
-  std::vector<SepItem> raw(n);
-  std::vector<uint64_t> key(packed ? n : 0), tmp(packed ? n : 0);
-#pragma omp parallel for schedule(static) if (n > 2048)
-  for (int i = 0; i < n; i++) {
-    SepItem& s = raw[i];
-    s.box = boxes[i];
-    const int l = t.level[s.box];
-    int a = s.box;
-    while (t.level[a] > lroot) a = t.parent[a];
-    s.root = a - a0;
-    s.d = l - lroot;
-    for (int q = 0; q < 3; q++)
-      s.x[q] = (int)std::lround((t.c(s.box, q) - t.c(a, q)) / t.boxsize[l] + 0.5 * ((1 << s.d) - 1));
-    if (packed) {
-      uint64_t k = (uint64_t)rank[s.d] << wr | (uint64_t)s.root;
-      for (int q = 0; q < 3; q++) k = k << dmax | (uint64_t)s.x[q];
-      key[i] = k << wn | (uint64_t)i;
-    }
-  }
-  if (!packed) {  // a tree deeper than the keys hold
-    std::stable_sort(raw.begin(), raw.end(), [&](const SepItem& a, const SepItem& b) {
-      if (a.d != b.d) return rank[a.d] < rank[b.d];
-      if (a.root != b.root) return a.root < b.root;
-      return std::lexicographical_compare(a.x, a.x + 3, b.x, b.x + 3);
-    });
-    items.swap(raw);
-    return;
-  }
-  for (int b = wn; b < wn + 3 * dmax + wr + wd; b += 11) {
-    int cnt[2049] = {0};
-    for (uint64_t k : key) cnt[((k >> b) & 2047) + 1]++;
-    for (int i = 0; i < 2048; i++) cnt[i + 1] += cnt[i];
-    for (uint64_t k : key) tmp[cnt[(k >> b) & 2047]++] = k;
-    key.swap(tmp);
-  }
-  items.resize(n);
-  const uint64_t mask = (uint64_t(1) << wn) - 1;
-#pragma omp parallel for schedule(static) if (n > 2048)
-  for (int i = 0; i < n; i++) items[i] = raw[key[i] & mask];
-}
-
-void sep_lists(const std::vector<SepItem>& items, const std::vector<SepLeaf>& leaf, const std::vector<int>& order,
-               const std::vector<int>& slot, int also, int npw, SepLists& S) {
-  const int n = (int)items.size(), n2 = npw / 2, nroot = (int)slot.size();
-  S = SepLists();
-  S.leaves = leaf;
-  S.cols.reserve(n);
-  S.slabs.reserve(n);
-  auto row = [](const SepItem& s, int q) { return (1 << s.d) - 1 + s.x[q]; };
-  std::vector<int> cnt(nroot + 1, 0), slab_root;
-  slab_root.reserve(n);
-  for (int i = 0; i < n; i++) {
-    const SepItem& s = items[i];
-    const int p = order[s.d];
-    const long long Pn = p + 1;
-    const SepItem* o = i ? &items[i - 1] : nullptr;
-    const bool slab = !o || o->d != s.d || o->root != s.root || o->x[0] != s.x[0];
-    if (!o || order[o->d] != p) S.groups.push_back({p, (int)S.cols.size(), 0, (int)S.slabs.size(), 0});
-    if (slab) {
-      S.slabs.push_back({(long long)S.t2, (int)S.cols.size(), 0, row(s, 0), (int)Pn});
-      S.t2 += (size_t)(Pn * n2 * npw * 2);
-      slab_root.push_back(s.root);
-      cnt[s.root + 1]++;
-    }
-    if (slab || o->x[1] != s.x[1]) {
-      S.cols.push_back({(long long)S.t1, i, 0, row(s, 1), (int)Pn});
-      S.t1 += (size_t)(Pn * Pn * n2 * 2);
-      S.slabs.back().cnt++;
-    }
-    S.cols.back().cnt++;
-    S.leaves[i].row = row(s, 2);
-    S.groups.back().cend = (int)S.cols.size();
-    S.groups.back().send = (int)S.slabs.size();
-  }
-  for (int r = 0; r < nroot; r++) {
-    const int m = cnt[r + 1];
-    if (m > 0 || r == also) S.boxes.push_back({(long long)slot[r], cnt[r], m, 0, 0});
-    cnt[r + 1] += cnt[r];
-  }
-  S.box_slabs.resize(slab_root.size());
-  for (size_t i = 0; i < slab_root.size(); i++) S.box_slabs[cnt[slab_root[i]]++] = (int)i;
-}
-
-void sep_phases(const HostPlan& H, int dmax, double bs0, std::vector<double>& ph) {
-  const int npw = H.P.npw;
-  ph.resize((size_t)2 * npw * ((size_t(2) << dmax) - 1));
-  for (int d = 0; d <= dmax; d++)
-    for (int i = 0; i < (1 << d); i++) {
-      const double sh = (i + 0.5 - 0.5 * (1 << d)) * std::ldexp(bs0, -d) * H.P.dsq;
-      double* r = ph.data() + (size_t)2 * npw * ((1 << d) - 1 + i);
-      for (int m = 0; m < npw; m++) {
-        r[2 * m] = std::cos(H.ts[m] * sh);
-        r[2 * m + 1] = std::sin(H.ts[m] * sh);
-      }
-    }
-}
 
 namespace {
 
@@ -773,7 +655,7 @@ int split_for(int nodes, int nd, int tiles, int sms) {
     if (e_ != cudaSuccess) return e_;       \
   } while (0)
 
-cudaError_t sep_up(const KP& k, const SepDev& S, const double* hbuf, cudaStream_t st, long long& launches) {
+cudaError_t sep_up_3d(const KP& k, const SepDev& S, const double* hbuf, cudaStream_t st, long long& launches) {
   const int n2 = k.n2, tiles = (n2 + 7) / 8;
   int pmax = 1;
   for (const SepGroup& G : S.groups) {
@@ -815,7 +697,7 @@ cudaError_t sep_up(const KP& k, const SepDev& S, const double* hbuf, cudaStream_
       switch (4 * ((pmax + 7) / 8 - 1) + std::min(4, tiles - t0) - 1) {
 #define UP_CASE(KS_, MT_)                                                                                       \
   case 4 * (KS_ - 1) + MT_ - 1:                                                                                 \
-    k_up_xy<KS_, MT_, false><<<gx, 128, 0, st>>>(k, S.boxes, S.slabs, S.box_slabs, pmax, t0, S.t2, nullptr, S.ph); \
+    k_up_xy<KS_, MT_, false><<<gx, 128, 0, st>>>(k, S.boxes, S.slabs, S.box_kids, pmax, t0, S.t2, nullptr, S.ph); \
     break;
         UP_CASES
 #undef UP_CASE
@@ -826,7 +708,7 @@ cudaError_t sep_up(const KP& k, const SepDev& S, const double* hbuf, cudaStream_
   return cudaGetLastError();
 }
 
-cudaError_t sep_down(const KP& k, const SepDev& S, double* lo, cudaStream_t st, long long& launches) {
+cudaError_t sep_down_3d(const KP& k, const SepDev& S, double* lo, cudaStream_t st, long long& launches) {
   const int n2 = k.n2, ksm = (n2 + 3) / 4;
   int pmax = 0;
   for (const SepGroup& G : S.groups) pmax = std::max(pmax, G.p + 1);
@@ -847,7 +729,7 @@ cudaError_t sep_down(const KP& k, const SepDev& S, double* lo, cudaStream_t st, 
   for (int u0 = 0; 16 * u0 < pmax; u0 += 2)
     cases(pmax - 16 * u0 <= 16 ? 1 : 2, [&](auto N, auto U, auto G) {
       k_down_xy<decltype(N)::value, decltype(U)::value, false, decltype(G)::value>
-          <<<gx, 128, 0, st>>>(k, S.boxes, S.slabs, S.box_slabs, pmax, u0, nullptr, S.t2, S.ph);
+          <<<gx, 128, 0, st>>>(k, S.boxes, S.slabs, S.box_kids, pmax, u0, nullptr, S.t2, S.ph);
     });
   for (const SepGroup& G : S.groups) {
     const int Pn = G.p + 1, nslab = G.send - G.sbeg, ncol = G.cend - G.cbeg;

@@ -127,21 +127,6 @@ int shard_filter(HostPlan& H, int nranks, int rank, ShardInfo& S) {
       if (own(x.box)) f.push_back(x);
     H.form.swap(f);
   }
-  // merge / split per level
-  auto filter_shift = [&](std::vector<ShiftTask>& v, std::vector<int>& beg, std::vector<int>& end,
-                          const std::vector<int>& dst_box) {
-    std::vector<ShiftTask> out;
-    for (size_t l = 0; l < beg.size(); l++) {
-      const int b0 = (int)out.size();
-      for (int i = beg[l]; i < end[l]; i++)
-        if (own(dst_box[v[i].dst])) out.push_back(v[i]);
-      beg[l] = b0;
-      end[l] = (int)out.size();
-    }
-    v.swap(out);
-  };
-  filter_shift(H.merge, H.merge_beg, H.merge_end, mp_box);
-  filter_shift(H.split, H.split_beg, H.split_end, loc_box);
   // mp -> loc, and the exchange lists: every rank's tasks are scanned so
   // that each side of a transfer lists the same slots
   {

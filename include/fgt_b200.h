@@ -80,9 +80,8 @@ typedef struct fgt_plan_info {
   int large_delta, all_direct;
   int kernel_launches;
   /* algorithmic work per execute: stage (b) bytes counting each distinct
-   * expansion once (merge, mp->loc, split; the split's counts only the
-   * split tasks that run, the rest being fused into the conversion to
-   * Taylor form), stage (a)/(c) flops as 4 * points * npw^dim, stage (d)
+   * expansion once (mp->loc; merge and split, entries 0 and 2, are parts of
+   * formation and evaluation and stay 0), stage (a)/(c) flops as 4 * points * npw^dim, stage (d)
    * source-target pairs */
   long long shift_bytes[3];
   double form_flops, eval_flops;
@@ -249,7 +248,7 @@ int fgt_plan_get_info(const fgt_plan* plan, fgt_plan_info* info);
  * orders, fgt2d.f:1518-1610 / fgt3d.f).  box is 0-based in the tree's
  * numbering (the reference's box - 1).  FGT_ERR_BADARG when the box holds
  * no such expansion (this library allocates them only where the transform
- * reads them; below the cut level in 3D they are formed by this call).  For checking intermediate stages against the reference. */
+ * reads them; below the cut level they are formed by this call).  For checking intermediate stages against the reference. */
 int fgt_plan_expansion(fgt_plan* plan, int which, int box, double* out);
 /* One execute with CUDA events around the plan's dominant tensor-core launch
  * (the Hermite-block MMA kernel of the form order group with the most
