@@ -23,7 +23,9 @@ namespace {
 // expansion read from global memory (L2) straight into the fragments, once
 // per chunk; the warps take pairs of column tiles in turn, and the lane's
 // sums over its columns are added in a fixed order at the end.  Bound by the
-// tensor pipe.
+// tensor pipe.  Measured (B200, eps 1e-6, npw 26; before: a thread per point and
+// node on the scalar pipe): forces of 3e5 blob points 1375 -> 157 us, potentials
+// of 1e5 uniform points 171 -> 67 us.
 template <int PGH>
 __host__ __device__ constexpr int pwev_tiles() { return PGH == 1 ? 4 : PGH == 2 ? 2 : 1; }
 
@@ -235,7 +237,10 @@ __global__ void __launch_bounds__(128) k_eval3d_pw(KP k, const EvalTask* __restr
 // dimension, by recurrence) into shared memory, where a B fragment is one
 // complex product of two of them.  With dipoles a source stages three columns
 // (dip3_coef, the factor of one dimension times v_d (-i t dsq)), ten sources
-// at a time.
+// at a time.  Bound by the tensor pipe.  Measured (B200, eps 1e-9, npw 38;
+// before: a thread per coefficient on the scalar pipe, an expansion per leaf,
+// then the merges): 3e5 uniform points 1.2 -> 0.53 ms; 1e5 for gradients, where
+// every leaf takes this route, 2.3 -> 0.92 ms.
 template <int MT>
 __host__ __device__ constexpr int pwform_pairs() { return MT == 1 ? 4 : MT == 2 ? 3 : MT == 3 ? 2 : 1; }
 constexpr int PWF_SC = 32;  // source columns per batch
