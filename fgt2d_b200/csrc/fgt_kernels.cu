@@ -2530,9 +2530,11 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
     // one density, one component per point: the random gather of the charges
     if (!pot && (nc == 1 || (!grad && !hess))) return;
     if (nd == 1 && nc == 1) k_gather1<<<gb, 256, 0, st>>>(in, inv, n, pot);
-    else
-      k_unsort<<<8 * D.sm_count, 256, 0, st>>>(in, inv, n, nd, nc > 1 ? P.dim * nd : 0, nc > 1 + P.dim ? nh * nd : 0,
-                                               pot, grad, hess);
+    else {
+      const int w1 = nc > 1 ? P.dim * nd : 0, w2 = nc > 1 + P.dim ? nh * nd : 0;
+      const long long ctas = ((long long)n * (nd + w1 + w2) + 255) / 256;
+      k_unsort<<<(int)std::min<long long>(8 * D.sm_count, ctas), 256, 0, st>>>(in, inv, n, nd, w1, w2, pot, grad, hess);
+    }
     launches++;
   };
   if (ph2 && P.ifpgh > 0 && P.ns > 0) unsort(D.psort, D.isrc_inv, P.ns, k.nc_s, outs.pot, outs.grad, outs.hess);
