@@ -1633,6 +1633,90 @@ cudaError_t device_pool_setup() {
   return cudaSuccess;
 }
 
+// What changes a plan's arithmetic is chosen by order from the tasks of the
+// whole transform (a shard's: of all its ranks).
+//
+// Formation: sources per partial block (chunk), and in 2D the orders whose
+// leaves (or chunks) take a warp each (k_form2d_mma).
+struct FormRules {
+  int chunk = 1 << 30;
+  std::vector<uint8_t> warp;
+};
+FormRules form_rules(const Params& P, const std::vector<FormTask>& tasks, int sms) {
+  FormRules R;
+  long long nsrc = 0;
+  for (const FormTask& f : tasks)
+    if (f.route == ROUTE_HERMITE) nsrc += f.n;
+  // Sources per partial block: at most 4096, fewer (whole batches of the
+  // kernel) where that leaves SMs without a CTA
+  if (P.dim == 3) {
+    const int batch = P.ifdipole ? FORM3_SB / 3 : FORM3_SB;
+    R.chunk = (int)std::min<long long>(4096 / batch, std::max<long long>(6, nsrc / (8LL * sms * batch))) * batch;
+    return R;
+  }
+  // 2D: about eight chunks per SM of at least 512 sources, whole passes of
+  // the kernels' four warps (four leaves of 75000 sources in four CTAs took
+  // 0.76 ms of a 0.80 ms execute, 0.02 of 0.08 cut up)
+  R.chunk = (int)std::max<long long>(512, (nsrc / (8LL * sms) + 255) / 256 * 256);
+  // leaves (or chunks) of about two blocks of source columns or less, a warp each
+  std::vector<long long> n(P.ntermmax + 1, 0), cnt(P.ntermmax + 1, 0);
+  for (const FormTask& f : tasks)
+    if (f.route == ROUTE_HERMITE) {
+      n[f.p] += f.n;
+      cnt[f.p] += f.n <= R.chunk ? 1 : (f.n + R.chunk - 1) / R.chunk;
+    }
+  R.warp.resize(n.size());
+  for (size_t p = 0; p < n.size(); p++) R.warp[p] = n[p] * (P.ifdipole ? 2 : 1) <= 80 * cnt[p];
+  return R;
+}
+// Taylor evaluation: the orders evaluated from blocks (the others from the
+// columns, 3D) and, in 2D, the warps per task of k_eval2d_mma (0: Horner).
+struct EvalRules {
+  std::vector<uint8_t> blocks, per;
+};
+EvalRules eval_rules(const Params& P, const std::vector<EvalTask>& tasks, int pgh) {
+  EvalRules R;
+  const int np = P.ntermmax + 1, n2 = P.npw / 2;
+  R.blocks.assign(np, P.dim == 2);
+  R.per.assign(np, 0);
+  if (P.dim == 2) {
+    // k_eval2d_mma where it is the faster one (its comment), with as many
+    // warps per task as have points
+    std::vector<long long> n(np, 0), cnt(np, 0);
+    for (const EvalTask& e : tasks)
+      if (e.route == ROUTE_TAYLOR) {
+        n[e.p] += e.n;
+        cnt[e.p] += e.n <= 256 ? 1 : (e.n + 255) / 256;
+      }
+    const long long tile = pgh <= 1 ? 16 : 8;
+    for (int p = 24; p < std::min(40, np); p++)
+      if (n[p] <= 72 * cnt[p]) R.per[p] = n[p] > 3 * tile * cnt[p] ? 4 : n[p] > tile * cnt[p] ? 2 : 1;
+    return R;
+  }
+  // Multiply-adds on the FP64 pipe of the two ways, each with what its
+  // kernels lose beside them (measured, 3D, eps 1e-6 and 1e-9): a leaf's
+  // block costs P^3 (n2 + 44) (44: its two passes over memory) and its
+  // points 2 P^3 per 32 begun; the column way 1.5 * 2 n2 P^2 per 8 points
+  // begun.  Mixed potentials up to order 15 are evaluated on the BF16
+  // tensor cores from the blocks; rows above 30 coefficients have no
+  // block evaluation.
+  std::vector<long long> leaves(np, 0), n32(np, 0), n8(np, 0);
+  for (size_t t = 0; t < tasks.size(); t++) {  // a leaf's tasks are consecutive
+    const EvalTask& e = tasks[t];
+    if (e.route != ROUTE_TAYLOR) continue;
+    leaves[e.p] += t == 0 || tasks[t - 1].box != e.box;
+    n32[e.p] += 32 * ((e.n + 31) / 32);
+    n8[e.p] += 8 * ((e.n + 7) / 8);
+  }
+  for (int p = 0; p < np; p++) {
+    const double Pn = p + 1, P3 = Pn * Pn * Pn;
+    const double cb = P3 * (n2 + 44) * leaves[p] + 2.0 * P3 * pgh * n32[p];
+    const double cc = 3.0 * n2 * Pn * Pn * pgh * n8[p];
+    R.blocks[p] = Pn <= 30 && ((Pn <= 16 && pgh == 1 && !P.ifdipole) || cb < cc);
+  }
+  return R;
+}
+
 cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_isrc, const int* d_itarg,
                                cudaStream_t pst, size_t* size_only) {
   const auto tnow = [] {
@@ -1723,7 +1807,8 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   std::vector<ColTask> ctask;
   uvector<SepItem> dn_items;
   std::vector<long long> first;   // first task of every item
-  std::vector<uint8_t> blocks;    // by order: evaluated from Taylor blocks
+  FormRules frules;
+  EvalRules erules;
   long long nh = 0, nct = 0;
   const int pgh = std::max(1, std::max(P.ifpgh, P.ifpghtarg)), cp = sep_col_points(pgh);
   auto build_up = [&] {
@@ -1733,19 +1818,9 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     std::vector<SepLeaf> leaf(D.form_hermite_n);
     std::vector<int> box(D.form_hermite_n);
     int ni = 0;
-    // Sources per partial block: at most 4096, fewer (whole batches of the
-    // kernel) where that leaves SMs without a CTA
-    long long nsrc = 0, hoff = 0;
-    for (int i = 0; i < D.form_hermite_n; i++) nsrc += form[i].n;
-    if (P.dim == 3) {
-      const int batch = P.ifdipole ? FORM3_SB / 3 : FORM3_SB;
-      D.form_chunk = (int)std::min<long long>(4096 / batch, std::max<long long>(6, nsrc / (8LL * D.sm_count * batch))) * batch;
-    } else {
-      // 2D: about eight chunks per SM of at least 512 sources, whole passes of
-      // the kernels' four warps (four leaves of 75000 sources in four CTAs took
-      // 0.76 ms of a 0.80 ms execute, 0.02 of 0.08 cut up)
-      D.form_chunk = (int)std::max<long long>(512, (nsrc / (8LL * D.sm_count) + 255) / 256 * 256);
-    }
+    long long hoff = 0;
+    frules = form_rules(P, H.form_of_all.empty() ? H.form : H.form_of_all, D.sm_count);
+    D.form_chunk = frules.chunk;
     const int chunk = D.form_chunk;
     for (const SepItem& s : sep_items) {
       const int i = s.num;
@@ -1806,39 +1881,17 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     }
   };
   auto build_down = [&] {
-    const int n2 = P.npw / 2;
     uvector<SepItem> items(sep_items.size());
     int ni = 0;
     for (const SepItem& s : sep_items)
       if (run[s.num].second > 0) items[ni++] = s;
     items.resize(ni);
-    blocks.assign(D.eval_pmax + 2, P.dim == 2);
-    for (size_t i = 0; i < items.size() && P.dim == 3;) {
-      // Multiply-adds on the FP64 pipe of the two ways, each with what its
-      // kernels lose beside them (measured, 3D, eps 1e-6 and 1e-9): a leaf's
-      // block costs P^3 (n2 + 44) (44: its two passes over memory) and its
-      // points 2 P^3 per 32 begun; the column way 1.5 * 2 n2 P^2 per 8 points
-      // begun.  Mixed potentials up to order 15 are evaluated on the BF16
-      // tensor cores from the blocks; rows above 30 coefficients have no
-      // block evaluation.
-      const int p = sep_order_of[items[i].d];
-      const double Pn = p + 1, P3 = Pn * Pn * Pn;
-      double cb = 0.0, cc = 0.0;
-      size_t j = i;
-      for (; j < items.size() && sep_order_of[items[j].d] == p; j++) {
-        cb += P3 * (n2 + 44);
-        for (int t = run[items[j].num].first; t < run[items[j].num].second; t++) {
-          cb += 2.0 * P3 * pgh * (32 * ((ev[t].n + 31) / 32));
-          cc += 3.0 * n2 * Pn * Pn * pgh * (8 * ((ev[t].n + 7) / 8));
-        }
-      }
-      blocks[p] = Pn <= 30 && ((Pn <= 16 && pgh == 1 && !P.ifdipole) || cb < cc);
-      i = j;
-    }
+    erules = eval_rules(P, H.eval_of_all.empty() ? H.eval : H.eval_of_all, pgh);
+    const std::vector<uint8_t>& blocks = erules.blocks;
     std::vector<long long> len(sep_order_of.size());  // doubles of a block, by depth
     for (size_t d = 0; d < len.size(); d++) {
       const long long p = sep_order_of[d], Pn = p + 1, E = (Pn + 1) & ~1LL;
-      len[d] = p < (int)blocks.size() && blocks[p] ? P.nd * Pn * E * (P.dim == 3 ? Pn : 1) : 0;
+      len[d] = blocks[p] ? P.nd * Pn * E * (P.dim == 3 ? Pn : 1) : 0;
     }
     std::vector<SepLeaf> leaf(ni);
     long long lo = 0;
@@ -1854,23 +1907,16 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
       G.blocks = blocks[G.p];
       const int step = G.blocks ? 256 : cp;
       const long long t0 = G.blocks ? nh : nct;
-      long long n = 0, at = t0;
+      long long at = t0;
       const int i0 = dn.cols[G.cbeg].beg, i1 = dn.cols[G.cend - 1].beg + dn.cols[G.cend - 1].cnt;
       for (int i = i0; i < i1; i++) {
         const std::pair<int, int> r = run[items[i].num];
         at0[i] = at;
-        for (int t = r.first; t < r.second; t++) {
-          at += ev[t].n <= step ? 1 : (ev[t].n + step - 1) / step;
-          n += ev[t].n;
-        }
+        for (int t = r.first; t < r.second; t++) at += ev[t].n <= step ? 1 : (ev[t].n + step - 1) / step;
       }
       (G.blocks ? nh : nct) = at;
       (G.blocks ? D.horner_groups : D.ctask_groups).push_back({G.p, (int)t0, (int)at});
-      // k_eval2d_mma where it is the faster one (its comment), with as many
-      // warps per task as have points
-      const long long cnt = at - t0, tile = pgh <= 1 ? 16 : 8;
-      if (P.dim == 2 && G.p >= 24 && G.p < 40 && n <= 72 * cnt)
-        D.horner_groups.back().per = n > 3 * tile * cnt ? 4 : n > tile * cnt ? 2 : 1;
+      if (G.blocks) D.horner_groups.back().per = erules.per[G.p];
     }
     dn_items.swap(items);
     first.swap(at0);
@@ -1885,11 +1931,9 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   // launch groups of equal order among the Hermite form tasks
   for (int t = 0; t < D.form_hermite_n;) {
     int u = t;
-    long long n = 0;
-    for (; u < D.form_hermite_n && form[u].p == form[t].p; u++) n += form[u].n;
+    while (u < D.form_hermite_n && form[u].p == form[t].p) u++;
     D.form_groups.push_back({form[t].p, t, u});
-    // 2D: leaves of about two blocks of source columns or less, a warp each
-    D.form_groups.back().warp = n * (P.ifdipole ? 2 : 1) <= 80LL * (u - t);
+    if (P.dim == 2 && sep) D.form_groups.back().warp = frules.warp[form[t].p];
     t = u;
   }
 
@@ -1919,7 +1963,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
         long long at = first[l];
         for (int t = r.first; t < r.second; t++) {
           const EvalTask& e = ev[t];
-          if (blocks[e.p])
+          if (erules.blocks[e.p])
             for (int q = 0; q < e.n; q += 256)
               horner[at++] = {e.box, e.set, e.i0 + q, std::min(256, e.n - q), e.p, dn.leaves[l].off};
           else

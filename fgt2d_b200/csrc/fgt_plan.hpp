@@ -87,6 +87,10 @@ struct HostPlan {
   std::vector<M2LTask> m2l;
   std::vector<M2LNbr> m2l_nbr;
   std::vector<EvalTask> eval;
+  // a shard's plan: the form and evaluation tasks of every rank, from which the
+  // kernels of an order are chosen (all ranks and the unsharded plan alike)
+  std::vector<FormTask> form_of_all;
+  std::vector<EvalTask> eval_of_all;
   uvector<DirTask> dir;
   uvector<SrcRange> dir_src;
   // The near-field arrays built on the GPU instead (build_near_tasks_device;

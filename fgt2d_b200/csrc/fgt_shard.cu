@@ -20,9 +20,11 @@
 // expansions that other ranks' mp -> loc tasks read and receives the ones
 // its own tasks read.  The near field needs no exchange because the source
 // coordinates and charges are replicated.  Every owned point is computed by
-// the same tasks in the same order as without the shard, so the sum of the
-// ranks' outputs (zero at the points a rank does not own) equals the
-// one-GPU result bit for bit.
+// the same tasks in the same order as without the shard, and every choice
+// that changes the arithmetic (sources per partial block, the kernels of an
+// order) is made from the tasks of all ranks, so the sum of the ranks' outputs
+// (zero at the points a rank does not own) equals the one-GPU result bit for
+// bit.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -126,6 +128,7 @@ int shard_filter(HostPlan& H, int nranks, int rank, ShardInfo& S) {
     for (const FormTask& x : H.form)
       if (own(x.box)) f.push_back(x);
     H.form.swap(f);
+    H.form_of_all.swap(f);
   }
   // mp -> loc, and the exchange lists: every rank's tasks are scanned so
   // that each side of a transfer lists the same slots
@@ -164,6 +167,7 @@ int shard_filter(HostPlan& H, int nranks, int rank, ShardInfo& S) {
     for (const EvalTask& x : H.eval)
       if (own(x.box)) e.push_back(x);
     H.eval.swap(e);
+    H.eval_of_all.swap(e);
   }
   // near field: the box of a task is the leaf holding its first point
   {
