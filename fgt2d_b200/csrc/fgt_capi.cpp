@@ -436,12 +436,11 @@ int transform_impl(fgt_ctx* ctx, int dim, int nd, double delta, double eps, int 
                    const double* rnormal, const double* dipstr,
                    int ifpgh, double* pot, double* grad, double* hess, int nt, const double* targ,
                    int ifpghtarg, double* pottarg, double* gradtarg, double* hesstarg) {
-  const bool on_device = tree_on_device(ctx, ns, targ ? nt : 0, targ == sources);
-  int st = check_args(dim, nd, delta, eps, ns, sources, ifcharge, ifdipole, ifpgh, nt, targ, ifpghtarg,
-                      !on_device);
+  // coordinates and strengths are looked at by the plan and its execute, on
+  // whichever side the tree is built: a refusal there zeroes the outputs below
+  int st = check_args(dim, nd, delta, eps, ns, sources, ifcharge, ifdipole, ifpgh, nt, targ, ifpghtarg, false);
   if (st != FGT_OK) return st;
   if (ns > 0 && ((ifcharge && !charge) || (ifdipole && (!rnormal || !dipstr)))) return FGT_ERR_BADARG;
-  if (!on_device && ns > 0 && ifcharge && !finite_all(charge, (size_t)ns * nd)) return FGT_ERR_BADARG;
   // outputs are written in full on success; zero them when nothing runs or
   // the call fails
   const size_t nh = dim == 2 ? 3 : 6;
