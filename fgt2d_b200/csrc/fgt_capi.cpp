@@ -365,12 +365,9 @@ int run_device(fgt_plan* p, const Inputs& in, const Outputs& o, cudaStream_t st,
   return FGT_OK;
 }
 
-// Finiteness of n source strengths on their way in: small arrays are looked
-// at on the host (the device check waits for its answer).
-int check_strengths(fgt_plan* p, const double* host, const double* dev, size_t n) {
-  if (n <= 16384) return finite_all(host, n) ? FGT_OK : FGT_ERR_BADARG;
-  return check_finite_device(p, dev, n);
-}
+// Arrays of up to this many source strengths are looked at on the host, before
+// anything is copied (the device check waits for its answer).
+constexpr size_t HOST_CHECKED = 16384;
 
 // Source strengths in from the host (charges and/or dipole directions and
 // strengths, as the plan's flags say), every execute output the plan
@@ -382,22 +379,32 @@ int exec_host(fgt_plan* p, const double* charge, const Outputs& host, const doub
   cudaStream_t st = p->ctx->stream;
   CKS(cudaSetDevice(p->ctx->device));
   const size_t ns = P.ns, nt = P.nt, nd = P.nd, nh = P.dim == 2 ? 3 : 6;
+  if ((P.ifcharge && !charge && ns) || (P.ifdipole && (!rnormal || !dipstr) && ns)) return FGT_ERR_BADARG;
+  struct Strengths {
+    const double *host, *pre;
+    double* dev;
+    size_t n;
+  };
+  const Strengths all[3] = {{P.ifcharge ? charge : nullptr, p->pre_q, p->d_chg, ns * nd},
+                            {P.ifdipole ? rnormal : nullptr, p->pre_rn, p->d_rn, ns * P.dim},
+                            {P.ifdipole ? dipstr : nullptr, p->pre_ds, p->d_ds, ns * nd}};
+  for (const Strengths& a : all)
+    if (a.host && a.n <= HOST_CHECKED && !finite_all(a.host, a.n)) {
+      // the caller has its arrays back: no upload of a one-shot call is still reading them
+      if (p->pre_done) CKS(cudaEventSynchronize(p->pre_done));
+      return FGT_ERR_BADARG;
+    }
   if (p->pre_done) CKS(cudaStreamWaitEvent(st, p->pre_done, 0));  // strengths uploaded with the points
+  for (const Strengths& a : all)
+    if (a.host && a.host != a.pre) CKS(cudaMemcpyAsync(a.dev, a.host, a.n * 8, cudaMemcpyHostToDevice, st));
+  for (const Strengths& a : all)
+    if (a.host && a.n > HOST_CHECKED) {
+      const int s = check_finite_device(p, a.dev, a.n);  // waits for the copies
+      if (s != FGT_OK) return s;
+    }
   Inputs in;
-  if (P.ifcharge) {
-    if (!charge && ns) return FGT_ERR_BADARG;
-    if (charge != p->pre_q) CKS(cudaMemcpyAsync(p->d_chg, charge, ns * nd * 8, cudaMemcpyHostToDevice, st));
-    int s = check_strengths(p, charge, p->d_chg, ns * nd);
-    if (s != FGT_OK) return s;
-    in.charge = p->d_chg;
-  }
+  if (P.ifcharge) in.charge = p->d_chg;
   if (P.ifdipole) {
-    if ((!rnormal || !dipstr) && ns) return FGT_ERR_BADARG;
-    if (rnormal != p->pre_rn) CKS(cudaMemcpyAsync(p->d_rn, rnormal, ns * P.dim * 8, cudaMemcpyHostToDevice, st));
-    if (dipstr != p->pre_ds) CKS(cudaMemcpyAsync(p->d_ds, dipstr, ns * nd * 8, cudaMemcpyHostToDevice, st));
-    int s = check_strengths(p, rnormal, p->d_rn, ns * P.dim);
-    if (s == FGT_OK) s = check_strengths(p, dipstr, p->d_ds, ns * nd);
-    if (s != FGT_OK) return s;
     in.rnormal = p->d_rn;
     in.dipstr = p->d_ds;
   }

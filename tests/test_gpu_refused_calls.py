@@ -30,3 +30,61 @@ def test_no_sources(fgt):
     ctx = fgt.Context(0)
     _, pt = fgt.transform(2, 1, 1e-3, 1e-6, np.zeros((0, 2)), np.zeros((0, 1)), trg, 0, 1, ctx=ctx)
     assert np.all(pt == 0.0)
+
+
+def _stalled(ctx, seconds=0.3):
+    """Work of about that long queued on the context's stream, and its end."""
+    import torch
+    s = torch.cuda.ExternalStream(ctx.stream)
+    end = torch.cuda.Event()
+    with torch.cuda.stream(s):
+        torch.cuda._sleep(int(seconds * 1.9e9))
+        end.record(s)
+    return end
+
+
+def test_refused_call_leaves_no_copy_behind(fgt):
+    """A one-shot call that is refused for its strengths returns when nothing
+    reads the caller's (pinned) arrays any more."""
+    import torch
+    ctx = fgt.Context(0)
+    rng = np.random.default_rng(3)
+    pin = [torch.from_numpy(a).pin_memory() for a in (rng.random((500, 2)), rng.random((500, 1)))]
+    src, q = (a.numpy() for a in pin)
+    fgt.transform(2, 1, 1e-3, 1e-6, src, q, ctx=ctx)
+    q[499] = np.inf
+    end = _stalled(ctx)
+    with pytest.raises(fgt.FGTError) as e:
+        fgt.transform(2, 1, 1e-3, 1e-6, src, q, ctx=ctx)
+    done = end.query()  # the uploads follow it
+    torch.cuda.synchronize()
+    assert e.value.status == 1 and done
+
+
+@pytest.mark.parametrize("bad", ["charge", "rnormal", "dipstr"])
+def test_refused_execute_copies_nothing(fgt, bad):
+    """Strengths that are looked at on the host are refused before any copy of
+    them is queued."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    ctx = fgt.Context(0)
+    rng = np.random.default_rng(4)
+    n = 500
+    plan = fgt.Plan(ctx, 2, 1, 1e-3, 1e-6, rng.random((n, 2)), None, 1, 0, 1, 1)
+    a = dict(charge=rng.random((n, 1)), rnormal=rng.random((n, 2)), dipstr=rng.random((n, 1)))
+    pot = np.zeros((n, 1))
+
+    def run():
+        p = lambda x: fgt._p(x)
+        return fgt.lib().fgt_plan_execute_host_full(plan._h, p(a["charge"]), p(a["rnormal"]), p(a["dipstr"]), p(pot),
+                                                    None, None, None, None, None)
+
+    assert run() == 0
+    a[bad][0, 0] = np.nan
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        st = run()
+        torch.cuda.synchronize()
+    copies = [e.name for e in prof.events() if "HtoD" in e.name]
+    plan.close()
+    assert st == 1 and not copies, copies
