@@ -202,8 +202,9 @@ int plan_device(fgt_plan* p, const double* src_host, const double* trg_host) {
   if (!P.large_delta) {
     CKS(device_plan_create(p->H, p->D));
     p->have_device = true;
-    CKS(device_plan_set_points(p->D, p->d_src, p->d_trg, st));
   }
+  CKS(cudaStreamSynchronize(st));  // the points are up: the caller may change its arrays
+  if (!P.large_delta) CKS(device_plan_set_points(p->D, p->d_src, p->d_trg, st));
   return FGT_OK;
 }
 
