@@ -200,7 +200,7 @@ int plan_device(fgt_plan* p, const double* src_host, const double* trg_host) {
   cudaStream_t st = p->ctx->stream;
   if (shard_filter(p->H, p->shard_n, p->shard_r, p->shard) != 0) return FGT_ERR_BADARG;
   if (!P.large_delta) {
-    CKS(device_plan_create(p->H, p->D));
+    CKS(device_plan_create(p->H, p->D, nullptr, nullptr, st));
     p->have_device = true;
   }
   CKS(cudaStreamSynchronize(st));  // the points are up: the caller may change its arrays

@@ -37,3 +37,30 @@ def test_points_may_change_after_plan_creation(fgt, delta, tree):
     got = plan.execute_host(src, q, trg)
     plan.close()
     assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1])
+
+
+@pytest.mark.parametrize("entry", ["plan", "call"])
+@pytest.mark.parametrize("tree", [None, "host"])
+def test_no_wait_for_the_default_stream(fgt, entry, tree):
+    """A plan, its execute and a drop-in call run beside work on the default
+    stream instead of after it."""
+    import torch
+    ctx = fgt.Context(0) if tree is None else fgt.Context(0, tree=tree)
+    rng = np.random.default_rng(9)
+    n = 900
+    src, q = rng.random((n, 2)), rng.random((n, 1))
+
+    def go():
+        if entry == "call":
+            return fgt.transform(2, 1, 1e-3, 1e-6, src, q, ctx=ctx)[0]
+        plan = fgt.Plan(ctx, 2, 1, 1e-3, 1e-6, src, None, 1, 0)
+        pot = plan.execute_host(src, q)[0]
+        plan.close()
+        return pot
+
+    ref = go()
+    end = _stall(torch.cuda.default_stream(), 0.5)
+    got = go()
+    waited = end.query()
+    torch.cuda.synchronize()
+    assert np.array_equal(got, ref) and not waited
