@@ -173,7 +173,7 @@ def _p(a):
 class Context:
     """One CUDA device, its stream and the precision mode."""
 
-    def __init__(self, device=0, precision="auto", host_threads=0, tree="device", scheme="planewave"):
+    def __init__(self, device=0, precision="auto", host_threads=0, tree="auto", scheme="planewave"):
         L = lib()
         h = _vp()
         _check(L.fgt_ctx_create(int(device), ctypes.byref(h)), "fgt_ctx_create")
@@ -185,8 +185,9 @@ class Context:
             L.fgt_ctx_set_host_threads(self._h, int(host_threads))
 
     def set_tree(self, where):
-        """Where plans build their tree: "device" (point work on the GPU) or "host"."""
-        _check(lib().fgt_ctx_set_tree(self._h, {"device": 0, "host": 1}[where]), "fgt_ctx_set_tree")
+        """Where plans build their tree: "device" (point work on the GPU), "host",
+        or "auto": the host up to 3000 points, else the device."""
+        _check(lib().fgt_ctx_set_tree(self._h, {"device": 0, "host": 1, "auto": 2}[where]), "fgt_ctx_set_tree")
 
     def set_scheme(self, scheme):
         """The algorithm of plans created afterwards: "planewave" (2d/planewave,

@@ -30,7 +30,7 @@ struct fgt_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   int precision = FGT_PREC_AUTO;
-  int tree = FGT_TREE_DEVICE;
+  int tree = FGT_TREE_AUTO;
   int nthreads = 0;
   int scheme = FGT_SCHEME_PLANEWAVE;  // the algorithm of the context's plans
   // uploads of a one-shot call's source strengths: they follow the points on
@@ -227,14 +227,18 @@ struct OmpTeam {
   ~OmpTeam() { omp_set_num_threads(old); }
 };
 
-// Whether a plan's tree is built on the device: the context's choice, but up
-// to 3000 points the host builds the same tree in less time than the device
-// build's read-backs take (B200 and 16 host cores, drop-in call with 1000 2D
-// points: 0.98 ms with the device build, 0.20 ms with the host's; at 4000
-// points the host build alone takes 0.3 to 1.3 ms, the device build 0.9).
+// Whether a plan's tree is built on the device: the context's choice, or for
+// FGT_TREE_AUTO from 3000 points on.  Up to there the host builds the same tree
+// in less time than the device build's read-backs take (B200 and 16 host cores,
+// drop-in calls, device build -> host's: 1000 points in 2D 0.98 -> 0.20 ms, in
+// 3D 0.81 -> 0.18; 2900 points in 2D, delta 1e-6 1.27 -> 0.57, on a circle 1.34
+// -> 0.90, in 3D 1.24 -> 0.93; at 4000 points the host build alone takes 0.3 to
+// 1.3 ms, the device build 0.9).  Targets that are the sources are built once
+// on the device and count there.
 constexpr int HOST_TREE_POINTS = 3000;
-bool tree_on_device(const fgt_ctx* c, int ns, int nt, bool same) {
-  return c->tree == FGT_TREE_DEVICE && (long long)ns + (same ? 0 : nt) > HOST_TREE_POINTS;
+bool tree_on_device(const fgt_ctx* c, int ns, const double* sources, int nt, const double* targ) {
+  if (c->tree != FGT_TREE_AUTO) return c->tree == FGT_TREE_DEVICE;
+  return (long long)ns + (targ && !(targ == sources && nt == ns) ? nt : 0) > HOST_TREE_POINTS;
 }
 
 int plan_create_device_tree(fgt_plan* p, int dim, int nd, double delta, double eps, int ns,
@@ -564,7 +568,7 @@ int fgt_ctx_set_precision(fgt_ctx* c, int precision) {
   return FGT_OK;
 }
 int fgt_ctx_set_tree(fgt_ctx* c, int where) {
-  if (!c || (where != FGT_TREE_DEVICE && where != FGT_TREE_HOST)) return FGT_ERR_BADARG;
+  if (!c || (where != FGT_TREE_DEVICE && where != FGT_TREE_HOST && where != FGT_TREE_AUTO)) return FGT_ERR_BADARG;
   c->tree = where;
   return FGT_OK;
 }
@@ -661,7 +665,7 @@ int plan_create_impl(fgt_ctx* ctx, int dim, int nd, double delta, double eps, in
                      const double* pre_rn, const double* pre_ds) {
   if (!ctx || !out) return FGT_ERR_BADARG;
   *out = nullptr;
-  const bool on_device = tree_on_device(ctx, ns, targ ? nt : 0, targ == sources);
+  const bool on_device = tree_on_device(ctx, ns, sources, nt, targ);
   int st = check_args(dim, nd, delta, eps, ns, sources, ifcharge, ifdipole, ifpgh, nt, targ, ifpghtarg,
                       !on_device);
   if (st != FGT_OK) return st;
@@ -682,7 +686,7 @@ int plan_create_impl(fgt_ctx* ctx, int dim, int nd, double delta, double eps, in
                                  nullptr, ifcharge, ifdipole);
   } else {
     // a small tree: one host thread (a team's start costs more than the work)
-    OmpTeam team(ctx, ctx->tree == FGT_TREE_DEVICE ? 1 : 0);
+    OmpTeam team(ctx, ctx->tree == FGT_TREE_AUTO ? 1 : 0);
     try {
       build_host_plan(p->H, dim, nd, delta, eps, ns, sources, nt, targ, ifpgh, ifpghtarg, ctx->nthreads,
                       ifcharge, ifdipole);
@@ -763,7 +767,7 @@ int fgt_plan_create_shard(fgt_ctx* ctx, int dim, int nd, double delta, double ep
   if (!ctx || !out || nranks < 1 || rank < 0 || rank >= nranks) return FGT_ERR_BADARG;
   *out = nullptr;
   int st = check_args(dim, nd, delta, eps, ns, sources, 1, 0, ifpgh, nt, targ, ifpghtarg,
-                      ctx->tree != FGT_TREE_DEVICE);
+                      ctx->tree == FGT_TREE_HOST);
   if (st != FGT_OK) return st;
   if (ns == 0) return FGT_ERR_BADARG;
   if (!targ) nt = 0;
@@ -774,7 +778,7 @@ int fgt_plan_create_shard(fgt_ctx* ctx, int dim, int nd, double delta, double ep
   p->shard_n = nranks;
   p->shard_r = rank;
   CKS(cudaSetDevice(ctx->device));
-  if (ctx->tree == FGT_TREE_DEVICE) {
+  if (ctx->tree != FGT_TREE_HOST) {
     st = plan_create_device_tree(p.get(), dim, nd, delta, eps, ns, sources, nt, targ, ifpgh, ifpghtarg);
   } else {
     try {

@@ -50,8 +50,10 @@ enum {
 };
 
 enum {
-  FGT_TREE_DEVICE = 0, /* tree build with its point work on the GPU (default) */
-  FGT_TREE_HOST = 1    /* tree build entirely on the host (OpenMP) */
+  FGT_TREE_DEVICE = 0, /* tree build with its point work on the GPU */
+  FGT_TREE_HOST = 1,   /* tree build entirely on the host (OpenMP) */
+  FGT_TREE_AUTO = 2    /* FGT_TREE_HOST on one thread up to 3000 points (sources and separate
+                        * targets), else FGT_TREE_DEVICE (default) */
 };
 
 /* Algorithm of a context's plans (fgt_ctx_set_scheme). */
@@ -99,8 +101,9 @@ int fgt_ctx_set_precision(fgt_ctx* ctx, int precision);
  * 8 (a server's contexts: the cores divided among its workers).  The calling
  * thread's own OpenMP setting is restored when each call returns. */
 int fgt_ctx_set_host_threads(fgt_ctx* ctx, int nthreads);
-/* where plans built with this context build their tree (FGT_TREE_DEVICE or
- * FGT_TREE_HOST); both give the same tree.  No counterpart in the reference,
+/* where plans built with this context build their tree (FGT_TREE_*); all
+ * give the same tree.  Shards (fgt_plan_create_shard) and a server's requests
+ * take the device for FGT_TREE_AUTO.  No counterpart in the reference,
  * whose tree is built on the host (pts_tree_build, pts_tree2d4.f:363-590). */
 int fgt_ctx_set_tree(fgt_ctx* ctx, int where);
 /* Accepted for older callers, without effect: the transforms have no
