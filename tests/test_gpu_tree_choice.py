@@ -32,5 +32,6 @@ def test_tree_choice(fgt, tree, src, trg, device):
         plan = fgt.Plan(ctx, 2, 1, 1e-3, 1e-6, src, trg, 1, 0 if trg is None else 1)
         torch.cuda.synchronize()
     plan.close()
+    # the device build reads counts and boxes back, the host build nothing
     names = {e.name for e in prof.events()}
-    assert any("k_bbox" in n for n in names) == device, names
+    assert any("DtoH" in n for n in names) == device, names
