@@ -38,7 +38,7 @@ struct Outputs {
   double* hesstarg = nullptr;
 };
 
-// n partial blocks of len doubles per density from off on (2D form)
+// n partial blocks of len doubles per density from off on (k_sum_blocks)
 struct BlockSum {
   long long off;
   int len, n;
@@ -191,8 +191,8 @@ struct DevicePlan {
   std::vector<double> group_flops;      // 2 n P^dim per form group (2D) / chunk group (3D)
   std::vector<double> group_alg_flops;  // 4 n npw^dim per form group (2D) / chunk group (3D)
   // Taylor evaluation from the leaves' blocks
-  BlockSum* form2_sums = nullptr;  // 2D: leaves of several partial blocks
-  int form2_nsums = 0;
+  BlockSum* form_sums = nullptr;  // leaves of several partial blocks (k_sum_blocks)
+  int form_nsums = 0;
   long long* form_hoff = nullptr;  // 2D MMA form: per form task, offset of its Hermite block in hbuf
   HornerTask* horner = nullptr;
   double* lo = nullptr;

@@ -296,9 +296,16 @@ __global__ void __launch_bounds__(128) k_form2d_mma(KP k, const FormTask* __rest
 // A leaf's partial Hermite blocks (one after the other, n of them) added into
 // the first: 32 coefficients per CTA, eight threads each with every eighth
 // block (a thread alone waits for hundreds of loads in a row: 37 us instead of
-// 5 at 586 blocks), added in a fixed order.
-__global__ void __launch_bounds__(256) k_sum_blocks2d(const BlockSum* __restrict__ sums, int nd,
-                                                      double* __restrict__ hbuf) {
+// 5 at 586 blocks), added in a fixed order.  In 2D all leaves of several
+// blocks; in 3D those of more than SUM_BLOCKS3D, since k_up_z adds blocks as it
+// reads them, 1.7 us each in a row but beside the other columns, and the launch
+// costs 4 to 7 (one leaf of 595 blocks among 1e6 sources, order 7 and 13: 1764
+// and 4303 us added there, 854 and 3189 here; of 126, 6e4 sources: 197 and 330,
+// 107 and 297; of 21: 109 and 302, 97 and 306; blob leaves of 9 to 16, forces:
+// 1720 and 1728).
+constexpr int SUM_BLOCKS3D = 32;
+__global__ void __launch_bounds__(256) k_sum_blocks(const BlockSum* __restrict__ sums, int nd,
+                                                    double* __restrict__ hbuf) {
   __shared__ double part[8][32];
   const BlockSum S = sums[blockIdx.x];
   const int len = S.len * nd, x = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1760,7 +1767,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     for (int t = D.eval_taylor_n; t < D.neval; t++)
       while (H.tree.level[ev[t].box] > lcut) ev[t].box = H.tree.parent[ev[t].box];
   SepLists up;
-  std::vector<BlockSum> sums2;  // 2D: the leaves of several partial blocks
+  std::vector<BlockSum> sums;   // leaves of several partial blocks
   std::vector<PwFormTask> pwf;  // 3D boxes formed from exponential sums
   std::vector<SrcRange> pwf_src;
   std::vector<double> sep_ph;
@@ -1833,9 +1840,11 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
       const int n = f.n <= chunk ? 1 : (f.n + chunk - 1) / chunk;
       items[ni] = s;
       box[ni] = s.box;
-      leaf[ni++] = {hoff, 0, n};
-      if (P.dim == 2 && n > 1) sums2.push_back({hoff * P.nd, (f.p + 1) * (f.p + 1), n});
-      hoff += (long long)n * (f.p + 1) * (f.p + 1) * (P.dim == 3 ? f.p + 1 : 1);
+      const int len = (f.p + 1) * (f.p + 1) * (P.dim == 3 ? f.p + 1 : 1);
+      const bool sum = n > (P.dim == 2 ? 1 : SUM_BLOCKS3D);
+      leaf[ni++] = {hoff, 0, sum ? 1 : n};
+      if (sum) sums.push_back({hoff * P.nd, len, n});
+      hoff += (long long)n * len;
     }
     hbuf_doubles = (size_t)hoff * P.nd;
     // the boxes formed from exponential sums; `add` where leaves below add to them
@@ -1858,7 +1867,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     D.up_leaf = leaf;
     sep_lists(P.dim, items, leaf, sep_order_of, mp_slot, -1, P.npw, up);
     // 2D: the source chunks as tasks of their own, each with its partial block
-    if (P.dim == 2 && sums2.empty()) {
+    if (P.dim == 2 && sums.empty()) {
       std::vector<long long> off(form.size());
       for (size_t t = 0; t < off.size(); t++) off[t] = D.up_leaf[t].off * P.nd;
       form_hoff.swap(off);
@@ -2030,7 +2039,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
                  bytes_of(fchunks) +
                  bytes_of(up.leaves) + bytes_of(up.cols) + bytes_of(up.slabs) + bytes_of(up.boxes) +
                  bytes_of(up.box_kids) + bytes_of(dn.cols) + bytes_of(dn.leaves) + bytes_of(dn.slabs) +
-                 bytes_of(dn.boxes) + bytes_of(dn.box_kids) + bytes_of(dn.col_slot) + bytes_of(dn.leaf_col) + bytes_of(sums2) + bytes_of(ctask) + bytes_of(pwf) + bytes_of(pwf_src) + bytes_of(sep_ph) +
+                 bytes_of(dn.boxes) + bytes_of(dn.box_kids) + bytes_of(dn.col_slot) + bytes_of(dn.leaf_col) + bytes_of(sums) + bytes_of(ctask) + bytes_of(pwf) + bytes_of(pwf_src) + bytes_of(sep_ph) +
                  al(std::max(up.t1, dn.t1) * nd * 8) + al(std::max(up.t2, dn.t2) * nd * 8) +
                  al(hbuf_doubles * 8) + bytes_of(form_hoff) + bytes_of(horner) +
                  al(lo_doubles * 8) + 4096;
@@ -2085,8 +2094,8 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     st.add(cur, D.dn.box_kids, dn.box_kids);
     st.add(cur, D.dn.col_slot, dn.col_slot);
     st.add(cur, D.dn.leaf_col, dn.leaf_col);
-    st.add(cur, D.form2_sums, sums2);
-    D.form2_nsums = (int)sums2.size();
+    st.add(cur, D.form_sums, sums);
+    D.form_nsums = (int)sums.size();
     st.add(cur, D.ctask, ctask);
     st.add(cur, D.pwf, pwf);
     st.add(cur, D.pwf_src, pwf_src);
@@ -2344,10 +2353,6 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
         }
         launches++;
       }
-      if (D.form2_nsums > 0) {
-        k_sum_blocks2d<<<dim3(D.form2_nsums, 32), 256, 0, st>>>(D.form2_sums, nd, D.hbuf);
-        launches++;
-      }
     }
     if (P.dim == 3 && D.form_hermite_n > 0) {
       for (size_t gi = 0; gi < D.fchunk_groups.size(); gi++) {
@@ -2397,6 +2402,10 @@ cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& 
         }
         launches++;
       }
+    }
+    if (D.form_nsums > 0) {
+      k_sum_blocks<<<dim3(D.form_nsums, 32), 256, 0, st>>>(D.form_sums, nd, D.hbuf);
+      launches++;
     }
     if (P.dim == 2 && D.form_pw_n > 0) {  // the NUFFT scheme's direct form
       const size_t sh = (size_t)FORM_CH * (P.npw + n2) * 16;

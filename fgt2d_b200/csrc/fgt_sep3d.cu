@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(128) k_up_z(KP k, const SepNode* __restrict__ 
           const int j = 8 * s + 2 * c + par;
           a[par][s] = j < Pn ? H[j * P2] : 0.0;
         }
-      for (int ch = 1; ch < L.n; ch++) {  // further partial blocks, in chunk order
+      for (int ch = 1; ch < L.n; ch++) {  // the few further partial blocks, in chunk order
         const double* Hc = H + (size_t)ch * P3 * k.nd;
 #pragma unroll
         for (int s = 0; s < KS; s++)
