@@ -698,9 +698,9 @@ def main():
     ap.add_argument("--workers", type=int, default=8, help="serving workload: server worker streams")
     ap.add_argument("--server-bytes", type=int, default=0, help="serving workload: device budget (0: 80%% free)")
     ap.add_argument("--server-sm-budget", type=int, default=0,
-                    help="serving workload: SMs a request's persistent kernels use (0: all)")
+                    help="serving workload: SMs a request's transforms size their grids for (0: all)")
     ap.add_argument("--server-grid-yield", action="store_true",
-                    help="serving workload: one CTA per task instead of persistent CTAs")
+                    help="serving workload: as many CTAs as a request's transforms have work for")
     args = ap.parse_args()
     if args.workload == "serving":
         return serving_arm(args)

@@ -196,11 +196,13 @@ class Context:
         _check(lib().fgt_ctx_set_scheme(self._h, {"planewave": 0, "nufft": 1}[scheme]), "fgt_ctx_set_scheme")
 
     def set_sm_budget(self, sms):
-        """Accepted, without effect (the transforms have no persistent kernels)."""
+        """SMs the transforms between the leaves and the cut level size their
+        grids for, in plans created afterwards (0: all)."""
         _check(lib().fgt_ctx_set_sm_budget(self._h, int(sms)), "fgt_ctx_set_sm_budget")
 
     def set_grid_yield(self, on):
-        """Accepted, without effect (the transforms have no persistent kernels)."""
+        """As many CTAs as those transforms have work for, instead of CTAs that
+        take several pieces in turn (plans created afterwards)."""
         _check(lib().fgt_ctx_set_grid_yield(self._h, int(bool(on))), "fgt_ctx_set_grid_yield")
 
     def set_precision(self, precision):

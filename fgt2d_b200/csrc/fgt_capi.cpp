@@ -32,6 +32,8 @@ struct fgt_ctx {
   int precision = FGT_PREC_AUTO;
   int tree = FGT_TREE_AUTO;
   int nthreads = 0;
+  int sm_budget = 0;         // SMs the plans' transforms size their grids for (0: all)
+  bool yield_grids = false;  // as many CTAs as there is work for
   int scheme = FGT_SCHEME_PLANEWAVE;  // the algorithm of the context's plans
   // uploads of a one-shot call's source strengths: they follow the points on
   // the copy engine while the tree build runs on `stream`
@@ -201,6 +203,7 @@ int plan_device(fgt_plan* p, const double* src_host, const double* trg_host) {
   if (shard_filter(p->H, p->shard_n, p->shard_r, p->shard) != 0) return FGT_ERR_BADARG;
   if (!P.large_delta) {
     CKS(device_plan_create(p->H, p->D, nullptr, nullptr, st));
+    device_plan_set_grids(p->D, p->ctx->sm_budget, p->ctx->yield_grids);
     p->have_device = true;
   }
   CKS(cudaStreamSynchronize(st));  // the points are up: the caller may change its arrays
@@ -311,6 +314,7 @@ int plan_create_device_tree(fgt_plan* p, int dim, int nd, double delta, double e
     if (st != FGT_OK) return st;
   }
   CKS(device_plan_create(p->H, p->D, d_isrc, d_itarg, s));
+  device_plan_set_grids(p->D, p->ctx->sm_budget, p->ctx->yield_grids);
   p->have_device = true;
   CKS(device_plan_set_points(p->D, p->d_src, p->d_trg, s));
   CKS(cudaStreamSynchronize(s));
@@ -579,10 +583,12 @@ int fgt_ctx_set_scheme(fgt_ctx* c, int scheme) {
 }
 int fgt_ctx_set_sm_budget(fgt_ctx* c, int sms) {
   if (!c || sms < 0) return FGT_ERR_BADARG;
+  c->sm_budget = sms;
   return FGT_OK;
 }
-int fgt_ctx_set_grid_yield(fgt_ctx* c, int) {
+int fgt_ctx_set_grid_yield(fgt_ctx* c, int on) {
   if (!c) return FGT_ERR_BADARG;
+  c->yield_grids = on != 0;
   return FGT_OK;
 }
 int fgt_ctx_set_host_threads(fgt_ctx* c, int nthreads) {

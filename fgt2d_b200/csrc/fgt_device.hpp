@@ -108,7 +108,7 @@ struct SepDev {
   std::vector<SepGroup> groups;
   double2* ph = nullptr;
   double *t1 = nullptr, *t2 = nullptr;
-  int sms = 148;
+  int sms = 148;  // SMs the grids are sized for (device_plan_set_grids)
 };
 
 struct StageTimes {
@@ -252,6 +252,10 @@ cudaError_t device_plan_set_points(DevicePlan& D, const double* src, const doubl
 // the cut level between the two).
 cudaError_t device_plan_execute(DevicePlan& D, const Inputs& in, const Outputs& out,
                                 int precision, cudaStream_t stream, StageTimes* times, int phase = 0);
+
+// SMs that the transforms between the leaves and the cut level size their
+// grids for: sms, or all (0); with yield a CTA for every four pieces of work.
+void device_plan_set_grids(DevicePlan& D, int sms, bool yield);
 
 // The multipole expansion of a box below the cut level after the last
 // execute (plane-wave scheme, which forms none there): its leaves' blocks

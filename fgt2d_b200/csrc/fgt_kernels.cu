@@ -2204,6 +2204,11 @@ void device_plan_destroy(DevicePlan& D) {
   D.base = nullptr;
 }
 
+void device_plan_set_grids(DevicePlan& D, int sms, bool yield) {
+  // no grid of theirs reaches 12 CTAs per SM of 2^24
+  D.up.sms = D.dn.sms = yield ? 1 << 24 : sms > 0 ? std::min(sms, D.sm_count) : D.sm_count;
+}
+
 static KP make_kp(const DevicePlan& D) {
   KP k;
   const Params& P = D.P;

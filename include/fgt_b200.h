@@ -106,10 +106,17 @@ int fgt_ctx_set_host_threads(fgt_ctx* ctx, int nthreads);
  * take the device for FGT_TREE_AUTO.  No counterpart in the reference,
  * whose tree is built on the host (pts_tree_build, pts_tree2d4.f:363-590). */
 int fgt_ctx_set_tree(fgt_ctx* ctx, int where);
-/* Accepted for older callers, without effect: the transforms have no
- * persistent kernels, so work that arrives on other streams gets SMs as soon
- * as any CTA finishes. */
+/* how many SMs the kernels between the leaves and the cut level, whose CTAs
+ * take several pieces of work in turn, size their grids for (the context's
+ * plans created after the call); 0 (the default) uses every SM.  A smaller
+ * budget leaves SMs free for work that arrives while a large transform runs
+ * (fgt_server_set_sm_budget).  The results do not depend on it.  No
+ * counterpart in the reference. */
 int fgt_ctx_set_sm_budget(fgt_ctx* ctx, int sms);
+/* on != 0: those kernels launch a CTA for every four pieces of work, whatever
+ * the budget, so that a large transform's launches let work on other
+ * (higher-priority) streams onto the SMs as soon as any of their CTAs finish.
+ * Default off.  No counterpart in the reference. */
 int fgt_ctx_set_grid_yield(fgt_ctx* ctx, int on);
 /* the algorithm of the plans created after the call (FGT_SCHEME_*): the
  * reference selects it by building 2d/planewave or 2d/nufft (3D likewise),
@@ -373,7 +380,7 @@ typedef struct fgt_server_stats {
 } fgt_server_stats;
 int fgt_server_create(int device, long long max_device_bytes, int nworkers, fgt_server** out);
 int fgt_server_set_precision(fgt_server* server, int precision);
-/* accepted, without effect (see fgt_ctx_set_sm_budget) */
+/* fgt_ctx_set_sm_budget and fgt_ctx_set_grid_yield for the requests planned afterwards */
 int fgt_server_set_sm_budget(fgt_server* server, int sms);
 int fgt_server_set_grid_yield(fgt_server* server, int on);
 int fgt_server_submit(fgt_server* server, const fgt_request* request, long long* id);
