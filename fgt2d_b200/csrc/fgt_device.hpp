@@ -56,11 +56,12 @@ struct HornerTask {
   long long off;
 };
 
-// A leaf below (or at) a root box, with its place in the root's grid of boxes
-// of its level: the root holds 2^d boxes per dimension at depth d.
+// A leaf below (or at) a root box, with its place in the root along every
+// dimension: among the 2^d boxes of its depth d, or among the places that
+// occur there (SepRows).
 struct SepItem {
   int box, root;  // box; root as its number among the boxes of the root level
-  int d, x[3];    // depth below the root, place in the root's grid
+  int d, x[3];    // depth below the root, places
   int num;        // number in the list that was sorted
 };
 // 3D plane-wave form: a box's expansion (slot) about its centre from the

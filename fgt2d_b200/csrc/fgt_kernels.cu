@@ -1773,6 +1773,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   std::vector<double> sep_ph;
   size_t hbuf_doubles = 0;  // the leaves' (partial) Hermite blocks
   std::vector<std::pair<int, int>> run;  // a leaf's Taylor tasks, by its number in the list below
+  SepRows sep_rows;
   uvector<SepItem> sep_items;  // every leaf at or below the cut level, in the order of the lists
   std::vector<int> sep_order_of;   // order by depth below the cut level
   if (sep) {
@@ -1800,8 +1801,8 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
       run[num[b]] = {t, u};
     }
     for (int l = lcut; l <= P.nlevels; l++) sep_order_of.push_back(H.nlocal[l]);
-    sep_order(tr, lcut, boxes, sep_rank(sep_order_of), sep_items);
-    sep_phases(H, P.nlevels - lcut, tr.boxsize[lcut], sep_ph);
+    sep_order(tr, lcut, boxes, sep_rank(sep_order_of), sep_items, sep_rows);
+    sep_phases(H, sep_rows, tr.boxsize[lcut], sep_ph);
   }
   std::vector<long long> form_hoff;
   // Taylor evaluation: point chunks of <= 256 that read a leaf's block
@@ -1865,7 +1866,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     }
     D.up_box.swap(box);
     D.up_leaf = leaf;
-    sep_lists(P.dim, items, leaf, sep_order_of, mp_slot, -1, P.npw, up);
+    sep_lists(P.dim, items, sep_rows, leaf, sep_order_of, mp_slot, -1, P.npw, up);
     // 2D: the source chunks as tasks of their own, each with its partial block
     if (P.dim == 2 && sums.empty()) {
       std::vector<long long> off(form.size());
@@ -1909,7 +1910,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
       lo += len[items[i].d];
     }
     lo_doubles = (size_t)lo;
-    sep_lists(P.dim, items, leaf, sep_order_of, H.loc_slot.data() + H.tree.lfirst[lcut], -1, P.npw, dn);
+    sep_lists(P.dim, items, sep_rows, leaf, sep_order_of, H.loc_slot.data() + H.tree.lfirst[lcut], -1, P.npw, dn);
     // first task of every item, the groups' ranges; the tasks below
     std::vector<long long> at0(ni);
     for (SepGroup& G : dn.groups) {
@@ -2639,15 +2640,16 @@ cudaError_t device_plan_box_expansion(const HostPlan& H, DevicePlan& D, int box,
   std::vector<int> order;
   for (int l = lb; l <= P.nlevels; l++) order.push_back(H.nlocal[l]);
   uvector<SepItem> items;
-  sep_order(t, lb, boxes, sep_rank(order), items);
+  SepRows rows;
+  sep_order(t, lb, boxes, sep_rank(order), items, rows);
   std::vector<SepLeaf> leaf;
   for (const SepItem& s : items) leaf.push_back(D.up_leaf[at[s.box]]);
   std::vector<int> slot(t.llast[lb] - t.lfirst[lb] + 1, -1);
   slot[box - t.lfirst[lb]] = 0;
   SepLists L;
-  sep_lists(P.dim, items, leaf, order, slot.data(), box - t.lfirst[lb], P.npw, L);
+  sep_lists(P.dim, items, rows, leaf, order, slot.data(), box - t.lfirst[lb], P.npw, L);
   std::vector<double> ph;
-  sep_phases(H, P.nlevels - lb, t.boxsize[lb], ph);
+  sep_phases(H, rows, t.boxsize[lb], ph);
   const std::vector<PwFormTask> pwt(1, pw);
   const size_t nd = P.nd, per = nd * P.nexp * 16;
   char* mem = nullptr;

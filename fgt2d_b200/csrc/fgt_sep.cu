@@ -35,8 +35,42 @@ std::vector<int> sep_rank(const std::vector<int>& order) {
 }
 
 void sep_order(const Tree& t, int lroot, const std::vector<int>& boxes, const std::vector<int>& rank,
-               uvector<SepItem>& items) {
-  const int n = (int)boxes.size(), a0 = t.lfirst[lroot], dmax = (int)rank.size() - 1;
+               uvector<SepItem>& items, SepRows& rows) {
+  const int n = (int)boxes.size(), a0 = t.lfirst[lroot], dmax = (int)rank.size() - 1, dim = t.dim;
+  const bool dense = dmax <= SEP_DENSE;
+  auto root_of = [&](int b) {
+    while (t.level[b] > lroot) b = t.parent[b];
+    return b;
+  };
+  const double bs0 = t.boxsize[lroot];
+  auto offset = [&](int b, int a, int d) { return (t.c(b, d) - t.c(a, d)) / bs0; };
+  rows.base.assign(dmax + 1, 0);
+  rows.at.clear();
+  if (dense) {
+    for (int d = 0; d <= dmax; d++) {
+      rows.base[d] = (1 << d) - 1;
+      for (int i = 0; i < (1 << d); i++) rows.at.push_back((i + 0.5) / (1 << d) - 0.5);
+    }
+  } else {
+    std::vector<std::vector<double>> at(dmax + 1);
+    for (int b : boxes) {
+      const int a = root_of(b);
+      for (int d = 0; d < dim; d++) at[t.level[b] - lroot].push_back(offset(b, a, d));
+    }
+    for (int d = 0; d <= dmax; d++) {
+      std::sort(at[d].begin(), at[d].end());
+      at[d].erase(std::unique(at[d].begin(), at[d].end()), at[d].end());
+      rows.base[d] = (int)rows.at.size();
+      rows.at.insert(rows.at.end(), at[d].begin(), at[d].end());
+    }
+  }
+  // the place of a box: its row less the first of its depth
+  auto place = [&](int b, int a, int dep, int d) {
+    const double v = offset(b, a, d);
+    if (dense) return std::max(0, std::min((1 << dep) - 1, (int)std::lround((v + 0.5) * (1 << dep) - 0.5)));
+    const auto first = rows.at.begin() + rows.base[dep];
+    return (int)(std::lower_bound(first, dep < dmax ? rows.at.begin() + rows.base[dep + 1] : rows.at.end(), v) - first);
+  };
   auto width = [](unsigned long long v) {
     int w = 0;
     while (v >> w) w++;
@@ -45,8 +79,8 @@ void sep_order(const Tree& t, int lroot, const std::vector<int>& boxes, const st
   // one key per item, (rank, root, x, y, z, number), sorted by digits of at
   // most 12 bits; the items are written once, in order
   const int wn = width(n), wr = width(t.llast[lroot] - a0), wd = width(dmax);
-  const int dim = t.dim;
-  const bool packed = dim * dmax + wr + wd + wn <= 64;
+  const int wx = dense ? dmax : width(rows.at.size());
+  const bool packed = dim * wx + wr + wd + wn <= 64;
   uvector<SepItem> raw(n);
   uvector<uint64_t> key(packed ? n : 0), tmp(packed ? n : 0);
 #pragma omp parallel for schedule(static) if (n > 2048)
@@ -54,23 +88,21 @@ void sep_order(const Tree& t, int lroot, const std::vector<int>& boxes, const st
     SepItem& s = raw[i];
     s.box = boxes[i];
     s.num = i;
-    const int l = t.level[s.box];
-    int a = s.box;
-    while (t.level[a] > lroot) a = t.parent[a];
+    const int a = root_of(s.box);
     s.root = a - a0;
-    s.d = l - lroot;
+    s.d = t.level[s.box] - lroot;
     s.x[2] = 0;
     for (int q = 0; q < dim; q++) {
       const int e = dim == 2 ? 1 - q : q;  // 2D: y, x
-      s.x[q] = (int)std::lround((t.c(s.box, e) - t.c(a, e)) / t.boxsize[l] + 0.5 * ((1 << s.d) - 1));
+      s.x[q] = place(s.box, a, s.d, e);
     }
     if (packed) {
       uint64_t k = (uint64_t)rank[s.d] << wr | (uint64_t)s.root;
-      for (int q = 0; q < dim; q++) k = k << dmax | (uint64_t)s.x[q];
+      for (int q = 0; q < dim; q++) k = k << wx | (uint64_t)s.x[q];
       key[i] = k << wn | (uint64_t)i;
     }
   }
-  if (!packed) {  // a tree deeper than the keys hold
+  if (!packed) {  // more roots and places than the keys hold
     std::stable_sort(raw.begin(), raw.end(), [&](const SepItem& a, const SepItem& b) {
       if (a.d != b.d) return rank[a.d] < rank[b.d];
       if (a.root != b.root) return a.root < b.root;
@@ -79,7 +111,7 @@ void sep_order(const Tree& t, int lroot, const std::vector<int>& boxes, const st
     items.swap(raw);
     return;
   }
-  const int bits = dim * dmax + wr + wd, digit = (bits + (bits + 11) / 12 - 1) / std::max(1, (bits + 11) / 12);
+  const int bits = dim * wx + wr + wd, digit = (bits + (bits + 11) / 12 - 1) / std::max(1, (bits + 11) / 12);
   for (int b = wn; b < wn + bits; b += digit) {
     int cnt[4097] = {0};
     const uint64_t dm = (uint64_t(1) << digit) - 1;
@@ -94,7 +126,7 @@ void sep_order(const Tree& t, int lroot, const std::vector<int>& boxes, const st
   for (int i = 0; i < n; i++) items[i] = raw[key[i] & mask];
 }
 
-void sep_lists(int dim, const uvector<SepItem>& items, std::vector<SepLeaf>& leaf,
+void sep_lists(int dim, const uvector<SepItem>& items, const SepRows& rows, std::vector<SepLeaf>& leaf,
                const std::vector<int>& order, const int* slot, int also, int npw, SepLists& out) {
   const int n = (int)items.size(), n2 = npw / 2;
   SepLists S;  // this thread's until it is whole
@@ -114,7 +146,7 @@ void sep_lists(int dim, const uvector<SepItem>& items, std::vector<SepLeaf>& lea
   size_t t1 = 0, t2 = 0;
   for (int i = 0; i < n;) {
     // the items of one depth
-    const int d = items[i].d, p = order[d], row0 = (1 << d) - 1;
+    const int d = items[i].d, p = order[d], row0 = rows.base[d];
     const long long Pn = p + 1;
     if (S.groups.empty() || S.groups.back().p != p) S.groups.push_back({p, nc, nc, ns, ns, i, i});
     runs.push_back(nk);
@@ -172,18 +204,17 @@ void sep_lists(int dim, const uvector<SepItem>& items, std::vector<SepLeaf>& lea
   out = std::move(S);
 }
 
-void sep_phases(const HostPlan& H, int dmax, double bs0, std::vector<double>& ph) {
+void sep_phases(const HostPlan& H, const SepRows& rows, double bs0, std::vector<double>& ph) {
   const int npw = H.P.npw;
-  ph.resize((size_t)2 * npw * ((size_t(2) << dmax) - 1));
-  for (int d = 0; d <= dmax; d++)
-    for (int i = 0; i < (1 << d); i++) {
-      const double sh = (i + 0.5 - 0.5 * (1 << d)) * std::ldexp(bs0, -d) * H.P.dsq;
-      double* r = ph.data() + (size_t)2 * npw * ((1 << d) - 1 + i);
-      for (int m = 0; m < npw; m++) {
-        r[2 * m] = std::cos(H.ts[m] * sh);
-        r[2 * m + 1] = std::sin(H.ts[m] * sh);
-      }
+  ph.resize((size_t)2 * npw * rows.at.size());
+  for (size_t i = 0; i < rows.at.size(); i++) {
+    const double sh = rows.at[i] * bs0 * H.P.dsq;
+    double* r = ph.data() + (size_t)2 * npw * i;
+    for (int m = 0; m < npw; m++) {
+      r[2 * m] = std::cos(H.ts[m] * sh);
+      r[2 * m + 1] = std::sin(H.ts[m] * sh);
     }
+  }
 }
 
 namespace {

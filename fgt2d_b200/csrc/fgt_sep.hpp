@@ -14,12 +14,22 @@ namespace fgtb {
 
 struct KP;
 
+// Phase rows: a row for every place that a box can have in its root along one
+// dimension (SepItem::x), by depth.  Up to depth SEP_DENSE every place of the
+// grid has one (row 2^d - 1 + i); in deeper trees, which only callers with a
+// tree of their own have, those that occur.
+constexpr int SEP_DENSE = 8;
+struct SepRows {
+  std::vector<int> base;   // first row of every depth
+  std::vector<double> at;  // offset of every row from the root's centre over the root's size
+};
+
 // The boxes as items, sorted by (rank[depth], root, x, y, z),
 // in 2D (rank[depth], root, y, x); roots are the
 // boxes of level lroot, numbered from its first.  rank: by depth, equal orders
 // next to one another.
 void sep_order(const Tree& t, int lroot, const std::vector<int>& boxes, const std::vector<int>& rank,
-               uvector<SepItem>& items);
+               uvector<SepItem>& items, SepRows& rows);
 // rank of sep_order from the orders by depth (increasing order, then depth)
 std::vector<int> sep_rank(const std::vector<int>& order_of_depth);
 
@@ -28,13 +38,12 @@ std::vector<int> sep_rank(const std::vector<int>& order_of_depth);
 // the rows are filled here); offsets and sizes per density.  slot: the
 // expansion slots by root; without any item root `also` (-1: none) gets an
 // empty box.
-void sep_lists(int dim, const uvector<SepItem>& items, std::vector<SepLeaf>& leaf,
+void sep_lists(int dim, const uvector<SepItem>& items, const SepRows& rows, std::vector<SepLeaf>& leaf,
                const std::vector<int>& order_of_depth, const int* slot, int also, int npw, SepLists& S);
 
-// Phase rows of depths 0..dmax: row 2^d - 1 + i holds exp(i t_m sh) of the
-// npw nodes, sh the offset of box i of 2^d from its root's centre over
+// The phase rows: exp(i t_m sh) of the npw nodes, sh the row's offset over
 // sqrt(delta) (bs0: the root's size).
-void sep_phases(const HostPlan& H, int dmax, double bs0, std::vector<double>& ph);
+void sep_phases(const HostPlan& H, const SepRows& rows, double bs0, std::vector<double>& ph);
 
 // 3D (fgt_sep3d.cu)
 cudaError_t sep_up_3d(const KP& k, const SepDev& S, const double* hbuf, cudaStream_t st, long long& launches);
