@@ -1080,8 +1080,8 @@ int fgt_plan_get_info(const fgt_plan* p, fgt_plan_info* o) {
   o->large_delta = P.large_delta; o->all_direct = P.all_direct;
   o->kernel_launches = p->last_launches;
   for (int i = 0; i < 3; i++) o->shift_bytes[i] = p->H.shift_bytes[i];
-  o->form_route_flops = p->H.form_route_flops;
-  o->eval_route_flops = p->H.eval_route_flops;
+  o->form_route_flops = p->D.form_route_flops;
+  o->eval_route_flops = p->D.eval_route_flops;
   double npwd = std::pow((double)P.npw, P.dim);
   o->form_flops = 4.0 * (double)p->H.form_sources * npwd;
   o->eval_flops = 4.0 * (double)p->H.eval_points * npwd;

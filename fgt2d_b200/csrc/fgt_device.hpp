@@ -201,6 +201,9 @@ struct DevicePlan {
   int sm_count = 148;
   // statistics copied from the host plan
   long long direct_pairs = 0, form_sources = 0, eval_points = 0;
+  // flops of this plan's tasks by the routes that they take (a multiply-add: 2),
+  // without padding: formation with the way up, the way down with evaluation
+  double form_route_flops = 0, eval_route_flops = 0;
   long long launches = 0;
 };
 

@@ -1818,6 +1818,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   FormRules frules;
   EvalRules erules;
   long long nh = 0, nct = 0;
+  double eval_flops = 0.0;  // per density, without the way down
   const int pgh = std::max(1, std::max(P.ifpgh, P.ifpghtarg)), cp = sep_col_points(pgh);
   auto build_up = [&] {
     const int* mp_slot = H.mp_slot.data() + H.tree.lfirst[lcut];
@@ -1917,13 +1918,19 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
       G.blocks = blocks[G.p];
       const int step = G.blocks ? 256 : cp;
       const long long t0 = G.blocks ? nh : nct;
-      long long at = t0;
+      long long n = 0, at = t0;
       const int i0 = dn.cols[G.cbeg].beg, i1 = dn.cols[G.cend - 1].beg + dn.cols[G.cend - 1].cnt;
       for (int i = i0; i < i1; i++) {
         const std::pair<int, int> r = run[items[i].num];
         at0[i] = at;
-        for (int t = r.first; t < r.second; t++) at += ev[t].n <= step ? 1 : (ev[t].n + step - 1) / step;
+        for (int t = r.first; t < r.second; t++) {
+          at += ev[t].n <= step ? 1 : (ev[t].n + step - 1) / step;
+          n += ev[t].n;
+        }
       }
+      const double Pn = G.p + 1, n2 = P.npw / 2;
+      // a block's Horner sums; from a column the z sums and the product with them
+      eval_flops += 2.0 * pgh * n * (G.blocks ? std::pow(Pn, P.dim) : 2.0 * n2 * Pn * (Pn + 1.0));
       (G.blocks ? nh : nct) = at;
       (G.blocks ? D.horner_groups : D.ctask_groups).push_back({G.p, (int)t0, (int)at});
       if (G.blocks) D.horner_groups.back().per = erules.per[G.p];
@@ -2020,6 +2027,21 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
         t = u;
       }
     }
+  }
+  // flops of the routes taken.  Plane-wave sums: in 3D two real products of half
+  // the nodes per coefficient, in 2D (the NUFFT scheme) a complex one
+  {
+    const double cols = P.ifdipole ? P.dim : 1, pw = (P.dim == 3 ? 4.0 : 8.0) * P.nexp;
+    double f = 0.0, e = eval_flops;
+    for (double g : D.group_flops) f += cols * g;  // the Hermite blocks, every density
+    for (int t = D.form_hermite_n; t < (int)form.size(); t++) f += cols * pw * form[t].n * P.nd;
+    for (int t = D.eval_taylor_n; t < D.neval; t++) e += pw * pgh * ev[t].n;
+    if (sep) {
+      f += P.nd * sep_flops(P.dim, true, up, P.npw);
+      e += sep_flops(P.dim, false, dn, P.npw);
+    }
+    D.form_route_flops = f;
+    D.eval_route_flops = P.nd * e;
   }
   size_t ns = P.ns, nt = P.nt, nd = P.nd, dim = P.dim;
   // FP32 coordinates of the mixed near field (charges only)

@@ -204,6 +204,21 @@ void sep_lists(int dim, const uvector<SepItem>& items, const SepRows& rows, std:
   out = std::move(S);
 }
 
+double sep_flops(int dim, bool up, const SepLists& S, int npw) {
+  const double n2 = npw / 2, w = npw, turn = up ? 8.0 : 16.0;
+  double f = 0.0;
+  for (const SepGroup& G : S.groups) {
+    const double P = G.p + 1, leaves = G.lend - G.lbeg, cols = G.cend - G.cbeg, slabs = G.send - G.sbeg;
+    if (dim == 2) {
+      f += leaves * (2 * P * P * n2 + 8 * P * n2) + cols * (4 * P * n2 * n2 + turn * n2 * n2);
+    } else {
+      if (G.blocks) f += leaves * (2 * P * P * P * n2 + 8 * P * P * n2);
+      f += cols * (4 * P * P * n2 * n2 + turn * P * n2 * n2) + slabs * (4 * P * n2 * n2 * w + turn * n2 * n2 * w);
+    }
+  }
+  return f;
+}
+
 void sep_phases(const HostPlan& H, const SepRows& rows, double bs0, std::vector<double>& ph) {
   const int npw = H.P.npw;
   ph.resize((size_t)2 * npw * rows.at.size());

@@ -45,6 +45,10 @@ void sep_lists(int dim, const uvector<SepItem>& items, const SepRows& rows, std:
 // sqrt(delta) (bs0: the root's size).
 void sep_phases(const HostPlan& H, const SepRows& rows, double bs0, std::vector<double>& ph);
 
+// Flops per density of the way up or down through the lists (a multiply-add:
+// 2): products with the node tables and turns to the nodes' phases.
+double sep_flops(int dim, bool up, const SepLists& S, int npw);
+
 // 3D (fgt_sep3d.cu)
 cudaError_t sep_up_3d(const KP& k, const SepDev& S, const double* hbuf, cudaStream_t st, long long& launches);
 cudaError_t sep_down_3d(const KP& k, const SepDev& S, double* lo, cudaStream_t st, long long& launches);

@@ -87,8 +87,10 @@ typedef struct fgt_plan_info {
    * source-target pairs */
   long long shift_bytes[3];
   double form_flops, eval_flops;
-  /* flops of the routes actually taken (Hermite/Taylor or plane wave),
-   * counting each multiply-add as 2 and complex ones as 8 */
+  /* flops of the routes actually taken (Hermite/Taylor or plane wave), a
+   * multiply-add counted as 2, without padding: form with the transforms up to
+   * the cut level (stages form and merge), eval with the transforms down to the
+   * leaves.  A shard counts its own tasks. */
   double form_route_flops, eval_route_flops;
 } fgt_plan_info;
 
