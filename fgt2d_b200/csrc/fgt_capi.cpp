@@ -14,6 +14,7 @@
 #include <memory>
 #include <mutex>
 #include <new>
+#include <stdexcept>
 #include <vector>
 
 #include <malloc.h>
@@ -82,6 +83,25 @@ struct fgt_plan {
 };
 
 namespace {
+// A plan that goes with its device memory when its creation stops.
+struct PlanDelete {
+  void operator()(fgt_plan* p) const { fgt_plan_destroy(p); }
+};
+typedef std::unique_ptr<fgt_plan, PlanDelete> PlanPtr;
+
+// The status of f; what the host cannot allocate is FGT_ERR_NOMEM, not an
+// exception past a C entry (or out of a server's worker).
+template <class F>
+int guarded(F&& f) {
+  try {
+    return f();
+  } catch (const std::bad_alloc&) {
+    return FGT_ERR_NOMEM;
+  } catch (const std::length_error&) {
+    return FGT_ERR_NOMEM;
+  }
+}
+
 thread_local int g_last_cuda = 0;
 
 double now_s() {
@@ -679,7 +699,7 @@ int plan_create_impl(fgt_ctx* ctx, int dim, int nd, double delta, double eps, in
   if (!targ) nt = 0;  // no target array: no targets in the tree either
   // the NUFFT scheme's 2D form takes charges only
   if (ctx->scheme == FGT_SCHEME_NUFFT && dim == 2 && ifdipole) return FGT_ERR_UNSUPPORTED;
-  std::unique_ptr<fgt_plan> p(new (std::nothrow) fgt_plan());
+  PlanPtr p(new (std::nothrow) fgt_plan());
   if (!p) return FGT_ERR_NOMEM;
   p->ctx = ctx;
   p->H.scheme = ctx->scheme;
@@ -687,24 +707,17 @@ int plan_create_impl(fgt_ctx* ctx, int dim, int nd, double delta, double eps, in
   p->pre_rn = pre_rn;
   p->pre_ds = pre_ds;
   CKS(cudaSetDevice(ctx->device));
-  if (on_device) {
-    st = plan_create_device_tree(p.get(), dim, nd, delta, eps, ns, sources, nt, targ, ifpgh, ifpghtarg,
-                                 nullptr, ifcharge, ifdipole);
-  } else {
+  st = guarded([&] {
+    if (on_device)
+      return plan_create_device_tree(p.get(), dim, nd, delta, eps, ns, sources, nt, targ, ifpgh, ifpghtarg,
+                                     nullptr, ifcharge, ifdipole);
     // a small tree: one host thread (a team's start costs more than the work)
     OmpTeam team(ctx, ctx->tree == FGT_TREE_AUTO ? 1 : 0);
-    try {
-      build_host_plan(p->H, dim, nd, delta, eps, ns, sources, nt, targ, ifpgh, ifpghtarg, ctx->nthreads,
-                      ifcharge, ifdipole);
-    } catch (const std::bad_alloc&) {
-      return FGT_ERR_NOMEM;
-    }
-    st = plan_device(p.get(), sources, targ);
-  }
-  if (st != FGT_OK) {
-    fgt_plan_destroy(p.release());
-    return st;
-  }
+    build_host_plan(p->H, dim, nd, delta, eps, ns, sources, nt, targ, ifpgh, ifpghtarg, ctx->nthreads,
+                    ifcharge, ifdipole);
+    return plan_device(p.get(), sources, targ);
+  });
+  if (st != FGT_OK) return st;
   *out = p.release();
   return FGT_OK;
 }
@@ -724,7 +737,7 @@ int fgt_plan_destroy(fgt_plan* p) {
     cudaStreamWaitEvent(p->ctx->stream, p->pre_done, 0);
     cudaEventDestroy(p->pre_done);
   }
-  if (p->have_device) {
+  if (p->D.base) {
     p->D.stream = p->ctx->stream;
     device_plan_destroy(p->D);
   }
@@ -777,50 +790,47 @@ int fgt_plan_create_shard(fgt_ctx* ctx, int dim, int nd, double delta, double ep
   if (st != FGT_OK) return st;
   if (ns == 0) return FGT_ERR_BADARG;
   if (!targ) nt = 0;
-  std::unique_ptr<fgt_plan> p(new (std::nothrow) fgt_plan());
+  PlanPtr p(new (std::nothrow) fgt_plan());
   if (!p) return FGT_ERR_NOMEM;
   p->ctx = ctx;
   p->H.scheme = ctx->scheme;
   p->shard_n = nranks;
   p->shard_r = rank;
   CKS(cudaSetDevice(ctx->device));
-  if (ctx->tree != FGT_TREE_HOST) {
-    st = plan_create_device_tree(p.get(), dim, nd, delta, eps, ns, sources, nt, targ, ifpgh, ifpghtarg);
-  } else {
-    try {
+  st = guarded([&]() -> int {
+    int st = FGT_OK;
+    if (ctx->tree != FGT_TREE_HOST) {
+      st = plan_create_device_tree(p.get(), dim, nd, delta, eps, ns, sources, nt, targ, ifpgh, ifpghtarg);
+    } else {
       build_host_plan(p->H, dim, nd, delta, eps, ns, sources, nt, targ, ifpgh, ifpghtarg, ctx->nthreads);
-    } catch (const std::bad_alloc&) {
-      return FGT_ERR_NOMEM;
+      st = plan_device(p.get(), sources, targ);
     }
-    st = plan_device(p.get(), sources, targ);
-  }
-  if (st == FGT_OK && nranks > 1) {
-    // the exchange lists on the device: every peer's send list, then every peer's receive list
-    std::vector<int> all;
-    p->xsend_off.assign(nranks + 1, 0);
-    p->xrecv_off.assign(nranks + 1, 0);
-    for (int r = 0; r < nranks; r++) {
-      all.insert(all.end(), p->shard.send[r].begin(), p->shard.send[r].end());
-      p->xsend_off[r + 1] = (long long)all.size();
+    if (st == FGT_OK && nranks > 1) {
+      // the exchange lists on the device: every peer's send list, then every peer's receive list
+      std::vector<int> all;
+      p->xsend_off.assign(nranks + 1, 0);
+      p->xrecv_off.assign(nranks + 1, 0);
+      for (int r = 0; r < nranks; r++) {
+        all.insert(all.end(), p->shard.send[r].begin(), p->shard.send[r].end());
+        p->xsend_off[r + 1] = (long long)all.size();
+      }
+      for (int r = 0; r < nranks; r++) {
+        p->xrecv_off[r] = (long long)all.size();
+        all.insert(all.end(), p->shard.recv[r].begin(), p->shard.recv[r].end());
+      }
+      p->xrecv_off[nranks] = (long long)all.size();
+      if (!all.empty()) {
+        cudaStream_t s = ctx->stream;
+        if (cudaMallocAsync(reinterpret_cast<void**>(&p->d_xslots), all.size() * sizeof(int), s) != cudaSuccess ||
+            cudaMemcpyAsync(p->d_xslots, all.data(), all.size() * sizeof(int), cudaMemcpyHostToDevice, s) !=
+                cudaSuccess ||
+            cudaStreamSynchronize(s) != cudaSuccess)
+          st = FGT_ERR_CUDA;
+      }
     }
-    for (int r = 0; r < nranks; r++) {
-      p->xrecv_off[r] = (long long)all.size();
-      all.insert(all.end(), p->shard.recv[r].begin(), p->shard.recv[r].end());
-    }
-    p->xrecv_off[nranks] = (long long)all.size();
-    if (!all.empty()) {
-      cudaStream_t s = ctx->stream;
-      if (cudaMallocAsync(reinterpret_cast<void**>(&p->d_xslots), all.size() * sizeof(int), s) != cudaSuccess ||
-          cudaMemcpyAsync(p->d_xslots, all.data(), all.size() * sizeof(int), cudaMemcpyHostToDevice, s) !=
-              cudaSuccess ||
-          cudaStreamSynchronize(s) != cudaSuccess)
-        st = FGT_ERR_CUDA;
-    }
-  }
-  if (st != FGT_OK) {
-    fgt_plan_destroy(p.release());
     return st;
-  }
+  });
+  if (st != FGT_OK) return st;
   *out = p.release();
   return FGT_OK;
 }
@@ -1032,8 +1042,7 @@ int fgt_plan_expansion(fgt_plan* p, int which, int box, double* out) {
     // below the cut level the transform forms none: formed here on request
     CKS(cudaSetDevice(p->ctx->device));
     if (p->done) CKS(cudaEventSynchronize(p->done));
-    CKS(device_plan_box_expansion(H, p->D, box, out, p->ctx->stream));
-    return FGT_OK;
+    return guarded([&] { return cuda_status(device_plan_box_expansion(H, p->D, box, out, p->ctx->stream)); });
   }
   int slot = slots[box], a = box;
   if (which == 1 && slot < 0 && H.P.scheme == 0 && H.tree.level[box] > lcut &&
@@ -1322,7 +1331,7 @@ static int main_gpu(int dim, const int* nd, const double* delta, const double* e
   fgt_ctx* c = fgt_default_ctx();
   if (!c) return FGT_ERR_NODEVICE;
   std::lock_guard<std::mutex> lk(c->mu);
-  std::unique_ptr<fgt_plan> p(new (std::nothrow) fgt_plan());
+  PlanPtr p(new (std::nothrow) fgt_plan());
   if (!p) return FGT_ERR_NOMEM;
   p->ctx = c;
   int nb = *nboxes, nlev = *nlevels, ns = *nsource, nt = *ntarget, D = dim;
@@ -1368,17 +1377,10 @@ static int main_gpu(int dim, const int* nd, const double* delta, const double* e
   P0.ifpgh = *ifpgh; P0.ifpghtarg = *ifpghtarg; P0.npwlevel = *npwlevel;
   P0.ifcharge = *ifcharge; P0.ifdipole = *ifdipole;
   std::vector<int> nl(nlocal, nlocal + nlev + 1);
-  try {
-    build_host_plan_from_tree(p->H, P0, nl, *pmax, *npw);
-  } catch (const std::bad_alloc&) {
-    return FGT_ERR_NOMEM;
-  }
+  build_host_plan_from_tree(p->H, P0, nl, *pmax, *npw);
   CKS(cudaSetDevice(c->device));
   st = plan_device(p.get(), sourcesort, targetsort);
-  if (st != FGT_OK) {
-    fgt_plan_destroy(p.release());
-    return st;
-  }
+  if (st != FGT_OK) return st;
   // outputs are incremented (fgt2dmain adds into pot/grad/hess)
   const size_t nh = dim == 2 ? 3 : 6, n1 = (size_t)ns * *nd, n2 = (size_t)nt * *nd;
   std::vector<double> po(n1), go(*ifpgh >= 2 ? n1 * dim : 0), ho(*ifpgh >= 3 ? n1 * nh : 0);
@@ -1387,7 +1389,7 @@ static int main_gpu(int dim, const int* nd, const double* delta, const double* e
   h.pot = po.data(); h.grad = go.data(); h.hess = ho.data();
   h.pottarg = pt.data(); h.gradtarg = gt.data(); h.hesstarg = ht.data();
   st = exec_host(p.get(), chargesort, h, rnormalsort, dipstrsort);
-  fgt_plan_destroy(p.release());
+  p.reset();
   if (st != FGT_OK) return st;
   auto add = [](double* out, const std::vector<double>& v) {
     if (out)
@@ -1417,10 +1419,10 @@ int fgt2dmain_gpu_(const int* nd, const double* delta, const double* eps, const 
                    double* gradtarg, double* hesstarg) {
   (void)iaddr; (void)rmlexp; (void)ltree; (void)iper;
   (void)ntermsh; (void)ntermmax;
-  return main_gpu<int>(2, nd, delta, eps, nsource, sourcesort, ifcharge, chargesort, ifdipole,
+  return guarded([&] { return main_gpu<int>(2, nd, delta, eps, nsource, sourcesort, ifcharge, chargesort, ifdipole,
                        rnormalsort, dipstrsort, ntarget, targetsort, itree, iptr, nlevels, npwlevel, nboxes, boxsize,
                        centers, laddr, isrcse, itargse, nlocal, pmax, npw, ifpgh, pot, grad, hess,
-                       ifpghtarg, pottarg, gradtarg, hesstarg);
+                       ifpghtarg, pottarg, gradtarg, hesstarg); });
 }
 
 int fgt3dmain_gpu_(const int* nd, const double* delta, const double* eps, const int* nsource,
@@ -1437,10 +1439,10 @@ int fgt3dmain_gpu_(const int* nd, const double* delta, const double* eps, const 
                    double* hesstarg) {
   (void)iaddr; (void)rmlexp; (void)ltree; (void)iper;
   (void)ndiv; (void)ntermsh; (void)ntermmax;
-  return main_gpu<long long>(3, nd, delta, eps, nsource, sourcesort, ifcharge, chargesort, ifdipole,
+  return guarded([&] { return main_gpu<long long>(3, nd, delta, eps, nsource, sourcesort, ifcharge, chargesort, ifdipole,
                              rnormalsort, dipstrsort, ntarget, targetsort, itree, iptr, nlevels, npwlevel, nboxes, boxsize,
                              centers, laddr, isrcse, itargse, nlocal, pmax, npw, ifpgh, pot, grad,
-                             hess, ifpghtarg, pottarg, gradtarg, hesstarg);
+                             hess, ifpghtarg, pottarg, gradtarg, hesstarg); });
 }
 
 }  // extern "C"
@@ -1539,7 +1541,7 @@ int server_run(fgt_server* S, fgt_ctx* ctx, const fgt_request& r) {
                             64LL * npts + (1 << 20);
   server_take(S, &S->in_pts, S->budget_pts, est_pts);
   long long plan_bytes = 0;
-  std::unique_ptr<fgt_plan> p(new (std::nothrow) fgt_plan());
+  PlanPtr p(new (std::nothrow) fgt_plan());
   if (!p) {
     server_give(S, &S->in_pts, est_pts);
     return FGT_ERR_NOMEM;
@@ -1553,8 +1555,10 @@ int server_run(fgt_server* S, fgt_ctx* ctx, const fgt_request& r) {
     server_take(S, &S->in_plan, S->budget_plan, plan_bytes);
     return FGT_OK;
   };
-  st = plan_create_device_tree(p.get(), r.dim, r.nd, r.delta, r.eps, r.ns, r.sources, nt, r.targ, r.ifpgh,
-                               r.ifpghtarg, &admit, ifcharge, ifdipole);
+  st = guarded([&] {
+    return plan_create_device_tree(p.get(), r.dim, r.nd, r.delta, r.eps, r.ns, r.sources, nt, r.targ, r.ifpgh,
+                                   r.ifpghtarg, &admit, ifcharge, ifdipole);
+  });
   if (st == FGT_OK) {
     Outputs h;
     h.pot = r.pot; h.grad = r.grad; h.hess = r.hess;

@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <memory>
+#include <new>
 #include <thread>
 #ifdef _OPENMP
 #include <omp.h>
@@ -111,6 +112,7 @@ static void build_near_tasks(HostPlan& H) {
     int* const curp = cur_buf.get();
     auto cur = [&](size_t i) -> int& { return curp[i]; };
     const int chunk = (s_hi + 1 + nth - 1) / nth;
+    bool room = true;  // an exception may not leave the parallel region
 #pragma omp parallel num_threads(nth) if (nth > 1)
     {
 #ifdef _OPENMP
@@ -134,7 +136,11 @@ static void build_near_tasks(HostPlan& H) {
 #pragma omp single
       {
         for (int a = 0; a < nb; a++) ioff[a + 1] += ioff[a];
-        into.assign(ioff[nb], 0);
+        try {
+          into.assign(ioff[nb], 0);
+        } catch (const std::bad_alloc&) {
+          room = false;
+        }
       }
 #pragma omp for schedule(static)
       for (int a = 0; a < nb; a++) {
@@ -145,10 +151,11 @@ static void build_near_tasks(HostPlan& H) {
           pos += n;
         }
       }
-      for (int s = s0; s < s1; s++)
+      for (int s = s0; room && s < s1; s++)
         if (L.ifhung[s])
           for (int k = L.l1off[s]; k < L.l1off[s + 1]; k++) into[c[L.l1[k]]++] = s;
     }
+    if (!room) throw std::bad_alloc();
   }
   // per leaf: its source ranges (ancestors' segments, leaf first) once per
   // evaluated point set, and its tasks of <= CH points; counted per leaf,

@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <stdexcept>
 #include <chrono>
 #include <cstdio>
@@ -592,10 +593,21 @@ void build_tree(Tree& t, int dim, const double* src, int ns, const double* trg, 
     count.resize(t.nboxes, 0);
     const int* fc = firstchild.data();
     const int c0 = t.lfirst[lev + 1], nnew = t.nboxes - c0;
-    // per-thread counts of the new boxes, summed afterwards (no atomics)
-#pragma omp parallel
+    // per-thread counts of the new boxes, summed afterwards (no atomics);
+    // allocated here, since an exception may not leave the parallel region
+    int nth = 1;
+#ifdef _OPENMP
+    nth = omp_get_max_threads();
+#endif
+    std::unique_ptr<int[]> counts(new int[(size_t)nth * nnew]);
+#pragma omp parallel num_threads(nth)
     {
-      std::vector<int> loc(nnew, 0);
+      int th = 0;
+#ifdef _OPENMP
+      th = omp_get_thread_num();
+#endif
+      int* const loc = counts.get() + (size_t)th * nnew;
+      std::fill(loc, loc + nnew, 0);
 #pragma omp for schedule(static) nowait
       for (int i = 0; i < ns; i++) {
         int box = pbox[i];
