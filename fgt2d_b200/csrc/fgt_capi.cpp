@@ -83,9 +83,14 @@ struct fgt_plan {
 };
 
 namespace {
-// A plan that goes with its device memory when its creation stops.
+// A plan that goes with its device memory when its creation stops, once no
+// upload reads the caller's arrays any more.
 struct PlanDelete {
-  void operator()(fgt_plan* p) const { fgt_plan_destroy(p); }
+  void operator()(fgt_plan* p) const {
+    if (p->d_io) cudaStreamSynchronize(p->ctx->stream);
+    if (p->pre_done) cudaEventSynchronize(p->pre_done);
+    fgt_plan_destroy(p);
+  }
 };
 typedef std::unique_ptr<fgt_plan, PlanDelete> PlanPtr;
 

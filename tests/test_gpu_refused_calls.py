@@ -88,3 +88,25 @@ def test_refused_execute_copies_nothing(fgt, bad):
     copies = [e.name for e in prof.events() if "HtoD" in e.name]
     plan.close()
     assert st == 1 and not copies, copies
+
+
+def test_refused_points_leave_no_upload_behind(fgt):
+    """The strengths of a one-shot call go up beside the tree build: a call
+    that is refused for its points returns when that upload has ended."""
+    import time
+
+    import torch
+    rng = np.random.default_rng(6)
+    ns, nd = 200000, 256
+    q = torch.zeros(ns, nd, dtype=torch.float64).pin_memory().numpy()  # 410 MB, about 8 ms
+    src = rng.random((ns, 2))
+    src[7, 1] = np.nan
+    ctx = fgt.Context(0)
+    after = []
+    for _ in range(3):
+        with pytest.raises(fgt.FGTError):
+            fgt.transform_pgh(2, nd, 1e-3, 1e-6, src, q, src[:1], 0, 1, ctx)
+        t0 = time.perf_counter()
+        torch.cuda.synchronize()
+        after.append(time.perf_counter() - t0)
+    assert min(after) < 1e-3, after
