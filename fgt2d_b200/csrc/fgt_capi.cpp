@@ -896,7 +896,7 @@ int fgt_plan_mp_unpack(fgt_plan* p, int peer, const double* d_buf, void* stream)
 struct fgt_host_shard {
   HostPlan H;
   ShardInfo S;
-  long long nform = 0, neval = 0, ndir = 0, nm2l = 0;
+  long long nform = 0, neval = 0, ndir = 0, nm2l = 0, nshift = 0;
   int nmp = 0;
 };
 
@@ -920,6 +920,7 @@ int fgt_host_shard_create(int dim, int nd, double delta, double eps, int ns, con
   h->neval = (long long)h->H.eval.size();
   h->ndir = (long long)h->H.dir.size();
   h->nm2l = (long long)h->H.m2l.size();
+  h->nshift = shift_pairs(h->H, h->S);
   h->nmp = h->H.nmp;
   *out = h.release();
   return FGT_OK;
@@ -945,7 +946,7 @@ int fgt_host_shard_stats(fgt_host_shard* h, long long* out8) {
   out8[3] = h->neval;
   out8[4] = h->ndir;
   out8[5] = h->nm2l;
-  out8[6] = 0;  // merge and split run with formation and evaluation
+  out8[6] = h->nshift;
   out8[7] = h->nmp;
   return FGT_OK;
 }

@@ -211,6 +211,23 @@ int shard_filter(HostPlan& H, int nranks, int rank, ShardInfo& S) {
   return 0;
 }
 
+long long shift_pairs(const HostPlan& H, const ShardInfo& S) {
+  const Tree& t = H.tree;
+  const Params& P = H.P;
+  if (P.all_direct || P.large_delta || P.scheme != 0) return 0;
+  auto points = [&](int b) { return (P.ifpgh > 0 ? t.ns(b) : 0) + (P.ifpghtarg > 0 ? t.nt(b) : 0); };
+  long long n = 0;
+  for (int l = std::max(P.npwlevel, 0); l < P.nlevels; l++)
+    for (int b = t.lfirst[l]; b <= t.llast[l]; b++) {
+      if (t.nchild[b] == 0 || (!S.owner.empty() && S.owner[b] != S.rank)) continue;
+      for (int j = 0; j < t.nch; j++) {
+        const int c = t.ch(b, j);
+        if (c >= 0) n += (t.ns(c) > 0) + (points(c) > 0);
+      }
+    }
+  return n;
+}
+
 // ---- device side: copies of cut-level mp expansions between a plan's pool
 // and a contiguous exchange buffer ([i][nd * nexp] complex per listed slot)
 namespace {

@@ -24,6 +24,12 @@ struct ShardInfo {
 // fills the exchange lists; 0 on success.
 int shard_filter(HostPlan& H, int nranks, int rank, ShardInfo& S);
 
+// Merges and splits (fgt2d.f:976-1009, 1082-1125) that the transforms between
+// the leaves and the cut level stand for: pairs of a box from the cut level on
+// and a child, both with sources (merge), both with points to evaluate (split).
+// Those of this rank's boxes, or all (S without owners).
+long long shift_pairs(const HostPlan& H, const ShardInfo& S);
+
 // Copies the nslot listed cut-level mp expansions (device slot list) of the
 // plan into buf (pack) or from buf into the plan's pool (unpack); buf holds
 // nslot * nd * nexp complex doubles.
