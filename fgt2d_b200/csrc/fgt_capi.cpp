@@ -230,9 +230,12 @@ int plan_device(fgt_plan* p, const double* src_host, const double* trg_host) {
     CKS(device_plan_create(p->H, p->D, nullptr, nullptr, st));
     device_plan_set_grids(p->D, p->ctx->sm_budget, p->ctx->yield_grids);
     p->have_device = true;
+    // the points are up (device_plan_create ends with the stream's copies): the
+    // caller may change its arrays
+    CKS(device_plan_set_points(p->D, p->d_src, p->d_trg, st));
+  } else {
+    CKS(cudaStreamSynchronize(st));
   }
-  CKS(cudaStreamSynchronize(st));  // the points are up: the caller may change its arrays
-  if (!P.large_delta) CKS(device_plan_set_points(p->D, p->d_src, p->d_trg, st));
   return FGT_OK;
 }
 

@@ -2144,6 +2144,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     k_shift_tables<<<blocks, 256, 0, s>>>(P.dim, P.npw, P.nexp, d_w1, D.wsh);
     CK(cudaGetLastError());
   }
+  std::vector<int> inv[2];  // until the copies below have ended
   if (d_isrc) {
     // permutations built on the device (fgt_devtree.cu): copy, invert there;
     // targets that are the sources share the sources' arrays
@@ -2172,13 +2173,12 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
   } else {
     CK(put(cur, D.isrc, H.tree.isrc, s));
     CK(put(cur, D.itarg, H.tree.itarg, s));
-    std::vector<int> inv(H.tree.isrc.size());
-    for (size_t i = 0; i < inv.size(); i++) inv[H.tree.isrc[i]] = (int)i;
-    CK(put(cur, D.isrc_inv, inv, s));
-    CK(cudaStreamSynchronize(s));
-    inv.assign(H.tree.itarg.size(), 0);
-    for (size_t i = 0; i < inv.size(); i++) inv[H.tree.itarg[i]] = (int)i;
-    CK(put(cur, D.itarg_inv, inv, s));
+    const std::vector<int>* perm[2] = {&H.tree.isrc, &H.tree.itarg};
+    for (int k = 0; k < 2; k++) {
+      inv[k].resize(perm[k]->size());
+      for (size_t i = 0; i < inv[k].size(); i++) inv[k][(*perm[k])[i]] = (int)i;
+      CK(put(cur, k ? D.itarg_inv : D.isrc_inv, inv[k], s));
+    }
   }
   if (H.dnear.mem) {
     D.dir = reinterpret_cast<DirTask*>(cur);
