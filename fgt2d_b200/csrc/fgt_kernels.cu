@@ -840,7 +840,9 @@ __global__ void __launch_bounds__(256) k_form2d_pw(KP k, const FormTask* __restr
 
 // ------------------------------------------------------------ (b) shifts
 // mp -> loc at the cut level: sum over the plane-wave list plus the box's own
-// multipole (g2dshiftpw_vec + g2dcopypwexp_vec, fgt2d.f:1048-1060)
+// multipole (g2dshiftpw_vec + g2dcopypwexp_vec, fgt2d.f:1048-1060).  Bound by the
+// L1 pipe (94%): an expansion entry and a table entry per coefficient and
+// neighbour, out of L2 (70%; DRAM 12%).
 __global__ void k_m2l(KP k, const M2LTask* __restrict__ tasks, const M2LNbr* __restrict__ nbr) {
   const M2LTask T = tasks[blockIdx.x];
   const size_t per = (size_t)k.nd * k.nexp;

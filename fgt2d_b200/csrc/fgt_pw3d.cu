@@ -237,7 +237,8 @@ __global__ void __launch_bounds__(128) k_eval3d_pw(KP k, const EvalTask* __restr
 // dimension, by recurrence) into shared memory, where a B fragment is one
 // complex product of two of them.  With dipoles a source stages three columns
 // (dip3_coef, the factor of one dimension times v_d (-i t dsq)), ten sources
-// at a time.  Bound by the tensor pipe.  Measured (B200, eps 1e-9, npw 38;
+// at a time.  Bound by the tensor pipe (45%) and by the barriers around the
+// factors' staging.  Measured (B200, eps 1e-9, npw 38;
 // before: a thread per coefficient on the scalar pipe, an expansion per leaf,
 // then the merges): 3e5 uniform points 1.2 -> 0.53 ms; 1e5 for gradients, where
 // every leaf takes this route, 2.3 -> 0.92 ms.

@@ -17,10 +17,11 @@
 // g3drouts.f:1565-1685) and the merge over the levels (g3dshiftpw_vec):
 // the same sums in another order.
 //
-// What bounds the kernels: the FP64 tensor pipe (mma.m8n8k4, 16 cycles per
-// SM sub-partition) in the z pass, memory in the others; every operand is
-// read once from global memory straight into the fragment that needs it, so
-// there is no shared memory and the warps are independent.  Measured against
+// What bounds the kernels: the latency of their operand loads at the few warps
+// that their registers allow (18 to 28% of the SM's; FP64 tensor pipe 20 to
+// 33%, DRAM 25 to 43% in ncu); every operand is read once from global memory
+// straight into the fragment that needs it, so there is no shared memory and
+// the warps are independent.  Measured against
 // a whole transform per leaf and level-by-level merges (B200, transforms and
 // merges of one execute): 4e6 blob sources, eps 1e-6, 2.75 -> 0.85 ms; 3e5
 // uniform points, eps 1e-9, delta 1e-3, 4.95 -> 1.38 ms; eps 1e-12, delta
@@ -436,7 +437,8 @@ __global__ void __launch_bounds__(128) k_down_z(KP k, const SepNode* __restrict_
 // (each element once per chunk), the warps taking the tiles of q in turn, two
 // at a time; the lane's sums of W[point][q] x^a y^b (and with the derivative
 // powers) are added over the lanes and warps at the end in a fixed order.
-// Bound by the tensor pipe and the operand loads.  Measured: 1e5 uniform
+// Bound by the tensor pipe (38 to 47%, each product waiting for the last) and
+// the operand loads.  Measured: 1e5 uniform
 // points, eps 1e-6 (24 points a leaf, order 21), 1.02 ms with blocks and
 // Horner -> 0.18 ms; 3e5 points, eps 1e-9, 3.2 -> 1.0 ms (orders 20 and 31);
 // gradients of 1e5 points at eps 1e-9, 37.5 -> 0.94 ms.
