@@ -1653,9 +1653,24 @@ struct FormRules {
 };
 FormRules form_rules(const Params& P, const std::vector<FormTask>& tasks, int sms) {
   FormRules R;
+  // sources and tasks by order; the tasks come level by level, so a run of one
+  // order is summed in registers
+  std::vector<long long> n(P.ntermmax + 1, 0), cnt(P.ntermmax + 1, 0);
   long long nsrc = 0;
-  for (const FormTask& f : tasks)
-    if (f.route == ROUTE_HERMITE) nsrc += f.n;
+  int most = 0;
+  for (size_t i = 0; i < tasks.size();) {
+    const int p = tasks[i].p;
+    long long sum = 0, num = 0;
+    for (; i < tasks.size() && tasks[i].p == p; i++)
+      if (tasks[i].route == ROUTE_HERMITE) {
+        sum += tasks[i].n;
+        num++;
+        most = std::max(most, tasks[i].n);
+      }
+    nsrc += sum;
+    n[p] += sum;
+    cnt[p] += num;
+  }
   // Sources per partial block: at most 4096, fewer (whole batches of the
   // kernel) where that leaves SMs without a CTA
   if (P.dim == 3) {
@@ -1668,12 +1683,9 @@ FormRules form_rules(const Params& P, const std::vector<FormTask>& tasks, int sm
   // 0.76 ms of a 0.80 ms execute, 0.02 of 0.08 cut up)
   R.chunk = (int)std::max<long long>(512, (nsrc / (8LL * sms) + 255) / 256 * 256);
   // leaves (or chunks) of about two blocks of source columns or less, a warp each
-  std::vector<long long> n(P.ntermmax + 1, 0), cnt(P.ntermmax + 1, 0);
-  for (const FormTask& f : tasks)
-    if (f.route == ROUTE_HERMITE) {
-      n[f.p] += f.n;
-      cnt[f.p] += f.n <= R.chunk ? 1 : (f.n + R.chunk - 1) / R.chunk;
-    }
+  if (most > R.chunk)
+    for (const FormTask& f : tasks)
+      if (f.route == ROUTE_HERMITE && f.n > R.chunk) cnt[f.p] += (f.n + R.chunk - 1) / R.chunk - 1;
   R.warp.resize(n.size());
   for (size_t p = 0; p < n.size(); p++) R.warp[p] = n[p] * (P.ifdipole ? 2 : 1) <= 80 * cnt[p];
   return R;
@@ -1683,7 +1695,7 @@ FormRules form_rules(const Params& P, const std::vector<FormTask>& tasks, int sm
 struct EvalRules {
   std::vector<uint8_t> blocks, per;
 };
-EvalRules eval_rules(const Params& P, const std::vector<EvalTask>& tasks, int pgh) {
+EvalRules eval_rules(const Params& P, const std::vector<int>& nlocal, const std::vector<EvalTask>& tasks, int pgh) {
   EvalRules R;
   const int np = P.ntermmax + 1, n2 = P.npw / 2;
   R.blocks.assign(np, P.dim == 2);
@@ -1691,12 +1703,21 @@ EvalRules eval_rules(const Params& P, const std::vector<EvalTask>& tasks, int pg
   if (P.dim == 2) {
     // k_eval2d_mma where it is the faster one (its comment), with as many
     // warps per task as have points
+    bool some = false;  // a level of such an order
+    for (int l = std::max(P.npwlevel, 0); l <= P.nlevels; l++) some = some || (nlocal[l] >= 24 && nlocal[l] < 40);
+    if (!some) return R;
     std::vector<long long> n(np, 0), cnt(np, 0);
-    for (const EvalTask& e : tasks)
-      if (e.route == ROUTE_TAYLOR) {
-        n[e.p] += e.n;
-        cnt[e.p] += e.n <= 256 ? 1 : (e.n + 255) / 256;
-      }
+    for (size_t i = 0; i < tasks.size();) {
+      const int p = tasks[i].p;
+      long long sum = 0, num = 0;
+      for (; i < tasks.size() && tasks[i].p == p; i++)
+        if (tasks[i].route == ROUTE_TAYLOR) {
+          sum += tasks[i].n;
+          num += tasks[i].n <= 256 ? 1 : (tasks[i].n + 255) / 256;
+        }
+      n[p] += sum;
+      cnt[p] += num;
+    }
     const long long tile = pgh <= 1 ? 16 : 8;
     for (int p = 24; p < std::min(40, np); p++)
       if (n[p] <= 72 * cnt[p]) R.per[p] = n[p] > 3 * tile * cnt[p] ? 4 : n[p] > tile * cnt[p] ? 2 : 1;
@@ -1710,12 +1731,19 @@ EvalRules eval_rules(const Params& P, const std::vector<EvalTask>& tasks, int pg
   // tensor cores from the blocks; rows above 30 coefficients have no
   // block evaluation.
   std::vector<long long> leaves(np, 0), n32(np, 0), n8(np, 0);
-  for (size_t t = 0; t < tasks.size(); t++) {  // a leaf's tasks are consecutive
-    const EvalTask& e = tasks[t];
-    if (e.route != ROUTE_TAYLOR) continue;
-    leaves[e.p] += t == 0 || tasks[t - 1].box != e.box;
-    n32[e.p] += 32 * ((e.n + 31) / 32);
-    n8[e.p] += 8 * ((e.n + 7) / 8);
+  for (size_t t = 0; t < tasks.size();) {
+    const int p = tasks[t].p;
+    long long num = 0, m32 = 0, m8 = 0;
+    for (; t < tasks.size() && tasks[t].p == p; t++) {
+      const EvalTask& e = tasks[t];
+      if (e.route != ROUTE_TAYLOR) continue;
+      num += t == 0 || tasks[t - 1].box != e.box;  // a leaf's tasks are consecutive
+      m32 += (e.n + 31) / 32;
+      m8 += (e.n + 7) / 8;
+    }
+    leaves[p] += num;
+    n32[p] += 32 * m32;
+    n8[p] += 8 * m8;
   }
   for (int p = 0; p < np; p++) {
     const double Pn = p + 1, P3 = Pn * Pn * Pn;
@@ -1899,7 +1927,7 @@ cudaError_t device_plan_create(const HostPlan& H, DevicePlan& D, const int* d_is
     for (const SepItem& s : sep_items)
       if (run[s.num].second > 0) items[ni++] = s;
     items.resize(ni);
-    erules = eval_rules(P, H.eval_of_all.empty() ? H.eval : H.eval_of_all, pgh);
+    erules = eval_rules(P, H.nlocal, H.eval_of_all.empty() ? H.eval : H.eval_of_all, pgh);
     const std::vector<uint8_t>& blocks = erules.blocks;
     std::vector<long long> len(sep_order_of.size());  // doubles of a block, by depth
     for (size_t d = 0; d < len.size(); d++) {
